@@ -192,3 +192,97 @@ def tolerance(case):
     """Gradients leave in bfloat16 after products with bfloat16 operands: against the same step in float64 they are off by
     2.1e-3 to 3.2e-3 (largest difference 3.5e-2 of the root mean square), the loss and its scalar gradients by 1e-6."""
     return {"rel": 1.2e-2, "max": 1.4e-1}
+
+
+def _loss_exact(rows, blocks, case):
+    """The streamed loss of bfloat16 ``rows`` against ``blocks`` (tensor, first row's number, how often) in float64:
+    the gradient of the rows and the twelve summands. An own cell's logit is the scale itself; a cosine whose inverse
+    norms' product reaches 100 counts as zero; a cell and its mirror both move the row, hence the factor two."""
+    ladder, count = _ladder(case), rows.shape[0]
+    live, beta, bias = count * sum(times for _, _, times in blocks), case["beta"], case["bias"]
+    q, edges = rows.double(), [0] + list(ladder.ends)
+    bands = list(zip(edges[:-1], edges[1:]))
+
+    def inverse_norms(values):
+        squares = torch.stack([values[:, a:b].square().sum(1) for a, b in bands]).cumsum(0)
+        return torch.where(squares > 0, squares.rsqrt(), torch.zeros_like(squares))
+
+    q_inverse = inverse_norms(q)
+    gradient, sums = torch.zeros_like(q), torch.zeros(12, dtype=torch.float64, device=q.device)
+    step = 1024
+    for block, base, times in blocks:
+        c = block.double()
+        c_inverse = inverse_norms(c)
+        columns = base + torch.arange(c.shape[0], device=q.device)[None, :]
+        for first in range(0, count, step):
+            part = slice(first, min(first + step, count))
+            numbers = torch.arange(part.start, part.stop, device=q.device)[:, None]
+            own = numbers == columns
+            z, mask = torch.full(own.shape, -1.0, dtype=torch.float64, device=q.device), torch.ones_like(own, dtype=torch.float64)
+            if case["positives"] == "pairs":
+                z[(numbers ^ 1) == columns] = 1.0
+            if case["diagonal"] == "own":
+                z[own] = 1.0
+            if case["diagonal"] == "skip":
+                mask[own] = 0.0
+            dots, raws = torch.zeros_like(z), []
+            for k, (a, b) in enumerate(bands):
+                dots = dots + q[part, a:b] @ c[:, a:b].T
+                inverse = q_inverse[k][part, None] * c_inverse[k][None, :]
+                floored = inverse >= 100.0
+                logit = beta * torch.where(own, 1.0, torch.where(floored, 0.0, dots * inverse))
+                s = z * (logit + bias)
+                cell = -mask * z * torch.sigmoid(-s) / live
+                loss = (mask * torch.nn.functional.softplus(-s)).sum() / live
+                sums[[0, 4 + k]] += times * loss
+                sums[1] += times * cell.sum()
+                sums[2] += times * (cell * logit).sum()
+                raws.append(torch.where(own | floored, 0.0, 2.0 * beta * cell * inverse))
+                fold = (raws[-1] * dots).sum(1) * q_inverse[k][part].square()
+                gradient[part, :b] -= times * fold[:, None] * q[part, :b]
+            suffix = torch.zeros_like(z)
+            for k in reversed(range(len(bands))):
+                a, b = bands[k]
+                suffix += raws[k]
+                gradient[part, a:b] += times * (suffix @ c[:, a:b])
+    return gradient, sums
+
+
+def _train_exact(case, state):
+    """One step of the trainer from the state that ``prepare`` leaves, in float64 from its bfloat16 weights on."""
+    trainer, batch = state["trainer"], state["batch"].to("cuda").double()
+    names = [name for name, _ in trainer.projector.named_parameters()]
+    weights = {name: value.double() for name, value in trainer.projector.state_dict().items()}
+    leaves = {name: weights[name].clone().requires_grad_() for name in names}
+    hidden = torch.nn.functional.gelu(batch @ leaves["fc1.weight"].T + leaves["fc1.bias"])
+    rows = hidden @ leaves["fc2.weight"].T + leaves["fc2.bias"]
+    gradient, sums = _loss_exact(rows.detach().to(torch.bfloat16), [(rows.detach().to(torch.bfloat16), 0, 1)], case)
+    rows.backward(gradient)
+    resumed = trainer.state_dict()["optimizer"]
+    values = list(leaves.values()) + [trainer.loss.logit_scale.detach().double(), trainer.loss.logit_bias.detach().double()]
+    gradients = [leaf.grad for leaf in leaves.values()] + [sums[2], sums[1]]
+    (first, second), count, updated = resumed["betas"], resumed["steps"] + 1, []
+    for value, g, m, v in zip(values, gradients, resumed["exp_avg"], resumed["exp_avg_sq"]):
+        m, v = first * m.double() + (1 - first) * g, second * v.double() + (1 - second) * g * g
+        move = (m / (1 - first ** count)) / ((v / (1 - second ** count)).sqrt() + resumed["eps"])
+        updated.append(value.detach() * (1 - resumed["lr"] * resumed["weight_decay"]) - resumed["lr"] * move)
+    return {"summands": sums, "parameters": dict(zip(names, updated)), "gradients": dict(zip(names, gradients)),
+            "scale": updated[-2], "bias": updated[-1]}
+
+
+def exact(case, seed):
+    kind, count = case["kind"], case["blocks"]
+    if kind == "train":
+        return _train_exact(case, prepare(case, seed))
+    generator = torch.Generator(device="cuda").manual_seed(seed)
+    distinct = [_embeddings(case, case["rows"], generator) for _ in range(count if kind in ("stream", "fused") else 1)]
+    distinct = [block.to(torch.bfloat16) for block in distinct]
+    blocks = [(block, index * case["rows"], 1) for index, block in enumerate(distinct)]
+    if kind == "simulate" and count > 1:  # blocks beyond the first hold no own copies and are all alike
+        blocks.append((distinct[0], case["rows"], count - 1))
+    gradient, sums = _loss_exact(distinct[0], blocks, case)
+    if kind == "module":
+        ladder = _ladder(case)
+        return {"loss": sums[0], "prefix_losses": sums[4:4 + ladder.count], "gradient": gradient,
+                "scale_gradient": sums[2], "bias_gradient": sums[1]}
+    return gradient, sums
