@@ -42,11 +42,6 @@ constexpr uint32_t fwd_rows = 128;
 constexpr uint32_t fwd_cols = 64;
 constexpr uint32_t fwd_depth = 64;
 constexpr uint32_t fwd_max_stages = 6;
-// Ladders of up to five prefixes leave room for six stages; longer ones keep more per-thread state and get five. The
-// fused kernel shares the shared memory with the gradient GEMM's stages and keeps three.
-__host__ __device__ constexpr uint32_t fwd_stages_for(uint32_t prefixes, bool fused) {
-    return fused ? 3u : (prefixes <= 5 ? 6u : 5u);
-}
 constexpr uint32_t fwd_max_slots = 8;
 // Tensor-memory slots of the score accumulators: all eight 64-column slots, or six when the last 128 columns hold the
 // gradient GEMM's accumulator.
@@ -72,18 +67,31 @@ constexpr uint32_t fz_max_tiles_per_run = 16;
 #endif
 constexpr uint32_t fwd_epilogue_warps = SC_FWD_EPILOGUE_WARPS; // 16: four per scheduler at 96 registers; 8: two at 168
 constexpr uint32_t fwd_epilogue_threads = fwd_epilogue_warps * 32;
-constexpr uint32_t fwd_chunk_columns = 16;                                  // columns handled per tensor-memory load
 constexpr uint32_t fwd_column_groups = fwd_epilogue_warps / 4;             // warps that share a lane quadrant
 constexpr uint32_t fwd_warp_columns = fwd_cols / fwd_column_groups;        // columns of a tile that one warp owns
-constexpr uint32_t fwd_warp_chunks = fwd_warp_columns / fwd_chunk_columns;
+// Columns a thread takes at a time: all bands' values of a chunk are held in registers together.
+// Ladders of seven and eight bands go band by band instead (`rolled`): the code of eight bands times three forms of the cell
+// math does not stay in the instruction cache, and their values do not fit the registers.
+__host__ __device__ constexpr bool fwd_rolled_for(int prefixes) { return prefixes >= 7; }
+__host__ __device__ constexpr int fwd_chunk_columns_for(int prefixes) { return prefixes <= 1 || fwd_rolled_for(prefixes) ? 16 : 8; }
+// The narrowest bands, where the registers have no room for them beside the others: their gradients are parked in the tensor
+// memory their dots came from until the suffix sums reach them, and their slots are released later than the others'.
+__host__ __device__ constexpr int fwd_parked_bands_for(int prefixes, bool fused) {
+    return fwd_rolled_for(prefixes) ? prefixes - 2 : (prefixes > (fused ? 4 : 5) ? prefixes - 4 : 0);
+}
+static_assert(fwd_warp_columns == 16, "a warp's store patch of a band is 32 rows x 16 columns");
 constexpr uint32_t fwd_producer_warp = fwd_epilogue_warps;
 constexpr uint32_t fwd_mma_warp = fwd_epilogue_warps + 1;
 constexpr uint32_t fwd_first_pull_warp = fwd_epilogue_warps + 2;
 constexpr uint32_t fwd_pull_warps = 1;
 constexpr uint32_t fz_mma_warp = fwd_epilogue_warps + 3; // fused kernel only; the pull warp doubles as its producer
-__host__ __device__ constexpr uint32_t fwd_threads_for(bool fused) {
-    return 32 * (fwd_epilogue_warps + 2 + fwd_pull_warps + (fused ? 1u : 0u));
-}
+// Twenty warps, five warpgroups: four of epilogue warps, one of helpers (the last helper works in the fused kernel only).
+// Launched with 96 registers a thread, of which the helpers' warpgroup hands most on: 512 x 104 + 128 x 64 = 640 x 96.
+constexpr uint32_t fwd_threads = 32 * (fwd_epilogue_warps + 4);
+constexpr uint32_t fwd_epilogue_registers = 104, fwd_helper_registers = 64, fwd_launch_registers = 96;
+static_assert(fwd_epilogue_threads * fwd_epilogue_registers + (fwd_threads - fwd_epilogue_threads) * fwd_helper_registers <=
+                  fwd_threads * fwd_launch_registers,
+              "the register split must not exceed what the block is launched with");
 constexpr uint32_t fwd_q_bytes = fwd_rows * fwd_depth * 2;
 constexpr uint32_t fwd_c_bytes = fwd_cols * fwd_depth * 2;
 constexpr uint32_t fwd_stage_bytes = fwd_q_bytes + fwd_c_bytes;
@@ -91,15 +99,22 @@ constexpr uint32_t fwd_tile_barriers = 8;
 constexpr float log2_e = 1.4426950408889634f;
 constexpr float easy_negative_limit = -8.0f; // (logit + bias) * log2(e) below this: e < 2^-8, the cubic series of log1p(e)
                                              // and e / (1 + e) are then exact to 2e-8 relative
+constexpr float left_out_logit = -1000.0f;   // a base-two exponential of zero
+constexpr float near_negative_limit = -5.0f; // the same for the series of five terms (e < 2^-5)
+
+constexpr uint32_t fwd_norm_slots = 4;
 
 struct fwd_tail {
     uint64_t stage_full[fwd_max_stages];
     uint64_t stage_empty[fwd_max_stages];
-    // Tile t's accumulators have been read by every epilogue warp (index t % fwd_slots): `early` covers the two widest
-    // bands, which the suffix pass reads first and whose slots the next tile's UMMAs want first; `late` covers the rest.
-    uint64_t tile_early[fwd_max_slots];
-    uint64_t tile_late[fwd_max_slots];
+    // Tile t's accumulators have been read by every epilogue warp (index t % fwd_slots): all bands', or, where the narrowest
+    // bands are parked, the others' (`tile_taken`, with a third of the tile's work still to come) and the parked ones'.
+    uint64_t tile_taken[fwd_max_slots];
+    uint64_t tile_parked_taken[fwd_max_slots];
     uint64_t tile_full[fwd_tile_barriers];
+    // The candidate norms of tile t are in ring entry t % fwd_norm_slots / have been read by every epilogue warp.
+    uint64_t norms_full[fwd_norm_slots];
+    uint64_t norms_empty[fwd_norm_slots];
     // Fused kernel: the gradient GEMM's stage ring, "this item's gradient patches are in memory" (one per scratch
     // buffer, an arrival per epilogue warp), and the hand-over of its single accumulator.
     uint64_t fz_stage_full[fz_stages];
@@ -111,21 +126,38 @@ struct fwd_tail {
     uint32_t abort_flag;
 };
 constexpr uint32_t fwd_tail_bytes = (sizeof(fwd_tail) + 127) / 128 * 128;
-// Per epilogue warp: [2 buffers][prefixes][16 columns] candidate inverse norms, then [2][8] tile maxima.
-constexpr uint32_t fwd_norm_floats_per_warp = 2 * (8 * fwd_warp_columns + 8);
-constexpr uint32_t fwd_norm_bytes = fwd_epilogue_warps * fwd_norm_floats_per_warp * 4;
-// Per epilogue thread: inverse norm, loss and coefficient of every prefix, laid out [3 * prefixes][thread].
-__host__ __device__ constexpr uint32_t fwd_state_bytes(uint32_t prefixes) { return 3 * prefixes * fwd_epilogue_threads * 4; }
-// Per epilogue warp two staging buffers (one per band of a pair) of [32 rows][16 columns] bfloat16 for each of the warp's
-// column chunks, from which the warp's patches of the gradient cube leave through TMA stores.
-constexpr uint32_t fwd_store_patch_bytes = 32 * fwd_chunk_columns * 2;
-constexpr uint32_t fwd_store_bytes = fwd_epilogue_warps * 2 * fwd_warp_chunks * fwd_store_patch_bytes;
+// Ring of candidate norms, one entry per tile in flight: [prefixes][64 columns] inverse norms, then the [8] tile maxima.
+__host__ __device__ constexpr uint32_t fwd_norm_floats(uint32_t prefixes) { return prefixes * fwd_cols + 8; }
+__host__ __device__ constexpr uint32_t fwd_norm_bytes(uint32_t prefixes) { return fwd_norm_slots * fwd_norm_floats(prefixes) * 4; }
+// Per epilogue thread and band the row factor beta / |q_k|: in shared memory where the bands' values leave no registers for
+// it (chunks of eight columns times four or more bands), in registers otherwise. Band by band, the row's loss and
+// coefficient as well.
+__host__ __device__ constexpr bool fwd_factors_in_shared(uint32_t prefixes, bool fused) { return !fused && prefixes >= 4; }
+__host__ __device__ constexpr uint32_t fwd_factor_bytes(uint32_t prefixes, bool fused) {
+    return (fwd_rolled_for(prefixes) ? 3u : (fwd_factors_in_shared(prefixes, fused) ? 1u : 0u)) * prefixes * fwd_epilogue_threads * 4;
+}
+// Per epilogue warp and band (four in rotation when the bands go one by one) a patch of [32 rows][16 columns] bfloat16, from
+// which the gradient cube is written by TMA stores.
+constexpr uint32_t fwd_store_patch_bytes = 32 * fwd_warp_columns * 2;
+__host__ __device__ constexpr uint32_t fwd_store_patches(uint32_t prefixes) { return fwd_rolled_for(prefixes) ? 4u : prefixes; }
+__host__ __device__ constexpr uint32_t fwd_store_bytes(uint32_t prefixes) {
+    return fwd_epilogue_warps * fwd_store_patches(prefixes) * fwd_store_patch_bytes;
+}
+// Stages of the score operands: as many as the rest of the shared memory leaves room for. The fused kernel keeps room for
+// the gradient GEMM's stages and runs the scores on two.
+constexpr uint32_t fwd_shared_limit = 227 * 1024;
+__host__ __device__ constexpr uint32_t fwd_stages_for(uint32_t prefixes, bool fused) {
+    uint32_t const rest = 1024 + (fused ? fz_stages * fz_stage_bytes : 0u) + fwd_store_bytes(prefixes) + fwd_tail_bytes + fwd_norm_bytes(prefixes) + fwd_factor_bytes(prefixes, fused);
+    uint32_t const fit = (fwd_shared_limit - rest) / fwd_stage_bytes;
+    return fit < fwd_max_stages ? fit : fwd_max_stages;
+}
+static_assert(fwd_stages_for(8, false) >= 3 && fwd_stages_for(fz_max_prefixes, true) >= 2, "the score operands need a ring of stages");
 __host__ __device__ constexpr uint32_t fwd_stage_region_bytes(uint32_t prefixes, bool fused) {
     return fwd_stages_for(prefixes, fused) * fwd_stage_bytes + (fused ? fz_stages * fz_stage_bytes : 0u);
 }
 __host__ __device__ constexpr uint32_t fwd_shared_bytes(uint32_t prefixes, bool fused) {
-    return 1024 + fwd_stage_region_bytes(prefixes, fused) + fwd_store_bytes + fwd_tail_bytes + fwd_norm_bytes +
-           fwd_state_bytes(prefixes);
+    return 1024 + fwd_stage_region_bytes(prefixes, fused) + fwd_store_bytes(prefixes) + fwd_tail_bytes + fwd_norm_bytes(prefixes) +
+           fwd_factor_bytes(prefixes, fused);
 }
 
 struct fwd_params {
@@ -208,26 +240,20 @@ struct phase_timer {
 #endif
 
 // ---- the cell math ----------------------------------------------------------------------------------------------
-// Accumulators are kept without the 1/N weight: `g` sums -mask*z*(1-sigmoid(s)), `ga` sums that times (logit+bias),
-// `loss` sums mask*softplus(-s); the weight is applied once when the partial record is written.
-struct row_constants {
-    float beta, bias, weight, raw_scale;
-};
-
-// The cell pass leaves each band's raw-dot gradients in tensor memory without the factor beta / |q_k| that is common to
-// the row and the band; the suffix pass multiplies it in while it sums the bands. The norms kernel writes an inverse
+// Accumulators are kept without the 1/N weight: `g` sums -mask*z*(1-sigmoid(s)), `loss` sums mask*softplus(-s),
+// `coefficient` sums raw gradient * dot; the weight is applied once when the partial record is written.
+// The cell pass forms each band's raw-dot gradients without the factor beta / |q_k| that is common to the row and the
+// band; the suffix pass multiplies it in while it sums the bands. The norms kernel writes an inverse
 // norm of 0 for a row of zero norm (factor 0, and its cosines are floored anyway); the cap only keeps a huge inverse
 // norm of a tiny row from turning 0 * factor into a NaN.
 __device__ __forceinline__ float row_factor(float beta, float inv_q) { return beta * fminf(inv_q, 1e30f); }
 
-// Any cell: positives, the diagonal, floored cosines. Only tiles that touch the diagonal or hold a floored norm come here,
-// so this is a real call (one copy of the code) rather than sixteen inlined ones: the kernel's hot loops stay small and
-// contiguous in the instruction cache. Returns what the cell adds to each of the row's sums.
+// Any cell: positives, the diagonal, floored cosines. Returns what the cell adds to each of the row's sums.
 struct cell_outcome {
-    float raw, loss, cell, cell_logit, coefficient;
+    float raw, loss, cell;
 };
-__device__ __noinline__ cell_outcome cell_general(float prefix_dot, float inv_q, float inv_c, float beta, float bias,
-                                                  float raw_scale, bool own, bool partner, uint32_t spec_code) {
+__device__ __forceinline__ cell_outcome cell_general(float prefix_dot, float inv_q, float inv_c, float beta, float bias,
+                                                     bool own, bool partner, uint32_t spec_code) {
     uint32_t const diagonal = (spec_code >> 1) & 3u; // 0 own, 1 negative, 2 skip
     float z = partner ? 1.0f : -1.0f;
     float mask = 1.0f;
@@ -238,22 +264,36 @@ __device__ __noinline__ cell_outcome cell_general(float prefix_dot, float inv_q,
     float const inverse_denominator = fminf(inv_q * inv_c, 100.0f);
     bool const floored = inverse_denominator >= 100.0f;
     float const cosine = floored ? 0.0f : prefix_dot * inverse_denominator;
-    float const logit = beta * (own ? 1.0f : cosine);
-    float const a = logit + bias;
-    float const s = z * a;
+    float const s = z * (beta * (own ? 1.0f : cosine) + bias);
     float const d = fast_ex2(-fabsf(s) * log2_e);
     float const complement = (s >= 0.0f ? d : 1.0f) * fast_rcp(1.0f + d);
     float const cell = -mask * z * complement;
-    float const raw = (own || floored) ? 0.0f : cell * inverse_denominator * raw_scale;
-    return cell_outcome{raw, mask * (fmaxf(-s, 0.0f) + log1p_unit(d)), cell, cell * a, raw * prefix_dot};
+    float const raw = (own || floored) ? 0.0f : cell * inverse_denominator * beta;
+    return cell_outcome{raw, mask * (fmaxf(-s, 0.0f) + log1p_unit(d)), cell};
 }
 
+template <int columns_> __device__ __forceinline__ void tmem_load(uint32_t taddr, uint32_t (&r)[columns_]) {
+    static_assert(columns_ == 8 || columns_ == 16, "tensor-memory loads of 8 or 16 columns");
+    if constexpr (columns_ == 16) {
+        tmem_load_16(taddr, r);
+    } else {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(taddr)
+                     : "memory");
+    }
+}
 __device__ __forceinline__ void tmem_store_16(uint32_t taddr, uint32_t const (&r)[16]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
         "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
+}
+__device__ __forceinline__ void tmem_store_8(uint32_t taddr, uint32_t const (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
 }
 __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -268,28 +308,47 @@ __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::
 #ifndef SC_FWD_HELPER_SLEEP
 #define SC_FWD_HELPER_SLEEP 1
 #endif
+// A CTA's items: every gridDim.x-th of the list.
+__device__ __forceinline__ uint32_t item_count(uint32_t items) { return (items + gridDim.x - 1 - blockIdx.x) / gridDim.x; }
+__device__ __forceinline__ uint32_t item_at(uint32_t, uint32_t n) { return blockIdx.x + n * gridDim.x; }
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, wait_context const& ctx, uint32_t site,
                                                uint32_t detail, uint32_t sleep_ns = 0) {
     if (SC_FWD_HELPER_SLEEP && sleep_ns != 0u)
         return __all_sync(0xFFFFFFFFu, mbar_wait_relaxed(bar, parity, ctx, site, detail, sleep_ns));
     return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, ctx, site, detail));
 }
-constexpr uint32_t sleep_producer_ns = 1000; // stages ahead of the issuer: nothing waits for this warp's wake-up
-constexpr uint32_t sleep_issuer_ns = 100;    // the epilogue may be waiting for the tile these UMMAs finish
+constexpr uint32_t sleep_producer_ns = 200; // stages ahead of the issuer: nothing waits for this warp's wake-up
+constexpr uint32_t sleep_issuer_ns = 20;    // the epilogue may be waiting for the tile these UMMAs finish
 constexpr uint32_t sleep_gemm_ns = 500;      // the fused kernel's gradient GEMM runs a whole item behind
 
+//
+// The producer also brings the candidates' inverse norms of a tile (and their maxima) into the ring the epilogue warps read
+// them from: plain loads at the start of the tile, stored once the tile's operand loads have been issued.
+template <int prefixes_>
 __device__ __forceinline__ void producer_role(CUtensorMap const* q_map, CUtensorMap const* c_map, fwd_params const& p,
-                                              uint32_t stages_base, fwd_tail* tail, wait_context const& ctx,
-                                              uint32_t const stages) {
+                                              uint32_t stages_base, float* norm_ring, fwd_tail* tail,
+                                              wait_context const& ctx, uint32_t const stages) {
     bool const elected = elect_one();
-    uint32_t stage = 0, phase = 0;
+    uint32_t const lane = threadIdx.x % 32;
+    uint32_t stage = 0, phase = 0, tile_local = 0;
     uint32_t const chunks = p.hidden / fwd_depth;
+    uint32_t const column_tiles = p.rows_c / fwd_cols;
     phase_timer timer(p);
     timer.only_if(elected);
-    for (uint32_t item = blockIdx.x; item < p.items; item += gridDim.x) {
+    for (uint32_t n = 0, count = item_count(p.items); n < count; ++n) {
+        uint32_t const item = item_at(p.items, n);
         uint32_t const strip = item / p.runs_per_strip, run = item % p.runs_per_strip;
-        for (uint32_t t = 0; t < p.tiles_per_run; ++t) {
+        for (uint32_t t = 0; t < p.tiles_per_run; ++t, ++tile_local) {
             uint32_t const column_tile = run * p.tiles_per_run + t;
+            float norms[2 * prefixes_], largest = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 2 * prefixes_; ++j) {
+                size_t const at = static_cast<size_t>(j / 2) * p.rows_c + column_tile * fwd_cols + (j % 2) * 32u + lane;
+                norms[j] = SC_IN_BOUNDS(at, static_cast<size_t>(prefixes_) * p.rows_c) ? __ldg(p.c_inv + at) : 0.0f;
+            }
+            if (lane < prefixes_ &&
+                SC_IN_BOUNDS(static_cast<size_t>(lane) * column_tiles + column_tile, static_cast<size_t>(prefixes_) * column_tiles))
+                largest = __ldg(p.c_tile_max + static_cast<size_t>(lane) * column_tiles + column_tile);
             for (int chunk = static_cast<int>(chunks) - 1; chunk >= 0; --chunk) {
                 timer.lap(0);
                 if (!mbar_wait_warp(smem_u32(&tail->stage_empty[stage]), phase ^ 1u, ctx, site_fwd_stage_empty, item, sleep_producer_ns))
@@ -306,6 +365,16 @@ __device__ __forceinline__ void producer_role(CUtensorMap const* q_map, CUtensor
                 __syncwarp();
                 if (++stage == stages) stage = 0, phase ^= 1u;
             }
+            uint32_t const entry = tile_local % fwd_norm_slots;
+            if (!mbar_wait_warp(smem_u32(&tail->norms_empty[entry]), ((tile_local / fwd_norm_slots) & 1u) ^ 1u, ctx,
+                                site_fwd_norms_empty, item, sleep_producer_ns))
+                return;
+            float* const into = norm_ring + entry * fwd_norm_floats(prefixes_);
+#pragma unroll
+            for (int j = 0; j < 2 * prefixes_; ++j) into[(j / 2) * fwd_cols + (j % 2) * 32u + lane] = norms[j];
+            if (lane < 8) into[prefixes_ * fwd_cols + lane] = largest;
+            __syncwarp();
+            if (elected) mbar_arrive(smem_u32(&tail->norms_full[entry]));
         }
     }
     timer.flush(p, 0, 2);
@@ -316,16 +385,42 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
                                          wait_context const& ctx) {
     constexpr uint32_t fwd_slots = fwd_slots_for(fused_);
     constexpr uint32_t idesc = umma_idesc_bf16(fwd_rows, fwd_cols);
+    constexpr uint32_t parked = fwd_parked_bands_for(prefixes_, fused_);
     constexpr uint32_t descriptor_high = (1024u >> 4) | (1u << 14) | (2u << 29); // stride 1024 B, version 1, 128-byte swizzle
     bool const elected = elect_one();
     uint32_t const chunks = p.hidden / fwd_depth;
     uint32_t const low_base = ((stages_base & 0x3FFFFu) >> 4) | (1u << 16);
-    uint32_t stage = 0, phase = 0, unit = 0, tile_local = 0, seen_early = 0, seen_late = 0;
+    uint32_t stage = 0, phase = 0, unit = 0, tile_local = 0, seen = 0, seen_parked = 0;
     phase_timer timer(p);
     timer.only_if(elected);
-    for (uint32_t item = blockIdx.x; item < p.items; item += gridDim.x) {
+    // The next band's slot, once it is free. The slot's last user was unit - fwd_slots, a band of tile `needed`; the
+    // epilogue must have read it out. Releases are observed here strictly in tile order, per barrier array, so a barrier's
+    // parity can never be a full turn ahead of the one waited for: tile X + fwd_slots cannot even be issued before tile X's release has been
+    // seen.
+    uint32_t slot_address = 0;
+    auto take_slot = [&]() -> bool {
+        if (unit >= fwd_slots) {
+            uint32_t const needed = (unit - fwd_slots) / prefixes_;
+            bool const was_parked = parked > 0 && (unit - fwd_slots) % prefixes_ >= prefixes_ - parked; // ranks run from the widest
+            uint64_t* const barriers = was_parked ? tail->tile_parked_taken : tail->tile_taken;
+            uint32_t& observed = was_parked ? seen_parked : seen;
+            timer.lap(0);
+            while (observed <= needed) {
+                if (!mbar_wait_warp(smem_u32(&barriers[observed % fwd_slots]), (observed / fwd_slots) & 1u, ctx,
+                                    site_fwd_slot_empty, unit, sleep_issuer_ns))
+                    return false;
+                ++observed;
+            }
+            timer.lap(2);
+            tcgen05_fence_after();
+        }
+        slot_address = tmem_base + unit % fwd_slots * fwd_slot_columns;
+        ++unit;
+        return true;
+    };
+    for (uint32_t n = 0, count = item_count(p.items); n < count; ++n) {
+        uint32_t const item = item_at(p.items, n);
         for (uint32_t t = 0; t < p.tiles_per_run; ++t) {
-            uint32_t slot_address = 0, accumulate = 0;
             for (int chunk = static_cast<int>(chunks) - 1; chunk >= 0; --chunk) {
                 uint32_t const starts = p.band_starts[chunk];
                 timer.lap(0);
@@ -334,47 +429,31 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
                 timer.lap(1);
                 tcgen05_fence_after();
                 uint32_t const low = low_base + stage * (fwd_stage_bytes >> 4);
-#pragma unroll
-                for (int sub = 3; sub >= 0; --sub) {
-                    if ((starts >> (8 * sub)) & 0xFFu) {
-                        // The slot's last user was unit - fwd_slots, band `rank` (counted from the widest) of tile `needed`;
-                        // the epilogue must have read it out. Releases are observed here strictly in tile order, per
-                        // barrier array, so a barrier's parity can never be a full turn ahead of the one waited for: tile
-                        // X + fwd_slots cannot even be issued before tile X's release has been seen.
-                        uint32_t const slot = unit % fwd_slots;
-                        if (unit >= fwd_slots) {
-                            uint32_t const needed = (unit - fwd_slots) / prefixes_, rank = (unit - fwd_slots) % prefixes_;
-                            timer.lap(0);
-                            if (rank < 2) {
-                                while (seen_early <= needed) {
-                                    if (!mbar_wait_warp(smem_u32(&tail->tile_early[seen_early % fwd_slots]),
-                                                        (seen_early / fwd_slots) & 1u, ctx, site_fwd_slot_empty, unit, sleep_issuer_ns))
-                                        return;
-                                    ++seen_early;
-                                }
-                            } else {
-                                while (seen_late <= needed) {
-                                    if (!mbar_wait_warp(smem_u32(&tail->tile_late[seen_late % fwd_slots]),
-                                                        (seen_late / fwd_slots) & 1u, ctx, site_fwd_slot_empty, unit, sleep_issuer_ns))
-                                        return;
-                                    ++seen_late;
-                                }
-                            }
-                            timer.lap(2);
-                        }
-                        tcgen05_fence_after();
-                        slot_address = tmem_base + slot * fwd_slot_columns;
-                        accumulate = 0;
-                        ++unit;
+                uint64_t q_descriptor, c_descriptor;
+                asm("mov.b64 %0, {%1, %2};" : "=l"(q_descriptor) : "r"(low), "r"(descriptor_high));
+                asm("mov.b64 %0, {%1, %2};" : "=l"(c_descriptor) : "r"(low + (fwd_q_bytes >> 4)), "r"(descriptor_high));
+                uint32_t const empty = smem_u32(&tail->stage_empty[stage]);
+                // A step of 16 channels advances both descriptors by 32 bytes. Steps run from the chunk's top down; a band
+                // that starts inside the chunk (its edge is not a multiple of 64) takes the step-by-step way.
+                if ((starts & 0x00FFFFFFu) == 0u) {
+                    if (starts != 0u && !take_slot()) return;
+                    if (elected) {
+                        umma_bf16(slot_address, q_descriptor + 6, c_descriptor + 6, idesc, starts != 0u ? 0u : 1u);
+                        umma_bf16(slot_address, q_descriptor + 4, c_descriptor + 4, idesc, 1u);
+                        umma_bf16(slot_address, q_descriptor + 2, c_descriptor + 2, idesc, 1u);
+                        umma_bf16(slot_address, q_descriptor, c_descriptor, idesc, 1u);
+                        umma_commit(empty);
                     }
-                    uint32_t const q_low = low + static_cast<uint32_t>(sub) * 2u; // 32 bytes per 16-channel step
-                    uint64_t q_descriptor, c_descriptor;
-                    asm("mov.b64 %0, {%1, %2};" : "=l"(q_descriptor) : "r"(q_low), "r"(descriptor_high));
-                    asm("mov.b64 %0, {%1, %2};" : "=l"(c_descriptor) : "r"(q_low + (fwd_q_bytes >> 4)), "r"(descriptor_high));
-                    if (elected) umma_bf16(slot_address, q_descriptor, c_descriptor, idesc, accumulate);
-                    accumulate = 1;
+                } else {
+#pragma unroll 1
+                    for (int sub = 3; sub >= 0; --sub) {
+                        bool const begins = ((starts >> (8 * sub)) & 0xFFu) != 0u;
+                        if (begins && !take_slot()) return;
+                        if (elected)
+                            umma_bf16(slot_address, q_descriptor + 2u * sub, c_descriptor + 2u * sub, idesc, begins ? 0u : 1u);
+                    }
+                    if (elected) umma_commit(empty);
                 }
-                if (elected) umma_commit(smem_u32(&tail->stage_empty[stage]));
                 __syncwarp();
                 if (++stage == fwd_stages_for(prefixes_, fused_)) stage = 0, phase ^= 1u;
             }
@@ -386,25 +465,19 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
     timer.flush(p, 2, 3);
 }
 
-// Position of a CTA in its fixed walk over (work item, tile of the run). The item's strip and run are carried along, so
-// the division by the runtime run count happens once per item and not once per tile.
+// Position of a CTA in its walk over (work item, tile of the run).
 struct tile_cursor {
-    uint32_t item, t, strip, run;
-    __device__ __forceinline__ static tile_cursor at(fwd_params const& p, uint32_t item) {
-        return tile_cursor{item, 0, item / p.runs_per_strip, item % p.runs_per_strip};
+    uint32_t n, t, strip, run;
+    __device__ __forceinline__ void go_to(fwd_params const& p, uint32_t to) {
+        uint32_t const item = item_at(p.items, to);
+        n = to, t = 0, strip = item / p.runs_per_strip, run = item % p.runs_per_strip;
     }
-    __device__ __forceinline__ bool valid(fwd_params const& p) const { return item < p.items; }
-    __device__ __forceinline__ tile_cursor next(fwd_params const& p) const {
-        return t + 1 < p.tiles_per_run ? tile_cursor{item, t + 1, strip, run} : at(p, item + gridDim.x);
+    __device__ __forceinline__ void advance(fwd_params const& p) {
+        if (++t == p.tiles_per_run) go_to(p, n + 1);
     }
     __device__ __forceinline__ uint32_t column_tile(fwd_params const& p) const { return run * p.tiles_per_run + t; }
 };
 
-// Epilogue warps: warp w owns tensor-memory lanes 32*(w%4).. (a quarter of the tile's rows) and the column group w/4 of
-// the tile (16 columns each with sixteen warps). The loop over prefixes is rolled (small code, few registers, four
-// warps per scheduler): a prefix's segment dots come out of tensor memory, its raw-dot gradients go back into the same
-// slot, and a second rolled pass reads them widest first, in pairs, to form the suffix sums. Per-thread sums that are
-// indexed by prefix live in shared memory.
 // Fused kernel: one warp's share of a finished accumulator of the gradient GEMM, added to the owner's rows. The
 // accumulator is [128 rows x width channels]; the warp owns the 32 rows of its lane quadrant and every fourth 16-column
 // chunk, starting at its column group. A real call: the code exists once and the hot loops keep their registers.
@@ -423,66 +496,119 @@ __device__ __noinline__ void fz_drain_chunks(float* destination, uint32_t chunks
     }
 }
 
+// Where band `band` of the tile whose widest band is unit `first_unit` of the ring has its slot.
+template <int prefixes_, bool fused_> __device__ __forceinline__ uint32_t band_slot(uint32_t first_unit, uint32_t band) {
+    return ((first_unit + (prefixes_ - 1 - band)) % fwd_slots_for(fused_)) * fwd_slot_columns;
+}
+
+// In a patch that the diagonal crosses, a row's own copy and its pair partner: each thread scores its two cells (where the
+// patch has them) band by band in their general form, and leaves the band's loss, coefficient and the partner's raw-dot
+// gradient (without the row factor; a row's own copy has none) in 16 bytes of shared memory per lane and band: the second half
+// of the lane's row in the warp's own store patches, which is idle until the last chunk is stored. The common path then
+// takes the patch with those cells left out. A real call with a rolled loop over the bands, so that the common path keeps its
+// registers. (Sending all of such a patch's cells through the general form, and the gradients back to the common path through
+// tensor memory, made a launch whose block holds the diagonal 28 us longer at 4096 rows.)
+struct special_sums {
+    float cell, own_logit;
+};
+__device__ __forceinline__ float pick_column(uint32_t const (&d)[16], uint32_t column) {
+    uint32_t eight[8], four[4], two[2];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) eight[c] = (column & 8u) ? d[c + 8] : d[c];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) four[c] = (column & 4u) ? eight[c + 4] : eight[c];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) two[c] = (column & 2u) ? four[c + 2] : four[c];
+    return __uint_as_float((column & 1u) ? two[1] : two[0]);
+}
+template <int prefixes_, bool fused_>
+__device__ __noinline__ special_sums special_cells(uint32_t lane_base, uint32_t first_unit, float const* norms,
+                                                   float const* q_inv, uint32_t rows_q, float beta, float bias,
+                                                   int own_column, int partner_column, uint32_t spec_code, uint32_t sums,
+                                                   uint32_t sums_stride) {
+    static_assert(fwd_warp_columns == 16, "a patch is sixteen columns wide");
+    special_sums total{0.0f, 0.0f};
+    float own_dot = 0.0f, partner_dot = 0.0f;
+#pragma unroll 1
+    for (int k = 0; k < prefixes_; ++k) {
+        uint32_t d[16];
+        tmem_load<16>(lane_base + band_slot<prefixes_, fused_>(first_unit, k), d);
+        float const inv_q = __ldg(q_inv + static_cast<size_t>(k) * rows_q);
+        float const row_beta = row_factor(beta, inv_q);
+        float const without_row_factor = row_beta != 0.0f ? __fdividef(1.0f, row_beta) : 0.0f;
+        float loss = 0.0f, coefficient = 0.0f, partner_raw = 0.0f;
+        tmem_load_wait();
+        own_dot += pick_column(d, static_cast<uint32_t>(own_column));
+        partner_dot += pick_column(d, static_cast<uint32_t>(partner_column));
+        if (own_column >= 0) {
+            cell_outcome const cell = cell_general(own_dot, inv_q, norms[k * fwd_cols + own_column], beta, bias, true, false, spec_code);
+            loss += cell.loss;
+            total.cell += cell.cell, total.own_logit += cell.cell * beta;
+        }
+        if (partner_column >= 0) {
+            cell_outcome const cell =
+                cell_general(partner_dot, inv_q, norms[k * fwd_cols + partner_column], beta, bias, false, true, spec_code);
+            loss += cell.loss;
+            total.cell += cell.cell;
+            partner_raw = cell.raw * without_row_factor;
+            coefficient = partner_raw * partner_dot;
+        }
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(sums + k * sums_stride), "f"(loss),
+                     "f"(coefficient), "f"(partner_raw), "f"(0.0f) : "memory");
+    }
+    return total;
+}
+
+// Epilogue warps: warp w owns tensor-memory lanes 32*(w%4).. (a quarter of the tile's rows) and the column group w/4 of
+// the tile (16 columns each with sixteen warps). A thread takes its columns in chunks; of a chunk it holds every band's
+// values in registers from the tensor-memory load to the store: segment dots come in, the prefix dots run up the ladder,
+// raw-dot gradients replace the dots, and the suffix sums run down the ladder straight from the same registers. Nothing is
+// parked in tensor memory in between, so a tile's slots go back to the issuer as soon as its last chunk has been loaded,
+// about half a tile before the epilogue is done with it.
+//
+// What bounds it: the packed float32 math (eleven instructions per pair of cells and prefix, two cycles each) and issue
+// slots.
 template <int prefixes_, bool fused_>
 __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_params const& p, fwd_tail* tail,
-                                              uint32_t store_base, float* norm_staging, float* thread_state,
-                                              uint32_t tmem_base, wait_context const& ctx, uint32_t warp, uint32_t lane) {
+                                              uint32_t store_base, float const* norm_ring, float* row_factors, uint32_t tmem_base,
+                                              wait_context const& ctx, uint32_t warp, uint32_t lane) {
     constexpr uint32_t fwd_slots = fwd_slots_for(fused_);
-    constexpr int columns = fwd_chunk_columns;
-    constexpr int chunks = fwd_warp_chunks;
+    constexpr int columns = fwd_chunk_columns_for(prefixes_);
+    constexpr int parked = fwd_parked_bands_for(prefixes_, fused_);
+    constexpr bool rolled = fwd_rolled_for(prefixes_);
     constexpr int warp_columns = fwd_warp_columns;
-    constexpr int norm_count = prefixes_ * warp_columns;
-    constexpr int ahead_count = (norm_count + 31) / 32;
     uint32_t const quadrant = warp % 4, group = warp / 4;
     uint32_t const row_local = quadrant * 32 + lane;
     uint32_t const lane_base = tmem_base + ((quadrant * 32u) << 16) + group * warp_columns;
-    uint32_t const column_tiles = p.rows_c / fwd_cols;
     uint32_t const quantities = 2 + 2 * prefixes_;
     float const beta = p.scalars != nullptr ? __ldg(p.scalars) : p.beta;
     float const bias = p.scalars != nullptr ? __ldg(p.scalars + 1) : p.bias;
-    row_constants const constants{beta, bias, p.weight, beta};
-    float* const staged_norms = norm_staging + warp * fwd_norm_floats_per_warp; // [2][8][warp_columns]
-    float* const staged_max = staged_norms + 2 * 8 * warp_columns;              // [2][8]
-    float* const mine = thread_state + threadIdx.x;                             // [3 * prefixes_] strided by the thread count
-    uint32_t tile_local = 0, buffer = 0;
-    uint32_t const warp_store_base = store_base + warp * (2u * chunks) * fwd_store_patch_bytes;
+    uint32_t tile_local = 0;
+    uint32_t const warp_store_base = store_base + warp * fwd_store_patches(prefixes_) * fwd_store_patch_bytes;
 
-    tile_cursor cursor = tile_cursor::at(p, blockIdx.x);
-    if (!cursor.valid(p)) return;
-    // Norms of a tile's candidates are fetched one tile ahead into registers and parked in this warp's shared-memory
-    // buffer, so the cell loop reads them with broadcast shared loads instead of waiting on global memory.
-    float ahead[ahead_count], ahead_max = 0.0f;
-    auto fetch = [&](tile_cursor const& where) {
-        uint32_t const column_tile = where.column_tile(p);
-#pragma unroll
-        for (int j = 0; j < ahead_count; ++j) {
-            uint32_t const index = lane + 32 * j; // (prefix, column) = (index / warp_columns, index % warp_columns)
-            if (index < norm_count &&
-                SC_IN_BOUNDS(static_cast<size_t>(index / warp_columns) * p.rows_c + column_tile * fwd_cols + group * warp_columns +
-                                 index % warp_columns,
-                             static_cast<size_t>(prefixes_) * p.rows_c))
-                ahead[j] = __ldg(p.c_inv + static_cast<size_t>(index / warp_columns) * p.rows_c + column_tile * fwd_cols +
-                                 group * warp_columns + index % warp_columns);
+    tile_cursor cursor;
+    cursor.go_to(p, 0);
+    uint32_t const items = item_count(p.items);
+    // Per-row sums of the item; `coefficient` is kept without the row factor beta / |q_k|, the thread's own words of shared
+    // memory or registers. Lane k of a warp holds the
+    // largest inverse norm of the warp's rows at band k.
+    constexpr bool shared_factors = fwd_factors_in_shared(prefixes_, fused_);
+    constexpr int factor_stride = shared_factors ? fwd_epilogue_threads : 1;
+    float own_factors[shared_factors ? 1 : prefixes_];
+    float* const row_beta = shared_factors ? row_factors + threadIdx.x : own_factors;
+    constexpr int sums_kept = rolled ? 1 : prefixes_;
+    float loss[sums_kept] = {}, coefficient[sums_kept] = {};
+    float* const band_sums = row_factors + threadIdx.x + prefixes_ * fwd_epilogue_threads; // rolled: [2 * prefixes_] strided
+    auto add_sums = [&](int k, float to_loss, float to_coefficient) {
+        if constexpr (rolled) {
+            band_sums[k * fwd_epilogue_threads] += to_loss;
+            band_sums[(prefixes_ + k) * fwd_epilogue_threads] += to_coefficient;
+        } else {
+            loss[k] += to_loss, coefficient[k] += to_coefficient;
         }
-        if (lane < prefixes_ &&
-            SC_IN_BOUNDS(static_cast<size_t>(lane) * column_tiles + column_tile, static_cast<size_t>(prefixes_) * column_tiles))
-            ahead_max = __ldg(p.c_tile_max + static_cast<size_t>(lane) * column_tiles + column_tile);
     };
-    auto park = [&](uint32_t into) {
-#pragma unroll
-        for (int j = 0; j < ahead_count; ++j) {
-            uint32_t const index = lane + 32 * j;
-            if (index < norm_count) staged_norms[into * 8 * warp_columns + index] = ahead[j];
-        }
-        if (lane < prefixes_) staged_max[into * 8 + lane] = ahead_max;
-        __syncwarp();
-    };
-    fetch(cursor);
-    park(0);
-
-    float g = 0.0f, ga = 0.0f;
+    float g = 0.0f, own_logit = 0.0f, rows_max = 0.0f;
     uint32_t row = 0;
-    uint64_t global_row = 0;
     phase_timer timer(p);
     timer.only_if(threadIdx.x == 0);
 
@@ -501,7 +627,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
                 break;
             }
             tcgen05_fence_after();
-            uint32_t const item = blockIdx.x + (drained / p.tile_count) * gridDim.x;
+            uint32_t const item = item_at(p.items, drained / p.tile_count);
             uint32_t const word = p.tiles[drained % p.tile_count];
             float* const destination = p.gradient +
                                        (static_cast<size_t>(item / p.runs_per_strip) * fwd_rows + row_local) * p.hidden +
@@ -519,305 +645,354 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
         return true;
     };
 
-    while (cursor.valid(p)) {
-        tile_cursor const following = cursor.next(p);
-        bool const more = following.valid(p);
-        if (more) fetch(following);
+    uint32_t strip_now = 0xFFFFFFFFu;
+    while (cursor.n < items) {
         if constexpr (fused_) drain(items_done * p.tile_count, false);
         uint32_t const strip = cursor.strip, run = cursor.run;
-        if (cursor.t == 0) {
+        if (strip != strip_now) {
+            strip_now = strip;
             row = strip * fwd_rows + row_local;
-            global_row = p.query_base + row;
 #pragma unroll
             for (int k = 0; k < prefixes_; ++k) {
-                mine[k * fwd_epilogue_threads] = __ldg(p.q_inv + static_cast<size_t>(k) * p.rows_q + row);
-                mine[(prefixes_ + k) * fwd_epilogue_threads] = 0.0f;
-                mine[(2 * prefixes_ + k) * fwd_epilogue_threads] = 0.0f;
+                float const inv_q = __ldg(p.q_inv + static_cast<size_t>(k) * p.rows_q + row);
+                // inverse norms are not negative, so their bits order as they do
+                float const band_max = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(inv_q)));
+                rows_max = lane == static_cast<uint32_t>(k) ? band_max : rows_max;
+                row_beta[k * factor_stride] = row_factor(beta, inv_q);
             }
-            g = 0.0f, ga = 0.0f;
         }
-        uint32_t const column_tile = cursor.column_tile(p);
-        uint32_t const column = column_tile * fwd_cols + group * warp_columns;
-        float const* const norms_now = staged_norms + buffer * 8 * warp_columns;
-        // Is every cell of this warp's patch a plain negative off the cosine floor? The patch is special when its columns
-        // come within one of its rows (a row's own copy, or its pair partner next to it), decided per warp so that a
-        // tile on the diagonal sends only the patches the diagonal crosses through the general cell.
+        if (cursor.t == 0) {
+#pragma unroll
+            for (int k = 0; k < prefixes_; ++k) {
+                if constexpr (rolled) band_sums[k * fwd_epilogue_threads] = 0.0f, band_sums[(prefixes_ + k) * fwd_epilogue_threads] = 0.0f;
+                else loss[k] = 0.0f, coefficient[k] = 0.0f;
+            }
+            g = 0.0f, own_logit = 0.0f;
+        }
+        uint32_t const column = cursor.column_tile(p) * fwd_cols + group * warp_columns;
+        uint32_t const entry = tile_local % fwd_norm_slots;
+        float const* const norms_now = norm_ring + entry * fwd_norm_floats(prefixes_) + group * warp_columns;
+        // Does the diagonal cross this warp's patch? It does when the patch's columns come within one of its rows (a row's
+        // own copy, or its pair partner next to it); then every cell takes its general form. Decided per warp, so that a
+        // tile on the diagonal sends only the patches the diagonal crosses that way.
         uint64_t const first_row = p.query_base + static_cast<uint64_t>(strip) * fwd_rows + quadrant * 32u;
         uint64_t const first_column = p.candidate_base + column;
-        bool special = first_column < first_row + 32u + 1 && first_row < first_column + warp_columns + 1;
-#pragma unroll
-        for (int k = 0; k < prefixes_; ++k) special |= mine[k * fwd_epilogue_threads] * staged_max[buffer * 8 + k] >= 100.0f;
-        special = __any_sync(0xFFFFFFFFu, special);
+        bool const special = first_column - first_row + warp_columns < 32u + 1 + warp_columns;
 
         timer.lap(0);
         if (!mbar_wait(smem_u32(&tail->tile_full[tile_local % fwd_tile_barriers]), (tile_local / fwd_tile_barriers) & 1u, ctx,
                        site_fwd_tile_full, tile_local))
             return;
         tcgen05_fence_after();
+        if (!mbar_wait(smem_u32(&tail->norms_full[entry]), (tile_local / fwd_norm_slots) & 1u, ctx, site_fwd_norms_full, tile_local))
+            return;
         timer.lap(1);
-
-        uint32_t const first_unit = tile_local * prefixes_;
-        pair_t prefix[chunks][columns / 2];
-#pragma unroll
-        for (int h = 0; h < chunks; ++h)
-#pragma unroll
-            for (int c = 0; c < columns / 2; ++c) prefix[h][c] = pack2(0.0f, 0.0f);
-        pair_t const bias2 = pack2(bias, bias);
-#pragma unroll 1
-        for (int k = 0; k < prefixes_; ++k) {
-            uint32_t const address = lane_base + ((first_unit + (prefixes_ - 1 - k)) % fwd_slots) * fwd_slot_columns;
-            uint32_t d[chunks][columns];
-#pragma unroll
-            for (int h = 0; h < chunks; ++h) tmem_load_16(address + h * columns, d[h]);
-            // Candidate norms are read from the warp's staging buffer pair by pair, right where they are used (broadcast
-            // shared loads), which keeps registers free for interleaving the cells.
-            pair_t const* const inv_c = reinterpret_cast<pair_t const*>(norms_now + k * warp_columns);
-            float const inv_q = mine[k * fwd_epilogue_threads];
-            float const row_beta = row_factor(beta, inv_q);
-            float loss = 0.0f, coefficient = 0.0f;
-            tmem_load_wait();
-            if (!special) {
-                pair_t const row_beta2 = pack2(row_beta, row_beta);
-                // First every cell's e = exp(logit + bias), computed in base two (the scale and the bias carry log2(e), so
-                // the exponential is a single MUFU), and the largest logit + bias of the thread's cells. Where the warp's
-                // patch is all easy negatives (every logit + bias below the limit, which is all but the hardest cells) e
-                // is the decay exp(-|logit + bias|) and the rest is a few packed multiply-adds: log1p(e) = e - e^2/2 +
-                // e^3/3 and 1 - sigmoid = e / (1 + e) = e - e^2 + e^3, both exact to better than 2e-8 relative below the
-                // limit. Otherwise the general form runs: the decay with the absolute value, reciprocal, select by sign,
-                // the full log1p polynomial, the hinge.
-                pair_t const row_beta2_binary = pack2(row_beta * log2_e, row_beta * log2_e);
-                pair_t const bias2_binary = pack2(bias * log2_e, bias * log2_e);
-                pair_t decay[chunks][columns / 2];
-                float largest0 = -INFINITY, largest1 = -INFINITY;
-#pragma unroll
-                for (int h = 0; h < chunks; ++h) {
-#pragma unroll
-                    for (int c = 0; c < columns / 2; ++c) {
-                        prefix[h][c] = add2(prefix[h][c], pack2(__uint_as_float(d[h][2 * c]), __uint_as_float(d[h][2 * c + 1])));
-                        pair_t const a = fma2(prefix[h][c], mul2(inv_c[h * (columns / 2) + c], row_beta2_binary), bias2_binary);
-                        float a0, a1;
-                        unpack2(a, a0, a1);
-                        decay[h][c] = pack2(fast_ex2(a0), fast_ex2(a1));
-                        largest0 = fmaxf(largest0, a0), largest1 = fmaxf(largest1, a1);
-                    }
-                }
-                float lo, hi, band_g;
-                pair_t loss2 = pack2(0.0f, 0.0f), coefficient2 = pack2(0.0f, 0.0f), g2 = pack2(0.0f, 0.0f);
-                if (__all_sync(0xFFFFFFFFu, fmaxf(largest0, largest1) < easy_negative_limit)) {
-                    pair_t singles = pack2(0.0f, 0.0f), squares = pack2(0.0f, 0.0f), cubes = pack2(0.0f, 0.0f);
-                    pair_t const minus_one = pack2(-1.0f, -1.0f);
-#pragma unroll
-                    for (int h = 0; h < chunks; ++h) {
-#pragma unroll
-                        for (int c = 0; c < columns / 2; ++c) {
-                            pair_t const e = decay[h][c];
-                            pair_t const square = mul2(e, e);
-                            singles = add2(singles, e);
-                            squares = add2(squares, square);
-                            cubes = fma2(square, e, cubes);
-                            pair_t const complement = fma2(square, add2(e, minus_one), e);
-                            pair_t const raw = mul2(complement, inv_c[h * (columns / 2) + c]);
-                            coefficient2 = fma2(raw, prefix[h][c], coefficient2);
-                            float raw0, raw1;
-                            unpack2(raw, raw0, raw1);
-                            d[h][2 * c] = __float_as_uint(raw0), d[h][2 * c + 1] = __float_as_uint(raw1);
-                        }
-                    }
-                    // Both sums are combinations of the power sums: loss e - e^2/2 + e^3/3, complement e - e^2 + e^3.
-                    loss2 = fma2(squares, pack2(-0.5f, -0.5f), singles);
-                    loss2 = fma2(cubes, pack2(1.0f / 3.0f, 1.0f / 3.0f), loss2);
-                    g2 = add2(fma2(squares, minus_one, singles), cubes);
-                } else {
-#pragma unroll
-                    for (int h = 0; h < chunks; ++h) {
-#pragma unroll
-                        for (int c = 0; c < columns / 2; ++c) {
-                            pair_t const scale = mul2(inv_c[h * (columns / 2) + c], row_beta2);
-                            float a0, a1, e0, e1, s0, s1;
-                            unpack2(fma2(prefix[h][c], scale, bias2), a0, a1);
-                            e0 = fast_ex2(-fabsf(a0) * log2_e), e1 = fast_ex2(-fabsf(a1) * log2_e);
-                            pair_t const e = pack2(e0, e1);
-                            unpack2(add2(e, pack2(1.0f, 1.0f)), s0, s1);
-                            pair_t const complement =
-                                mul2(pack2(a0 >= 0.0f ? 1.0f : e0, a1 >= 0.0f ? 1.0f : e1), pack2(fast_rcp(s0), fast_rcp(s1)));
-                            loss2 = add2(fma2(log1p_ratio2(e), e, loss2), pack2(fmaxf(a0, 0.0f), fmaxf(a1, 0.0f)));
-                            g2 = add2(g2, complement);
-                            pair_t const raw = mul2(complement, inv_c[h * (columns / 2) + c]);
-                            coefficient2 = fma2(raw, prefix[h][c], coefficient2);
-                            float raw0, raw1;
-                            unpack2(raw, raw0, raw1);
-                            d[h][2 * c] = __float_as_uint(raw0), d[h][2 * c + 1] = __float_as_uint(raw1);
-                        }
-                    }
-                }
-                unpack2(loss2, lo, hi);
-                loss = lo + hi;
-                unpack2(coefficient2, lo, hi);
-                coefficient = row_beta * (lo + hi);
-                unpack2(g2, lo, hi);
-                band_g = lo + hi;
-                g += band_g;
-                // sum of complement * (logit + bias) = sum of raw * dot + bias * sum of complement
-                ga += fmaf(bias, band_g, coefficient);
-            } else {
-                // Which of this warp's columns, if any, is the row's own copy or its pair partner.
-                int64_t const first = static_cast<int64_t>(p.candidate_base + column);
-                int64_t const own_at = static_cast<int64_t>(global_row) - first;
-                int64_t const partner_at = static_cast<int64_t>(global_row ^ 1ull) - first;
-                int const own_column = own_at >= 0 && own_at < warp_columns ? static_cast<int>(own_at) : -1;
-                int const partner_column =
-                    (p.spec_code & 1u) != 0u && partner_at >= 0 && partner_at < warp_columns ? static_cast<int>(partner_at) : -1;
-                float const without_row_factor = row_beta != 0.0f ? __fdividef(1.0f, row_beta) : 0.0f;
-#pragma unroll
-                for (int h = 0; h < chunks; ++h) {
-#pragma unroll
-                    for (int c = 0; c < columns / 2; ++c) {
-                        prefix[h][c] = add2(prefix[h][c], pack2(__uint_as_float(d[h][2 * c]), __uint_as_float(d[h][2 * c + 1])));
-                        float dot0, dot1, norm0, norm1;
-                        unpack2(prefix[h][c], dot0, dot1);
-                        unpack2(inv_c[h * (columns / 2) + c], norm0, norm1);
-                        int const at = h * columns + 2 * c;
-                        cell_outcome const first_cell = cell_general(dot0, inv_q, norm0, constants.beta, constants.bias,
-                                                                     constants.raw_scale, at == own_column, at == partner_column,
-                                                                     p.spec_code);
-                        cell_outcome const second_cell =
-                            cell_general(dot1, inv_q, norm1, constants.beta, constants.bias, constants.raw_scale,
-                                         at + 1 == own_column, at + 1 == partner_column, p.spec_code);
-                        d[h][2 * c] = __float_as_uint(first_cell.raw * without_row_factor);
-                        d[h][2 * c + 1] = __float_as_uint(second_cell.raw * without_row_factor);
-                        loss += first_cell.loss + second_cell.loss;
-                        g += first_cell.cell + second_cell.cell;
-                        ga += first_cell.cell_logit + second_cell.cell_logit;
-                        coefficient += first_cell.coefficient + second_cell.coefficient;
-                    }
-                }
-            }
-#pragma unroll
-            for (int h = 0; h < chunks; ++h) tmem_store_16(address + h * columns, d[h]);
-            mine[(prefixes_ + k) * fwd_epilogue_threads] += loss;
-            mine[(2 * prefixes_ + k) * fwd_epilogue_threads] += coefficient;
+        // Bands in which some cosine of the patch may sit on the floor (one bit each).
+        uint32_t floors = 0;
+        {
+            bool const may = lane < prefixes_ &&
+                             rows_max * norm_ring[entry * fwd_norm_floats(prefixes_) + prefixes_ * fwd_cols + lane % 8u] >= 100.0f;
+            floors = __ballot_sync(0xFFFFFFFFu, may);
         }
-        tmem_store_wait();
-        timer.lap(2);
-        // Suffix sums, widest band first: band k's gradient cube holds the sum over bands >= k.
-        pair_t running[chunks][columns / 2];
+
+        // The staging patches are rewritten below: the stores of the tile before must have finished reading them.
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        __syncwarp();
+        uint32_t const first_unit = tile_local * prefixes_;
+        // Which of this warp's columns, if any, is the row's own copy or its pair partner: bit c for a cell scored apart, bit
+        // 16 + c for the partner's.
+        uint32_t apart = 0;
+        uint32_t const sums = warp_store_base + (rolled ? lane * 16u : lane * 32u + (((lane >> 2) & 1u) ^ 1u) * 16u);
+        constexpr uint32_t sums_stride = rolled ? 512u : fwd_store_patch_bytes;
+        if (special) {
+            uint64_t const global_row = p.query_base + row;
+            int64_t const first = static_cast<int64_t>(p.candidate_base + column);
+            int64_t const own_at = static_cast<int64_t>(global_row) - first;
+            int64_t const partner_at = static_cast<int64_t>(global_row ^ 1ull) - first;
+            int own_column = -1, partner_column = -1;
+            if (own_at >= 0 && own_at < warp_columns) own_column = static_cast<int>(own_at);
+            if ((p.spec_code & 1u) != 0u && partner_at >= 0 && partner_at < warp_columns) partner_column = static_cast<int>(partner_at);
+            special_sums const total =
+                special_cells<prefixes_, fused_>(lane_base, first_unit, norms_now, p.q_inv + row, p.rows_q, beta, bias, own_column,
+                                                 partner_column, p.spec_code, sums, sums_stride);
+            g += total.cell, own_logit += total.own_logit;
+            apart = (own_column >= 0 ? 1u << own_column : 0u) | (partner_column >= 0 ? 0x10001u << partner_column : 0u);
 #pragma unroll
-        for (int h = 0; h < chunks; ++h)
-#pragma unroll
-            for (int c = 0; c < columns / 2; ++c) running[h][c] = pack2(0.0f, 0.0f);
-        // Bands are taken two at a time: both loads are in flight together, both patches are staged behind one proxy
-        // fence, and both leave in one bulk group, so a tile pays the load -> convert -> stage -> fence -> store latency
-        // chain three times for five bands instead of five times. A [32 rows x 16 columns] patch of a band goes to one of
-        // the warp's staging buffers (32 bytes per row) and leaves as a TMA store issued by lane 0, so no load/store-unit
-        // instruction touches global memory and no other warp is waited for. Before the buffers are rewritten, the
-        // stores that read them (the previous group) must have finished reading.
-        auto band_address = [&](int band) {
-            return lane_base + ((first_unit + (prefixes_ - 1 - band)) % fwd_slots) * fwd_slot_columns;
+            for (int k = 0; k < prefixes_; ++k) {
+                float band_loss, band_coefficient;
+                asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(band_loss), "=f"(band_coefficient)
+                             : "r"(sums + k * sums_stride) : "memory");
+                add_sums(k, band_loss, band_coefficient);
+            }
+        }
+        // Stores the patches from `patch` on to bands `band` and up (one band when they go one by one, else all) of the block's
+        // gradient cube at the tile's place, or (fused kernel) of this CTA's scratch buffer of the item,
+        // [band][128 rows][tiles_per_run * 64 candidates], at the tile's place in the run.
+        auto store_patches = [&](int patch, int band) {
+            uint32_t const store_x = fused_ ? cursor.t * fwd_cols + group * warp_columns : column;
+            uint32_t const store_y = fused_ ? quadrant * 32u : strip * fwd_rows + quadrant * 32u;
+            uint32_t const store_z = fused_ ? (blockIdx.x * 2u + (items_done & 1u)) * prefixes_ : 0u;
+            asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+                             reinterpret_cast<uint64_t>(cube_map)),
+                         "r"(warp_store_base + patch * fwd_store_patch_bytes), "r"(store_x), "r"(store_y), "r"(store_z + band)
+                         : "memory");
         };
-        auto fold_and_pack = [&](uint32_t const (&d)[chunks][columns], int band, uint32_t (&packed)[chunks][columns / 2]) {
-            float const factor = row_factor(beta, mine[band * fwd_epilogue_threads]);
-            pair_t const factor2 = pack2(factor, factor);
+        // A cell scored apart takes no part: its decay, and with it all that the cell adds, becomes zero.
+        auto without_special = [&](pair_t a, int at) {
+            a.x = apart & (1u << at) ? left_out_logit : a.x;
+            a.y = apart & (2u << at) ? left_out_logit : a.y;
+            return a;
+        };
+#pragma unroll 1
+        for (int first = 0; first < warp_columns; first += columns) {
+            pair_t prefix[columns / 2], running[columns / 2];
+            if constexpr (rolled) {
 #pragma unroll
-            for (int h = 0; h < chunks; ++h)
+                for (int c = 0; c < columns / 2; ++c) prefix[c] = running[c] = pack2(0.0f, 0.0f);
+            }
+            pair_t const bias2_binary = pack2(bias * log2_e, bias * log2_e);
+            // One band of the chunk: the dots in `dk` become raw-dot gradients.
+            auto score_band = [&](int const k, uint32_t (&dk)[columns]) {
+                    // The candidates' inverse norms (broadcast shared loads). A cell on the cosine floor has cosine and
+                    // gradient zero, which is what an inverse norm of zero gives it.
+                    pair_t inv_c[columns / 2];
+#pragma unroll
+                    for (int c = 0; c < columns / 2; c += 2) {
+                        float4 const quad = *reinterpret_cast<float4 const*>(norms_now + k * fwd_cols + first + 2 * c);
+                        inv_c[c] = pack2(quad.x, quad.y), inv_c[c + 1] = pack2(quad.z, quad.w);
+                    }
+                    if ((floors >> k) & 1u) {
+                        float const inv_q = __ldg(p.q_inv + static_cast<size_t>(k) * p.rows_q + row);
+#pragma unroll
+                        for (int c = 0; c < columns / 2; ++c) {
+                            inv_c[c].x = inv_q * inv_c[c].x >= 100.0f ? 0.0f : inv_c[c].x;
+                            inv_c[c].y = inv_q * inv_c[c].y >= 100.0f ? 0.0f : inv_c[c].y;
+                        }
+                    }
+                    // First every cell's logit + bias, in base two (the scale and the bias carry log2(e), so that an
+                    // exponential is a single MUFU), and the largest of the thread's cells. Where the warp's cells are all
+                    // easy negatives (every logit + bias below the limit, which is all but the hardest cells) the rest is
+                    // the exponential e and a few packed multiply-adds: log1p(e) = e - e^2/2 + e^3/3 and 1 - sigmoid =
+                    // e / (1 + e) = e - e^2 + e^3, both exact to better than 2e-8 relative below the limit. Up to the second
+                    // limit two more terms of both series do. Otherwise the general form runs: the decay with the absolute
+                    // value, reciprocal, select by sign, the full log1p polynomial, the hinge.
+                    float const row_beta_binary = row_beta[k * factor_stride] * log2_e;
+                    pair_t const row_beta2_binary = pack2(row_beta_binary, row_beta_binary);
+                    pair_t logits[columns / 2];
+                    float largest = -INFINITY;
+#pragma unroll
+                    for (int c = 0; c < columns / 2; ++c) {
+                        pair_t const dots = pack2(__uint_as_float(dk[2 * c]), __uint_as_float(dk[2 * c + 1]));
+                        prefix[c] = !rolled && k == 0 ? dots : add2(prefix[c], dots);
+                        logits[c] = fma2(prefix[c], mul2(inv_c[c], row_beta2_binary), bias2_binary);
+                    }
+                    if (special) {
+#pragma unroll
+                        for (int c = 0; c < columns / 2; ++c) logits[c] = without_special(logits[c], 2 * c);
+                    }
+#pragma unroll
+                    for (int c = 0; c < columns / 2; ++c) largest = fmaxf(fmaxf(largest, logits[c].x), logits[c].y);
+                    pair_t complements = pack2(0.0f, 0.0f), coefficient2 = pack2(0.0f, 0.0f);
+                    float band_loss, band_g;
+                    if (__all_sync(0xFFFFFFFFu, largest < easy_negative_limit)) {
+                        // With u = e^2 - e the complement is c = e + e u, and e^2 and e^3 = c + u are combinations of the two:
+                        // the loss's sum is that of e / 2 - u / 6 + c / 3, so three sums serve both.
+                        pair_t singles, lower;
+#pragma unroll
+                        for (int c = 0; c < columns / 2; ++c) {
+                            pair_t const e = pack2(fast_ex2(logits[c].x), fast_ex2(logits[c].y));
+                            pair_t const u = fma2(e, e, pack2(-e.x, -e.y));
+                            pair_t const complement = fma2(e, u, e);
+                            singles = c == 0 ? e : add2(singles, e);
+                            lower = c == 0 ? u : add2(lower, u);
+                            complements = c == 0 ? complement : add2(complements, complement);
+                            pair_t const raw = mul2(complement, inv_c[c]);
+                            coefficient2 = c == 0 ? mul2(raw, prefix[c]) : fma2(raw, prefix[c], coefficient2);
+                            dk[2 * c] = __float_as_uint(raw.x), dk[2 * c + 1] = __float_as_uint(raw.y);
+                        }
+                        band_g = complements.x + complements.y;
+                        band_loss = fmaf(0.5f, singles.x + singles.y, fmaf(-1.0f / 6.0f, lower.x + lower.y, (1.0f / 3.0f) * band_g));
+                    } else if (__all_sync(0xFFFFFFFFu, largest < near_negative_limit)) {
+                        pair_t const minus_one = pack2(-1.0f, -1.0f);
+                        pair_t loss2 = pack2(0.0f, 0.0f);
+#pragma unroll
+                        for (int c = 0; c < columns / 2; ++c) {
+                            pair_t const e = pack2(fast_ex2(logits[c].x), fast_ex2(logits[c].y));
+                            pair_t s = fma2(e, pack2(-0.2f, -0.2f), pack2(0.25f, 0.25f)); // minus the series of log1p(e) / e
+                            pair_t h = add2(e, minus_one);                                // minus that of 1 / (1 + e)
+                            h = fma2(e, h, pack2(1.0f, 1.0f)), s = fma2(e, s, pack2(-1.0f / 3.0f, -1.0f / 3.0f));
+                            h = fma2(e, h, minus_one), s = fma2(e, s, pack2(0.5f, 0.5f));
+                            h = fma2(e, h, pack2(1.0f, 1.0f)), s = fma2(e, s, minus_one);
+                            loss2 = fma2(e, s, loss2);
+                            pair_t const complement = mul2(e, h);
+                            complements = add2(complements, complement);
+                            pair_t const raw = mul2(complement, inv_c[c]);
+                            coefficient2 = fma2(raw, prefix[c], coefficient2);
+                            dk[2 * c] = __float_as_uint(raw.x), dk[2 * c + 1] = __float_as_uint(raw.y);
+                        }
+                        band_g = complements.x + complements.y;
+                        band_loss = -(loss2.x + loss2.y);
+                    } else {
+                        pair_t hinges = pack2(0.0f, 0.0f), loss2 = pack2(0.0f, 0.0f);
+                        float const factor = row_beta[k * factor_stride];
+                        pair_t const row_beta2 = pack2(factor, factor);
+#pragma unroll
+                        for (int c = 0; c < columns / 2; ++c) {
+                            // In natural units: a hard cell's gradient is large, and is rounded as the special cells' are.
+                            pair_t a = fma2(prefix[c], mul2(inv_c[c], row_beta2), pack2(bias, bias));
+                            a = without_special(a, 2 * c);
+                            pair_t const e = pack2(fast_ex2(-fabsf(a.x) * log2_e), fast_ex2(-fabsf(a.y) * log2_e));
+                            pair_t const whole = add2(e, pack2(1.0f, 1.0f));
+                            pair_t const complement = mul2(pack2(a.x >= 0.0f ? 1.0f : e.x, a.y >= 0.0f ? 1.0f : e.y),
+                                                           pack2(fast_rcp(whole.x), fast_rcp(whole.y)));
+                            loss2 = fma2(log1p_ratio2(e), e, loss2);
+                            hinges = add2(hinges, pack2(fmaxf(a.x, 0.0f), fmaxf(a.y, 0.0f)));
+                            complements = add2(complements, complement);
+                            pair_t const raw = mul2(complement, inv_c[c]);
+                            coefficient2 = fma2(raw, prefix[c], coefficient2);
+                            dk[2 * c] = __float_as_uint(raw.x), dk[2 * c + 1] = __float_as_uint(raw.y);
+                        }
+                        band_g = complements.x + complements.y;
+                        band_loss = (hinges.x + hinges.y) + (loss2.x + loss2.y);
+                    }
+                    if (special) {
+                        float raw;
+                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(raw) : "r"(sums + k * sums_stride + 8u) : "memory");
+#pragma unroll
+                        for (int c = 0; c < columns; ++c) dk[c] = apart & (0x10000u << c) ? __float_as_uint(raw) : dk[c];
+                    }
+                    add_sums(k, band_loss, coefficient2.x + coefficient2.y);
+                    g += band_g;
+            };
+            // Suffix sums, widest band first: band k's gradient cube holds the sum over bands >= k, each with its row
+            // factor beta / |q_k|. A warp's patch of a band is [32 rows x 16 columns] bfloat16, 32 bytes per row, under the
+            // 32-byte swizzle (the two 16-byte halves of a row change places in every second group of four rows), so that
+            // the eight lanes of a store phase cover all banks: unswizzled, every phase had two lanes on each bank.
+            auto sum_band = [&](int const k, uint32_t const (&dk)[columns], int const patch) {
+                float const factor = row_beta[k * factor_stride];
+                pair_t const factor2 = pack2(factor, factor);
+                uint32_t packed[columns / 2];
 #pragma unroll
                 for (int c = 0; c < columns / 2; ++c) {
-                    running[h][c] =
-                        fma2(pack2(__uint_as_float(d[h][2 * c]), __uint_as_float(d[h][2 * c + 1])), factor2, running[h][c]);
-                    float lo, hi;
-                    unpack2(running[h][c], lo, hi);
-                    packed[h][c] = pack_bf16x2(lo, hi);
+                    pair_t const raw = pack2(__uint_as_float(dk[2 * c]), __uint_as_float(dk[2 * c + 1]));
+                    running[c] = !rolled && k == prefixes_ - 1 ? mul2(raw, factor2) : fma2(raw, factor2, running[c]);
+                    packed[c] = pack_bf16x2(running[c].x, running[c].y);
                 }
-        };
-        auto stage_patches = [&](uint32_t const (&packed)[chunks][columns / 2], uint32_t half) {
 #pragma unroll
-            for (int h = 0; h < chunks; ++h) {
-                uint32_t const patch = warp_store_base + (half * chunks + h) * fwd_store_patch_bytes + lane * 32u;
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(patch), "r"(packed[h][0]), "r"(packed[h][1]),
-                             "r"(packed[h][2]), "r"(packed[h][3]) : "memory");
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(patch + 16u), "r"(packed[h][4]), "r"(packed[h][5]),
-                             "r"(packed[h][6]), "r"(packed[h][7]) : "memory");
-            }
-        };
-        // Where the warp's patches go: into the block's gradient cube at the tile's place, or (fused kernel) into this
-        // CTA's scratch buffer of the item, [band][128 rows][tiles_per_run * 64 candidates], at the tile's place in the run.
-        uint32_t const store_x = fused_ ? cursor.t * fwd_cols + group * warp_columns : column;
-        uint32_t const store_y = fused_ ? quadrant * 32u : strip * fwd_rows + quadrant * 32u;
-        uint32_t const store_z = fused_ ? (blockIdx.x * 2u + (items_done & 1u)) * prefixes_ : 0u;
-        auto send_patches = [&](uint32_t half, int band) {
+                for (int part = 0; part < columns; part += 8) {
+                    uint32_t const half = static_cast<uint32_t>(first + part) / 8u;
+                    uint32_t const at = warp_store_base + patch * fwd_store_patch_bytes + lane * 32u + (((half & 1u) ^ ((lane >> 2) & 1u)) * 16u);
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(packed[part / 2]),
+                                 "r"(packed[part / 2 + 1]), "r"(packed[part / 2 + 2]), "r"(packed[part / 2 + 3]) : "memory");
+                }
+            };
+            auto load_bands = [&](auto& d, int const from, int const to) {
 #pragma unroll
-            for (int h = 0; h < chunks; ++h)
-                asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
-                                 reinterpret_cast<uint64_t>(cube_map)),
-                             "r"(warp_store_base + (half * chunks + h) * fwd_store_patch_bytes), "r"(store_x + h * columns),
-                             "r"(store_y), "r"(store_z + band)
-                             : "memory");
-        };
-        auto release = [&](uint64_t* barriers) {
-            tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&barriers[tile_local % fwd_slots]));
-        };
-        int k = prefixes_ - 1;
+                for (int k = from; k < to; ++k) tmem_load<columns>(lane_base + band_slot<prefixes_, fused_>(first_unit, k) + first, d[k - from]);
+                tmem_load_wait();
+            };
+            auto release_slots = [&](uint64_t* barriers) { // this warp is done with the tile's slots (or one kind of them)
+                if (first + columns != warp_columns) return;
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&barriers[tile_local % fwd_slots]));
+            };
+            if constexpr (rolled) {
 #pragma unroll 1
-        for (; k >= 1; k -= 2) {
-            uint32_t upper[chunks][columns], lower[chunks][columns];
+                for (int k = 0; k < prefixes_; ++k) {
+                    uint32_t const address = lane_base + band_slot<prefixes_, fused_>(first_unit, k);
+                    uint32_t d[columns];
+                    tmem_load<columns>(address, d);
+                    tmem_load_wait();
+                    score_band(k, d);
+                    tmem_store_16(address, d);
+                }
+                tmem_store_wait();
+                // Two bands at a time, widest first: both loads in flight, both patches behind one proxy fence and in one bulk
+                // group; a pair's patches are rewritten two pairs later, once their stores have read them.
+#pragma unroll 1
+                for (int k = prefixes_ - 1; k >= 0; k -= 2) {
+                    int const below = k > 0 ? k - 1 : 0, patch = ((prefixes_ - 1 - k) / 2 % 2) * 2;
+                    uint32_t upper[columns], lower[columns];
+                    tmem_load<columns>(lane_base + band_slot<prefixes_, fused_>(first_unit, k), upper);
+                    tmem_load<columns>(lane_base + band_slot<prefixes_, fused_>(first_unit, below), lower);
+                    tmem_load_wait();
+                    if (k == prefixes_ - 1) release_slots(tail->tile_taken);
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                    __syncwarp();
+                    sum_band(k, upper, patch);
+                    if (k > 0) sum_band(below, lower, patch + 1);
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) {
+                        store_patches(patch, k);
+                        if (k > 0) store_patches(patch + 1, below);
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    }
+                }
+                release_slots(tail->tile_parked_taken);
+            } else {
+            if constexpr (parked > 0) {
+                uint32_t d[parked][columns];
+                load_bands(d, 0, parked);
 #pragma unroll
-            for (int h = 0; h < chunks; ++h) tmem_load_16(band_address(k) + h * columns, upper[h]);
+                for (int k = 0; k < parked; ++k) {
+                    score_band(k, d[k]);
+                    tmem_store_8(lane_base + band_slot<prefixes_, fused_>(first_unit, k) + first, d[k]);
+                }
+            }
+            {
+                uint32_t d[prefixes_ - parked][columns];
+                load_bands(d, parked, prefixes_);
+                release_slots(tail->tile_taken);
 #pragma unroll
-            for (int h = 0; h < chunks; ++h) tmem_load_16(band_address(k - 1) + h * columns, lower[h]);
-            tmem_load_wait();
-            if (k == prefixes_ - 1) release(tail->tile_early);
-            uint32_t packed_upper[chunks][columns / 2], packed_lower[chunks][columns / 2];
-            fold_and_pack(upper, k, packed_upper);
-            fold_and_pack(lower, k - 1, packed_lower);
-            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            __syncwarp();
-            stage_patches(packed_upper, 0);
-            stage_patches(packed_lower, 1);
+                for (int k = parked; k < prefixes_; ++k) score_band(k, d[k - parked]);
+#pragma unroll
+                for (int k = prefixes_ - 1; k >= parked; --k) sum_band(k, d[k - parked], k);
+            }
+            if constexpr (parked > 0) {
+                uint32_t d[parked][columns];
+                tmem_store_wait();
+                load_bands(d, 0, parked);
+                release_slots(tail->tile_parked_taken);
+#pragma unroll
+                for (int k = parked - 1; k >= 0; --k) sum_band(k, d[k], k);
+            }
+            }
+            apart >>= columns; // the next chunk's cells
+        }
+        timer.lap(2);
+        if constexpr (!rolled) {
+            // The tile's patches, all bands of them, leave as one TMA store issued by one lane.
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) {
-                send_patches(0, k);
-                send_patches(1, k - 1);
+                store_patches(0, 0);
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
         }
-        if (k == 0) {
-            uint32_t last[chunks][columns];
-#pragma unroll
-            for (int h = 0; h < chunks; ++h) tmem_load_16(band_address(0) + h * columns, last[h]);
-            tmem_load_wait();
-            if (prefixes_ == 1) release(tail->tile_early);
-            uint32_t packed_last[chunks][columns / 2];
-            fold_and_pack(last, 0, packed_last);
-            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            __syncwarp();
-            stage_patches(packed_last, 0);
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) {
-                send_patches(0, 0);
-                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            }
-        }
+        if (lane == 0) mbar_arrive(smem_u32(&tail->norms_empty[entry])); // every lane's reads are behind a __syncwarp above
         timer.lap(3);
-        // This warp is done with the tile's slots.
-        release(tail->tile_late);
-        if (more) park(buffer ^ 1u);
         if (cursor.t + 1 == p.tiles_per_run) {
             // One partial record per (run, column group, row); the 1/N weight and the mirror cell's factor two go in here.
             uint32_t const slot = run * fwd_column_groups + group;
             float* record = p.partials + static_cast<size_t>(slot) * quantities * p.rows_q + row;
             if (SC_IN_BOUNDS((static_cast<size_t>(slot) * quantities + quantities - 1) * p.rows_q + row,
                              static_cast<size_t>(p.runs_per_strip) * fwd_column_groups * quantities * p.rows_q)) {
-            record[0] = p.weight * g;
-            record[static_cast<size_t>(1) * p.rows_q] = p.weight * (ga - bias * g);
+                // sum of cell gradient * logit: the coefficients are exactly that, except for a row's own copy, whose logit
+                // is the scale itself and which moves no dot product
+                float logits = own_logit;
 #pragma unroll
-            for (int k = 0; k < prefixes_; ++k) {
-                record[static_cast<size_t>(2 + k) * p.rows_q] = p.weight * mine[(prefixes_ + k) * fwd_epilogue_threads];
-                record[static_cast<size_t>(2 + prefixes_ + k) * p.rows_q] =
-                    2.0f * p.weight * mine[(2 * prefixes_ + k) * fwd_epilogue_threads];
-            }
+                for (int k = 0; k < prefixes_; ++k) {
+                    float const band_loss = rolled ? band_sums[k * fwd_epilogue_threads] : loss[rolled ? 0 : k];
+                    float const band_coefficient = rolled ? band_sums[(prefixes_ + k) * fwd_epilogue_threads] : coefficient[rolled ? 0 : k];
+                    float const whole = row_beta[k * factor_stride] * band_coefficient;
+                    logits += whole;
+                    record[static_cast<size_t>(2 + k) * p.rows_q] = p.weight * band_loss;
+                    record[static_cast<size_t>(2 + prefixes_ + k) * p.rows_q] = 2.0f * p.weight * whole;
+                }
+                record[0] = p.weight * g;
+                record[static_cast<size_t>(1) * p.rows_q] = p.weight * logits;
             }
             if constexpr (fused_) {
                 // The item's patches of this warp are in memory once its bulk stores have completed (not merely been
@@ -833,8 +1008,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
                 if (!drain((items_done - 1) * p.tile_count, true)) return;
             }
         }
-        cursor = following;
-        buffer ^= 1u;
+        cursor.advance(p);
         ++tile_local;
     }
     timer.flush(p, 5, 4);
@@ -853,7 +1027,8 @@ __device__ __forceinline__ void fz_producer_role(fz_maps const* maps, fwd_params
     uint32_t stage = 0, phase = 0, local = 0;
     phase_timer timer(p);
     timer.only_if(elected);
-    for (uint32_t item = blockIdx.x; item < p.items; item += gridDim.x, ++local) {
+    for (uint32_t count = item_count(p.items); local < count; ++local) {
+        uint32_t const item = item_at(p.items, local);
         uint32_t const buffer = local & 1u;
         timer.lap(0);
         if (!mbar_wait_warp(smem_u32(&tail->fz_item_stored[buffer]), (local >> 1) & 1u, ctx, site_fz_item_stored, item, sleep_producer_ns))
@@ -904,7 +1079,8 @@ __device__ __forceinline__ void fz_mma_role(fwd_params const& p, uint32_t stages
     uint32_t stage = 0, phase = 0, unit = 0;
     phase_timer timer(p);
     timer.only_if(elected);
-    for (uint32_t item = blockIdx.x; item < p.items; item += gridDim.x) {
+    for (uint32_t n = 0, count = item_count(p.items); n < count; ++n) {
+        uint32_t const item = item_at(p.items, n);
         for (uint32_t which = 0; which < p.tile_count; ++which, ++unit) {
             uint32_t const idesc = umma_idesc_bf16(128, (p.tiles[which] >> 16) * 16u);
             // The accumulator's previous contents must have left tensor memory (an arrival per epilogue warp).
@@ -959,7 +1135,7 @@ __device__ __forceinline__ void pull_role(pull_request const& request, uint32_t 
 }
 
 template <int prefixes_, bool fused_>
-__global__ void __launch_bounds__(fwd_threads_for(fused_), 1)
+__global__ void __launch_bounds__(fwd_threads, 1)
     forward_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap c_map,
                    const __grid_constant__ CUtensorMap cube_map, const __grid_constant__ fz_maps gemm_maps,
                    const fwd_params p) {
@@ -970,7 +1146,7 @@ __global__ void __launch_bounds__(fwd_threads_for(fused_), 1)
     uint32_t const stages_base = (raw_address + 1023u) & ~1023u;
     uint32_t const gemm_stages_base = stages_base + stages * fwd_stage_bytes;
     uint32_t const store_base = stages_base + fwd_stage_region_bytes(prefixes_, fused_);
-    fwd_tail* tail = reinterpret_cast<fwd_tail*>(raw_shared + (store_base - raw_address) + fwd_store_bytes);
+    fwd_tail* tail = reinterpret_cast<fwd_tail*>(raw_shared + (store_base - raw_address) + fwd_store_bytes(prefixes_));
     uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 
     if (threadIdx.x == 0) {
@@ -980,10 +1156,14 @@ __global__ void __launch_bounds__(fwd_threads_for(fused_), 1)
             mbar_init(smem_u32(&tail->stage_empty[i]), 1);
         }
         for (uint32_t i = 0; i < fwd_slots; ++i) {
-            mbar_init(smem_u32(&tail->tile_early[i]), fwd_epilogue_warps);
-            mbar_init(smem_u32(&tail->tile_late[i]), fwd_epilogue_warps);
+            mbar_init(smem_u32(&tail->tile_taken[i]), fwd_epilogue_warps);
+            mbar_init(smem_u32(&tail->tile_parked_taken[i]), fwd_epilogue_warps);
         }
         for (uint32_t i = 0; i < fwd_tile_barriers; ++i) mbar_init(smem_u32(&tail->tile_full[i]), 1);
+        for (uint32_t i = 0; i < fwd_norm_slots; ++i) {
+            mbar_init(smem_u32(&tail->norms_full[i]), 1);
+            mbar_init(smem_u32(&tail->norms_empty[i]), fwd_epilogue_warps);
+        }
         if constexpr (fused_) {
             for (uint32_t i = 0; i < fz_stages; ++i) {
                 mbar_init(smem_u32(&tail->fz_stage_full[i]), 1);
@@ -1018,12 +1198,15 @@ __global__ void __launch_bounds__(fwd_threads_for(fused_), 1)
     uint32_t const tmem_base = tail->tmem_base;
     wait_context const ctx{p.status, p.budget_ns, &tail->abort_flag};
 
+    float* const norm_ring = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(tail) + fwd_tail_bytes);
     if (warp < fwd_epilogue_warps) {
-        float* const norm_staging = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(tail) + fwd_tail_bytes);
-        epilogue_role<prefixes_, fused_>(&cube_map, p, tail, store_base, norm_staging, norm_staging + fwd_norm_bytes / 4,
-                                         tmem_base, ctx, warp, lane);
-    } else if (warp == fwd_producer_warp) {
-        producer_role(&q_map, &c_map, p, stages_base, tail, ctx, stages);
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(fwd_epilogue_registers));
+        epilogue_role<prefixes_, fused_>(&cube_map, p, tail, store_base, norm_ring, norm_ring + fwd_norm_bytes(prefixes_) / 4, tmem_base, ctx, warp,
+                                         lane);
+    } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(fwd_helper_registers));
+    if (warp == fwd_producer_warp) {
+        producer_role<prefixes_>(&q_map, &c_map, p, stages_base, norm_ring, tail, ctx, stages);
     } else if (warp == fwd_mma_warp) {
         mma_role<prefixes_, fused_>(p, stages_base, tail, tmem_base, ctx);
     } else if (warp == fwd_first_pull_warp) {
@@ -1033,6 +1216,7 @@ __global__ void __launch_bounds__(fwd_threads_for(fused_), 1)
         if constexpr (fused_) fz_producer_role(&gemm_maps, p, gemm_stages_base, tail, ctx, prefixes_);
     } else if (warp == fz_mma_warp) {
         if constexpr (fused_) fz_mma_role(p, gemm_stages_base, tail, tmem_base, ctx);
+    }
     }
 
     tcgen05_fence_before();
@@ -1069,7 +1253,7 @@ void launch_instance(CUtensorMap const& q_map, CUtensorMap const& c_map, CUtenso
                 "raising the forward kernel's shared memory");
         prepared_device = device;
     }
-    forward_kernel<prefixes_, fused_><<<blocks, fwd_threads_for(fused_), fwd_shared_bytes(prefixes_, fused_), stream>>>(
+    forward_kernel<prefixes_, fused_><<<blocks, fwd_threads, fwd_shared_bytes(prefixes_, fused_), stream>>>(
         q_map, c_map, cube_map, gemm_maps, p);
 }
 
@@ -1183,12 +1367,13 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
     CUtensorMap const& c_map = operand_map(a.candidates_bf16, a.hidden, a.rows_c, fwd_depth, fwd_cols);
     fz_maps gemm_maps{};
     if (!a.fused) {
-        // The warps' patches of the gradient cube [K, rows_q, rows_c]: boxes of 32 rows x 16 candidates, unswizzled.
+        // The warps' patches of the gradient cube [K, rows_q, rows_c]: boxes of all bands x 32 rows x 16 candidates, staged under the
+        // 32-byte swizzle.
         cuuint64_t const dims[3] = {a.rows_c, a.rows_q, a.ladder.count};
         cuuint64_t const strides[2] = {static_cast<cuuint64_t>(a.rows_c) * 2, static_cast<cuuint64_t>(a.rows_c) * a.rows_q * 2};
-        cuuint32_t const box[3] = {fwd_chunk_columns, 32, 1};
+        cuuint32_t const box[3] = {fwd_warp_columns, 32, fwd_rolled_for(static_cast<int>(a.ladder.count)) ? 1u : a.ladder.count};
         CUtensorMap const& cube_map =
-            cached_map(a.gradient_cube_bf16, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE);
+            cached_map(a.gradient_cube_bf16, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
         launch_for_count<false>(a.ladder.count, q_map, c_map, cube_map, gemm_maps, p, blocks, stream);
     } else {
         p.gradient = a.query_gradient, p.gradient_scale = a.gradient_scale;
@@ -1199,14 +1384,14 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
                 p.tiles[p.tile_count++] = band | ((channel / 16) << 4) | (((left < fz_max_width ? left : fz_max_width) / 16) << 16);
             }
         // Scratch of gradient patches: [CTA and buffer][band][128 rows][run of candidates], written in the warps' boxes
-        // (unswizzled), read back as the GEMM's A operand (128 rows x 64 candidates, swizzled).
+        // (under the 32-byte swizzle), read back as the GEMM's A operand (128 rows x 64 candidates, swizzled).
         uint64_t const run = static_cast<uint64_t>(a.tiles_per_run) * fwd_cols;
         cuuint64_t const dims[3] = {run, fwd_rows, static_cast<cuuint64_t>(blocks) * 2 * a.ladder.count};
         cuuint64_t const strides[2] = {run * 2, run * fwd_rows * 2};
-        cuuint32_t const store_box[3] = {fwd_chunk_columns, 32, 1};
+        cuuint32_t const store_box[3] = {fwd_warp_columns, 32, a.ladder.count};
         cuuint32_t const load_box[3] = {fz_depth, fwd_rows, 1};
         CUtensorMap const& store_map =
-            cached_map(a.fused_scratch_bf16, 3, dims, strides, store_box, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE);
+            cached_map(a.fused_scratch_bf16, 3, dims, strides, store_box, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
         gemm_maps.patches =
             cached_map(a.fused_scratch_bf16, 3, dims, strides, load_box, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
         for (uint32_t index = 0; index < fz_candidate_maps; ++index) {
