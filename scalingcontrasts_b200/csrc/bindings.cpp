@@ -141,6 +141,11 @@ struct loss_plan {
         scored = 0;
     }
 
+    void clear_gradient(cudaStream_t stream) {
+        runtime_check(cudaMemsetAsync(pointer<void>(query_gradient), 0, static_cast<size_t>(rows_q) * hidden * 4, stream),
+                      "cudaMemsetAsync");
+    }
+
     void launch_pending_on_side() {
         runtime_check(cudaStreamWaitEvent(side, forward_done[pending_slot], 0), "cudaStreamWaitEvent");
         sc::launch_backward(pending_backward, side);
@@ -160,6 +165,11 @@ struct loss_plan {
             sc::launch_backward(pending_backward, stream);
             pending = false;
         }
+        if (scored == 0) { // a step that scored no block: its sums are zero
+            clear_gradient(stream);
+            runtime_check(cudaMemsetAsync(pointer<void>(accumulators), 0, static_cast<size_t>(rows_q) * quantities * 4, stream),
+                          "cudaMemsetAsync");
+        }
         scored = 0;
     }
 
@@ -174,6 +184,7 @@ struct loss_plan {
         uint64_t const cube = slot ? gradients_alt : gradients;
         // this cube was last read by the backward of the block before the previous one
         if (overlapping && scored >= 2) runtime_check(cudaStreamWaitEvent(stream, backward_done[slot], 0), "cudaStreamWaitEvent");
+        if (fused && scored == 0) clear_gradient(stream); // items of the fused kernel add in no fixed order
         if (transposing) sc::launch_transpose(pointer<void>(candidates), pointer<void>(transposed), rows_c, hidden, stream);
         sc::forward_arguments a{};
         a.queries_bf16 = pointer<void>(queries), a.candidates_bf16 = pointer<void>(candidates);
@@ -201,7 +212,8 @@ struct loss_plan {
             runtime_check(cudaEventRecord(rejoined[slot], front), "cudaEventRecord");
             runtime_check(cudaStreamWaitEvent(stream, rejoined[slot], 0), "cudaStreamWaitEvent");
         } else sc::launch_forward(a, stream);
-        sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows_q, partial_slots, quantities, stream);
+        sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows_q, partial_slots, quantities, scored == 0,
+                                 stream);
         if (!fused) {
             sc::backward_arguments b{};
             b.gradient_cube_bf16 = pointer<void>(cube);
@@ -210,6 +222,9 @@ struct loss_plan {
             b.query_gradient = pointer<float>(query_gradient), b.status = pointer<uint32_t>(status);
             b.rows_q = rows_q, b.rows_c = rows_c, b.hidden = hidden, b.ladder = ladder, b.split = backward_split;
             b.scale = static_cast<float>(2.0 / live), b.budget_ns = budget_ns;
+            // a step's first block replaces what the step before left; its partial sums of a split launch need zeros to start from
+            b.overwrite = scored == 0 && backward_split == 1;
+            if (scored == 0 && backward_split != 1) clear_gradient(stream);
             if (!overlapping) sc::launch_backward(b, stream);
             else {
                 runtime_check(cudaEventRecord(forward_done[slot], stream), "cudaEventRecord");
@@ -326,15 +341,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     });
     m.def("fold_partials", [](uint64_t partials, uint64_t accumulators, uint32_t rows, uint32_t slots, uint32_t quantities,
                               uint64_t stream) {
-        sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows, slots, quantities, stream_of(stream));
+        sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows, slots, quantities, false, stream_of(stream));
     });
-    m.def("finalize", [](uint64_t queries, uint64_t inverse_norms, uint64_t accumulators, uint64_t query_gradient, uint64_t out,
-                         uint32_t rows, uint32_t hidden, std::vector<uint32_t> const& ends, uint64_t stream) {
-        sc::launch_finalize(pointer<void>(queries), pointer<float>(inverse_norms), pointer<float>(accumulators),
-                            pointer<float>(query_gradient), pointer<void>(out), rows, hidden, ladder_of(ends), stream_of(stream));
-    });
-    m.def("sum_summands", [](uint64_t accumulators, uint64_t summands, uint32_t rows, uint32_t prefixes, uint64_t stream) {
-        sc::launch_sum_summands(pointer<float>(accumulators), pointer<float>(summands), rows, prefixes, stream_of(stream));
+    m.def("finish", [](uint64_t queries, uint64_t inverse_norms, uint64_t accumulators, uint64_t query_gradient, uint64_t out,
+                       uint64_t summands, uint32_t rows, uint32_t hidden, std::vector<uint32_t> const& ends, uint64_t stream) {
+        sc::launch_finish(pointer<void>(queries), pointer<float>(inverse_norms), pointer<float>(accumulators),
+                          pointer<float>(query_gradient), pointer<void>(out), pointer<float>(summands), rows, hidden, ladder_of(ends),
+                          stream_of(stream));
     });
     py::class_<loss_plan, std::shared_ptr<loss_plan>>(m, "LossPlan")
         .def(py::init([](uint32_t rows_q, uint32_t rows_c, uint32_t hidden, std::vector<uint32_t> const& ends,

@@ -5,9 +5,9 @@
 //                     largest inverse norm, which lets a tile prove that no cosine of it sits on the floor
 //   transpose         [R, H] -> [H, R] so that the gradient tiles read candidates K-major
 //   pull              peer block -> local staging by plain 16-byte loads and stores
-//   fold_partials     per row, adds the forward kernel's per-run partials in run order (deterministic)
-//   finalize          folds the L2-normalisation's self term into the query gradient and casts to bfloat16
-//   sum_summands      fixed-tree sums of the row accumulators into the loss summands
+//   fold_partials     per row, adds the forward kernel's per-run partials in a fixed order (deterministic)
+//   finish            folds the L2-normalisation's self term into the query gradient and casts to bfloat16; fixed-tree sums
+//                     of the row accumulators into the loss summands
 //
 // Parity: transpose_cuda_, prefix_inverse_norms_cuda_, fold_partials_cuda_, finalize_cuda_, sum_summands_cuda_
 // (scalingcontrasts.cuh:660-686, 1138-1177); keyed_* and count_* (scalingcontrasts.cu:48-105). The staging pull
@@ -35,60 +35,78 @@ ladder_t to_device(ladder_host const& host) {
     return ladder;
 }
 
-// One warp per row. Each lane reads 16-byte vectors (8 channels); band edges are multiples of 16 channels, so a vector
-// never straddles two bands.
-__global__ void __launch_bounds__(256)
+// A block takes 64 rows, a warp two of them with the loads of both in flight; the block then has the rows' largest inverse
+// norm per band at hand, which had a launch of its own before (2.9 us). Each lane reads 16-byte vectors (8 channels); band
+// edges are multiples of 16 channels, so a vector never straddles two bands.
+constexpr uint32_t norm_rows = 64, norm_warps = 32;
+__global__ void __launch_bounds__(norm_warps * 32)
     prefix_norms_kernel(uint4 const* __restrict__ rows, uint4* __restrict__ copy, float* __restrict__ inverse_norms,
-                        uint32_t row_count, uint32_t hidden, ladder_t ladder) {
+                        float* __restrict__ tile_max, uint32_t row_count, uint32_t hidden, ladder_t ladder) {
+    constexpr uint32_t each = norm_rows / norm_warps;
+    __shared__ float largest[norm_warps][8];
     uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    uint32_t const row = blockIdx.x * 8 + warp;
-    if (row >= row_count) return;
+    uint32_t const first = blockIdx.x * norm_rows + warp * each;
     uint32_t const vectors = hidden / 8;
-    float sums[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (uint32_t v = lane; v < vectors; v += 32) {
-        if (!SC_IN_BOUNDS(static_cast<size_t>(row) * vectors + v, static_cast<size_t>(row_count) * vectors)) continue;
-        uint4 const packed = rows[static_cast<size_t>(row) * vectors + v];
-        if (copy != nullptr) copy[static_cast<size_t>(row) * vectors + v] = packed;
-        uint32_t const words[4] = {packed.x, packed.y, packed.z, packed.w};
-        float square = 0;
+    float sums[each][8];
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            float const lo = __uint_as_float(words[w] << 16), hi = __uint_as_float(words[w] & 0xFFFF0000u);
-            square = fmaf(lo, lo, square);
-            square = fmaf(hi, hi, square);
+    for (uint32_t r = 0; r < each; ++r)
+#pragma unroll
+        for (int band = 0; band < 8; ++band) sums[r][band] = 0.0f;
+    for (uint32_t v = lane; v < vectors; v += 32) {
+        uint4 packed[each];
+#pragma unroll
+        for (uint32_t r = 0; r < each; ++r) {
+            packed[r] = make_uint4(0u, 0u, 0u, 0u);
+            if (first + r < row_count && SC_IN_BOUNDS(static_cast<size_t>(first + r) * vectors + v, static_cast<size_t>(row_count) * vectors))
+                packed[r] = rows[static_cast<size_t>(first + r) * vectors + v];
         }
         uint32_t const channel = v * 8;
 #pragma unroll
-        for (int band = 0; band < 8; ++band)
-            if (band < ladder.count && channel >= ladder.begin(band) && channel < ladder.ends[band]) sums[band] += square;
+        for (uint32_t r = 0; r < each; ++r) {
+            if (copy != nullptr && first + r < row_count) copy[static_cast<size_t>(first + r) * vectors + v] = packed[r];
+            uint32_t const words[4] = {packed[r].x, packed[r].y, packed[r].z, packed[r].w};
+            float square = 0;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                float const lo = __uint_as_float(words[w] << 16), hi = __uint_as_float(words[w] & 0xFFFF0000u);
+                square = fmaf(lo, lo, square);
+                square = fmaf(hi, hi, square);
+            }
+#pragma unroll
+            for (int band = 0; band < 8; ++band)
+                if (band < ladder.count && channel >= ladder.begin(band) && channel < ladder.ends[band]) sums[r][band] += square;
+        }
     }
-    float running = 0;
+    float running[each];
+#pragma unroll
+    for (uint32_t r = 0; r < each; ++r) running[r] = 0.0f;
 #pragma unroll
     for (int band = 0; band < 8; ++band) {
         if (band >= ladder.count) break;
-        float total = sums[band];
+        float warp_max = 0.0f;
 #pragma unroll
-        for (int offset = 16; offset > 0; offset >>= 1) total += __shfl_xor_sync(0xFFFFFFFFu, total, offset);
-        running += total;
-        if (lane == 0 && SC_IN_BOUNDS(static_cast<size_t>(band) * row_count + row, static_cast<size_t>(ladder.count) * row_count))
-            inverse_norms[static_cast<size_t>(band) * row_count + row] = running > 0.0f ? rsqrtf(running) : 0.0f;
+        for (uint32_t r = 0; r < each; ++r) {
+            float total = sums[r][band];
+#pragma unroll
+            for (int offset = 16; offset > 0; offset >>= 1) total += __shfl_xor_sync(0xFFFFFFFFu, total, offset);
+            running[r] += total;
+            float const inverse = running[r] > 0.0f ? rsqrtf(running[r]) : 0.0f;
+            if (lane == 0 && first + r < row_count &&
+                SC_IN_BOUNDS(static_cast<size_t>(band) * row_count + first + r, static_cast<size_t>(ladder.count) * row_count))
+                inverse_norms[static_cast<size_t>(band) * row_count + first + r] = inverse;
+            warp_max = fmaxf(warp_max, inverse);
+        }
+        if (lane == 0) largest[warp][band] = warp_max;
     }
-}
-
-// tile_max[band, t] = max over rows [64 t, 64 t + 64) of inverse_norms[band, row].
-__global__ void tile_max_kernel(float const* __restrict__ inverse_norms, float* __restrict__ tile_max, uint32_t row_count,
-                                uint32_t bands) {
-    uint32_t const tiles = row_count / 64;
-    uint32_t const index = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    uint32_t const lane = threadIdx.x % 32;
-    if (index >= tiles * bands) return;
-    uint32_t const band = index / tiles, tile = index % tiles;
-    float const* base = inverse_norms + static_cast<size_t>(band) * row_count + tile * 64;
-    if (!SC_IN_BOUNDS(static_cast<size_t>(band) * row_count + tile * 64 + lane + 32, static_cast<size_t>(bands) * row_count)) return;
-    float value = fmaxf(base[lane], base[lane + 32]);
+    if (tile_max == nullptr) return;
+    __syncthreads();
+    // tile_max[band, t] = max over rows [64 t, 64 t + 64) of inverse_norms[band, row]; warp b takes band b.
+    if (warp < ladder.count) {
+        float value = largest[lane][warp];
 #pragma unroll
-    for (int offset = 16; offset > 0; offset >>= 1) value = fmaxf(value, __shfl_xor_sync(0xFFFFFFFFu, value, offset));
-    if (lane == 0) tile_max[static_cast<size_t>(band) * tiles + tile] = value;
+        for (int offset = 16; offset > 0; offset >>= 1) value = fmaxf(value, __shfl_xor_sync(0xFFFFFFFFu, value, offset));
+        if (lane == 0) tile_max[static_cast<size_t>(warp) * (row_count / norm_rows) + blockIdx.x] = value;
+    }
 }
 
 __global__ void __launch_bounds__(256)
@@ -128,48 +146,150 @@ __global__ void __launch_bounds__(256) pull_kernel(pull_request request) {
                          request.bytes[part] / 16, thread, threads);
 }
 
-__global__ void __launch_bounds__(256)
+// A block takes 128 rows of one quantity: a lane four rows (one 16-byte load per record), a warp every eighth record, four
+// of them in flight; the warps' sums are then added in warp order, so the result is the same from run to run. Bound by the
+// latency of its loads: with a thread per row and all records in one chain, 128 records of 4096 rows took 20 us.
+constexpr uint32_t fold_warps = 8;
+// Four rows from `row` on; without `vector_` (rows or pointers that are no whole, aligned vectors) word by word.
+template <bool vector_> __device__ __forceinline__ float4 load_rows(float const* quantity, uint32_t row, uint32_t rows) {
+    if constexpr (vector_) {
+        return row < rows ? *reinterpret_cast<float4 const*>(quantity + row) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    } else {
+        return make_float4(row < rows ? quantity[row] : 0.0f, row + 1 < rows ? quantity[row + 1] : 0.0f,
+                           row + 2 < rows ? quantity[row + 2] : 0.0f, row + 3 < rows ? quantity[row + 3] : 0.0f);
+    }
+}
+template <bool vector_>
+__global__ void __launch_bounds__(fold_warps * 32)
     fold_partials_kernel(float const* __restrict__ partials, float* __restrict__ accumulators, uint32_t rows, uint32_t slots,
-                         uint32_t quantities) {
-    uint32_t const row = blockIdx.x * blockDim.x + threadIdx.x;
+                         uint32_t quantities, bool overwrite) {
+    __shared__ float4 sums[fold_warps][32];
+    uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    uint32_t const row = blockIdx.x * 128 + lane * 4;
     uint32_t const quantity = blockIdx.y;
-    if (row >= rows) return;
-    float total = 0;
-#pragma unroll 8
-    for (uint32_t slot = 0; slot < slots; ++slot)
-        if (SC_IN_BOUNDS((static_cast<size_t>(slot) * quantities + quantity) * rows + row, static_cast<size_t>(slots) * quantities * rows))
-            total += partials[(static_cast<size_t>(slot) * quantities + quantity) * rows + row];
-    accumulators[static_cast<size_t>(quantity) * rows + row] += total;
+    float4 total = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    size_t const stride = static_cast<size_t>(quantities) * rows;
+    float const* const first = partials + static_cast<size_t>(quantity) * rows;
+#pragma unroll 4
+    for (uint32_t slot = warp; slot < slots; slot += fold_warps)
+        if (SC_IN_BOUNDS(slot * stride + static_cast<size_t>(quantity) * rows + rows - 1, static_cast<size_t>(slots) * stride)) {
+            float4 const record = load_rows<vector_>(first + slot * stride, row, rows);
+            total.x += record.x, total.y += record.y, total.z += record.z, total.w += record.w;
+        }
+    sums[warp][lane] = total;
+    __syncthreads();
+    if (warp != 0) return;
+#pragma unroll
+    for (uint32_t w = 1; w < fold_warps; ++w) {
+        float4 const other = sums[w][lane];
+        total.x += other.x, total.y += other.y, total.z += other.z, total.w += other.w;
+    }
+    float* const into = accumulators + static_cast<size_t>(quantity) * rows;
+    float4 const before = overwrite ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : load_rows<vector_>(into, row, rows);
+    float4 const after = make_float4(before.x + total.x, before.y + total.y, before.z + total.z, before.w + total.w);
+    if constexpr (vector_) {
+        if (row < rows) *reinterpret_cast<float4*>(into + row) = after;
+    } else {
+        if (row < rows) into[row] = after.x;
+        if (row + 1 < rows) into[row + 1] = after.y;
+        if (row + 2 < rows) into[row + 2] = after.z;
+        if (row + 3 < rows) into[row + 3] = after.w;
+    }
 }
 
-// Row accumulators are laid out [quantity, row] with quantities: 0 bias grad, 1 log-beta grad, 2..2+K prefix losses,
-// 2+K..2+2K self coefficients.
-__global__ void __launch_bounds__(128)
-    finalize_kernel(uint4 const* __restrict__ queries, float const* __restrict__ inverse_norms,
-                    float const* __restrict__ accumulators, float const* __restrict__ query_gradient,
-                    uint4* __restrict__ gradient_out, uint32_t rows, uint32_t hidden, ladder_t ladder) {
-    uint32_t const row = blockIdx.x;
-    __shared__ float fold_from[8]; // fold_from[b] = sum over bands k >= b of coefficient_k * inverse_norm_k^2
-    if (threadIdx.x == 0) {
-        float running = 0;
-        for (int band = static_cast<int>(ladder.count) - 1; band >= 0; --band) {
-            float const inverse = inverse_norms[static_cast<size_t>(band) * rows + row];
-            float const coefficient = accumulators[static_cast<size_t>(2 + ladder.count + band) * rows + row];
-            running += coefficient * inverse * inverse;
-            fold_from[band] = running;
-        }
+// The end of a step, one launch. Row accumulators are laid out [quantity, row] with quantities: 0 bias grad, 1 log-beta
+// grad, 2..2+K prefix losses, 2+K..2+2K self coefficients. Block 0 reduces the first 2 + K of them to the summands; it is
+// the first to start and done before the others (a launch of its own with one pass per quantity took 9 us at 4096 rows).
+// Every other block takes eight rows, a warp each: the self term of the normalisation is folded into the gradient, which
+// leaves as bfloat16. Bound by memory.
+constexpr uint32_t finish_warps = 8;
+
+// A fixed reduction tree, so the bits do not depend on anything but the inputs. All quantities go in one pass: a thread has
+// a 16-byte load of every quantity in flight at once, and the block meets twice instead of twice per quantity.
+template <uint32_t prefixes_>
+__device__ __forceinline__ void sum_summands(float const* __restrict__ accumulators, float* __restrict__ summands, uint32_t rows) {
+    constexpr uint32_t quantities = 2 + prefixes_, prefixes = prefixes_, warps = finish_warps;
+    __shared__ float scratch[quantities][warps];
+    __shared__ float totals[quantities];
+    uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    float partial[quantities];
+#pragma unroll
+    for (uint32_t quantity = 0; quantity < quantities; ++quantity) partial[quantity] = 0.0f;
+    uint32_t const count = rows / 4; // rows are a multiple of 4, so a quantity's rows are whole, aligned vectors
+#pragma unroll 2
+    for (uint32_t index = threadIdx.x; index < count; index += warps * 32) {
+        float4 held[quantities];
+#pragma unroll
+        for (uint32_t quantity = 0; quantity < quantities; ++quantity)
+            held[quantity] = reinterpret_cast<float4 const*>(accumulators + static_cast<size_t>(quantity) * rows)[index];
+#pragma unroll
+        for (uint32_t quantity = 0; quantity < quantities; ++quantity)
+            partial[quantity] += (held[quantity].x + held[quantity].y) + (held[quantity].z + held[quantity].w);
+    }
+#pragma unroll
+    for (uint32_t quantity = 0; quantity < quantities; ++quantity) {
+#pragma unroll
+        for (int offset = 16; offset > 0; offset >>= 1) partial[quantity] += __shfl_xor_sync(0xFFFFFFFFu, partial[quantity], offset);
+        if (lane == 0) scratch[quantity][warp] = partial[quantity];
     }
     __syncthreads();
+    if (threadIdx.x < quantities) {
+        float value = 0.0f;
+#pragma unroll
+        for (uint32_t w = 0; w < warps; ++w) value += scratch[threadIdx.x][w];
+        totals[threadIdx.x] = value;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float loss = 0;
+        for (uint32_t band = 0; band < prefixes; ++band) loss += totals[2 + band];
+        summands[0] = loss;
+        summands[1] = totals[0];
+        summands[2] = totals[1];
+        summands[3] = 0.0f;
+        for (uint32_t band = 0; band < 8; ++band) summands[4 + band] = band < prefixes ? totals[2 + band] : 0.0f;
+    }
+}
+
+template <uint32_t prefixes_>
+__global__ void __launch_bounds__(finish_warps * 32)
+    finish_kernel(uint4 const* __restrict__ queries, float const* __restrict__ inverse_norms,
+                  float const* __restrict__ accumulators, float const* __restrict__ query_gradient,
+                  uint4* __restrict__ gradient_out, float* __restrict__ summands, uint32_t rows, uint32_t hidden, ladder_t ladder) {
+    if (blockIdx.x == 0) {
+        sum_summands<prefixes_>(accumulators, summands, rows);
+        return;
+    }
+    __shared__ float folds[finish_warps][8]; // per row, [b] = sum over bands k >= b of coefficient_k * inverse_norm_k^2
+    uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    uint32_t const row = (blockIdx.x - 1) * finish_warps + warp;
+    if (row >= rows) return;
+    if (lane == 0) {
+        float inverse[prefixes_], coefficient[prefixes_], running = 0;
+#pragma unroll
+        for (uint32_t band = 0; band < prefixes_; ++band) {
+            inverse[band] = inverse_norms[static_cast<size_t>(band) * rows + row];
+            coefficient[band] = accumulators[static_cast<size_t>(2 + prefixes_ + band) * rows + row];
+        }
+#pragma unroll
+        for (int band = static_cast<int>(prefixes_) - 1; band >= 0; --band) {
+            running += coefficient[band] * inverse[band] * inverse[band];
+            folds[warp][band] = running;
+        }
+    }
+    __syncwarp();
     uint32_t const vectors = hidden / 8;
-    for (uint32_t v = threadIdx.x; v < vectors; v += blockDim.x) {
+#pragma unroll 3
+    for (uint32_t v = lane; v < vectors; v += 32) {
         uint32_t const channel = v * 8;
-        uint32_t band = 0;
-        while (band + 1 < ladder.count && channel >= ladder.ends[band]) ++band;
-        float const fold = fold_from[band];
         if (!SC_IN_BOUNDS(static_cast<size_t>(row) * hidden + channel + 7, static_cast<size_t>(rows) * hidden)) continue;
         uint4 const packed = queries[static_cast<size_t>(row) * vectors + v];
         float4 const g0 = *reinterpret_cast<float4 const*>(query_gradient + static_cast<size_t>(row) * hidden + channel);
         float4 const g1 = *reinterpret_cast<float4 const*>(query_gradient + static_cast<size_t>(row) * hidden + channel + 4);
+        uint32_t band = 0;
+#pragma unroll
+        for (uint32_t b = 0; b + 1 < prefixes_; ++b) band += channel >= ladder.ends[b] ? 1u : 0u;
+        float const fold = folds[warp][band];
         uint32_t const words[4] = {packed.x, packed.y, packed.z, packed.w};
         float const g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
         uint32_t out[4];
@@ -179,51 +299,6 @@ __global__ void __launch_bounds__(128)
             out[w] = pack_bf16x2(fmaf(-fold, lo, g[2 * w]), fmaf(-fold, hi, g[2 * w + 1]));
         }
         gradient_out[static_cast<size_t>(row) * vectors + v] = make_uint4(out[0], out[1], out[2], out[3]);
-    }
-}
-
-// One block; a fixed reduction tree, so the bits do not depend on anything but the inputs.
-__global__ void __launch_bounds__(1024)
-    sum_summands_kernel(float const* __restrict__ accumulators, float* __restrict__ summands, uint32_t rows, uint32_t prefixes) {
-    __shared__ float scratch[32];
-    __shared__ float totals[10];
-    uint32_t const quantities = 2 + prefixes;
-    for (uint32_t quantity = 0; quantity < quantities; ++quantity) {
-        // Four 16-byte loads in flight per thread before anything is added (rows are a multiple of 128, so a quantity's
-        // rows are whole, aligned vectors): one round trip to memory per quantity instead of one per row a thread owns.
-        float partial = 0;
-        float4 const* const vectors = reinterpret_cast<float4 const*>(accumulators + static_cast<size_t>(quantity) * rows);
-        uint32_t const count = rows / 4;
-        for (uint32_t first = threadIdx.x; first < count; first += 4 * blockDim.x) {
-            float4 held[4];
-#pragma unroll
-            for (uint32_t u = 0; u < 4; ++u) {
-                uint32_t const index = first + u * blockDim.x;
-                held[u] = index < count ? vectors[index] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
-#pragma unroll
-            for (uint32_t u = 0; u < 4; ++u) partial += (held[u].x + held[u].y) + (held[u].z + held[u].w);
-        }
-#pragma unroll
-        for (int offset = 16; offset > 0; offset >>= 1) partial += __shfl_xor_sync(0xFFFFFFFFu, partial, offset);
-        if (threadIdx.x % 32 == 0) scratch[threadIdx.x / 32] = partial;
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            float value = threadIdx.x < blockDim.x / 32 ? scratch[threadIdx.x] : 0.0f;
-#pragma unroll
-            for (int offset = 16; offset > 0; offset >>= 1) value += __shfl_xor_sync(0xFFFFFFFFu, value, offset);
-            if (threadIdx.x == 0) totals[quantity] = value;
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        float loss = 0;
-        for (uint32_t band = 0; band < prefixes; ++band) loss += totals[2 + band];
-        summands[0] = loss;
-        summands[1] = totals[0];
-        summands[2] = totals[1];
-        summands[3] = 0.0f;
-        for (uint32_t band = 0; band < 8; ++band) summands[4 + band] = band < prefixes ? totals[2 + band] : 0.0f;
     }
 }
 
@@ -285,16 +360,10 @@ SC_DEFINE_BOUNDS_READER(bounds_record_small)
 void launch_prefix_norms(void const* rows_bf16, void* copy_bf16, float* inverse_norms, float* tile_max, uint32_t rows,
                          uint32_t hidden, ladder_host const& ladder, cudaStream_t stream) {
     if (hidden % 8) throw std::runtime_error("prefix_norms: hidden must be a multiple of 8");
-    prefix_norms_kernel<<<blocks_of(rows, 8), 256, 0, stream>>>(static_cast<uint4 const*>(rows_bf16),
-                                                               static_cast<uint4*>(copy_bf16), inverse_norms, rows, hidden,
-                                                               to_device(ladder));
+    if (tile_max != nullptr && rows % norm_rows) throw std::runtime_error("prefix_norms: rows must be a multiple of 64 for tile maxima");
+    prefix_norms_kernel<<<blocks_of(rows, norm_rows), norm_warps * 32, 0, stream>>>(
+        static_cast<uint4 const*>(rows_bf16), static_cast<uint4*>(copy_bf16), inverse_norms, tile_max, rows, hidden, to_device(ladder));
     check_launch("prefix_norms");
-    if (tile_max != nullptr) {
-        if (rows % 64) throw std::runtime_error("prefix_norms: rows must be a multiple of 64 for tile maxima");
-        uint32_t const items = rows / 64 * ladder.count;
-        tile_max_kernel<<<blocks_of(items, 8), 256, 0, stream>>>(inverse_norms, tile_max, rows, ladder.count);
-        check_launch("tile_max");
-    }
 }
 
 void launch_transpose(void const* rows_bf16, void* transposed_bf16, uint32_t rows, uint32_t hidden, cudaStream_t stream) {
@@ -315,27 +384,37 @@ void launch_pull(void const* src0, void* dst0, size_t bytes0, void const* src1, 
 }
 
 void launch_fold_partials(float const* partials, float* row_accumulators, uint32_t rows, uint32_t slots,
-                          uint32_t quantities, cudaStream_t stream) {
-    fold_partials_kernel<<<dim3(blocks_of(rows, 256), quantities), 256, 0, stream>>>(partials, row_accumulators, rows, slots,
-                                                                                   quantities);
+                          uint32_t quantities, bool overwrite, cudaStream_t stream) {
+    bool const vectors = rows % 4 == 0 && reinterpret_cast<uintptr_t>(partials) % 16 == 0 &&
+                         reinterpret_cast<uintptr_t>(row_accumulators) % 16 == 0;
+    dim3 const grid(blocks_of(rows, 128), quantities);
+    if (vectors) fold_partials_kernel<true><<<grid, fold_warps * 32, 0, stream>>>(partials, row_accumulators, rows, slots, quantities, overwrite);
+    else fold_partials_kernel<false><<<grid, fold_warps * 32, 0, stream>>>(partials, row_accumulators, rows, slots, quantities, overwrite);
     check_launch("fold_partials");
 }
 
-void launch_finalize(void const* queries_bf16, float const* inverse_norms, float const* row_accumulators,
-                     float const* query_gradient, void* gradient_out_bf16, uint32_t rows, uint32_t hidden,
-                     ladder_host const& ladder, cudaStream_t stream) {
-    finalize_kernel<<<rows, 128, 0, stream>>>(static_cast<uint4 const*>(queries_bf16), inverse_norms, row_accumulators,
-                                              query_gradient, static_cast<uint4*>(gradient_out_bf16), rows, hidden,
-                                              to_device(ladder));
-    check_launch("finalize");
-}
-
-void launch_sum_summands(float const* row_accumulators, float* summands, uint32_t rows, uint32_t prefixes,
-                         cudaStream_t stream) {
-    if (rows % 4 || reinterpret_cast<uintptr_t>(row_accumulators) % 16)
-        throw std::runtime_error("sum_summands: rows must be a multiple of 4 and the accumulators 16-byte aligned");
-    sum_summands_kernel<<<1, 1024, 0, stream>>>(row_accumulators, summands, rows, prefixes);
-    check_launch("sum_summands");
+void launch_finish(void const* queries_bf16, float const* inverse_norms, float const* row_accumulators,
+                   float const* query_gradient, void* gradient_out_bf16, float* summands, uint32_t rows, uint32_t hidden,
+                   ladder_host const& ladder, cudaStream_t stream) {
+    if (rows % 4 || hidden % 8 || reinterpret_cast<uintptr_t>(row_accumulators) % 16)
+        throw std::runtime_error("finish: rows must be a multiple of 4, hidden of 8 and the accumulators 16-byte aligned");
+    auto launch = [&](auto kernel) {
+        kernel<<<1 + blocks_of(rows, finish_warps), finish_warps * 32, 0, stream>>>(
+            static_cast<uint4 const*>(queries_bf16), inverse_norms, row_accumulators, query_gradient,
+            static_cast<uint4*>(gradient_out_bf16), summands, rows, hidden, to_device(ladder));
+    };
+    switch (ladder.count) {
+    case 1: launch(finish_kernel<1>); break;
+    case 2: launch(finish_kernel<2>); break;
+    case 3: launch(finish_kernel<3>); break;
+    case 4: launch(finish_kernel<4>); break;
+    case 5: launch(finish_kernel<5>); break;
+    case 6: launch(finish_kernel<6>); break;
+    case 7: launch(finish_kernel<7>); break;
+    case 8: launch(finish_kernel<8>); break;
+    default: throw std::runtime_error("finish: a ladder holds one to eight prefixes");
+    }
+    check_launch("finish");
 }
 
 void launch_keyed_embeddings(void* rows_bf16, uint32_t rows, uint32_t hidden, uint64_t salt, float scale,

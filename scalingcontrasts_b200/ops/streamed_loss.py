@@ -196,11 +196,9 @@ class StreamedLoss:
         return sum(t.numel() * t.element_size() for t in tensors)
 
     def begin(self, queries: torch.Tensor, stream=None, query_norms: Optional[BlockNorms] = None) -> None:
-        """Clears the per-row accumulators and takes the queries' prefix norms (computed here unless supplied)."""
+        """Starts a step: takes the queries' prefix norms (computed here unless supplied). The first block scored replaces
+        what the accumulators hold from the step before."""
         self._check_queries(queries)
-        with torch.cuda.stream(stream) if stream is not None else _NullContext():
-            self.query_gradient.zero_()
-            self.row_accumulators.zero_()
         if query_norms is None:
             compute_block_norms(queries, self.ladder, self.query_norms, stream=stream)
             self._query_norms_view = self.query_norms
@@ -248,9 +246,8 @@ class StreamedLoss:
         ext, s = native(), _stream(stream)
         qn = self._query_norms_view
         self._plan.join(s)
-        ext.finalize(queries.data_ptr(), qn.inverse.data_ptr(), self.row_accumulators.data_ptr(),
-                     self.query_gradient.data_ptr(), gradient_out.data_ptr(), self.rows, self.hidden, list(self.ladder.ends), s)
-        ext.sum_summands(self.row_accumulators.data_ptr(), summands.data_ptr(), self.rows, self.ladder.count, s)
+        ext.finish(queries.data_ptr(), qn.inverse.data_ptr(), self.row_accumulators.data_ptr(), self.query_gradient.data_ptr(),
+                   gradient_out.data_ptr(), summands.data_ptr(), self.rows, self.hidden, list(self.ladder.ends), s)
         self._begun = False
         return gradient_out, summands
 
@@ -266,14 +263,6 @@ class StreamedLoss:
         _check_block(queries)
         if tuple(queries.shape) != (self.rows, self.hidden):
             raise ValueError(f"queries must be [{self.rows}, {self.hidden}], got {tuple(queries.shape)}")
-
-
-class _NullContext:
-    def __enter__(self):
-        return None
-
-    def __exit__(self, *args):
-        return False
 
 
 def keyed_embeddings_device(rows: int, hidden: int, salt: int, scale: float, device=None) -> torch.Tensor:
