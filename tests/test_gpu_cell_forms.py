@@ -1,0 +1,118 @@
+"""The forward kernel's forms of the cell math (series for easy and near negatives, the general form, cells scored apart on
+the diagonal, cells on the cosine floor) at every ladder length, and what the kernels around it do at their edges."""
+import pytest
+import torch
+
+from scalingcontrasts_b200 import LossSpec, Matryoshka, StreamedLoss
+from scalingcontrasts_b200.cpu.streamed import CpuStreamedLoss
+
+pytestmark = pytest.mark.gpu
+
+LADDERS = {
+    1: (256,), 2: (112, 256), 3: (64, 176, 320), 4: (16, 208, 576, 832), 5: (48, 96, 192, 384, 768),
+    6: (32, 48, 128, 208, 272, 320), 7: (16, 32, 64, 128, 256, 272, 512), 8: (16, 32, 48, 96, 176, 256, 400, 448),
+}
+
+
+def _rows(rows, hidden, seed):
+    generator = torch.Generator(device="cuda").manual_seed(seed)
+    values = torch.randn(rows, hidden, device="cuda", generator=generator)
+    values[1::2] = 0.6 * values[0::2] + 0.8 * values[1::2]  # partners are alike, so that positives matter
+    return torch.nn.functional.normalize(values, dim=1).to(torch.bfloat16)
+
+
+def _relative(measured, expected):
+    return float((measured.double() - expected.double()).norm() / expected.double().norm().clamp_min(1e-30))
+
+
+# Series and general form agree with the exact functions to about 1e-7 relative; the summands add up to rows * columns such
+# terms in float32, the gradient leaves through bfloat16 gradient cubes and a bfloat16 store (2^-9 each, at random).
+SUMMAND_TOLERANCE, GRADIENT_TOLERANCE = 2e-5, 8e-3
+
+
+@pytest.mark.parametrize("beta,bias", [(10.0, -10.0), (10.0, -6.0), (20.0, -3.0), (1.0, 2.0)])
+@pytest.mark.parametrize("spec", [LossSpec("self"), LossSpec("pairs"), LossSpec("pairs", "skip")], ids=lambda s: f"{s.positives}-{s.diagonal}")
+@pytest.mark.parametrize("prefixes", sorted(LADDERS))
+def test_forms_of_the_cell_math_against_float64(prefixes, spec, beta, bias):
+    ladder = Matryoshka(LADDERS[prefixes])
+    rows, hidden = (128 if prefixes % 2 else 384), ladder.hidden
+    blocks = [_rows(rows, hidden, seed) for seed in (1, 2)]
+    reference = CpuStreamedLoss(rows, hidden, ladder, spec, torch.float64, "cuda")
+    reference.begin(blocks[0])
+    for index, block in enumerate(blocks):
+        reference.score(blocks[0], block, 0, index * rows, beta, bias, 2 * rows)
+    expected, expected_summands = reference.finish(blocks[0], torch.empty(rows, hidden, dtype=torch.float64, device="cuda"))
+    for fused in ([False, True] if prefixes <= 6 else [False]):
+        loss = StreamedLoss(rows, hidden, ladder, spec, "cuda", fused=fused)
+        for scratch in (loss.query_gradient, loss.row_accumulators, loss.partials, loss.similarity_gradients):
+            scratch.fill_(float("nan"))  # the first block replaces whatever is there
+        for _ in range(2):
+            loss.begin(blocks[0])
+            for index, block in enumerate(blocks):
+                loss.score(blocks[0], block, 0, index * rows, beta, bias, 2 * rows)
+            gradient, summands = loss.finish(blocks[0])
+        loss.check()
+        assert _relative(summands[:3], expected_summands[:3]) < SUMMAND_TOLERANCE
+        assert _relative(summands[4:], expected_summands[4:]) < SUMMAND_TOLERANCE
+        assert _relative(gradient, expected) < GRADIENT_TOLERANCE
+
+
+@pytest.mark.parametrize("prefixes", [1, 4, 8])
+def test_every_cosine_on_the_floor(prefixes):
+    """Rows so short that every product of inverse norms is past the floor: cosines and gradients are exactly zero."""
+    ladder = Matryoshka(LADDERS[prefixes])
+    rows, hidden = 128, ladder.hidden
+    queries, candidates = (_rows(rows, hidden, seed) * 2.0 ** -7 for seed in (3, 4))
+    loss = StreamedLoss(rows, hidden, ladder, LossSpec("self"), "cuda")
+    loss.begin(queries)
+    loss.score(queries, candidates, 0, rows, 10.0, -10.0, 2 * rows)
+    gradient, summands = loss.finish(queries)
+    loss.check()
+    assert not gradient.any()
+    per_prefix = rows * torch.nn.functional.softplus(torch.tensor(-10.0, dtype=torch.float64)) / 2
+    assert torch.allclose(summands[4:4 + prefixes].double().cpu(), per_prefix.expand(prefixes), rtol=1e-5)
+
+
+def test_a_step_without_blocks_is_zero():
+    ladder = Matryoshka(LADDERS[5])
+    queries = _rows(128, ladder.hidden, 5)
+    loss = StreamedLoss(128, ladder.hidden, ladder, LossSpec("self"), "cuda")
+    loss.begin(queries)
+    loss.score(queries, queries, 0, 0, 10.0, -10.0, 128)
+    loss.finish(queries)
+    loss.begin(queries)
+    gradient, summands = loss.finish(queries)
+    assert not gradient.any() and not summands.any()
+
+
+@pytest.mark.parametrize("rows,slots,offset", [(128, 1, 0), (128, 9, 0), (384, 70, 0), (132, 8, 0), (130, 5, 0), (128, 3, 1)])
+def test_fold_of_the_partials(rows, slots, offset):
+    """Whole vectors, ragged rows and buffers that start off a 16-byte boundary."""
+    from scalingcontrasts_b200._ext import native
+
+    quantities = 4
+    generator = torch.Generator(device="cuda").manual_seed(slots)
+    storage = torch.randn(slots * quantities * rows + 1, device="cuda", generator=generator)
+    partials = storage[offset:offset + slots * quantities * rows]
+    sums = torch.ones(quantities, rows, device="cuda")
+    native().fold_partials(partials.data_ptr(), sums.data_ptr(), rows, slots, quantities, torch.cuda.current_stream().cuda_stream)
+    expected = 1.0 + partials.view(slots, quantities, rows).double().sum(dim=0)
+    assert torch.allclose(sums.double(), expected, rtol=0.0, atol=slots * 4 * 2.0 ** -23)
+
+
+@pytest.mark.parametrize("rows,hidden", [(64, 64), (192, 832), (37, 128)])
+def test_norms_and_their_maxima(rows, hidden):
+    from scalingcontrasts_b200._ext import native
+
+    block = torch.randn(rows, hidden, device="cuda").to(torch.bfloat16)
+    ends = [16, hidden // 2 // 16 * 16, hidden]
+    inverse = torch.full((3, rows), float("nan"), device="cuda")
+    maxima = torch.full((3, max(1, rows // 64)), float("nan"), device="cuda")
+    copy = torch.zeros_like(block)
+    native().prefix_norms(block.data_ptr(), copy.data_ptr(), inverse.data_ptr(), maxima.data_ptr() if rows % 64 == 0 else 0, rows, hidden,
+                          ends, torch.cuda.current_stream().cuda_stream)
+    expected = torch.stack([block.double()[:, :end].norm(dim=1).reciprocal() for end in ends])
+    assert torch.allclose(inverse.double(), expected, rtol=2e-6)
+    assert torch.equal(copy, block)
+    if rows % 64 == 0:
+        assert torch.equal(maxima, inverse.view(3, rows // 64, 64).amax(dim=2))
