@@ -75,7 +75,7 @@ void launch_prefix_norms(void const* rows_bf16, void* copy_bf16, float* inverse_
 void launch_transpose(void const* rows_bf16, void* transposed_bf16, uint32_t rows, uint32_t hidden, cudaStream_t stream);
 void launch_pull(void const* src0, void* dst0, size_t bytes0, void const* src1, void* dst1, size_t bytes1, int blocks,
                  cudaStream_t stream);
-// With `overwrite` the sums replace what the accumulators hold (a step's first block).
+// With `overwrite` the sums replace what the accumulators hold.
 void launch_fold_partials(float const* partials, float* row_accumulators, uint32_t rows, uint32_t slots,
                           uint32_t quantities, bool overwrite, cudaStream_t stream);
 void launch_finish(void const* queries_bf16, float const* inverse_norms, float const* row_accumulators,
@@ -116,6 +116,7 @@ struct forward_arguments {
     float const* scalars;            // optional device {beta, bias}; overrides the two floats above when set
     uint64_t query_base, candidate_base;
     uint32_t spec_code;
+    bool accumulate;       // add to the partial records instead of replacing them (a step's blocks after the first)
     uint64_t budget_ns;
     pull_request pull;               // optional: bytes == 0 means nothing to pull
     // Optional phase timers, live only in a build with -DSC_FWD_TRACE=1 and ignored otherwise (device array of

@@ -103,6 +103,7 @@ struct loss_plan {
     cudaEvent_t forward_done[2] = {nullptr, nullptr}, backward_done[2] = {nullptr, nullptr};
     cudaEvent_t forked[2] = {nullptr, nullptr}, rejoined[2] = {nullptr, nullptr};
     uint32_t scored = 0;
+    bool fold_due = false;
     bool pending = false;
     uint32_t pending_slot = 0;
     sc::backward_arguments pending_backward{};
@@ -139,6 +140,7 @@ struct loss_plan {
     void begin_step() {
         if (pending) throw std::runtime_error("LossPlan: begin_step with a backward still pending (join() was not called)");
         scored = 0;
+        fold_due = false;
     }
 
     void clear_gradient(cudaStream_t stream) {
@@ -153,6 +155,15 @@ struct loss_plan {
         pending = false;
     }
 
+    // The row accumulators from the partial records, which gather over the blocks of a step: folded when somebody reads them
+    // (at the end of a step, or earlier on request) instead of once per block.
+    void fold(uint64_t stream_handle) {
+        if (!fold_due) return;
+        sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows_q, partial_slots, quantities, true,
+                                 stream_of(stream_handle));
+        fold_due = false;
+    }
+
     // Ends a step on `stream`: everything the side stream still runs is waited for, and the last block's backward runs
     // here with the whole chip.
     void join(uint64_t stream_handle) {
@@ -165,6 +176,7 @@ struct loss_plan {
             sc::launch_backward(pending_backward, stream);
             pending = false;
         }
+        fold(stream_handle);
         if (scored == 0) { // a step that scored no block: its sums are zero
             clear_gradient(stream);
             runtime_check(cudaMemsetAsync(pointer<void>(accumulators), 0, static_cast<size_t>(rows_q) * quantities * 4, stream),
@@ -196,6 +208,7 @@ struct loss_plan {
         a.tiles_per_run = tiles_per_run, a.beta = beta, a.bias = bias, a.weight = static_cast<float>(1.0 / live);
         a.scalars = pointer<float>(scalars);
         a.query_base = query_base, a.candidate_base = candidate_base, a.spec_code = spec_code, a.budget_ns = budget_ns;
+        a.accumulate = scored != 0;
         a.pull.src[0] = pointer<void>(pull_src0), a.pull.dst[0] = pointer<void>(pull_dst0), a.pull.bytes[0] = pull_bytes0;
         a.pull.src[1] = pointer<void>(pull_src1), a.pull.dst[1] = pointer<void>(pull_dst1), a.pull.bytes[1] = pull_bytes1;
         // a forward that has the previous block's backward beside it leaves that kernel its multiprocessors
@@ -212,8 +225,7 @@ struct loss_plan {
             runtime_check(cudaEventRecord(rejoined[slot], front), "cudaEventRecord");
             runtime_check(cudaStreamWaitEvent(stream, rejoined[slot], 0), "cudaStreamWaitEvent");
         } else sc::launch_forward(a, stream);
-        sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows_q, partial_slots, quantities, scored == 0,
-                                 stream);
+        fold_due = true;
         if (!fused) {
             sc::backward_arguments b{};
             b.gradient_cube_bf16 = pointer<void>(cube);
@@ -373,6 +385,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def("enable_overlap", &loss_plan::enable_overlap, py::arg("second_cube"), py::arg("backward_multiprocessors"))
         .def("begin_step", &loss_plan::begin_step)
         .def("join", &loss_plan::join, py::arg("stream"))
+        .def("fold", &loss_plan::fold, py::arg("stream"))
         .def("score", &loss_plan::score);
     m.attr("BOUNDS_BUILD") = sc::bounds_build();
     m.def("bounds_records", []() {

@@ -174,6 +174,7 @@ struct fwd_params {
     float const* scalars; // optional device copy of {beta, bias}: learnable values never visit the host
     uint64_t query_base, candidate_base;
     uint32_t spec_code;
+    uint32_t accumulate; // non-zero: the partial records are added to what is there (a step's blocks after the first)
     uint64_t budget_ns;
     pull_request pull;
     unsigned long long* trace; // optional: phase cycle counters of CTA 0 (see forward_trace_slots in api.h)
@@ -979,6 +980,13 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
             float* record = p.partials + static_cast<size_t>(slot) * quantities * p.rows_q + row;
             if (SC_IN_BOUNDS((static_cast<size_t>(slot) * quantities + quantities - 1) * p.rows_q + row,
                              static_cast<size_t>(p.runs_per_strip) * fwd_column_groups * quantities * p.rows_q)) {
+                // One writer per word and launch, launches in stream order: the sums do not depend on scheduling. The reductions
+                // are fire and forget; a load of the old value would stand at the end of every item.
+                auto put = [&](uint32_t quantity, float value) {
+                    float* const at = record + static_cast<size_t>(quantity) * p.rows_q;
+                    if (p.accumulate != 0u) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(at), "f"(value) : "memory");
+                    else *at = value;
+                };
                 // sum of cell gradient * logit: the coefficients are exactly that, except for a row's own copy, whose logit
                 // is the scale itself and which moves no dot product
                 float logits = own_logit;
@@ -988,11 +996,11 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
                     float const band_coefficient = rolled ? band_sums[(prefixes_ + k) * fwd_epilogue_threads] : coefficient[rolled ? 0 : k];
                     float const whole = row_beta[k * factor_stride] * band_coefficient;
                     logits += whole;
-                    record[static_cast<size_t>(2 + k) * p.rows_q] = p.weight * band_loss;
-                    record[static_cast<size_t>(2 + prefixes_ + k) * p.rows_q] = 2.0f * p.weight * whole;
+                    put(2 + k, p.weight * band_loss);
+                    put(2 + prefixes_ + k, 2.0f * p.weight * whole);
                 }
-                record[0] = p.weight * g;
-                record[static_cast<size_t>(1) * p.rows_q] = p.weight * logits;
+                put(0, p.weight * g);
+                put(1, p.weight * logits);
             }
             if constexpr (fused_) {
                 // The item's patches of this warp are in memory once its bulk stores have completed (not merely been
@@ -1336,6 +1344,7 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
     p.beta = a.beta, p.bias = a.bias, p.weight = a.weight;
     p.scalars = a.scalars;
     p.query_base = a.query_base, p.candidate_base = a.candidate_base, p.spec_code = a.spec_code;
+    p.accumulate = a.accumulate ? 1u : 0u;
     p.budget_ns = a.budget_ns;
     p.pull = a.pull;
     p.trace = a.trace;

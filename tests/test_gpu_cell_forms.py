@@ -85,6 +85,25 @@ def test_a_step_without_blocks_is_zero():
     assert not gradient.any() and not summands.any()
 
 
+@pytest.mark.parametrize("fused", [False, True])
+def test_row_accumulators_between_blocks(fused):
+    """The partial records gather over the blocks; read in mid-step the accumulators hold what was scored so far."""
+    ladder = Matryoshka(LADDERS[5])
+    rows, hidden = 256, ladder.hidden
+    blocks = [_rows(rows, hidden, seed) for seed in (6, 7, 8)]
+    loss = StreamedLoss(rows, hidden, ladder, LossSpec("pairs"), "cuda", fused=fused)
+    reference = CpuStreamedLoss(rows, hidden, ladder, LossSpec("pairs"), torch.float64, "cuda")
+    loss.begin(blocks[0]), reference.begin(blocks[0])
+    for index, block in enumerate(blocks):
+        loss.score(blocks[0], block, 0, index * rows, 10.0, -10.0, 3 * rows)
+        reference.score(blocks[0], block, 0, index * rows, 10.0, -10.0, 3 * rows)
+        if index != 1:
+            assert _relative(loss.row_accumulators[0], reference.row_bias_grad) < SUMMAND_TOLERANCE
+            assert _relative(loss.row_accumulators[2:7], reference.row_loss) < SUMMAND_TOLERANCE
+            assert _relative(loss.row_accumulators[7:], reference.self_coefficients) < 10 * SUMMAND_TOLERANCE  # signed terms
+    loss.finish(blocks[0])
+
+
 @pytest.mark.parametrize("rows,slots,offset", [(128, 1, 0), (128, 9, 0), (384, 70, 0), (132, 8, 0), (130, 5, 0), (128, 3, 1)])
 def test_fold_of_the_partials(rows, slots, offset):
     """Whole vectors, ragged rows and buffers that start off a 16-byte boundary."""
