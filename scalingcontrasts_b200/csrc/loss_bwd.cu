@@ -57,7 +57,13 @@ struct bwd_tail {
 };
 // The ring of stages: 208 KB; a stage is the CTA's row blocks of the cube plus the candidates of the tile's own width.
 constexpr uint32_t bwd_ring_bytes = 208 * 1024;
-constexpr uint32_t bwd_shared_bytes = 1024 + bwd_ring_bytes + sizeof(bwd_tail);
+// Shared launches (two CTAs on a multiprocessor, see plan_tiles) have half the ring and half the tensor memory.
+constexpr uint32_t bwd_shared_width = 128;
+constexpr uint32_t bwd_half_ring_bytes = 104 * 1024;
+constexpr uint32_t bwd_shared_bytes_for(uint32_t ring) { return 1024 + ring + sizeof(bwd_tail); }
+constexpr uint32_t bwd_shared_bytes = bwd_shared_bytes_for(bwd_ring_bytes);
+static_assert(2 * (bwd_shared_bytes_for(bwd_half_ring_bytes) + 1024) <= 228 * 1024, "two CTAs of a shared launch must fit one multiprocessor");
+static_assert(3 * (bwd_a_bytes + bwd_shared_width * bwd_depth * 2) <= bwd_half_ring_bytes, "three stages of a shared launch's widest tile must fit");
 static_assert(3 * bwd_stage_bytes <= bwd_ring_bytes, "three of the largest stages must fit the ring");
 static_assert(bwd_shared_bytes <= 227 * 1024, "the kernel's shared memory must fit one CTA's maximum");
 constexpr uint32_t bwd_candidate_maps = 5;                          // boxes of 16, 32, 64, 128 and 256 channels
@@ -81,6 +87,7 @@ struct bwd_params {
     uint32_t* status;
     uint32_t rows_q, rows_c, hidden;
     uint32_t tile_count, split;
+    uint32_t ring_bytes, tmem_columns; // of one CTA
     uint32_t overwrite; // non-zero: the gradient is stored instead of added to (one CTA per output element)
     float scale; // applied to every product before it is added: the loss's 2/N (mirror cell and weight)
     uint64_t budget_ns;
@@ -101,7 +108,7 @@ __global__ void __launch_bounds__(bwd_threads, 1)
     extern __shared__ uint8_t raw_shared[];
     uint32_t const raw_address = smem_u32(raw_shared);
     uint32_t const stages_base = (raw_address + 1023u) & ~1023u;
-    bwd_tail* tail = reinterpret_cast<bwd_tail*>(raw_shared + (stages_base - raw_address) + bwd_ring_bytes);
+    bwd_tail* tail = reinterpret_cast<bwd_tail*>(raw_shared + (stages_base - raw_address) + p.ring_bytes);
     uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     uint32_t tile_index = 0; // the first tile of the group this CTA falls into, then the CTA's own tile within it
     while (tile_index + p.tiles[tile_index].group < p.tile_count &&
@@ -119,7 +126,7 @@ __global__ void __launch_bounds__(bwd_threads, 1)
     // One-block tiles (small launches) take as deep a ring as fits: 0.187 -> 0.181 ms per 4096-row block. Two-block tiles
     // stay at three stages: deeper rings for the narrow, DRAM-bound ones made a 16384-row launch slower (1.82 -> 1.85 ms per
     // block), their CTAs then take bandwidth from the wide ones that finish last.
-    uint32_t const stages = tile.blocks == 2 ? 3u : min(bwd_stages, bwd_ring_bytes / stage_bytes);
+    uint32_t const stages = tile.blocks == 2 ? 3u : min(bwd_stages, p.ring_bytes / stage_bytes);
     uint32_t const b_offset = tile.blocks * bwd_a_bytes;
     uint32_t const first_block = within / group * tile.blocks;
     uint32_t const blocks = min(tile.blocks, p.rows_q / bwd_rows - first_block);
@@ -140,7 +147,7 @@ __global__ void __launch_bounds__(bwd_threads, 1)
     __syncthreads();
     if (tail->abort_flag != 0u || chunk_begin >= chunk_end) return;
     if (warp == 5) {
-        tmem_alloc(smem_u32(&tail->tmem_base), bwd_tmem_columns);
+        tmem_alloc(smem_u32(&tail->tmem_base), p.tmem_columns);
         tmem_relinquish();
     }
     if (warp == 4 && lane == 0) {
@@ -272,27 +279,36 @@ __global__ void __launch_bounds__(bwd_threads, 1)
     __syncthreads();
     if (warp == 5) {
         tcgen05_fence_after();
-        tmem_dealloc(tmem_base, bwd_tmem_columns);
+        tmem_dealloc(tmem_base, p.tmem_columns);
     }
 }
 
 // The launch's tile table: which (band, channels, row blocks per CTA) tiles there are and which CTAs of the
 // one-dimensional grid belong to each. Pure arithmetic on the shape, so that it can be checked without a GPU.
 uint32_t plan_tiles(uint32_t rows_q, ladder_host const& ladder, uint32_t split, int multiprocessors, bwd_tile* tiles,
-                    uint32_t& tile_count) {
+                    uint32_t& tile_count, bool& shared) {
     tile_count = 0;
     // Two row blocks per CTA once that still leaves at least two CTAs per multiprocessor with tiles of 256 channels. Only
     // then (a launch bound by the cube's bytes, not by its tail) does a band of 257..384 channels go to one-block CTAs
     // that take it whole; a small launch prefers more and shorter CTAs.
     uint32_t const row_blocks = rows_q / bwd_rows;
-    uint32_t plain_tiles = 0, begin = 0;
+    uint32_t plain_tiles = 0, narrow_tiles = 0, begin = 0;
     for (uint32_t band = 0; band < ladder.count; ++band) {
         uint32_t const end = ladder.ends[band];
         if (end % 16 || end <= begin) throw std::runtime_error("backward: band edges must ascend in multiples of 16");
         plain_tiles += (end - begin + bwd_max_width - 1) / bwd_max_width;
+        narrow_tiles += (end - begin + bwd_shared_width - 1) / bwd_shared_width;
         begin = end;
     }
     bool const two_blocks = static_cast<uint64_t>(row_blocks / 2) * plain_tiles * split >= 2ull * static_cast<uint64_t>(multiprocessors);
+    // One-block tiles that make a little more than one CTA per multiprocessor leave most of the chip idle in a second round
+    // (4096 rows, H=768, K=5: 192 CTAs on 148, 58 us). Cut to 128 channels they run two to a multiprocessor, each with half
+    // the ring and half the tensor memory, as long as all of them are resident at once: 47 us. A launch of one round stays
+    // with 256 channels, and so does one with more CTAs than two per multiprocessor, which would start a third round.
+    uint64_t const rounds_of = static_cast<uint64_t>(row_blocks) * split;
+    shared = !two_blocks && rounds_of * plain_tiles > static_cast<uint64_t>(multiprocessors) && narrow_tiles <= bwd_max_tiles &&
+             rounds_of * narrow_tiles <= 2ull * static_cast<uint64_t>(multiprocessors);
+    uint32_t const widest = shared ? bwd_shared_width : bwd_max_width;
     begin = 0;
     for (uint32_t band = 0; band < ladder.count; ++band) {
         uint32_t const end = ladder.ends[band];
@@ -300,7 +316,7 @@ uint32_t plan_tiles(uint32_t rows_q, ladder_host const& ladder, uint32_t split, 
             if (tile_count == bwd_max_tiles) throw std::runtime_error("backward: too many channel tiles for one launch");
             uint32_t const left = end - channel;
             bool const whole_band = two_blocks && left == end - begin && left > bwd_max_width && left <= bwd_wide_width;
-            uint32_t const width = whole_band || left <= bwd_max_width ? left : bwd_max_width;
+            uint32_t const width = whole_band || left <= widest ? left : widest;
             tiles[tile_count++] = bwd_tile{band, channel, width, two_blocks && !whole_band ? 2u : 1u, 0u, 1u};
             channel += width;
         }
@@ -357,7 +373,11 @@ void launch_backward(backward_arguments const& a, cudaStream_t stream) {
         if (cudaDeviceGetAttribute(&multiprocessors, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) multiprocessors = 148;
         counted_device = device;
     }
-    uint32_t const ctas = plan_tiles(a.rows_q, a.ladder, a.split, multiprocessors, p.tiles, p.tile_count);
+    bool shared = false;
+    uint32_t const ctas = plan_tiles(a.rows_q, a.ladder, a.split, multiprocessors, p.tiles, p.tile_count, shared);
+    p.ring_bytes = shared ? bwd_half_ring_bytes : bwd_ring_bytes;
+    p.tmem_columns = shared ? bwd_tmem_columns / 2 : bwd_tmem_columns;
+    uint32_t const shared_bytes = bwd_shared_bytes_for(p.ring_bytes);
     bool const mn_major = a.candidates_row_major != nullptr && a.hidden >= 64;
     if (!mn_major && a.transposed_candidates == nullptr) throw std::runtime_error("backward: no candidates given");
     // Everything above is checked before the first driver or runtime call.
@@ -389,8 +409,8 @@ void launch_backward(backward_arguments const& a, cudaStream_t stream) {
         prepared_device = device;
     }
     dim3 const grid(ctas, a.split, 1);
-    if (mn_major) backward_kernel<true><<<grid, bwd_threads, bwd_shared_bytes, stream>>>(cube_map, candidates, p);
-    else backward_kernel<false><<<grid, bwd_threads, bwd_shared_bytes, stream>>>(cube_map, candidates, p);
+    if (mn_major) backward_kernel<true><<<grid, bwd_threads, shared_bytes, stream>>>(cube_map, candidates, p);
+    else backward_kernel<false><<<grid, bwd_threads, shared_bytes, stream>>>(cube_map, candidates, p);
     cudaError_t const error = cudaGetLastError();
     if (error != cudaSuccess) throw std::runtime_error(std::string("backward launch failed: ") + cudaGetErrorString(error));
     note_launch();
@@ -402,7 +422,8 @@ std::vector<std::array<uint32_t, 6>> backward_plan(uint32_t rows_q, ladder_host 
     if (rows_q % bwd_rows || split < 1) throw std::runtime_error("backward_plan: rows must be a multiple of 128 and split positive");
     bwd_tile tiles[bwd_max_tiles];
     uint32_t count = 0;
-    uint32_t const total = plan_tiles(rows_q, ladder, split, multiprocessors, tiles, count);
+    bool shared = false;
+    uint32_t const total = plan_tiles(rows_q, ladder, split, multiprocessors, tiles, count, shared);
     if (ctas) *ctas = total;
     std::vector<std::array<uint32_t, 6>> out;
     for (uint32_t i = 0; i < count; ++i)

@@ -135,3 +135,26 @@ def test_norms_and_their_maxima(rows, hidden):
     assert torch.equal(copy, block)
     if rows % 64 == 0:
         assert torch.equal(maxima, inverse.view(3, rows // 64, 64).amax(dim=2))
+
+
+@pytest.mark.parametrize("rows_q,ends", [(3200, [48, 96, 192, 384, 768]), (4096, [64, 128, 256, 512, 1024]), (3200, [16, 208, 576, 832])])
+def test_backward_with_two_ctas_to_a_multiprocessor(rows_q, ends):
+    """Launches of more than one CTA per multiprocessor and at most two: 128-channel tiles with half the ring. Float32 sums
+    of bfloat16 products against the same in float64; 192 candidates, so the half ring wraps."""
+    from scalingcontrasts_b200._ext import native
+
+    ext, hidden, rows_c = native(), ends[-1], 192
+    tiles, ctas = ext.backward_plan(rows_q, ends, 1, 148)
+    assert 148 < ctas <= 296 and max(t[2] for t in tiles) <= 128
+    generator = torch.Generator(device="cuda").manual_seed(9)
+    cube = (torch.randn(len(ends), rows_q, rows_c, device="cuda", generator=generator) * 0.1).to(torch.bfloat16)
+    candidates = torch.randn(rows_c, hidden, device="cuda", generator=generator).to(torch.bfloat16)
+    gradient = torch.ones(rows_q, hidden, device="cuda")
+    status = torch.zeros(8, dtype=torch.int32, device="cuda")
+    ext.backward(cube.data_ptr(), 0, gradient.data_ptr(), status.data_ptr(), rows_q, rows_c, hidden, ends, 1, 0.5, 2 * 10 ** 9,
+                 torch.cuda.current_stream().cuda_stream, candidates.data_ptr())
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0
+    begins = [0] + ends[:-1]
+    expected = 0.5 * torch.cat([cube[b].double() @ candidates.double()[:, begins[b]:ends[b]] for b in range(len(ends))], dim=1)
+    assert _relative(gradient, expected + 1.0) < 1e-5
