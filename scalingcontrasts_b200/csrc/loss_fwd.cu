@@ -8,22 +8,28 @@
 // slot of tensor memory and the UMMAs of a 16-channel step accumulate into the slot of the band that contains the
 // step, so each channel is multiplied exactly once (depth H per cell, where a sweep-and-subtract scheme spends up to
 // 2H). The eight slots form a ring: while the epilogue warps drain the K slots of tile t, the issuing thread already
-// fills the widest bands of tile t+1. The epilogue walks the bands narrowest first, adding each band's segment dots to
-// a running prefix dot in registers, runs the cell math, parks the band's raw-dot gradients (without the factor
-// beta / |q_k| that the row and band share) in the tensor-memory slot the dots came from, and then walks the bands
-// widest first, two at a time, to form the suffix sums that go to the gradient cube. A tile's slots go back to the
-// issuer in two steps: the two widest bands' as soon as the suffix pass has read them (the next tile's narrow bands
-// wait for exactly those slots), the rest when the pass is done.
+// fills the widest bands of tile t+1. A thread of the epilogue takes its columns eight at a time and holds all bands' values
+// of a chunk in registers: the segment dots come in, the prefix dots run up the ladder, the raw-dot gradients (without the
+// factor beta / |q_k| that the row and band share) replace the dots, and the suffix sums that go to the gradient cube run
+// down the ladder. A tile's slots go back to the issuer when its last chunk has been loaded. Ladders of six and more bands
+// keep some or all of their gradients in the tensor-memory slots the dots came from until the suffix sums reach them
+// (fwd_parked_bands_for, fwd_rolled_for).
 //
-// Warp roles (608 threads): warps 0-15 epilogue (warp w owns tensor-memory lanes 32*(w%4).. and the 16 columns w/4 of
-// the tile; four warps per scheduler keep the issue slots busy), warp 16 TMA producer, warp 17 UMMA issuer and
-// tensor-memory owner (both run warp-wide, with the TMA / UMMA / commit instructions under one elected lane), warp 18
-// peer pull (plain 16-byte loads from the peer's replica, plain stores to local staging; never a TMA load from another
-// GPU's memory).
+// Warp roles (640 threads): warps 0-15 epilogue (warp w owns tensor-memory lanes 32*(w%4).. and the 16 columns w/4 of
+// the tile; four warps per scheduler keep the issue slots busy), warp 16 TMA producer (and the candidates' norms), warp 17
+// UMMA issuer and tensor-memory owner (both run warp-wide, with the TMA / UMMA / commit instructions under one elected
+// lane), warp 18 peer pull (plain 16-byte loads from the peer's replica, plain stores to local staging; never a TMA load
+// from another GPU's memory), warp 19 the fused kernel's second issuer. The epilogue's four warpgroups run with 104
+// registers a thread, the helpers' with 64.
+//
+// What bounds it (B200, 4096 rows, H=768, K=5, 90 us): nothing alone. Taking one resource away at a time gained little:
+// three of four UMMAs 4 us, the queries' loads 2 us, four of five bands' math 4 us, the cube's stores 6 us. A tile is a chain
+// (operands, UMMAs, epilogue, slots back to the issuer) of which two tiles are under way at once; tensor memory has no room
+// for a third. The issuer is busy 78 % of a tile's time, the epilogue 85 %.
 //
 // A CTA walks work items (row strip, run of consecutive candidate tiles) in a fixed round-robin order and writes one
-// partial record per (run, column quarter, row): the fold over runs happens later in run order, so the loss summands do
-// not depend on scheduling.
+// partial record per (run, column quarter, row), added to by a step's later blocks: the fold over records happens once, in
+// a fixed order, so the loss summands do not depend on scheduling.
 //
 // Parity: forward_tile_cuda_ and score_forward_row_ (scalingcontrasts.cuh:688-1040) and fold of its row partials;
 // the staging copy of streamed_loss_t::score (scalingcontrasts.cuh:1262-1265) is what the pull warps replace.
@@ -62,16 +68,15 @@ constexpr uint32_t fz_accumulator_column = 6 * fwd_slot_columns;
 constexpr uint32_t fz_max_tiles = 48;
 constexpr uint32_t fz_candidate_maps = 4; // boxes of 16, 32, 64 and 128 channels
 constexpr uint32_t fz_max_tiles_per_run = 16;
-#ifndef SC_FWD_EPILOGUE_WARPS
-#define SC_FWD_EPILOGUE_WARPS 16
-#endif
-constexpr uint32_t fwd_epilogue_warps = SC_FWD_EPILOGUE_WARPS; // 16: four per scheduler at 96 registers; 8: two at 168
+constexpr uint32_t fwd_epilogue_warps = 16; // four per scheduler
 constexpr uint32_t fwd_epilogue_threads = fwd_epilogue_warps * 32;
 constexpr uint32_t fwd_column_groups = fwd_epilogue_warps / 4;             // warps that share a lane quadrant
 constexpr uint32_t fwd_warp_columns = fwd_cols / fwd_column_groups;        // columns of a tile that one warp owns
 // Columns a thread takes at a time: all bands' values of a chunk are held in registers together.
-// Ladders of seven and eight bands go band by band instead (`rolled`): the code of eight bands times three forms of the cell
-// math does not stay in the instruction cache, and their values do not fit the registers.
+// Ladders of seven and eight bands go band by band instead (`rolled`), sixteen columns at a time: their values do not fit the
+// registers, and eight bands times three forms of the cell math are more code than the instruction cache likes. One block
+// of 4096 rows, H=1024, K=8: 215 us with half the bands parked, 190 us band by band; at six bands 150 us either way, and 153
+// against 161 us where every cell takes the general form, so six stay with two bands parked.
 __host__ __device__ constexpr bool fwd_rolled_for(int prefixes) { return prefixes >= 7; }
 __host__ __device__ constexpr int fwd_chunk_columns_for(int prefixes) { return prefixes <= 1 || fwd_rolled_for(prefixes) ? 16 : 8; }
 // The narrowest bands, where the registers have no room for them beside the others: their gradients are parked in the tensor
@@ -304,25 +309,22 @@ __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::
 // values the compiler can keep in uniform registers, which is where those instructions take their operands from. (Run
 // by a single lane inside a divergent branch, every operand would cross from a vector to a uniform register first.)
 // Every lane waits; the answer is the same in every lane.
-// Their waits sleep between attempts (`sleep_ns`; 0 polls back to back): a helper warp shares its scheduler with four
-// epilogue warps, and a warp that polls an mbarrier without pause issues about as many instructions as one of them.
-#ifndef SC_FWD_HELPER_SLEEP
-#define SC_FWD_HELPER_SLEEP 1
-#endif
-// A CTA's items: every gridDim.x-th of the list.
-__device__ __forceinline__ uint32_t item_count(uint32_t items) { return (items + gridDim.x - 1 - blockIdx.x) / gridDim.x; }
-__device__ __forceinline__ uint32_t item_at(uint32_t, uint32_t n) { return blockIdx.x + n * gridDim.x; }
+// Their waits sleep between attempts: a helper warp shares its scheduler with four epilogue warps, and a warp that polls an
+// mbarrier without pause issues about as many instructions as one of them. (The polling wait's timed part is a function of
+// the epilogue warps alone: one function cannot serve both sides of the register split.)
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, wait_context const& ctx, uint32_t site,
-                                               uint32_t detail, uint32_t sleep_ns = 0) {
-    if (SC_FWD_HELPER_SLEEP && sleep_ns != 0u)
-        return __all_sync(0xFFFFFFFFu, mbar_wait_relaxed(bar, parity, ctx, site, detail, sleep_ns));
-    return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, ctx, site, detail));
+                                               uint32_t detail, uint32_t sleep_ns) {
+    return __all_sync(0xFFFFFFFFu, mbar_wait_relaxed(bar, parity, ctx, site, detail, sleep_ns));
 }
 constexpr uint32_t sleep_producer_ns = 200; // stages ahead of the issuer: nothing waits for this warp's wake-up
 constexpr uint32_t sleep_issuer_ns = 20;    // the epilogue may be waiting for the tile these UMMAs finish
 constexpr uint32_t sleep_gemm_ns = 500;      // the fused kernel's gradient GEMM runs a whole item behind
 
-//
+
+// A CTA's items: every gridDim.x-th of the list.
+__device__ __forceinline__ uint32_t item_count(uint32_t items) { return (items + gridDim.x - 1 - blockIdx.x) / gridDim.x; }
+__device__ __forceinline__ uint32_t item_at(uint32_t n) { return blockIdx.x + n * gridDim.x; }
+
 // The producer also brings the candidates' inverse norms of a tile (and their maxima) into the ring the epilogue warps read
 // them from: plain loads at the start of the tile, stored once the tile's operand loads have been issued.
 template <int prefixes_>
@@ -337,7 +339,7 @@ __device__ __forceinline__ void producer_role(CUtensorMap const* q_map, CUtensor
     phase_timer timer(p);
     timer.only_if(elected);
     for (uint32_t n = 0, count = item_count(p.items); n < count; ++n) {
-        uint32_t const item = item_at(p.items, n);
+        uint32_t const item = item_at(n);
         uint32_t const strip = item / p.runs_per_strip, run = item % p.runs_per_strip;
         for (uint32_t t = 0; t < p.tiles_per_run; ++t, ++tile_local) {
             uint32_t const column_tile = run * p.tiles_per_run + t;
@@ -420,7 +422,7 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
         return true;
     };
     for (uint32_t n = 0, count = item_count(p.items); n < count; ++n) {
-        uint32_t const item = item_at(p.items, n);
+        uint32_t const item = item_at(n);
         for (uint32_t t = 0; t < p.tiles_per_run; ++t) {
             for (int chunk = static_cast<int>(chunks) - 1; chunk >= 0; --chunk) {
                 uint32_t const starts = p.band_starts[chunk];
@@ -470,7 +472,7 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
 struct tile_cursor {
     uint32_t n, t, strip, run;
     __device__ __forceinline__ void go_to(fwd_params const& p, uint32_t to) {
-        uint32_t const item = item_at(p.items, to);
+        uint32_t const item = item_at(to);
         n = to, t = 0, strip = item / p.runs_per_strip, run = item % p.runs_per_strip;
     }
     __device__ __forceinline__ void advance(fwd_params const& p) {
@@ -567,8 +569,9 @@ __device__ __noinline__ special_sums special_cells(uint32_t lane_base, uint32_t 
 // parked in tensor memory in between, so a tile's slots go back to the issuer as soon as its last chunk has been loaded,
 // about half a tile before the epilogue is done with it.
 //
-// What bounds it: the packed float32 math (eleven instructions per pair of cells and prefix, two cycles each) and issue
-// slots.
+// What it costs: eleven packed float32 instructions per pair of cells and prefix, two cycles each, and one exponential per
+// cell, eight cycles; about 5000 cycles of a tile's 9700 at K=5 are bound by these. One block of 4096 rows, H=768, K=5: 98 ->
+// 90 us off the diagonal, 123 -> 92 us on it, against the form that parked every band in tensor memory.
 template <int prefixes_, bool fused_>
 __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_params const& p, fwd_tail* tail,
                                               uint32_t store_base, float const* norm_ring, float* row_factors, uint32_t tmem_base,
@@ -628,7 +631,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
                 break;
             }
             tcgen05_fence_after();
-            uint32_t const item = item_at(p.items, drained / p.tile_count);
+            uint32_t const item = item_at(drained / p.tile_count);
             uint32_t const word = p.tiles[drained % p.tile_count];
             float* const destination = p.gradient +
                                        (static_cast<size_t>(item / p.runs_per_strip) * fwd_rows + row_local) * p.hidden +
@@ -1036,7 +1039,7 @@ __device__ __forceinline__ void fz_producer_role(fz_maps const* maps, fwd_params
     phase_timer timer(p);
     timer.only_if(elected);
     for (uint32_t count = item_count(p.items); local < count; ++local) {
-        uint32_t const item = item_at(p.items, local);
+        uint32_t const item = item_at(local);
         uint32_t const buffer = local & 1u;
         timer.lap(0);
         if (!mbar_wait_warp(smem_u32(&tail->fz_item_stored[buffer]), (local >> 1) & 1u, ctx, site_fz_item_stored, item, sleep_producer_ns))
@@ -1088,7 +1091,7 @@ __device__ __forceinline__ void fz_mma_role(fwd_params const& p, uint32_t stages
     phase_timer timer(p);
     timer.only_if(elected);
     for (uint32_t n = 0, count = item_count(p.items); n < count; ++n) {
-        uint32_t const item = item_at(p.items, n);
+        uint32_t const item = item_at(n);
         for (uint32_t which = 0; which < p.tile_count; ++which, ++unit) {
             uint32_t const idesc = umma_idesc_bf16(128, (p.tiles[which] >> 16) * 16u);
             // The accumulator's previous contents must have left tensor memory (an arrival per epilogue warp).

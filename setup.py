@@ -16,16 +16,9 @@ SOURCES = [os.path.join(CSRC, name) for name in (
     "collectives.cu", "loss_small.cu", "loss_fwd.cu", "loss_bwd.cu", "no_alloc.cu", "tower.cu", "optim.cu",
 )]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a", "--expt-relaxed-constexpr"]
-# Tuning knob of the forward kernel (16 or 8 epilogue warps); the default is the measured best.
-if os.environ.get("SC_FWD_EPILOGUE_WARPS"):
-    NVCC_FLAGS.append("-DSC_FWD_EPILOGUE_WARPS=" + os.environ["SC_FWD_EPILOGUE_WARPS"])
 # Diagnostic build of the forward kernel with in-kernel phase timers (the `trace` argument of `forward`).
 if os.environ.get("SC_FWD_TRACE"):
     NVCC_FLAGS.append("-DSC_FWD_TRACE=" + os.environ["SC_FWD_TRACE"])
-
-# A/B switch for the helper warps' sleeping waits in the forward kernel (1: sleep between polls, 0: poll back to back).
-if os.environ.get("SC_FWD_HELPER_SLEEP"):
-    NVCC_FLAGS.append("-DSC_FWD_HELPER_SLEEP=" + os.environ["SC_FWD_HELPER_SLEEP"])
 
 EXTENSIONS = [CUDAExtension(
     name="scalingcontrasts_b200._C",
