@@ -149,7 +149,7 @@ __host__ __device__ constexpr uint32_t fwd_store_bytes(uint32_t prefixes) {
     return fwd_epilogue_warps * fwd_store_patches(prefixes) * fwd_store_patch_bytes;
 }
 // Stages of the score operands: as many as the rest of the shared memory leaves room for. The fused kernel keeps room for
-// the gradient GEMM's stages and runs the scores on two.
+// the gradient GEMM's stages and runs the scores on what is left (three at five prefixes, two at six).
 constexpr uint32_t fwd_shared_limit = 227 * 1024;
 __host__ __device__ constexpr uint32_t fwd_stages_for(uint32_t prefixes, bool fused) {
     uint32_t const rest = 1024 + (fused ? fz_stages * fz_stage_bytes : 0u) + fwd_store_bytes(prefixes) + fwd_tail_bytes + fwd_norm_bytes(prefixes) + fwd_factor_bytes(prefixes, fused);

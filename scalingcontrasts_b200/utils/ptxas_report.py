@@ -79,11 +79,14 @@ def render(rows: List[Dict[str, object]]) -> str:
         lines.append(f"| `{row['source']}` | `{row['name']}` | {row['registers']} | {row['spill_stores']} | {row['spill_loads']} | "
                      f"{row['stack']} | {row['shared']} |")
     lines += ["",
-              "Dynamic shared memory (set by the launchers), K the number of prefixes: `forward_kernel<K, false>` 199,040 + 6,144 K",
-              "bytes for K <= 5 (six 24 KB stages; 229,760 at K = 5) and 174,464 + 6,144 K for K >= 6 (five stages);",
-              "`forward_kernel<K, true>` (fused) 190,848 + 6,144 K (three 24 KB scoring stages and two 32 KB stages of the gradient",
-              "GEMM; 221,568 at K = 5); `backward_kernel` 214,128 bytes (a 208 KB ring of three to six stages, a stage being the CTA's row blocks of the cube plus its tile's candidates). Threads per block: 608",
-              "(forward), 640 (fused forward), 192 (backward), 512 (bandwidth collectives), up to 1024 (one-round all-reduce).", ""]
+              "Dynamic shared memory (set by the launchers), K the number of prefixes: `forward_kernel<K, false>` as many 24 KB stages as",
+              "fit beside 16 KB of store patches per band (four bands in rotation from K = 7 on), norms and row factors: six for K <= 4",
+              "(226,944 bytes at K = 4), five at K = 5 (221,824), four above; `forward_kernel<K, true>` (fused) two 32 KB stages of the",
+              "gradient GEMM and six to two scoring stages (227,968 bytes, three stages, at K = 5); `backward_kernel` 214,128 bytes (a 208 KB",
+              "ring of three to six stages, a stage being the CTA's row blocks of the cube plus its tile's candidates), or half the ring",
+              "where two CTAs share a multiprocessor. Threads per block: 640 (forward; 96 registers at launch, 104 in the epilogue's",
+              "warpgroups and 64 in the helpers' after the hand-over), 192 (backward), 512 (bandwidth collectives), up to 1024 (one-round",
+              "all-reduce, norms).", ""]
     return "\n".join(lines)
 
 
