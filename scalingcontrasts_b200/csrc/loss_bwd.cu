@@ -384,8 +384,8 @@ void launch_backward(backward_arguments const& a, cudaStream_t stream) {
     cuuint64_t const cube_dims[3] = {a.rows_c, a.rows_q, a.ladder.count};
     cuuint64_t const cube_strides[2] = {static_cast<cuuint64_t>(a.rows_c) * 2, static_cast<cuuint64_t>(a.rows_c) * a.rows_q * 2};
     cuuint32_t const cube_box[3] = {bwd_depth, bwd_rows, 1};
-    CUtensorMap const& cube_map = cached_map(a.gradient_cube_bf16, 3, cube_dims, cube_strides, cube_box, CU_TENSOR_MAP_SWIZZLE_128B,
-                                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    CUtensorMap const cube_map = cached_map(a.gradient_cube_bf16, 3, cube_dims, cube_strides, cube_box, CU_TENSOR_MAP_SWIZZLE_128B,
+                                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     bwd_candidate_boxes candidates;
     for (uint32_t index = 0; index < bwd_candidate_maps; ++index) {
         if (mn_major) {

@@ -1246,11 +1246,6 @@ __global__ void __launch_bounds__(fwd_threads, 1)
 }
 
 // ---- host side --------------------------------------------------------------------------------------------------
-// Rows of `inner` bfloat16 values, `outer` of them, read in boxes under the 128-byte swizzle.
-CUtensorMap const& operand_map(void const* base, uint64_t inner, uint64_t outer, uint32_t box_inner, uint32_t box_outer) {
-    return cached_operand_map(base, inner, outer, box_inner, box_outer);
-}
-
 template <int prefixes_, bool fused_>
 void launch_instance(CUtensorMap const& q_map, CUtensorMap const& c_map, CUtensorMap const& cube_map, fz_maps const& gemm_maps,
                      fwd_params const& p, int blocks, cudaStream_t stream) {
@@ -1375,8 +1370,8 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
             throw std::runtime_error("forward: the fused kernel needs its scratch, the transposed candidates and the gradient");
     }
     // Everything above is checked before the first driver or runtime call.
-    CUtensorMap const& q_map = operand_map(a.queries_bf16, a.hidden, a.rows_q, fwd_depth, fwd_rows);
-    CUtensorMap const& c_map = operand_map(a.candidates_bf16, a.hidden, a.rows_c, fwd_depth, fwd_cols);
+    CUtensorMap const q_map = cached_operand_map(a.queries_bf16, a.hidden, a.rows_q, fwd_depth, fwd_rows);
+    CUtensorMap const c_map = cached_operand_map(a.candidates_bf16, a.hidden, a.rows_c, fwd_depth, fwd_cols);
     fz_maps gemm_maps{};
     if (!a.fused) {
         // The warps' patches of the gradient cube [K, rows_q, rows_c]: boxes of all bands x 32 rows x 16 candidates, staged under the
@@ -1384,7 +1379,7 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
         cuuint64_t const dims[3] = {a.rows_c, a.rows_q, a.ladder.count};
         cuuint64_t const strides[2] = {static_cast<cuuint64_t>(a.rows_c) * 2, static_cast<cuuint64_t>(a.rows_c) * a.rows_q * 2};
         cuuint32_t const box[3] = {fwd_warp_columns, 32, fwd_rolled_for(static_cast<int>(a.ladder.count)) ? 1u : a.ladder.count};
-        CUtensorMap const& cube_map =
+        CUtensorMap const cube_map =
             cached_map(a.gradient_cube_bf16, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
         launch_for_count<false>(a.ladder.count, q_map, c_map, cube_map, gemm_maps, p, blocks, stream);
     } else {
@@ -1402,7 +1397,7 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
         cuuint64_t const strides[2] = {run * 2, run * fwd_rows * 2};
         cuuint32_t const store_box[3] = {fwd_warp_columns, 32, a.ladder.count};
         cuuint32_t const load_box[3] = {fz_depth, fwd_rows, 1};
-        CUtensorMap const& store_map =
+        CUtensorMap const store_map =
             cached_map(a.fused_scratch_bf16, 3, dims, strides, store_box, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
         gemm_maps.patches =
             cached_map(a.fused_scratch_bf16, 3, dims, strides, load_box, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
@@ -1410,7 +1405,7 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
             // A box may not be taller than the tensor; such a box is never asked for either (tiles are at most `hidden` wide).
             uint32_t const channels = 16u << index;
             gemm_maps.candidates[index] =
-                operand_map(a.transposed_candidates, a.rows_c, a.hidden, fz_depth, channels <= a.hidden ? channels : 16u);
+                cached_operand_map(a.transposed_candidates, a.rows_c, a.hidden, fz_depth, channels <= a.hidden ? channels : 16u);
         }
         launch_for_count<true>(a.ladder.count, q_map, c_map, store_map, gemm_maps, p, blocks, stream);
     }
