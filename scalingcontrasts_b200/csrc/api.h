@@ -75,9 +75,8 @@ void launch_prefix_norms(void const* rows_bf16, void* copy_bf16, float* inverse_
 void launch_transpose(void const* rows_bf16, void* transposed_bf16, uint32_t rows, uint32_t hidden, cudaStream_t stream);
 void launch_pull(void const* src0, void* dst0, size_t bytes0, void const* src1, void* dst1, size_t bytes1, int blocks,
                  cudaStream_t stream);
-// With `overwrite` the sums replace what the accumulators hold.
 void launch_fold_partials(float const* partials, float* row_accumulators, uint32_t rows, uint32_t slots,
-                          uint32_t quantities, bool overwrite, cudaStream_t stream);
+                          uint32_t quantities, cudaStream_t stream);
 void launch_finish(void const* queries_bf16, float const* inverse_norms, float const* row_accumulators,
                    float const* query_gradient, void* gradient_out_bf16, float* summands, uint32_t rows, uint32_t hidden,
                    ladder_host const& ladder, cudaStream_t stream);
@@ -116,7 +115,6 @@ struct forward_arguments {
     float const* scalars;            // optional device {beta, bias}; overrides the two floats above when set
     uint64_t query_base, candidate_base;
     uint32_t spec_code;
-    bool accumulate;       // add to the partial records instead of replacing them (a step's blocks after the first)
     uint64_t budget_ns;
     pull_request pull;               // optional: bytes == 0 means nothing to pull
     // Optional phase timers, live only in a build with -DSC_FWD_TRACE=1 and ignored otherwise (device array of
@@ -156,7 +154,6 @@ struct backward_arguments {
     uint32_t split;                     // candidate-range splits (1: deterministic read-modify-write)
     float scale;                        // multiplies every product before accumulation (the loss passes 2 / live)
     uint64_t budget_ns;
-    bool overwrite;                     // the gradient is stored instead of added to (a step's first block)
 };
 void launch_backward(backward_arguments const& arguments, cudaStream_t stream);
 // The backward launch's tile table for a shape, without launching: one {band, first channel, width, row blocks per CTA,

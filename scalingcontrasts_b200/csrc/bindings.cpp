@@ -103,7 +103,6 @@ struct loss_plan {
     cudaEvent_t forward_done[2] = {nullptr, nullptr}, backward_done[2] = {nullptr, nullptr};
     cudaEvent_t forked[2] = {nullptr, nullptr}, rejoined[2] = {nullptr, nullptr};
     uint32_t scored = 0;
-    bool fold_due = false;
     bool pending = false;
     uint32_t pending_slot = 0;
     sc::backward_arguments pending_backward{};
@@ -136,15 +135,14 @@ struct loss_plan {
         gradients_alt = second_cube, backward_multiprocessors = reserved, overlap = true;
     }
 
-    // Starts a step: no backward is in flight (join() ended the last one).
-    void begin_step() {
+    // Starts a step: no backward is in flight (join() ended the last one). The gradient and the row accumulators behind it are
+    // cleared here, and every block adds to both, whatever came before it: what a launch does never hangs on what this object
+    // remembers, so blocks captured in a graph and replayed any number of times sum up like blocks scored one by one.
+    void begin_step(uint64_t stream_handle) {
         if (pending) throw std::runtime_error("LossPlan: begin_step with a backward still pending (join() was not called)");
         scored = 0;
-        fold_due = false;
-    }
-
-    void clear_gradient(cudaStream_t stream) {
-        runtime_check(cudaMemsetAsync(pointer<void>(query_gradient), 0, static_cast<size_t>(rows_q) * hidden * 4, stream),
+        runtime_check(cudaMemsetAsync(pointer<void>(query_gradient), 0, static_cast<size_t>(rows_q) * (hidden + quantities) * 4,
+                                      stream_of(stream_handle)),
                       "cudaMemsetAsync");
     }
 
@@ -153,15 +151,6 @@ struct loss_plan {
         sc::launch_backward(pending_backward, side);
         runtime_check(cudaEventRecord(backward_done[pending_slot], side), "cudaEventRecord");
         pending = false;
-    }
-
-    // The row accumulators from the partial records, which gather over the blocks of a step: folded when somebody reads them
-    // (at the end of a step, or earlier on request) instead of once per block.
-    void fold(uint64_t stream_handle) {
-        if (!fold_due) return;
-        sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows_q, partial_slots, quantities, true,
-                                 stream_of(stream_handle));
-        fold_due = false;
     }
 
     // Ends a step on `stream`: everything the side stream still runs is waited for, and the last block's backward runs
@@ -175,12 +164,6 @@ struct loss_plan {
         if (pending) {
             sc::launch_backward(pending_backward, stream);
             pending = false;
-        }
-        fold(stream_handle);
-        if (scored == 0) { // a step that scored no block: its sums are zero
-            clear_gradient(stream);
-            runtime_check(cudaMemsetAsync(pointer<void>(accumulators), 0, static_cast<size_t>(rows_q) * quantities * 4, stream),
-                          "cudaMemsetAsync");
         }
         scored = 0;
     }
@@ -196,7 +179,6 @@ struct loss_plan {
         uint64_t const cube = slot ? gradients_alt : gradients;
         // this cube was last read by the backward of the block before the previous one
         if (overlapping && scored >= 2) runtime_check(cudaStreamWaitEvent(stream, backward_done[slot], 0), "cudaStreamWaitEvent");
-        if (fused && scored == 0) clear_gradient(stream); // items of the fused kernel add in no fixed order
         if (transposing) sc::launch_transpose(pointer<void>(candidates), pointer<void>(transposed), rows_c, hidden, stream);
         sc::forward_arguments a{};
         a.queries_bf16 = pointer<void>(queries), a.candidates_bf16 = pointer<void>(candidates);
@@ -208,7 +190,6 @@ struct loss_plan {
         a.tiles_per_run = tiles_per_run, a.beta = beta, a.bias = bias, a.weight = static_cast<float>(1.0 / live);
         a.scalars = pointer<float>(scalars);
         a.query_base = query_base, a.candidate_base = candidate_base, a.spec_code = spec_code, a.budget_ns = budget_ns;
-        a.accumulate = scored != 0;
         a.pull.src[0] = pointer<void>(pull_src0), a.pull.dst[0] = pointer<void>(pull_dst0), a.pull.bytes[0] = pull_bytes0;
         a.pull.src[1] = pointer<void>(pull_src1), a.pull.dst[1] = pointer<void>(pull_dst1), a.pull.bytes[1] = pull_bytes1;
         // a forward that has the previous block's backward beside it leaves that kernel its multiprocessors
@@ -225,7 +206,7 @@ struct loss_plan {
             runtime_check(cudaEventRecord(rejoined[slot], front), "cudaEventRecord");
             runtime_check(cudaStreamWaitEvent(stream, rejoined[slot], 0), "cudaStreamWaitEvent");
         } else sc::launch_forward(a, stream);
-        fold_due = true;
+        sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows_q, partial_slots, quantities, stream);
         if (!fused) {
             sc::backward_arguments b{};
             b.gradient_cube_bf16 = pointer<void>(cube);
@@ -234,9 +215,6 @@ struct loss_plan {
             b.query_gradient = pointer<float>(query_gradient), b.status = pointer<uint32_t>(status);
             b.rows_q = rows_q, b.rows_c = rows_c, b.hidden = hidden, b.ladder = ladder, b.split = backward_split;
             b.scale = static_cast<float>(2.0 / live), b.budget_ns = budget_ns;
-            // a step's first block replaces what the step before left; its partial sums of a split launch need zeros to start from
-            b.overwrite = scored == 0 && backward_split == 1;
-            if (scored == 0 && backward_split != 1) clear_gradient(stream);
             if (!overlapping) sc::launch_backward(b, stream);
             else {
                 runtime_check(cudaEventRecord(forward_done[slot], stream), "cudaEventRecord");
@@ -353,7 +331,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     });
     m.def("fold_partials", [](uint64_t partials, uint64_t accumulators, uint32_t rows, uint32_t slots, uint32_t quantities,
                               uint64_t stream) {
-        sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows, slots, quantities, false, stream_of(stream));
+        sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows, slots, quantities, stream_of(stream));
     });
     m.def("finish", [](uint64_t queries, uint64_t inverse_norms, uint64_t accumulators, uint64_t query_gradient, uint64_t out,
                        uint64_t summands, uint32_t rows, uint32_t hidden, std::vector<uint32_t> const& ends, uint64_t stream) {
@@ -374,6 +352,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                  plan->gradients = gradients, plan->gradients_bytes = gradients_bytes, plan->transposed = transposed;
                  plan->query_gradient = query_gradient, plan->partials = partials, plan->accumulators = accumulators;
                  plan->status = status, plan->budget_ns = budget_ns, plan->multiprocessors = multiprocessors;
+                 if (accumulators != query_gradient + static_cast<uint64_t>(rows_q) * hidden * 4)
+                     throw std::runtime_error("LossPlan: the row accumulators must lie directly behind the gradient");
                  return plan;
              }),
              py::arg("rows_q"), py::arg("rows_c"), py::arg("hidden"), py::arg("ends"), py::arg("tiles_per_run"),
@@ -383,9 +363,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def_readwrite("transpose_candidates", &loss_plan::transpose_candidates)
         .def_readonly("overlap", &loss_plan::overlap)
         .def("enable_overlap", &loss_plan::enable_overlap, py::arg("second_cube"), py::arg("backward_multiprocessors"))
-        .def("begin_step", &loss_plan::begin_step)
+        .def("begin_step", &loss_plan::begin_step, py::arg("stream"))
         .def("join", &loss_plan::join, py::arg("stream"))
-        .def("fold", &loss_plan::fold, py::arg("stream"))
         .def("score", &loss_plan::score);
     m.attr("BOUNDS_BUILD") = sc::bounds_build();
     m.def("bounds_records", []() {

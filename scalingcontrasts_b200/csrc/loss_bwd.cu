@@ -15,8 +15,7 @@
 // Warp roles (192 threads): warps 0-3 epilogue (tensor-memory lanes 32*w..), warp 4 TMA producer, warp 5 UMMA issuer
 // and tensor-memory owner. The producer and the issuer run warp-wide with only the TMA / UMMA / commit instructions
 // under the elected lane, so that their operands are warp-uniform values. The epilogue adds its scaled accumulators with
-// vector reductions (fire and forget: no read of the old value comes back to the SM), or stores them when the launch is a
-// step's first block, which saves a pass that clears the gradient. With `split == 1` each output
+// vector reductions (fire and forget: no read of the old value comes back to the SM). With `split == 1` each output
 // element receives exactly one addition per launch, so the sum's order is the launches' stream order and the result
 // is deterministic; with a larger split the candidate range is divided and the order of a launch's partial sums is not.
 //
@@ -88,7 +87,6 @@ struct bwd_params {
     uint32_t rows_q, rows_c, hidden;
     uint32_t tile_count, split;
     uint32_t ring_bytes, tmem_columns; // of one CTA
-    uint32_t overwrite; // non-zero: the gradient is stored instead of added to (one CTA per output element)
     float scale; // applied to every product before it is added: the loss's 2/N (mirror cell and weight)
     uint64_t budget_ns;
     bwd_tile tiles[bwd_max_tiles];
@@ -256,15 +254,11 @@ __global__ void __launch_bounds__(bwd_threads, 1)
                 tmem_load_16(lane_base + column, values);
                 tmem_load_wait();
 #pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    float4 const sum = make_float4(p.scale * __uint_as_float(values[4 * v]), p.scale * __uint_as_float(values[4 * v + 1]),
-                                                   p.scale * __uint_as_float(values[4 * v + 2]), p.scale * __uint_as_float(values[4 * v + 3]));
-                    if (p.overwrite != 0u)
-                        *reinterpret_cast<float4*>(destination + column + 4 * v) = sum;
-                    else
-                        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(destination + column + 4 * v), "f"(sum.x),
-                                     "f"(sum.y), "f"(sum.z), "f"(sum.w) : "memory");
-                }
+                for (int v = 0; v < 4; ++v)
+                    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(destination + column + 4 * v),
+                                 "f"(p.scale * __uint_as_float(values[4 * v])), "f"(p.scale * __uint_as_float(values[4 * v + 1])),
+                                 "f"(p.scale * __uint_as_float(values[4 * v + 2])), "f"(p.scale * __uint_as_float(values[4 * v + 3]))
+                                 : "memory");
             }
           }
         }
@@ -363,8 +357,6 @@ void launch_backward(backward_arguments const& a, cudaStream_t stream) {
     p.query_gradient = a.query_gradient, p.status = a.status;
     p.rows_q = a.rows_q, p.rows_c = a.rows_c, p.hidden = a.hidden;
     p.split = a.split, p.budget_ns = a.budget_ns, p.scale = a.scale;
-    if (a.overwrite && a.split != 1) throw std::runtime_error("backward: only a launch without split can overwrite the gradient");
-    p.overwrite = a.overwrite ? 1u : 0u;
     // Per device, once: the multiprocessor count (a runtime query that needs no context of its own).
     static int counted_device = -1, multiprocessors = 148;
     int device = 0;

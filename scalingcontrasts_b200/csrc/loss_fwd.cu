@@ -28,8 +28,8 @@
 // for a third. The issuer is busy 78 % of a tile's time, the epilogue 85 %.
 //
 // A CTA walks work items (row strip, run of consecutive candidate tiles) in a fixed round-robin order and writes one
-// partial record per (run, column quarter, row), added to by a step's later blocks: the fold over records happens once, in
-// a fixed order, so the loss summands do not depend on scheduling.
+// partial record per (run, column quarter, row); the fold over records happens in a fixed order elsewhere, so the loss
+// summands do not depend on scheduling.
 //
 // Parity: forward_tile_cuda_ and score_forward_row_ (scalingcontrasts.cuh:688-1040) and fold of its row partials;
 // the staging copy of streamed_loss_t::score (scalingcontrasts.cuh:1262-1265) is what the pull warps replace.
@@ -179,7 +179,6 @@ struct fwd_params {
     float const* scalars; // optional device copy of {beta, bias}: learnable values never visit the host
     uint64_t query_base, candidate_base;
     uint32_t spec_code;
-    uint32_t accumulate; // non-zero: the partial records are added to what is there (a step's blocks after the first)
     uint64_t budget_ns;
     pull_request pull;
     unsigned long long* trace; // optional: phase cycle counters of CTA 0 (see forward_trace_slots in api.h)
@@ -983,13 +982,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
             float* record = p.partials + static_cast<size_t>(slot) * quantities * p.rows_q + row;
             if (SC_IN_BOUNDS((static_cast<size_t>(slot) * quantities + quantities - 1) * p.rows_q + row,
                              static_cast<size_t>(p.runs_per_strip) * fwd_column_groups * quantities * p.rows_q)) {
-                // One writer per word and launch, launches in stream order: the sums do not depend on scheduling. The reductions
-                // are fire and forget; a load of the old value would stand at the end of every item.
-                auto put = [&](uint32_t quantity, float value) {
-                    float* const at = record + static_cast<size_t>(quantity) * p.rows_q;
-                    if (p.accumulate != 0u) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(at), "f"(value) : "memory");
-                    else *at = value;
-                };
+                auto put = [&](uint32_t quantity, float value) { record[static_cast<size_t>(quantity) * p.rows_q] = value; };
                 // sum of cell gradient * logit: the coefficients are exactly that, except for a row's own copy, whose logit
                 // is the scale itself and which moves no dot product
                 float logits = own_logit;
@@ -1342,7 +1335,6 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
     p.beta = a.beta, p.bias = a.bias, p.weight = a.weight;
     p.scalars = a.scalars;
     p.query_base = a.query_base, p.candidate_base = a.candidate_base, p.spec_code = a.spec_code;
-    p.accumulate = a.accumulate ? 1u : 0u;
     p.budget_ns = a.budget_ns;
     p.pull = a.pull;
     p.trace = a.trace;

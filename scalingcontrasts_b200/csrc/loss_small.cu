@@ -162,7 +162,7 @@ template <bool vector_> __device__ __forceinline__ float4 load_rows(float const*
 template <bool vector_>
 __global__ void __launch_bounds__(fold_warps * 32)
     fold_partials_kernel(float const* __restrict__ partials, float* __restrict__ accumulators, uint32_t rows, uint32_t slots,
-                         uint32_t quantities, bool overwrite) {
+                         uint32_t quantities) {
     __shared__ float4 sums[fold_warps][32];
     uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     uint32_t const row = blockIdx.x * 128 + lane * 4;
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(fold_warps * 32)
         total.x += other.x, total.y += other.y, total.z += other.z, total.w += other.w;
     }
     float* const into = accumulators + static_cast<size_t>(quantity) * rows;
-    float4 const before = overwrite ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : load_rows<vector_>(into, row, rows);
+    float4 const before = load_rows<vector_>(into, row, rows);
     float4 const after = make_float4(before.x + total.x, before.y + total.y, before.z + total.z, before.w + total.w);
     if constexpr (vector_) {
         if (row < rows) *reinterpret_cast<float4*>(into + row) = after;
@@ -384,12 +384,12 @@ void launch_pull(void const* src0, void* dst0, size_t bytes0, void const* src1, 
 }
 
 void launch_fold_partials(float const* partials, float* row_accumulators, uint32_t rows, uint32_t slots,
-                          uint32_t quantities, bool overwrite, cudaStream_t stream) {
+                          uint32_t quantities, cudaStream_t stream) {
     bool const vectors = rows % 4 == 0 && reinterpret_cast<uintptr_t>(partials) % 16 == 0 &&
                          reinterpret_cast<uintptr_t>(row_accumulators) % 16 == 0;
     dim3 const grid(blocks_of(rows, 128), quantities);
-    if (vectors) fold_partials_kernel<true><<<grid, fold_warps * 32, 0, stream>>>(partials, row_accumulators, rows, slots, quantities, overwrite);
-    else fold_partials_kernel<false><<<grid, fold_warps * 32, 0, stream>>>(partials, row_accumulators, rows, slots, quantities, overwrite);
+    if (vectors) fold_partials_kernel<true><<<grid, fold_warps * 32, 0, stream>>>(partials, row_accumulators, rows, slots, quantities);
+    else fold_partials_kernel<false><<<grid, fold_warps * 32, 0, stream>>>(partials, row_accumulators, rows, slots, quantities);
     check_launch("fold_partials");
 }
 

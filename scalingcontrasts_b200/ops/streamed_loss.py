@@ -10,10 +10,12 @@ A rank owns ``rows`` query rows. Each ``score`` runs, on the calling stream,
    bfloat16 patches in a per-CTA scratch buffer, which the same CTA folds into the query gradient with a tensor-core
    GEMM while its epilogue warps already score the next item: no ``[K, R, R]`` gradient cube exists. Optionally the
    same launch pulls the next block from a peer's memory into local staging,
-4. (two-kernel form) the gradient GEMM over the block's cube.
+4. the deterministic fold of the partials into ``row_accumulators``, and in the two-kernel form the gradient GEMM over the
+   block's cube into ``query_gradient``.
 
-The per-row partial sums gather over a step's blocks and are folded, in a fixed order, when ``finish`` (or a reader of
-``row_accumulators``) needs them.
+``begin`` clears both on the device and every block adds to them, in stream order: they hold the blocks scored so far, and a
+``score`` captured in a CUDA graph may be replayed any number of times between ``begin`` and ``finish`` (with
+``overlap_backward`` only whole steps can be captured: a block's gradient GEMM is launched with the block after it).
 
 The default is the two-kernel form (``fused=False``; the only one for ladders of seven or eight prefixes): the forward
 kernel writes the bfloat16 gradient cube ``[K, R, R]`` and a separate backward tile kernel folds it, reading the candidates
@@ -145,8 +147,11 @@ class StreamedLoss:
         bf16 = dict(dtype=torch.bfloat16, device=self.device)
         self.query_norms = BlockNorms(k, rows, device=self.device)
         self.candidate_norms = BlockNorms(k, self.candidate_rows, device=self.device)
-        self.query_gradient = torch.zeros(rows, hidden, **f32)
-        self._row_accumulators = torch.zeros(self.quantities, rows, **f32)
+        # One span, the gradient and the row accumulators behind it, so that a step clears both with one launch.
+        sums = torch.zeros(rows * (hidden + self.quantities), **f32)
+        self.query_gradient = sums[:rows * hidden].view(rows, hidden)
+        # Bias gradient, log-scale gradient, prefix losses, self coefficients of the blocks scored so far.
+        self.row_accumulators = sums[rows * hidden:].view(self.quantities, rows)
         self.partials = torch.empty(self.partial_slots, self.quantities, rows, **f32)
         if self.fused:
             # Gradient patches of the items in flight: two buffers per CTA, independent of the block's size.
@@ -168,7 +173,7 @@ class StreamedLoss:
                                   self.quantities, self.backward_split, spec.code(), self.fused,
                                   self.similarity_gradients.data_ptr(), self.similarity_gradients.numel() * 2,
                                   self.transposed_candidates.data_ptr(), self.query_gradient.data_ptr(),
-                                  self.partials.data_ptr(), self._row_accumulators.data_ptr(), self.status.data_ptr(),
+                                  self.partials.data_ptr(), self.row_accumulators.data_ptr(), self.status.data_ptr(),
                                   self.budget_ns, self.multiprocessors)
         self._plan.transpose_candidates = self.transpose_candidates
         # With ``overlap_backward`` a block's gradient GEMM runs on a second stream, on a few multiprocessors, beside the
@@ -193,29 +198,20 @@ class StreamedLoss:
     # ------------------------------------------------------------------------------------------------------
     def bytes(self) -> int:
         """Bytes of scratch this object holds; does not grow with the number of blocks scored."""
-        tensors = (self.query_norms.storage, self.candidate_norms.storage, self.query_gradient, self._row_accumulators,
+        tensors = (self.query_norms.storage, self.candidate_norms.storage, self.query_gradient, self.row_accumulators,
                    self.partials, self.similarity_gradients, self.similarity_gradients_alt, self.transposed_candidates,
                    self.status)
         return sum(t.numel() * t.element_size() for t in tensors)
 
-    @property
-    def row_accumulators(self) -> torch.Tensor:
-        """``[quantities, rows]``: bias gradient, log-scale gradient, prefix losses, self coefficients of the blocks scored so
-        far. The forward launches gather them in partial records, which are folded here (on the current stream) if a block
-        was scored since the last fold, and by ``finish``."""
-        self._plan.fold(torch.cuda.current_stream(self.device).cuda_stream)
-        return self._row_accumulators
-
     def begin(self, queries: torch.Tensor, stream=None, query_norms: Optional[BlockNorms] = None) -> None:
-        """Starts a step: takes the queries' prefix norms (computed here unless supplied). The first block scored replaces
-        what the accumulators hold from the step before."""
+        """Clears the gradient and the row accumulators and takes the queries' prefix norms (computed here unless supplied)."""
         self._check_queries(queries)
+        self._plan.begin_step(_stream(stream))
         if query_norms is None:
             compute_block_norms(queries, self.ladder, self.query_norms, stream=stream)
             self._query_norms_view = self.query_norms
         else:
             self._query_norms_view = query_norms
-        self._plan.begin_step()
         self._begun = True
 
     def score(self, queries: torch.Tensor, candidates: torch.Tensor, query_base: int, candidate_base: int, beta: float,
@@ -257,7 +253,7 @@ class StreamedLoss:
         ext, s = native(), _stream(stream)
         qn = self._query_norms_view
         self._plan.join(s)
-        ext.finish(queries.data_ptr(), qn.inverse.data_ptr(), self._row_accumulators.data_ptr(), self.query_gradient.data_ptr(),
+        ext.finish(queries.data_ptr(), qn.inverse.data_ptr(), self.row_accumulators.data_ptr(), self.query_gradient.data_ptr(),
                    gradient_out.data_ptr(), summands.data_ptr(), self.rows, self.hidden, list(self.ladder.ends), s)
         self._begun = False
         return gradient_out, summands
