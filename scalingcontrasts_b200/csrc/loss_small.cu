@@ -63,7 +63,9 @@ __global__ void __launch_bounds__(norm_warps * 32)
         uint32_t const channel = v * 8;
 #pragma unroll
         for (uint32_t r = 0; r < each; ++r) {
-            if (copy != nullptr && first + r < row_count) copy[static_cast<size_t>(first + r) * vectors + v] = packed[r];
+            if (copy != nullptr && first + r < row_count &&
+                SC_IN_BOUNDS(static_cast<size_t>(first + r) * vectors + v, static_cast<size_t>(row_count) * vectors))
+                copy[static_cast<size_t>(first + r) * vectors + v] = packed[r];
             uint32_t const words[4] = {packed[r].x, packed[r].y, packed[r].z, packed[r].w};
             float square = 0;
 #pragma unroll
@@ -105,7 +107,8 @@ __global__ void __launch_bounds__(norm_warps * 32)
         float value = largest[lane][warp];
 #pragma unroll
         for (int offset = 16; offset > 0; offset >>= 1) value = fmaxf(value, __shfl_xor_sync(0xFFFFFFFFu, value, offset));
-        if (lane == 0) tile_max[static_cast<size_t>(warp) * (row_count / norm_rows) + blockIdx.x] = value;
+        size_t const tiles = row_count / norm_rows;
+        if (lane == 0 && SC_IN_BOUNDS(warp * tiles + blockIdx.x, ladder.count * tiles)) tile_max[warp * tiles + blockIdx.x] = value;
     }
 }
 

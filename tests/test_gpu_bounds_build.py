@@ -1,7 +1,8 @@
-"""The kernels' index arithmetic under the bounds-checked debug build: the loss, domain and trainer GPU tests are run once
-more in a child process that loads ``_C_bounds`` (same sources, ``-DSC_BOUNDS=1``: every computed global index is compared
-with its limit, a miss is recorded and the access skipped, nothing traps). The child's session fails if a miss was
-recorded (tests/conftest.py). No bad input is fed to a kernel here; the launchers' refusals are tested on the CPU."""
+"""The kernels' index arithmetic under the bounds-checked debug build: the GPU tests of the loss (its cell forms and step state
+among them), the domain and the trainer are run once more in a child process that loads ``_C_bounds`` (same sources,
+``-DSC_BOUNDS=1``: every computed global index is compared with its limit, a miss is recorded and the access skipped, nothing
+traps). The child's session fails if a miss was recorded (tests/conftest.py). No bad input is fed to a kernel here; the
+launchers' refusals are tested on the CPU."""
 import glob
 import os
 import subprocess
@@ -20,7 +21,8 @@ def test_gpu_suite_under_the_bounds_checked_build():
     environment = dict(os.environ, PYTHONPATH=ROOT, SC_NATIVE_VARIANT="bounds")
     result = subprocess.run([sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider",
                              os.path.join(ROOT, "tests", "test_gpu_loss.py"), os.path.join(ROOT, "tests", "test_gpu_domain.py"),
-                             os.path.join(ROOT, "tests", "test_gpu_trainer.py"), os.path.join(ROOT, "tests", "test_launcher_validation.py")],
+                             os.path.join(ROOT, "tests", "test_gpu_trainer.py"), os.path.join(ROOT, "tests", "test_launcher_validation.py"),
+                             os.path.join(ROOT, "tests", "test_gpu_cell_forms.py"), os.path.join(ROOT, "tests", "test_gpu_step_state.py")],
                             cwd=ROOT, env=environment, capture_output=True, text=True, timeout=900)
     assert result.returncode == 0, result.stdout[-4000:] + result.stderr[-2000:]
     assert " passed" in result.stdout and "out-of-range" not in result.stdout

@@ -50,3 +50,15 @@ def test_every_device_wait_is_bounded():
         for loop in re.finditer(r"for \(;;\) \{", text):
             body = text[loop.end():loop.end() + 900]
             assert "budget_ns" in body, "a spin loop without a budget"
+
+
+def test_stores_of_the_norms_kernel_are_bounds_checked():
+    """The bounds-checked build can only find a bad index where one is compared: every global store of the kernel that the other
+    kernels' inputs come from stands behind a comparison of its own."""
+    text = _code_only(_read("loss_small.cu"))
+    kernel = text[text.index("prefix_norms_kernel(uint4"):text.index("transpose_kernel(")]
+    for target in ("copy", "inverse_norms", "tile_max"):
+        stores = list(re.finditer(rf"\n[^\n]*\b{target}\[[^\n]*\] = ", kernel))
+        assert len(stores) == 1, target
+        statement = kernel[:stores[0].end()].rsplit("if (", 1)[1]
+        assert "SC_IN_BOUNDS(" in statement and ";" not in statement, target
