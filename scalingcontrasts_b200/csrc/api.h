@@ -154,6 +154,11 @@ struct backward_arguments {
     uint32_t split;                     // candidate-range splits (1: deterministic read-modify-write)
     float scale;                        // multiplies every product before accumulation (the loss passes 2 / live)
     uint64_t budget_ns;
+    // Optional (null: none): the forward launch's partial records, folded into the row accumulators by warps that would
+    // otherwise wait for the first accumulator. The same sums in the same order as launch_fold_partials; only without split.
+    float const* partials;
+    float* row_accumulators;
+    uint32_t partial_slots, quantities;
 };
 void launch_backward(backward_arguments const& arguments, cudaStream_t stream);
 // The backward launch's tile table for a shape, without launching: one {band, first channel, width, row blocks per CTA,

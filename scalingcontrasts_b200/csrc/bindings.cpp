@@ -206,7 +206,10 @@ struct loss_plan {
             runtime_check(cudaEventRecord(rejoined[slot], front), "cudaEventRecord");
             runtime_check(cudaStreamWaitEvent(stream, rejoined[slot], 0), "cudaStreamWaitEvent");
         } else sc::launch_forward(a, stream);
-        sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows_q, partial_slots, quantities, stream);
+        // The block's records are folded by the backward kernel, unless there is none, it comes later (the next block's records
+        // are written before it has run) or its CTAs need not all run (split).
+        bool const folds = !fused && !overlapping && backward_split == 1;
+        if (!folds) sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows_q, partial_slots, quantities, stream);
         if (!fused) {
             sc::backward_arguments b{};
             b.gradient_cube_bf16 = pointer<void>(cube);
@@ -215,6 +218,10 @@ struct loss_plan {
             b.query_gradient = pointer<float>(query_gradient), b.status = pointer<uint32_t>(status);
             b.rows_q = rows_q, b.rows_c = rows_c, b.hidden = hidden, b.ladder = ladder, b.split = backward_split;
             b.scale = static_cast<float>(2.0 / live), b.budget_ns = budget_ns;
+            if (folds) {
+                b.partials = pointer<float>(partials), b.row_accumulators = pointer<float>(accumulators);
+                b.partial_slots = partial_slots, b.quantities = quantities;
+            }
             if (!overlapping) sc::launch_backward(b, stream);
             else {
                 runtime_check(cudaEventRecord(forward_done[slot], stream), "cudaEventRecord");

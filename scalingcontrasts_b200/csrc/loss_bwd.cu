@@ -12,8 +12,8 @@
 // 257 to 384 channels, one block x the whole band, so that the band's cube, the traffic this kernel is bound by, is read
 // from DRAM once instead of once per 256-channel tile.
 //
-// Warp roles (192 threads): warps 0-3 epilogue (tensor-memory lanes 32*w..), warp 4 TMA producer, warp 5 UMMA issuer
-// and tensor-memory owner. The producer and the issuer run warp-wide with only the TMA / UMMA / commit instructions
+// Warp roles (192 threads): warps 0-3 epilogue (tensor-memory lanes 32*w..; before that the fold of the forward launch's
+// partial records, if asked for), warp 4 TMA producer, warp 5 UMMA issuer and tensor-memory owner. The producer and the issuer run warp-wide with only the TMA / UMMA / commit instructions
 // under the elected lane, so that their operands are warp-uniform values. The epilogue adds its scaled accumulators with
 // vector reductions (fire and forget: no read of the old value comes back to the SM). With `split == 1` each output
 // element receives exactly one addition per launch, so the sum's order is the launches' stream order and the result
@@ -89,6 +89,9 @@ struct bwd_params {
     uint32_t ring_bytes, tmem_columns; // of one CTA
     float scale; // applied to every product before it is added: the loss's 2/N (mirror cell and weight)
     uint64_t budget_ns;
+    float const* partials; // optional: the block's partial records and the sums they are folded into
+    float* row_accumulators;
+    uint32_t partial_slots, quantities;
     bwd_tile tiles[bwd_max_tiles];
 };
 
@@ -98,6 +101,41 @@ struct bwd_params {
 // candidates make one atom, atoms follow each other every 1024 bytes along K (the stride offset), boxes of 64 channels
 // every 8192 bytes along N (the leading offset); a step of 16 candidates is two atoms, 2048 bytes.
 constexpr uint32_t bwd_mn_box_bytes = 64 * bwd_depth * 2;
+
+// The fold of the forward launch's partial records into the row accumulators, by the epilogue warps before their accumulators
+// are ready. A warp takes sixteen rows of one quantity: a lane four rows (one 16-byte load per record) of every eighth record,
+// eight of them in flight. The eight lanes' sums are then added in order, which gives bit for bit what the fold's own kernel
+// gives. Bound by the latency of its loads, which the GEMM beside it hides: as a launch of its own between the two tile kernels
+// the fold took 4.7 us a block of 4096 rows (72 blocks 11.52 -> 11.19 ms) and 9 us one of 2944 (three blocks 337 -> 310 us).
+// With 128 rows of a quantity to a warp and all its records in eight chains of one lane, the latter took 329 us.
+__device__ __forceinline__ void fold_share(bwd_params const& p, uint32_t warp, uint32_t lane) {
+    constexpr uint32_t chains = 8, rows = 16;
+    uint32_t const groups = p.rows_q / rows, units = groups * p.quantities;
+    size_t const stride = static_cast<size_t>(p.quantities) * p.rows_q;
+    for (uint32_t unit = blockIdx.x + warp * gridDim.x; unit < units; unit += 4 * gridDim.x) {
+        size_t const at = static_cast<size_t>(unit / groups) * p.rows_q + unit % groups * rows + lane % 4 * 4;
+        float4 total = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 8
+        for (uint32_t slot = lane / 4; slot < p.partial_slots; slot += chains)
+            if (SC_IN_BOUNDS(slot * stride + at + 3, p.partial_slots * stride)) {
+                float4 const record = *reinterpret_cast<float4 const*>(p.partials + slot * stride + at);
+                total.x += record.x, total.y += record.y, total.z += record.z, total.w += record.w;
+            }
+        __syncwarp();
+        float4 const own = total;
+#pragma unroll
+        for (uint32_t c = 1; c < chains; ++c) {
+            uint32_t const from = c * 4 + lane % 4;
+            total.x += __shfl_sync(0xFFFFFFFFu, own.x, from), total.y += __shfl_sync(0xFFFFFFFFu, own.y, from);
+            total.z += __shfl_sync(0xFFFFFFFFu, own.z, from), total.w += __shfl_sync(0xFFFFFFFFu, own.w, from);
+        }
+        if (lane < 4 && SC_IN_BOUNDS(at + 3, stride)) { // these lanes began with the first sums
+            float4* const into = reinterpret_cast<float4*>(p.row_accumulators + at);
+            float4 const before = *into;
+            *into = make_float4(before.x + total.x, before.y + total.y, before.z + total.z, before.w + total.w);
+        }
+    }
+}
 
 template <bool mn_major_>
 __global__ void __launch_bounds__(bwd_threads, 1)
@@ -240,6 +278,7 @@ __global__ void __launch_bounds__(bwd_threads, 1)
         if (ok && elected) umma_commit(smem_u32(&tail->accumulated));
         __syncwarp();
     } else {
+        if (p.partials != nullptr) fold_share(p, warp, lane);
         if (mbar_wait(smem_u32(&tail->accumulated), 0u, ctx, site_bwd_accumulated, tile_index)) {
             tcgen05_fence_after();
           for (uint32_t block = 0; block < blocks; ++block) {
@@ -357,6 +396,10 @@ void launch_backward(backward_arguments const& a, cudaStream_t stream) {
     p.query_gradient = a.query_gradient, p.status = a.status;
     p.rows_q = a.rows_q, p.rows_c = a.rows_c, p.hidden = a.hidden;
     p.split = a.split, p.budget_ns = a.budget_ns, p.scale = a.scale;
+    if (a.partials != nullptr && (a.split != 1 || a.row_accumulators == nullptr))
+        throw std::runtime_error("backward: the partial records are folded by launches without split, into row accumulators");
+    p.partials = a.partials, p.row_accumulators = a.row_accumulators;
+    p.partial_slots = a.partial_slots, p.quantities = a.quantities;
     // Per device, once: the multiprocessor count (a runtime query that needs no context of its own).
     static int counted_device = -1, multiprocessors = 148;
     int device = 0;

@@ -11,7 +11,7 @@ A rank owns ``rows`` query rows. Each ``score`` runs, on the calling stream,
    GEMM while its epilogue warps already score the next item: no ``[K, R, R]`` gradient cube exists. Optionally the
    same launch pulls the next block from a peer's memory into local staging,
 4. the deterministic fold of the partials into ``row_accumulators``, and in the two-kernel form the gradient GEMM over the
-   block's cube into ``query_gradient``.
+   block's cube into ``query_gradient`` (one launch for both, unless the GEMM is split or overlapped).
 
 ``begin`` clears both on the device and every block adds to them, in stream order: they hold the blocks scored so far, and a
 ``score`` captured in a CUDA graph may be replayed any number of times between ``begin`` and ``finish`` (with

@@ -90,3 +90,32 @@ def test_sums_read_in_mid_step_follow_the_step(fused):
     loss.finish(queries, stream=side)
     side.synchronize()
     loss.check()
+
+
+@pytest.mark.parametrize("rows,candidate_rows,ends,tiles_per_run", [
+    (128, 128, (64,), 2),                                # one CTA, four records: half of the fold's chains are empty
+    (128, 640, (48, 96, 192, 384, 768), 1),              # forty records
+    (384, 1152, (16, 32, 48, 96, 176, 256, 400, 448), 2),  # thirty-six: the chains' lengths differ
+    (2944, 1408, (16, 208, 576, 832), 1),                # more sums than the launch's warps take in one pass
+    (4096, 512, (256,), 2),
+    (9600, 256, (16, 32, 48, 96, 176, 256, 400, 448), 4),  # two row blocks to a CTA, the last one alone
+])
+def test_fold_in_the_backward_launch(rows, candidate_rows, ends, tiles_per_run):
+    """The records' fold rides in the backward launch, or is a launch of its own where that launch is split: the same bits."""
+    ladder = Matryoshka(ends)
+    generator = torch.Generator(device="cuda").manual_seed(5)
+    queries, *blocks = (torch.nn.functional.normalize(torch.randn(n, ladder.hidden, device="cuda", generator=generator), dim=1).bfloat16()
+                        for n in (rows, candidate_rows, candidate_rows))
+    sums = []
+    for split in (1, 2):
+        loss = StreamedLoss(rows, ladder.hidden, ladder, LossSpec("pairs"), "cuda", candidate_rows=candidate_rows,
+                            tiles_per_run=tiles_per_run, backward_split=split)
+        loss.partials.fill_(float("nan"))
+        loss.begin(queries)
+        for index, block in enumerate(blocks):
+            loss.score(queries, block, 0, rows + index * candidate_rows, 10.0, -10.0, rows)
+        loss.check()
+        sums.append((loss.row_accumulators.clone(), loss.query_gradient.clone()))
+        loss.finish(queries)
+    assert torch.equal(sums[0][0], sums[1][0]) and sums[0][0].isfinite().all() and sums[0][0][0].all()
+    assert _relative(sums[0][1], sums[1][1]) < 1e-6  # float32 sums, of a split launch in no fixed order
