@@ -70,8 +70,10 @@ void launch_expect_arrivals(control_view const& control, uint32_t arrivals, cuda
 void preload_collective_kernels();
 
 // -------- small loss kernels (loss_small.cu) ---------------------------------------------------------------------
+// `clear` (optional): `clear_floats` words, whole 16-byte vectors, that the same launch sets to zero.
 void launch_prefix_norms(void const* rows_bf16, void* copy_bf16, float* inverse_norms, float* tile_max, uint32_t rows,
-                         uint32_t hidden, ladder_host const& ladder, cudaStream_t stream);
+                         uint32_t hidden, ladder_host const& ladder, cudaStream_t stream,
+                         float* clear = nullptr, size_t clear_floats = 0);
 void launch_transpose(void const* rows_bf16, void* transposed_bf16, uint32_t rows, uint32_t hidden, cudaStream_t stream);
 void launch_pull(void const* src0, void* dst0, size_t bytes0, void const* src1, void* dst1, size_t bytes1, int blocks,
                  cudaStream_t stream);

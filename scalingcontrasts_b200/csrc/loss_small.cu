@@ -12,6 +12,7 @@
 // Parity: transpose_cuda_, prefix_inverse_norms_cuda_, fold_partials_cuda_, finalize_cuda_, sum_summands_cuda_
 // (scalingcontrasts.cuh:660-686, 1138-1177); keyed_* and count_* (scalingcontrasts.cu:48-105). The staging pull
 // replaces the reference's cudaMemcpyAsync (scalingcontrasts.cuh:1262-1265).
+#include <algorithm>
 #include <stdexcept>
 #include <string>
 
@@ -41,12 +42,16 @@ ladder_t to_device(ladder_host const& host) {
 constexpr uint32_t norm_rows = 64, norm_warps = 32;
 __global__ void __launch_bounds__(norm_warps * 32)
     prefix_norms_kernel(uint4 const* __restrict__ rows, uint4* __restrict__ copy, float* __restrict__ inverse_norms,
-                        float* __restrict__ tile_max, uint32_t row_count, uint32_t hidden, ladder_t ladder) {
+                        float* __restrict__ tile_max, uint32_t row_count, uint32_t hidden, ladder_t ladder,
+                        float4* __restrict__ clear, size_t clear_vectors) {
     constexpr uint32_t each = norm_rows / norm_warps;
     __shared__ float largest[norm_warps][8];
     uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     uint32_t const first = blockIdx.x * norm_rows + warp * each;
     uint32_t const vectors = hidden / 8;
+    for (size_t v = blockIdx.x * blockDim.x + threadIdx.x; v < clear_vectors; v += static_cast<size_t>(gridDim.x) * blockDim.x)
+        clear[v] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (blockIdx.x * norm_rows >= row_count) return; // a block that only clears
     float sums[each][8];
 #pragma unroll
     for (uint32_t r = 0; r < each; ++r)
@@ -361,11 +366,17 @@ bool bounds_build() { return SC_BOUNDS != 0; }
 SC_DEFINE_BOUNDS_READER(bounds_record_small)
 
 void launch_prefix_norms(void const* rows_bf16, void* copy_bf16, float* inverse_norms, float* tile_max, uint32_t rows,
-                         uint32_t hidden, ladder_host const& ladder, cudaStream_t stream) {
+                         uint32_t hidden, ladder_host const& ladder, cudaStream_t stream, float* clear, size_t clear_floats) {
     if (hidden % 8) throw std::runtime_error("prefix_norms: hidden must be a multiple of 8");
     if (tile_max != nullptr && rows % norm_rows) throw std::runtime_error("prefix_norms: rows must be a multiple of 64 for tile maxima");
-    prefix_norms_kernel<<<blocks_of(rows, norm_rows), norm_warps * 32, 0, stream>>>(
-        static_cast<uint4 const*>(rows_bf16), static_cast<uint4*>(copy_bf16), inverse_norms, tile_max, rows, hidden, to_device(ladder));
+    if (clear_floats % 4 || reinterpret_cast<uintptr_t>(clear) % 16)
+        throw std::runtime_error("prefix_norms: the span to clear must be whole, aligned vectors");
+    // A few rows make a few blocks, which would clear a wide gradient slowly: up to one block per multiprocessor helps them.
+    size_t const clearing = (clear_floats / 4 + norm_warps * 32 - 1) / (norm_warps * 32);
+    int const blocks = std::max(blocks_of(rows, norm_rows), static_cast<int>(std::min<size_t>(clearing, 148)));
+    prefix_norms_kernel<<<blocks, norm_warps * 32, 0, stream>>>(
+        static_cast<uint4 const*>(rows_bf16), static_cast<uint4*>(copy_bf16), inverse_norms, tile_max, rows, hidden, to_device(ladder),
+        reinterpret_cast<float4*>(clear), clear_floats / 4);
     check_launch("prefix_norms");
 }
 

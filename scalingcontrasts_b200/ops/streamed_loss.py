@@ -147,7 +147,7 @@ class StreamedLoss:
         bf16 = dict(dtype=torch.bfloat16, device=self.device)
         self.query_norms = BlockNorms(k, rows, device=self.device)
         self.candidate_norms = BlockNorms(k, self.candidate_rows, device=self.device)
-        # One span, the gradient and the row accumulators behind it, so that a step clears both with one launch.
+        # One span, the gradient and the row accumulators behind it, so that a step clears both at once.
         sums = torch.zeros(rows * (hidden + self.quantities), **f32)
         self.query_gradient = sums[:rows * hidden].view(rows, hidden)
         # Bias gradient, log-scale gradient, prefix losses, self coefficients of the blocks scored so far.
@@ -206,11 +206,12 @@ class StreamedLoss:
     def begin(self, queries: torch.Tensor, stream=None, query_norms: Optional[BlockNorms] = None) -> None:
         """Clears the gradient and the row accumulators and takes the queries' prefix norms (computed here unless supplied)."""
         self._check_queries(queries)
-        self._plan.begin_step(_stream(stream))
         if query_norms is None:
-            compute_block_norms(queries, self.ladder, self.query_norms, stream=stream)
-            self._query_norms_view = self.query_norms
+            own = self.query_norms
+            self._plan.begin_step(queries.data_ptr(), own.inverse.data_ptr(), own.tile_max.data_ptr(), _stream(stream))
+            self._query_norms_view = own
         else:
+            self._plan.begin_step(0, 0, 0, _stream(stream))
             self._query_norms_view = query_norms
         self._begun = True
 
