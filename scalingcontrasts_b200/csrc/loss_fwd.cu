@@ -11,7 +11,7 @@
 // fills the widest bands of tile t+1. A thread of the epilogue takes its columns eight at a time and holds all bands' values
 // of a chunk in registers: the segment dots come in, the prefix dots run up the ladder, the raw-dot gradients (without the
 // factor beta / |q_k| that the row and band share) replace the dots, and the suffix sums that go to the gradient cube run
-// down the ladder. A tile's slots go back to the issuer when its last chunk has been loaded. Ladders of six and more bands
+// down the ladder. A tile's slots go back to the issuer when its last chunk has been loaded. Ladders of five and more bands
 // keep some or all of their gradients in the tensor-memory slots the dots came from until the suffix sums reach them
 // (fwd_parked_bands_for, fwd_rolled_for).
 //
@@ -79,10 +79,13 @@ constexpr uint32_t fwd_warp_columns = fwd_cols / fwd_column_groups;        // co
 // against 161 us where every cell takes the general form, so six stay with two bands parked.
 __host__ __device__ constexpr bool fwd_rolled_for(int prefixes) { return prefixes >= 7; }
 __host__ __device__ constexpr int fwd_chunk_columns_for(int prefixes) { return prefixes <= 1 || fwd_rolled_for(prefixes) ? 16 : 8; }
-// The narrowest bands, where the registers have no room for them beside the others: their gradients are parked in the tensor
-// memory their dots came from until the suffix sums reach them, and their slots are released later than the others'.
-__host__ __device__ constexpr int fwd_parked_bands_for(int prefixes, bool fused) {
-    return fwd_rolled_for(prefixes) ? prefixes - 2 : (prefixes > (fused ? 4 : 5) ? prefixes - 4 : 0);
+// The narrowest bands, where the registers have no room for them beside four others: their gradients are parked in the tensor
+// memory their dots came from until the suffix sums reach them, and their slots are released later than the others'. With all
+// five bands of K=5 in registers the kernel spilled 72 bytes each way: one block of 4096 rows, H=768, took 90.7 us and, with every
+// cell in the general form, 133.9 us; with one band parked it takes 87.9 and 125.0; two blocks of 16384 rows as a
+// whole step 4.06 and 5.22 ms against 4.06 and 5.14 (at that size the GPU runs at its power limit).
+__host__ __device__ constexpr int fwd_parked_bands_for(int prefixes) {
+    return fwd_rolled_for(prefixes) ? prefixes - 2 : (prefixes > 4 ? prefixes - 4 : 0);
 }
 static_assert(fwd_warp_columns == 16, "a warp's store patch of a band is 32 rows x 16 columns");
 constexpr uint32_t fwd_producer_warp = fwd_epilogue_warps;
@@ -387,7 +390,7 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
                                          wait_context const& ctx) {
     constexpr uint32_t fwd_slots = fwd_slots_for(fused_);
     constexpr uint32_t idesc = umma_idesc_bf16(fwd_rows, fwd_cols);
-    constexpr uint32_t parked = fwd_parked_bands_for(prefixes_, fused_);
+    constexpr uint32_t parked = fwd_parked_bands_for(prefixes_);
     constexpr uint32_t descriptor_high = (1024u >> 4) | (1u << 14) | (2u << 29); // stride 1024 B, version 1, 128-byte swizzle
     bool const elected = elect_one();
     uint32_t const chunks = p.hidden / fwd_depth;
@@ -577,7 +580,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
                                               wait_context const& ctx, uint32_t warp, uint32_t lane) {
     constexpr uint32_t fwd_slots = fwd_slots_for(fused_);
     constexpr int columns = fwd_chunk_columns_for(prefixes_);
-    constexpr int parked = fwd_parked_bands_for(prefixes_, fused_);
+    constexpr int parked = fwd_parked_bands_for(prefixes_);
     constexpr bool rolled = fwd_rolled_for(prefixes_);
     constexpr int warp_columns = fwd_warp_columns;
     uint32_t const quadrant = warp % 4, group = warp / 4;
@@ -841,9 +844,11 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
                         pair_t const row_beta2 = pack2(factor, factor);
 #pragma unroll
                         for (int c = 0; c < columns / 2; ++c) {
-                            // In natural units: a hard cell's gradient is large, and is rounded as the special cells' are.
+                            // In natural units: a hard cell's gradient is large, and is rounded as the special cells' are. The cells
+                            // scored apart are looked for only in patches that have any: for every patch it cost 2 % at four bands,
+                            // 3 % at five and 6 % at six.
                             pair_t a = fma2(prefix[c], mul2(inv_c[c], row_beta2), pack2(bias, bias));
-                            a = without_special(a, 2 * c);
+                            if (special) a = without_special(a, 2 * c);
                             pair_t const e = pack2(fast_ex2(-fabsf(a.x) * log2_e), fast_ex2(-fabsf(a.y) * log2_e));
                             pair_t const whole = add2(e, pack2(1.0f, 1.0f));
                             pair_t const complement = mul2(pack2(a.x >= 0.0f ? 1.0f : e.x, a.y >= 0.0f ? 1.0f : e.y),
