@@ -337,7 +337,8 @@ uint32_t plan_tiles(uint32_t rows_q, ladder_host const& ladder, uint32_t split, 
     // One-block tiles that make a little more than one CTA per multiprocessor leave most of the chip idle in a second round
     // (4096 rows, H=768, K=5: 192 CTAs on 148, 58 us). Cut to 128 channels they run two to a multiprocessor, each with half
     // the ring and half the tensor memory, as long as all of them are resident at once: 47 us. A launch of one round stays
-    // with 256 channels, and so does one with more CTAs than two per multiprocessor, which would start a third round.
+    // with 256 channels, and so does one with more CTAs than two per multiprocessor, which would start a third round (neither line
+    // has been measured closely: launches that fill a part of one round, and widths between 128 and 256 channels, have not).
     uint64_t const rounds_of = static_cast<uint64_t>(row_blocks) * split;
     shared = !two_blocks && rounds_of * plain_tiles > static_cast<uint64_t>(multiprocessors) && narrow_tiles <= bwd_max_tiles &&
              rounds_of * narrow_tiles <= 2ull * static_cast<uint64_t>(multiprocessors);
