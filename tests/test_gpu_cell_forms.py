@@ -30,6 +30,28 @@ def _relative(measured, expected):
 SUMMAND_TOLERANCE, GRADIENT_TOLERANCE = 2e-5, 8e-3
 
 
+def _absolute_sums(blocks, ladder, spec, beta, bias):
+    """Sums over all cells, in float64, of |d loss / d bias| and |d loss / d log scale|, without the weight 1 / live: what the
+    signed sums' rounding errors are measured against."""
+    queries, rows = blocks[0].double(), blocks[0].shape[0]
+    candidates = torch.cat(blocks).double()
+    numbers = torch.arange(rows, device="cuda")[:, None]
+    columns = torch.arange(candidates.shape[0], device="cuda")[None, :]
+    own, positive = numbers == columns, torch.zeros(rows, candidates.shape[0], dtype=torch.bool, device="cuda")
+    if spec.pairs:
+        positive |= (numbers ^ 1) == columns
+    if spec.diagonal == "own":
+        positive |= own
+    mask = ~own if spec.diagonal == "skip" else torch.ones_like(own)
+    sums = torch.zeros(2, dtype=torch.float64, device="cuda")
+    for end in ladder.ends:
+        cosine = torch.nn.functional.normalize(queries[:, :end], dim=1) @ torch.nn.functional.normalize(candidates[:, :end], dim=1).T
+        logit = beta * torch.where(own, 1.0, cosine)
+        cell = mask * torch.sigmoid(torch.where(positive, -1.0, 1.0) * (logit + bias))
+        sums += torch.stack([cell.sum(), (cell * logit.abs()).sum()])
+    return sums
+
+
 @pytest.mark.parametrize("beta,bias", [(10.0, -10.0), (10.0, -6.0), (20.0, -3.0), (1.0, 2.0)])
 @pytest.mark.parametrize("spec", [LossSpec("self"), LossSpec("pairs"), LossSpec("pairs", "skip")], ids=lambda s: f"{s.positives}-{s.diagonal}")
 @pytest.mark.parametrize("prefixes", sorted(LADDERS))
@@ -42,10 +64,11 @@ def test_forms_of_the_cell_math_against_float64(prefixes, spec, beta, bias):
     for index, block in enumerate(blocks):
         reference.score(blocks[0], block, 0, index * rows, beta, bias, 2 * rows)
     expected, expected_summands = reference.finish(blocks[0], torch.empty(rows, hidden, dtype=torch.float64, device="cuda"))
+    absolute = _absolute_sums(blocks, ladder, spec, beta, bias)
     for fused in ([False, True] if prefixes <= 6 else [False]):
         loss = StreamedLoss(rows, hidden, ladder, spec, "cuda", fused=fused)
         for scratch in (loss.query_gradient, loss.row_accumulators, loss.partials, loss.similarity_gradients):
-            scratch.fill_(float("nan"))  # the first block replaces whatever is there
+            scratch.fill_(float("nan"))  # a step starts from whatever is there
         for _ in range(2):
             loss.begin(blocks[0])
             for index, block in enumerate(blocks):
@@ -54,6 +77,10 @@ def test_forms_of_the_cell_math_against_float64(prefixes, spec, beta, bias):
         loss.check()
         assert _relative(summands[:3], expected_summands[:3]) < SUMMAND_TOLERANCE
         assert _relative(summands[4:], expected_summands[4:]) < SUMMAND_TOLERANCE
+        # each by itself: the losses are sums of positive terms, the two scalar gradients of signed ones
+        losses = [0] + list(range(4, 4 + prefixes))
+        assert torch.allclose(summands[losses].double(), expected_summands[losses].double(), rtol=SUMMAND_TOLERANCE, atol=0.0)
+        assert ((summands[1:3].double() - expected_summands[1:3].double()).abs() <= SUMMAND_TOLERANCE * absolute / (2 * rows)).all()
         assert _relative(gradient, expected) < GRADIENT_TOLERANCE
 
 
@@ -87,7 +114,7 @@ def test_a_step_without_blocks_is_zero():
 
 @pytest.mark.parametrize("fused", [False, True])
 def test_row_accumulators_between_blocks(fused):
-    """The partial records gather over the blocks; read in mid-step the accumulators hold what was scored so far."""
+    """Read in mid-step the accumulators hold what was scored so far."""
     ladder = Matryoshka(LADDERS[5])
     rows, hidden = 256, ladder.hidden
     blocks = [_rows(rows, hidden, seed) for seed in (6, 7, 8)]
