@@ -13,8 +13,7 @@
 // from DRAM once instead of once per 256-channel tile.
 //
 // Warp roles (192 threads): warps 0-3 epilogue (tensor-memory lanes 32*w..; before that the fold of the forward launch's
-// partial records, if asked for), warp 4 TMA producer, warp 5 UMMA issuer and tensor-memory owner. The producer and the issuer run warp-wide with only the TMA / UMMA / commit instructions
-// under the elected lane, so that their operands are warp-uniform values. The epilogue adds its scaled accumulators with
+// partial records, if asked for), warp 4 TMA producer, warp 5 UMMA issuer and tensor-memory owner. The producer's and the issuer's loops are run by one elected lane each. The epilogue adds its scaled accumulators with
 // vector reductions (fire and forget: no read of the old value comes back to the SM). With `split == 1` each output
 // element receives exactly one addition per launch, so the sum's order is the launches' stream order and the result
 // is deterministic; with a larger split the candidate range is divided and the order of a launch's partial sums is not.
@@ -196,17 +195,17 @@ __global__ void __launch_bounds__(bwd_threads, 1)
     uint32_t const tmem_base = tail->tmem_base;
     wait_context const ctx{p.status, p.budget_ns, &tail->abort_flag};
 
+    // The producer's and the issuer's loops are run by one elected lane each, as in the forward kernel (walked by the whole warp a
+    // launch of 2944 rows, H=832, K=4 took 31 us instead of 29, one of 2048 rows, H=2048, K=8 41 instead of 36).
     if (warp == 4) {
-        bool const elected = elect_one();
-        uint32_t stage = 0, phase = 0;
-        uint32_t const boxes = (tile.width + 63u) / 64u; // MN-major: whole boxes of 64 channels, the last one partly used
-        uint32_t const bytes = blocks * bwd_a_bytes + (mn_major_ ? boxes * bwd_mn_box_bytes : tile.width * bwd_depth * 2);
-        for (uint32_t chunk = chunk_begin; chunk < chunk_end; ++chunk) {
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&tail->stage_empty[stage]), phase ^ 1u, ctx, site_bwd_stage_empty, chunk)))
-                break;
-            uint32_t const full = smem_u32(&tail->stage_full[stage]);
-            uint32_t const destination = stages_base + stage * stage_bytes;
-            if (elected) {
+        if (elect_one()) {
+            uint32_t stage = 0, phase = 0;
+            uint32_t const boxes = (tile.width + 63u) / 64u; // MN-major: whole boxes of 64 channels, the last one partly used
+            uint32_t const bytes = blocks * bwd_a_bytes + (mn_major_ ? boxes * bwd_mn_box_bytes : tile.width * bwd_depth * 2);
+            for (uint32_t chunk = chunk_begin; chunk < chunk_end; ++chunk) {
+                if (!mbar_wait(smem_u32(&tail->stage_empty[stage]), phase ^ 1u, ctx, site_bwd_stage_empty, chunk)) break;
+                uint32_t const full = smem_u32(&tail->stage_full[stage]);
+                uint32_t const destination = stages_base + stage * stage_bytes;
                 mbar_arrive_expect_tx(full, bytes);
                 for (uint32_t block = 0; block < blocks; ++block)
                     tma_load_3d(destination + block * bwd_a_bytes, &cube_map, full, static_cast<int>(chunk * bwd_depth),
@@ -230,38 +229,36 @@ __global__ void __launch_bounds__(bwd_threads, 1)
                         }
                     }
                 }
+                if (++stage == stages) stage = 0, phase ^= 1u;
             }
-            __syncwarp();
-            if (++stage == stages) stage = 0, phase ^= 1u;
         }
     } else if (warp == 5) {
-        bool const elected = elect_one();
-        // A tile wider than one UMMA's 256 columns is issued in two pieces; the second starts 256 channels on, which is
-        // 32 KB into the candidate stage in either layout (four 8 KB boxes, or 256 rows of 128 bytes).
-        uint32_t const major = mn_major_ ? umma_idesc_b_mn_major : 0u;
-        uint32_t const width0 = wide ? bwd_max_width : tile.width;
-        uint32_t const idesc0 = umma_idesc_bf16(bwd_rows, width0) | major;
-        uint32_t const idesc1 = wide ? (umma_idesc_bf16(bwd_rows, tile.width - bwd_max_width) | major) : 0u;
-        constexpr uint32_t descriptor_high = (1024u >> 4) | (1u << 14) | (2u << 29); // stride 1024 B, version 1, 128-byte swizzle
-        uint32_t const low_base = ((stages_base & 0x3FFFFu) >> 4) | (1u << 16);
-        // The B operand's leading offset (bits 16-29 of the low word) and its advance per 16 candidates.
-        constexpr uint32_t b_leading = mn_major_ ? ((bwd_mn_box_bytes >> 4) << 16) : (1u << 16);
-        constexpr uint32_t b_step = mn_major_ ? (2048u >> 4) : 2u;
-        uint32_t stage = 0, phase = 0, accumulate = 0;
-        bool ok = true;
-        for (uint32_t chunk = chunk_begin; chunk < chunk_end; ++chunk) {
-            ok = __all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&tail->stage_full[stage]), phase, ctx, site_bwd_stage_full, chunk));
-            if (!ok) break;
-            tcgen05_fence_after();
-            uint32_t const a_low = low_base + ((stage * stage_bytes) >> 4);
-            uint32_t const b_low = (a_low & 0xFFFFu) + (b_offset >> 4) + b_leading;
-            for (uint32_t block = 0; block < blocks; ++block) {
+        if (elect_one()) {
+            // A tile wider than one UMMA's 256 columns is issued in two pieces; the second starts 256 channels on, which is
+            // 32 KB into the candidate stage in either layout (four 8 KB boxes, or 256 rows of 128 bytes).
+            uint32_t const major = mn_major_ ? umma_idesc_b_mn_major : 0u;
+            uint32_t const width0 = wide ? bwd_max_width : tile.width;
+            uint32_t const idesc0 = umma_idesc_bf16(bwd_rows, width0) | major;
+            uint32_t const idesc1 = wide ? (umma_idesc_bf16(bwd_rows, tile.width - bwd_max_width) | major) : 0u;
+            constexpr uint32_t descriptor_high = (1024u >> 4) | (1u << 14) | (2u << 29); // stride 1024 B, version 1, 128-byte swizzle
+            uint32_t const low_base = ((stages_base & 0x3FFFFu) >> 4) | (1u << 16);
+            // The B operand's leading offset (bits 16-29 of the low word) and its advance per 16 candidates.
+            constexpr uint32_t b_leading = mn_major_ ? ((bwd_mn_box_bytes >> 4) << 16) : (1u << 16);
+            constexpr uint32_t b_step = mn_major_ ? (2048u >> 4) : 2u;
+            uint32_t stage = 0, phase = 0, accumulate = 0;
+            bool ok = true;
+            for (uint32_t chunk = chunk_begin; chunk < chunk_end; ++chunk) {
+                ok = mbar_wait(smem_u32(&tail->stage_full[stage]), phase, ctx, site_bwd_stage_full, chunk);
+                if (!ok) break;
+                tcgen05_fence_after();
+                uint32_t const a_low = low_base + ((stage * stage_bytes) >> 4);
+                uint32_t const b_low = (a_low & 0xFFFFu) + (b_offset >> 4) + b_leading;
+                for (uint32_t block = 0; block < blocks; ++block) {
 #pragma unroll
-                for (uint32_t step = 0; step < bwd_depth / 16; ++step) {
-                    uint64_t a_descriptor, b_descriptor;
-                    asm("mov.b64 %0, {%1, %2};" : "=l"(a_descriptor) : "r"(a_low + block * (bwd_a_bytes >> 4) + step * 2u), "r"(descriptor_high));
-                    asm("mov.b64 %0, {%1, %2};" : "=l"(b_descriptor) : "r"(b_low + step * b_step), "r"(descriptor_high));
-                    if (elected) {
+                    for (uint32_t step = 0; step < bwd_depth / 16; ++step) {
+                        uint64_t a_descriptor, b_descriptor;
+                        asm("mov.b64 %0, {%1, %2};" : "=l"(a_descriptor) : "r"(a_low + block * (bwd_a_bytes >> 4) + step * 2u), "r"(descriptor_high));
+                        asm("mov.b64 %0, {%1, %2};" : "=l"(b_descriptor) : "r"(b_low + step * b_step), "r"(descriptor_high));
                         umma_bf16(tmem_base + block * bwd_block_columns, a_descriptor, b_descriptor, idesc0,
                                   step == 0 ? accumulate : 1u);
                         if (wide)
@@ -269,14 +266,12 @@ __global__ void __launch_bounds__(bwd_threads, 1)
                                       idesc1, step == 0 ? accumulate : 1u);
                     }
                 }
+                accumulate = 1;
+                umma_commit(smem_u32(&tail->stage_empty[stage]));
+                if (++stage == stages) stage = 0, phase ^= 1u;
             }
-            accumulate = 1;
-            if (elected) umma_commit(smem_u32(&tail->stage_empty[stage]));
-            __syncwarp();
-            if (++stage == stages) stage = 0, phase ^= 1u;
+            if (ok) umma_commit(smem_u32(&tail->accumulated));
         }
-        if (ok && elected) umma_commit(smem_u32(&tail->accumulated));
-        __syncwarp();
     } else {
         if (p.partials != nullptr) fold_share(p, warp, lane);
         if (mbar_wait(smem_u32(&tail->accumulated), 0u, ctx, site_bwd_accumulated, tile_index)) {

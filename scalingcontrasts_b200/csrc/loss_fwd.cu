@@ -17,8 +17,7 @@
 //
 // Warp roles (640 threads): warps 0-15 epilogue (warp w owns tensor-memory lanes 32*(w%4).. and the 16 columns w/4 of
 // the tile; four warps per scheduler keep the issue slots busy), warp 16 TMA producer (and the candidates' norms), warp 17
-// UMMA issuer and tensor-memory owner (both run warp-wide, with the TMA / UMMA / commit instructions under one elected
-// lane), warp 18 peer pull (plain 16-byte loads from the peer's replica, plain stores to local staging; never a TMA load
+// UMMA issuer and tensor-memory owner (each loop run by one elected lane), warp 18 peer pull (plain 16-byte loads from the peer's replica, plain stores to local staging; never a TMA load
 // from another GPU's memory), warp 19 the fused kernel's second issuer. The epilogue's four warpgroups run with 104
 // registers a thread, the helpers' with 64.
 //
@@ -308,22 +307,19 @@ __device__ __forceinline__ void tmem_store_8(uint32_t taddr, uint32_t const (&r)
 __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ---- roles ------------------------------------------------------------------------------------------------------
-// The producer and UMMA roles are run by all 32 lanes of their warp, with only the TMA / UMMA / commit instructions
-// themselves under the elected lane's predicate: loop counters, stage addresses and descriptors are then warp-uniform
-// values the compiler can keep in uniform registers, which is where those instructions take their operands from. (Run
-// by a single lane inside a divergent branch, every operand would cross from a vector to a uniform register first.)
-// Every lane waits; the answer is the same in every lane.
-// Their waits sleep between attempts: a helper warp shares its scheduler with four epilogue warps, and a warp that polls an
-// mbarrier without pause issues about as many instructions as one of them. (The polling wait's timed part is a function of
-// the epilogue warps alone: one function cannot serve both sides of the register split.)
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, wait_context const& ctx, uint32_t site,
-                                               uint32_t detail, uint32_t sleep_ns) {
-    return __all_sync(0xFFFFFFFFu, mbar_wait_relaxed(bar, parity, ctx, site, detail, sleep_ns));
+// The producer and UMMA roles' loops are run by one elected lane: a chunk of the issue loop costs 228 cycles (192 of them its four
+// UMMAs), where the whole warp walking it, with only the TMA / UMMA / commit instructions under the elected lane's predicate,
+// took 379 (votes over the waits' answers, reconvergence after every predicated block). One block of 4096 rows, H=768, K=5:
+// 88.9 -> 81 us, H=1024, K=1: 72.6 -> 58 us. They wait on their barriers without sleeping in between (the suspended wait takes
+// no issue slots worth counting; with naps of 200 and 20 ns the same blocks take 82.4 and 60.4 us).
+// (The timed part of the epilogue's wait is a function of its own: one function cannot serve both sides of the register split.)
+__device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, wait_context const& ctx, uint32_t site, uint32_t detail) {
+#pragma unroll 1
+    for (int spin = 0; spin < 16; ++spin)
+        if (mbar_try_wait(bar, parity)) return true;
+    return mbar_wait_sleeping(bar, parity, ctx.status, ctx.budget_ns, ctx.abort_flag, site, detail, 0u);
 }
-constexpr uint32_t sleep_producer_ns = 200; // stages ahead of the issuer: nothing waits for this warp's wake-up
-constexpr uint32_t sleep_issuer_ns = 20;    // the epilogue may be waiting for the tile these UMMAs finish
-constexpr uint32_t sleep_gemm_ns = 500;      // the fused kernel's gradient GEMM runs a whole item behind
-
+constexpr uint32_t sleep_gemm_ns = 500; // the fused kernel's gradient GEMM runs a whole item behind
 
 // A CTA's items: every gridDim.x-th of the list.
 __device__ __forceinline__ uint32_t item_count(uint32_t items) { return (items + gridDim.x - 1 - blockIdx.x) / gridDim.x; }
@@ -356,25 +352,26 @@ __device__ __forceinline__ void producer_role(CUtensorMap const* q_map, CUtensor
             if (lane < prefixes_ &&
                 SC_IN_BOUNDS(static_cast<size_t>(lane) * column_tiles + column_tile, static_cast<size_t>(prefixes_) * column_tiles))
                 largest = __ldg(p.c_tile_max + static_cast<size_t>(lane) * column_tiles + column_tile);
-            for (int chunk = static_cast<int>(chunks) - 1; chunk >= 0; --chunk) {
-                timer.lap(0);
-                if (!mbar_wait_warp(smem_u32(&tail->stage_empty[stage]), phase ^ 1u, ctx, site_fwd_stage_empty, item, sleep_producer_ns))
-                    return;
-                timer.lap(1);
-                uint32_t const full = smem_u32(&tail->stage_full[stage]);
-                uint32_t const destination = stages_base + stage * fwd_stage_bytes;
-                if (elected) {
+            bool ok = true;
+            if (elected) {
+                for (int chunk = static_cast<int>(chunks) - 1; chunk >= 0; --chunk) {
+                    timer.lap(0);
+                    ok = mbar_wait_lane(smem_u32(&tail->stage_empty[stage]), phase ^ 1u, ctx, site_fwd_stage_empty, item);
+                    if (!ok) break;
+                    timer.lap(1);
+                    uint32_t const full = smem_u32(&tail->stage_full[stage]);
+                    uint32_t const destination = stages_base + stage * fwd_stage_bytes;
                     mbar_arrive_expect_tx(full, fwd_stage_bytes);
                     tma_load_2d(destination, q_map, full, chunk * static_cast<int>(fwd_depth), static_cast<int>(strip * fwd_rows));
                     tma_load_2d(destination + fwd_q_bytes, c_map, full, chunk * static_cast<int>(fwd_depth),
                                 static_cast<int>(column_tile * fwd_cols));
+                    if (++stage == stages) stage = 0, phase ^= 1u;
                 }
-                __syncwarp();
-                if (++stage == stages) stage = 0, phase ^= 1u;
             }
+            if (!__all_sync(0xFFFFFFFFu, ok)) return;
             uint32_t const entry = tile_local % fwd_norm_slots;
-            if (!mbar_wait_warp(smem_u32(&tail->norms_empty[entry]), ((tile_local / fwd_norm_slots) & 1u) ^ 1u, ctx,
-                                site_fwd_norms_empty, item, sleep_producer_ns))
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait_lane(smem_u32(&tail->norms_empty[entry]), ((tile_local / fwd_norm_slots) & 1u) ^ 1u,
+                                                        ctx, site_fwd_norms_empty, item)))
                 return;
             float* const into = norm_ring + entry * fwd_norm_floats(prefixes_);
 #pragma unroll
@@ -394,12 +391,11 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
     constexpr uint32_t idesc = umma_idesc_bf16(fwd_rows, fwd_cols);
     constexpr uint32_t parked = fwd_parked_bands_for(prefixes_);
     constexpr uint32_t descriptor_high = (1024u >> 4) | (1u << 14) | (2u << 29); // stride 1024 B, version 1, 128-byte swizzle
-    bool const elected = elect_one();
+    if (!elect_one()) return;
     uint32_t const chunks = p.hidden / fwd_depth;
     uint32_t const low_base = ((stages_base & 0x3FFFFu) >> 4) | (1u << 16);
     uint32_t stage = 0, phase = 0, unit = 0, tile_local = 0, seen = 0, seen_parked = 0;
     phase_timer timer(p);
-    timer.only_if(elected);
     // The next band's slot, once it is free. The slot's last user was unit - fwd_slots, a band of tile `needed`; the
     // epilogue must have read it out. Releases are observed here strictly in tile order, per barrier array, so a barrier's
     // parity can never be a full turn ahead of the one waited for: tile X + fwd_slots cannot even be issued before tile X's release has been
@@ -413,8 +409,7 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
             uint32_t& observed = was_parked ? seen_parked : seen;
             timer.lap(0);
             while (observed <= needed) {
-                if (!mbar_wait_warp(smem_u32(&barriers[observed % fwd_slots]), (observed / fwd_slots) & 1u, ctx,
-                                    site_fwd_slot_empty, unit, sleep_issuer_ns))
+                if (!mbar_wait_lane(smem_u32(&barriers[observed % fwd_slots]), (observed / fwd_slots) & 1u, ctx, site_fwd_slot_empty, unit))
                     return false;
                 ++observed;
             }
@@ -431,7 +426,7 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
             for (int chunk = static_cast<int>(chunks) - 1; chunk >= 0; --chunk) {
                 uint32_t const starts = p.band_starts[chunk];
                 timer.lap(0);
-                if (!mbar_wait_warp(smem_u32(&tail->stage_full[stage]), phase, ctx, site_fwd_stage_full, tile_local, sleep_issuer_ns))
+                if (!mbar_wait_lane(smem_u32(&tail->stage_full[stage]), phase, ctx, site_fwd_stage_full, tile_local))
                     return;
                 timer.lap(1);
                 tcgen05_fence_after();
@@ -444,28 +439,22 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
                 // that starts inside the chunk (its edge is not a multiple of 64) takes the step-by-step way.
                 if ((starts & 0x00FFFFFFu) == 0u) {
                     if (starts != 0u && !take_slot()) return;
-                    if (elected) {
-                        umma_bf16(slot_address, q_descriptor + 6, c_descriptor + 6, idesc, starts != 0u ? 0u : 1u);
-                        umma_bf16(slot_address, q_descriptor + 4, c_descriptor + 4, idesc, 1u);
-                        umma_bf16(slot_address, q_descriptor + 2, c_descriptor + 2, idesc, 1u);
-                        umma_bf16(slot_address, q_descriptor, c_descriptor, idesc, 1u);
-                        umma_commit(empty);
-                    }
+                    umma_bf16(slot_address, q_descriptor + 6, c_descriptor + 6, idesc, starts != 0u ? 0u : 1u);
+                    umma_bf16(slot_address, q_descriptor + 4, c_descriptor + 4, idesc, 1u);
+                    umma_bf16(slot_address, q_descriptor + 2, c_descriptor + 2, idesc, 1u);
+                    umma_bf16(slot_address, q_descriptor, c_descriptor, idesc, 1u);
                 } else {
 #pragma unroll 1
                     for (int sub = 3; sub >= 0; --sub) {
                         bool const begins = ((starts >> (8 * sub)) & 0xFFu) != 0u;
                         if (begins && !take_slot()) return;
-                        if (elected)
-                            umma_bf16(slot_address, q_descriptor + 2u * sub, c_descriptor + 2u * sub, idesc, begins ? 0u : 1u);
+                        umma_bf16(slot_address, q_descriptor + 2u * sub, c_descriptor + 2u * sub, idesc, begins ? 0u : 1u);
                     }
-                    if (elected) umma_commit(empty);
                 }
-                __syncwarp();
+                umma_commit(empty);
                 if (++stage == fwd_stages_for(prefixes_, fused_)) stage = 0, phase ^= 1u;
             }
-            if (elected) umma_commit(smem_u32(&tail->tile_full[tile_local % fwd_tile_barriers]));
-            __syncwarp();
+            umma_commit(smem_u32(&tail->tile_full[tile_local % fwd_tile_barriers]));
             ++tile_local;
         }
     }
@@ -1045,15 +1034,14 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
 // [width channels x 64 candidates]. Both K-major under the 128-byte swizzle.
 __device__ __forceinline__ void fz_producer_role(fz_maps const* maps, fwd_params const& p, uint32_t stages_base,
                                                  fwd_tail* tail, wait_context const& ctx, uint32_t const prefixes) {
-    bool const elected = elect_one();
+    if (!elect_one()) return;
     uint32_t stage = 0, phase = 0, local = 0;
     phase_timer timer(p);
-    timer.only_if(elected);
     for (uint32_t count = item_count(p.items); local < count; ++local) {
         uint32_t const item = item_at(local);
         uint32_t const buffer = local & 1u;
         timer.lap(0);
-        if (!mbar_wait_warp(smem_u32(&tail->fz_item_stored[buffer]), (local >> 1) & 1u, ctx, site_fz_item_stored, item, sleep_producer_ns))
+        if (!mbar_wait_relaxed(smem_u32(&tail->fz_item_stored[buffer]), (local >> 1) & 1u, ctx, site_fz_item_stored, item, sleep_gemm_ns))
             return;
         timer.lap(1);
         fence_proxy_async_all();
@@ -1063,28 +1051,25 @@ __device__ __forceinline__ void fz_producer_role(fz_maps const* maps, fwd_params
             uint32_t const band = word & 0xFu, channel0 = ((word >> 4) & 0xFFFu) * 16u, width = (word >> 16) * 16u;
             for (uint32_t block = 0; block < p.tiles_per_run; ++block) {
                 timer.lap(0);
-                if (!mbar_wait_warp(smem_u32(&tail->fz_stage_empty[stage]), phase ^ 1u, ctx, site_fz_stage_empty, which, sleep_gemm_ns))
+                if (!mbar_wait_lane(smem_u32(&tail->fz_stage_empty[stage]), phase ^ 1u, ctx, site_fz_stage_empty, which))
                     return;
                 timer.lap(2);
                 uint32_t const full = smem_u32(&tail->fz_stage_full[stage]);
                 uint32_t const destination = stages_base + stage * fz_stage_bytes;
-                if (elected) {
-                    mbar_arrive_expect_tx(full, fz_a_bytes + width * fz_depth * 2u);
-                    tma_load_3d(destination, &maps->patches, full, static_cast<int>(block * fz_depth), 0,
-                                static_cast<int>((blockIdx.x * 2u + buffer) * prefixes + band));
-                    // Largest boxes first; 16 channels are 2048 bytes of the stage (rows of 128 bytes under the swizzle).
-                    uint32_t done = 0;
+                mbar_arrive_expect_tx(full, fz_a_bytes + width * fz_depth * 2u);
+                tma_load_3d(destination, &maps->patches, full, static_cast<int>(block * fz_depth), 0,
+                            static_cast<int>((blockIdx.x * 2u + buffer) * prefixes + band));
+                // Largest boxes first; 16 channels are 2048 bytes of the stage (rows of 128 bytes under the swizzle).
+                uint32_t done = 0;
 #pragma unroll
-                    for (int index = static_cast<int>(fz_candidate_maps) - 1; index >= 0; --index) {
-                        uint32_t const box = 16u << index;
-                        if (width - done >= box) {
-                            tma_load_2d(destination + fz_a_bytes + done * 128u, &maps->candidates[index], full,
-                                        static_cast<int>(first_candidate + block * fz_depth), static_cast<int>(channel0 + done));
-                            done += box;
-                        }
+                for (int index = static_cast<int>(fz_candidate_maps) - 1; index >= 0; --index) {
+                    uint32_t const box = 16u << index;
+                    if (width - done >= box) {
+                        tma_load_2d(destination + fz_a_bytes + done * 128u, &maps->candidates[index], full,
+                                    static_cast<int>(first_candidate + block * fz_depth), static_cast<int>(channel0 + done));
+                        done += box;
                     }
                 }
-                __syncwarp();
                 if (++stage == fz_stages) stage = 0, phase ^= 1u;
             }
         }
@@ -1095,12 +1080,11 @@ __device__ __forceinline__ void fz_producer_role(fz_maps const* maps, fwd_params
 __device__ __forceinline__ void fz_mma_role(fwd_params const& p, uint32_t stages_base, fwd_tail* tail, uint32_t tmem_base,
                                             wait_context const& ctx) {
     constexpr uint32_t descriptor_high = (1024u >> 4) | (1u << 14) | (2u << 29); // stride 1024 B, version 1, 128-byte swizzle
-    bool const elected = elect_one();
+    if (!elect_one()) return;
     uint32_t const low_base = ((stages_base & 0x3FFFFu) >> 4) | (1u << 16);
     uint32_t const accumulator = tmem_base + fz_accumulator_column;
     uint32_t stage = 0, phase = 0, unit = 0;
     phase_timer timer(p);
-    timer.only_if(elected);
     for (uint32_t n = 0, count = item_count(p.items); n < count; ++n) {
         uint32_t const item = item_at(n);
         for (uint32_t which = 0; which < p.tile_count; ++which, ++unit) {
@@ -1108,12 +1092,12 @@ __device__ __forceinline__ void fz_mma_role(fwd_params const& p, uint32_t stages
             // The accumulator's previous contents must have left tensor memory (an arrival per epilogue warp).
             timer.lap(0);
             if (unit != 0 &&
-                !mbar_wait_warp(smem_u32(&tail->fz_accumulator_empty), (unit - 1) & 1u, ctx, site_fz_accumulator_empty, unit, sleep_gemm_ns))
+                !mbar_wait_relaxed(smem_u32(&tail->fz_accumulator_empty), (unit - 1) & 1u, ctx, site_fz_accumulator_empty, unit, sleep_gemm_ns))
                 return;
             timer.lap(1);
             tcgen05_fence_after();
             for (uint32_t block = 0; block < p.tiles_per_run; ++block) {
-                if (!mbar_wait_warp(smem_u32(&tail->fz_stage_full[stage]), phase, ctx, site_fz_stage_full, unit, sleep_gemm_ns)) return;
+                if (!mbar_wait_lane(smem_u32(&tail->fz_stage_full[stage]), phase, ctx, site_fz_stage_full, unit)) return;
                 timer.lap(2);
                 tcgen05_fence_after();
                 uint32_t const a_low = low_base + stage * (fz_stage_bytes >> 4);
@@ -1123,14 +1107,12 @@ __device__ __forceinline__ void fz_mma_role(fwd_params const& p, uint32_t stages
                     uint64_t a_descriptor, b_descriptor;
                     asm("mov.b64 %0, {%1, %2};" : "=l"(a_descriptor) : "r"(a_low + step * 2u), "r"(descriptor_high));
                     asm("mov.b64 %0, {%1, %2};" : "=l"(b_descriptor) : "r"(b_low + step * 2u), "r"(descriptor_high));
-                    if (elected) umma_bf16(accumulator, a_descriptor, b_descriptor, idesc, (block | step) != 0u ? 1u : 0u);
+                    umma_bf16(accumulator, a_descriptor, b_descriptor, idesc, (block | step) != 0u ? 1u : 0u);
                 }
-                if (elected) umma_commit(smem_u32(&tail->fz_stage_empty[stage]));
-                __syncwarp();
+                umma_commit(smem_u32(&tail->fz_stage_empty[stage]));
                 if (++stage == fz_stages) stage = 0, phase ^= 1u;
             }
-            if (elected) umma_commit(smem_u32(&tail->fz_accumulator_full));
-            __syncwarp();
+            umma_commit(smem_u32(&tail->fz_accumulator_full));
         }
     }
     timer.flush(p, 12, 3);
