@@ -134,6 +134,7 @@ struct forward_arguments {
     void const* transposed_candidates; // [hidden, rows_c]
     float* query_gradient;             // [rows_q, hidden], accumulated
     float gradient_scale;              // the loss passes 2 / live
+    bool ordinary_launch;              // true: starts only once everything before it in the stream is complete (see launch.h)
 };
 // Returns the number of partial slots the launch fills: (column groups per tile) * rows_c / 64 / tiles_per_run.
 uint32_t forward_partial_slots(uint32_t rows_c, uint32_t tiles_per_run);
@@ -161,6 +162,7 @@ struct backward_arguments {
     float const* partials;
     float* row_accumulators;
     uint32_t partial_slots, quantities;
+    bool ordinary_launch; // as above
 };
 void launch_backward(backward_arguments const& arguments, cudaStream_t stream);
 // The backward launch's tile table for a shape, without launching: one {band, first channel, width, row blocks per CTA,

@@ -200,6 +200,7 @@ struct loss_plan {
         a.fused = fused, a.fused_scratch_bf16 = pointer<void>(cube), a.fused_scratch_bytes = gradients_bytes;
         a.transposed_candidates = pointer<void>(transposed), a.query_gradient = pointer<float>(query_gradient);
         a.gradient_scale = static_cast<float>(2.0 / live);
+        a.ordinary_launch = overlapping; // between streams, behind events
         if (overlapping && pending) {
             runtime_check(cudaEventRecord(forked[slot], stream), "cudaEventRecord");
             runtime_check(cudaStreamWaitEvent(front, forked[slot], 0), "cudaStreamWaitEvent");
@@ -220,7 +221,7 @@ struct loss_plan {
             b.candidates_row_major = transposing ? nullptr : pointer<void>(candidates);
             b.query_gradient = pointer<float>(query_gradient), b.status = pointer<uint32_t>(status);
             b.rows_q = rows_q, b.rows_c = rows_c, b.hidden = hidden, b.ladder = ladder, b.split = backward_split;
-            b.scale = static_cast<float>(2.0 / live), b.budget_ns = budget_ns;
+            b.scale = static_cast<float>(2.0 / live), b.budget_ns = budget_ns, b.ordinary_launch = overlapping;
             if (folds) {
                 b.partials = pointer<float>(partials), b.row_accumulators = pointer<float>(accumulators);
                 b.partial_slots = partial_slots, b.quantities = quantities;

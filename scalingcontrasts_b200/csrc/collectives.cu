@@ -27,6 +27,7 @@
 
 #include "api.h"
 #include "common.cuh"
+#include "launch.h"
 
 namespace sc {
 
@@ -101,6 +102,7 @@ __device__ __forceinline__ void leave(control_view const& c, uint32_t round) {
 }
 
 __global__ void barrier_kernel(control_view c) {
+    wait_for_kernels_before(); // and lets nothing start before it is done: it waits for other ranks
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     if (status_poisoned(c.status)) return;
     uint32_t const round = *reinterpret_cast<uint32_t volatile*>(c.own_round);
@@ -312,6 +314,7 @@ __global__ void __launch_bounds__(small_threads)
     all_reduce_small_kernel(control_view c, char* own_payload, char* slots, replica_list slot_replicas, char* own_slots,
                             uint32_t vectors, uint32_t slot_bytes, float scale) {
     __shared__ uint32_t shared_round, shared_ok;
+    wait_for_kernels_before(); // and lets nothing start before it is done: it waits for other ranks
     if (threadIdx.x == 0) {
         shared_round = *reinterpret_cast<uint32_t volatile*>(c.own_round);
         shared_ok = status_poisoned(c.status) ? 0u : 1u;
@@ -419,7 +422,7 @@ int last_collective_path() { return last_path.load(); }
 SC_DEFINE_BOUNDS_READER(bounds_record_collectives)
 
 void launch_barrier(control_view const& control, cudaStream_t stream) {
-    barrier_kernel<<<1, 32, 0, stream>>>(control);
+    launch_dependent(true, barrier_kernel, 1, 32, 0, stream, control);
     check_launch("barrier");
     last_path.store(control.multicast_flag != nullptr ? 1 : 0);
 }
@@ -469,11 +472,11 @@ void launch_all_reduce_small(control_view const& control, void* own_payload, voi
     char* const mine = static_cast<char*>(own_slots);
     uint32_t const v = static_cast<uint32_t>(vectors), bytes = static_cast<uint32_t>(slot_bytes);
     if (type == payload_type::f32) {
-        if (multicast_path) all_reduce_small_kernel<payload_type::f32, true><<<1, threads, 0, stream>>>(control, payload, mc, list, mine, v, bytes, scale);
-        else all_reduce_small_kernel<payload_type::f32, false><<<1, threads, 0, stream>>>(control, payload, mc, list, mine, v, bytes, scale);
+        if (multicast_path) launch_dependent(true, all_reduce_small_kernel<payload_type::f32, true>, 1, threads, 0, stream, control, payload, mc, list, mine, v, bytes, scale);
+        else launch_dependent(true, all_reduce_small_kernel<payload_type::f32, false>, 1, threads, 0, stream, control, payload, mc, list, mine, v, bytes, scale);
     } else {
-        if (multicast_path) all_reduce_small_kernel<payload_type::bf16, true><<<1, threads, 0, stream>>>(control, payload, mc, list, mine, v, bytes, scale);
-        else all_reduce_small_kernel<payload_type::bf16, false><<<1, threads, 0, stream>>>(control, payload, mc, list, mine, v, bytes, scale);
+        if (multicast_path) launch_dependent(true, all_reduce_small_kernel<payload_type::bf16, true>, 1, threads, 0, stream, control, payload, mc, list, mine, v, bytes, scale);
+        else launch_dependent(true, all_reduce_small_kernel<payload_type::bf16, false>, 1, threads, 0, stream, control, payload, mc, list, mine, v, bytes, scale);
     }
     check_launch("all_reduce_small");
     last_path.store(multicast_path ? 1 : 0);

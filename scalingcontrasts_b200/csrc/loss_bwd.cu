@@ -27,6 +27,7 @@
 #include "api.h"
 #include "common.cuh"
 #include "driver.h"
+#include "launch.h"
 
 namespace sc {
 
@@ -171,7 +172,6 @@ __global__ void __launch_bounds__(bwd_threads, 1)
     uint32_t const chunk_end = min(chunk_begin + chunks_per_split, chunks_total);
 
     if (threadIdx.x == 0) {
-        tail->abort_flag = status_poisoned(p.status) ? 1u : 0u;
         for (uint32_t i = 0; i < bwd_stages; ++i) {
             mbar_init(smem_u32(&tail->stage_full[i]), 1);
             mbar_init(smem_u32(&tail->stage_empty[i]), 1);
@@ -179,8 +179,11 @@ __global__ void __launch_bounds__(bwd_threads, 1)
         mbar_init(smem_u32(&tail->accumulated), 1);
         fence_barrier_init();
     }
-    __syncthreads();
-    if (tail->abort_flag != 0u || chunk_begin >= chunk_end) return;
+    let_dependents_start();
+    if (chunk_begin >= chunk_end) { // a split with nothing left
+        wait_for_kernels_before();
+        return;
+    }
     if (warp == 5) {
         tmem_alloc(smem_u32(&tail->tmem_base), p.tmem_columns);
         tmem_relinquish();
@@ -189,6 +192,9 @@ __global__ void __launch_bounds__(bwd_threads, 1)
         tma_prefetch_descriptor(&cube_map);
         for (uint32_t i = 0; i < bwd_candidate_maps; ++i) tma_prefetch_descriptor(&candidates.maps[i]);
     }
+    // Everything up to here may run beside the end of the kernel before.
+    wait_for_kernels_before();
+    if (threadIdx.x == 0) tail->abort_flag = status_poisoned(p.status) ? 1u : 0u;
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
@@ -197,7 +203,9 @@ __global__ void __launch_bounds__(bwd_threads, 1)
 
     // The producer's and the issuer's loops are run by one elected lane each, as in the forward kernel (walked by the whole warp a
     // launch of 2944 rows, H=832, K=4 took 31 us instead of 29, one of 2048 rows, H=2048, K=8 41 instead of 36).
-    if (warp == 4) {
+    bool const poisoned = tail->abort_flag != 0u; // by an earlier kernel: nothing is added
+    if (poisoned) {
+    } else if (warp == 4) {
         if (elect_one()) {
             uint32_t stage = 0, phase = 0;
             uint32_t const boxes = (tile.width + 63u) / 64u; // MN-major: whole boxes of 64 channels, the last one partly used
@@ -300,7 +308,7 @@ __global__ void __launch_bounds__(bwd_threads, 1)
 
     tcgen05_fence_before();
     __syncthreads();
-    if (tail->abort_flag != 0u) {
+    if (!poisoned && tail->abort_flag != 0u) {
         uint64_t const start = global_timer_ns();
         while (global_timer_ns() - start < 200000ull) __nanosleep(1000);
     }
@@ -440,8 +448,8 @@ void launch_backward(backward_arguments const& a, cudaStream_t stream) {
         prepared_device = device;
     }
     dim3 const grid(ctas, a.split, 1);
-    if (mn_major) backward_kernel<true><<<grid, bwd_threads, shared_bytes, stream>>>(cube_map, candidates, p);
-    else backward_kernel<false><<<grid, bwd_threads, shared_bytes, stream>>>(cube_map, candidates, p);
+    launch_dependent(!a.ordinary_launch, mn_major ? backward_kernel<true> : backward_kernel<false>, grid, bwd_threads, shared_bytes, stream,
+                     cube_map, candidates, p);
     cudaError_t const error = cudaGetLastError();
     if (error != cudaSuccess) throw std::runtime_error(std::string("backward launch failed: ") + cudaGetErrorString(error));
     note_launch();

@@ -39,6 +39,7 @@
 #include "api.h"
 #include "common.cuh"
 #include "driver.h"
+#include "launch.h"
 
 namespace sc {
 
@@ -347,11 +348,11 @@ __device__ __forceinline__ void producer_role(CUtensorMap const* q_map, CUtensor
 #pragma unroll
             for (int j = 0; j < 2 * prefixes_; ++j) {
                 size_t const at = static_cast<size_t>(j / 2) * p.rows_c + column_tile * fwd_cols + (j % 2) * 32u + lane;
-                norms[j] = SC_IN_BOUNDS(at, static_cast<size_t>(prefixes_) * p.rows_c) ? __ldg(p.c_inv + at) : 0.0f;
+                norms[j] = SC_IN_BOUNDS(at, static_cast<size_t>(prefixes_) * p.rows_c) ? *(p.c_inv + at) : 0.0f;
             }
             if (lane < prefixes_ &&
                 SC_IN_BOUNDS(static_cast<size_t>(lane) * column_tiles + column_tile, static_cast<size_t>(prefixes_) * column_tiles))
-                largest = __ldg(p.c_tile_max + static_cast<size_t>(lane) * column_tiles + column_tile);
+                largest = *(p.c_tile_max + static_cast<size_t>(lane) * column_tiles + column_tile);
             bool ok = true;
             if (elected) {
                 for (int chunk = static_cast<int>(chunks) - 1; chunk >= 0; --chunk) {
@@ -529,7 +530,7 @@ __device__ __noinline__ special_sums special_cells(uint32_t lane_base, uint32_t 
     for (int k = 0; k < prefixes_; ++k) {
         uint32_t d[16];
         tmem_load<16>(lane_base + band_slot<prefixes_, fused_>(first_unit, k), d);
-        float const inv_q = __ldg(q_inv + static_cast<size_t>(k) * rows_q);
+        float const inv_q = *(q_inv + static_cast<size_t>(k) * rows_q);
         float const row_beta = row_factor(beta, inv_q);
         float const without_row_factor = row_beta != 0.0f ? __fdividef(1.0f, row_beta) : 0.0f;
         float loss = 0.0f, coefficient = 0.0f, partner_raw = 0.0f;
@@ -579,8 +580,8 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
     uint32_t const row_local = quadrant * 32 + lane;
     uint32_t const lane_base = tmem_base + ((quadrant * 32u) << 16) + group * warp_columns;
     uint32_t const quantities = 2 + 2 * prefixes_;
-    float const beta = p.scalars != nullptr ? __ldg(p.scalars) : p.beta;
-    float const bias = p.scalars != nullptr ? __ldg(p.scalars + 1) : p.bias;
+    float const beta = p.scalars != nullptr ? *p.scalars : p.beta;
+    float const bias = p.scalars != nullptr ? *(p.scalars + 1) : p.bias;
     uint32_t tile_local = 0;
     uint32_t const warp_store_base = store_base + warp * fwd_store_patches(prefixes_) * fwd_store_patch_bytes;
 
@@ -651,7 +652,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
             row = strip * fwd_rows + row_local;
 #pragma unroll
             for (int k = 0; k < prefixes_; ++k) {
-                float const inv_q = __ldg(p.q_inv + static_cast<size_t>(k) * p.rows_q + row);
+                float const inv_q = *(p.q_inv + static_cast<size_t>(k) * p.rows_q + row);
                 // inverse norms are not negative, so their bits order as they do
                 float const band_max = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(inv_q)));
                 rows_max = lane == static_cast<uint32_t>(k) ? band_max : rows_max;
@@ -759,7 +760,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
                     inv_c[c] = pack2(quad.x, quad.y), inv_c[c + 1] = pack2(quad.z, quad.w);
                 }
                 if ((floors >> k) & 1u) {
-                    float const inv_q = __ldg(p.q_inv + static_cast<size_t>(k) * p.rows_q + row);
+                    float const inv_q = *(p.q_inv + static_cast<size_t>(k) * p.rows_q + row);
 #pragma unroll
                     for (int c = 0; c < columns / 2; ++c) {
                         inv_c[c].x = inv_q * inv_c[c].x >= 100.0f ? 0.0f : inv_c[c].x;
@@ -1154,7 +1155,6 @@ __global__ void __launch_bounds__(fwd_threads, 1)
     uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 
     if (threadIdx.x == 0) {
-        tail->abort_flag = status_poisoned(p.status) ? 1u : 0u;
         for (uint32_t i = 0; i < fwd_max_stages; ++i) {
             mbar_init(smem_u32(&tail->stage_full[i]), 1);
             mbar_init(smem_u32(&tail->stage_empty[i]), 1);
@@ -1180,8 +1180,6 @@ __global__ void __launch_bounds__(fwd_threads, 1)
         }
         fence_barrier_init();
     }
-    __syncthreads();
-    if (tail->abort_flag != 0u) return; // a poisoned status block: nothing was allocated, every thread leaves
     if (warp == fwd_mma_warp) {
         tmem_alloc(smem_u32(&tail->tmem_base), fwd_tmem_columns);
         tmem_relinquish();
@@ -1196,6 +1194,10 @@ __global__ void __launch_bounds__(fwd_threads, 1)
             for (uint32_t i = 0; i < fz_candidate_maps; ++i) tma_prefetch_descriptor(&gemm_maps.candidates[i]);
         }
     }
+    // Everything up to here may run beside the end of the kernel before.
+    let_dependents_start();
+    wait_for_kernels_before();
+    if (threadIdx.x == 0) tail->abort_flag = status_poisoned(p.status) ? 1u : 0u;
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
@@ -1203,7 +1205,9 @@ __global__ void __launch_bounds__(fwd_threads, 1)
     wait_context const ctx{p.status, p.budget_ns, &tail->abort_flag};
 
     float* const norm_ring = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(tail) + fwd_tail_bytes);
-    if (warp < fwd_epilogue_warps) {
+    bool const poisoned = tail->abort_flag != 0u; // by an earlier kernel: nothing is scored
+    if (poisoned) {
+    } else if (warp < fwd_epilogue_warps) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(fwd_epilogue_registers));
         epilogue_role<prefixes_, fused_>(&cube_map, p, tail, store_base, norm_ring, norm_ring + fwd_norm_bytes(prefixes_) / 4, tmem_base, ctx, warp,
                                          lane);
@@ -1225,7 +1229,7 @@ __global__ void __launch_bounds__(fwd_threads, 1)
 
     tcgen05_fence_before();
     __syncthreads();
-    if (tail->abort_flag != 0u) {
+    if (!poisoned && tail->abort_flag != 0u) {
         // Something gave up. Give copies and UMMAs that are still in flight a bounded time to land before the tensor
         // memory goes back.
         uint64_t const start = global_timer_ns();
@@ -1241,7 +1245,7 @@ __global__ void __launch_bounds__(fwd_threads, 1)
 // ---- host side --------------------------------------------------------------------------------------------------
 template <int prefixes_, bool fused_>
 void launch_instance(CUtensorMap const& q_map, CUtensorMap const& c_map, CUtensorMap const& cube_map, fz_maps const& gemm_maps,
-                     fwd_params const& p, int blocks, cudaStream_t stream) {
+                     fwd_params const& p, int blocks, cudaStream_t stream, bool overlap) {
     // The attribute is per device; a process drives one GPU, but a second one costs only the repeat of a cheap call.
     static int prepared_device = -1;
     int device = 0;
@@ -1252,24 +1256,24 @@ void launch_instance(CUtensorMap const& q_map, CUtensorMap const& c_map, CUtenso
                 "raising the forward kernel's shared memory");
         prepared_device = device;
     }
-    forward_kernel<prefixes_, fused_><<<blocks, fwd_threads, fwd_shared_bytes(prefixes_, fused_), stream>>>(
-        q_map, c_map, cube_map, gemm_maps, p);
+    launch_dependent(overlap, forward_kernel<prefixes_, fused_>, blocks, fwd_threads, fwd_shared_bytes(prefixes_, fused_), stream, q_map, c_map,
+                     cube_map, gemm_maps, p);
 }
 
 template <bool fused_>
 void launch_for_count(uint32_t count, CUtensorMap const& q_map, CUtensorMap const& c_map, CUtensorMap const& cube_map,
-                      fz_maps const& gemm_maps, fwd_params const& p, int blocks, cudaStream_t stream) {
+                      fz_maps const& gemm_maps, fwd_params const& p, int blocks, cudaStream_t stream, bool overlap) {
     switch (count) {
-    case 1: launch_instance<1, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream); break;
-    case 2: launch_instance<2, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream); break;
-    case 3: launch_instance<3, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream); break;
-    case 4: launch_instance<4, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream); break;
-    case 5: launch_instance<5, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream); break;
-    case 6: launch_instance<6, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream); break;
+    case 1: launch_instance<1, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
+    case 2: launch_instance<2, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
+    case 3: launch_instance<3, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
+    case 4: launch_instance<4, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
+    case 5: launch_instance<5, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
+    case 6: launch_instance<6, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
     default:
         if constexpr (!fused_) {
-            if (count == 7) launch_instance<7, false>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream);
-            else launch_instance<8, false>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream);
+            if (count == 7) launch_instance<7, false>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap);
+            else launch_instance<8, false>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap);
         }
         break;
     }
@@ -1373,7 +1377,7 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
         cuuint32_t const box[3] = {fwd_warp_columns, 32, fwd_rolled_for(static_cast<int>(a.ladder.count)) ? 1u : a.ladder.count};
         CUtensorMap const cube_map =
             cached_map(a.gradient_cube_bf16, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
-        launch_for_count<false>(a.ladder.count, q_map, c_map, cube_map, gemm_maps, p, blocks, stream);
+        launch_for_count<false>(a.ladder.count, q_map, c_map, cube_map, gemm_maps, p, blocks, stream, !a.ordinary_launch);
     } else {
         p.gradient = a.query_gradient, p.gradient_scale = a.gradient_scale;
         for (uint32_t band = 0, begin = 0; band < a.ladder.count; begin = a.ladder.ends[band++])
@@ -1399,7 +1403,7 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
             gemm_maps.candidates[index] =
                 cached_operand_map(a.transposed_candidates, a.rows_c, a.hidden, fz_depth, channels <= a.hidden ? channels : 16u);
         }
-        launch_for_count<true>(a.ladder.count, q_map, c_map, store_map, gemm_maps, p, blocks, stream);
+        launch_for_count<true>(a.ladder.count, q_map, c_map, store_map, gemm_maps, p, blocks, stream, !a.ordinary_launch);
     }
     cudaError_t const error = cudaGetLastError();
     if (error != cudaSuccess) throw std::runtime_error(std::string("forward launch failed: ") + cudaGetErrorString(error));

@@ -18,6 +18,7 @@
 
 #include "api.h"
 #include "common.cuh"
+#include "launch.h"
 
 namespace sc {
 
@@ -41,14 +42,15 @@ ladder_t to_device(ladder_host const& host) {
 // edges are multiples of 16 channels, so a vector never straddles two bands.
 constexpr uint32_t norm_rows = 64, norm_warps = 32;
 __global__ void __launch_bounds__(norm_warps * 32)
-    prefix_norms_kernel(uint4 const* __restrict__ rows, uint4* __restrict__ copy, float* __restrict__ inverse_norms,
-                        float* __restrict__ tile_max, uint32_t row_count, uint32_t hidden, ladder_t ladder,
-                        float4* __restrict__ clear, size_t clear_vectors) {
+    prefix_norms_kernel(uint4 const* rows, uint4* copy, float* inverse_norms, float* tile_max, uint32_t row_count, uint32_t hidden, ladder_t ladder,
+                        float4* clear, size_t clear_vectors) {
     constexpr uint32_t each = norm_rows / norm_warps;
     __shared__ float largest[norm_warps][8];
     uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     uint32_t const first = blockIdx.x * norm_rows + warp * each;
     uint32_t const vectors = hidden / 8;
+    let_dependents_start();
+    wait_for_kernels_before();
     for (size_t v = blockIdx.x * blockDim.x + threadIdx.x; v < clear_vectors; v += static_cast<size_t>(gridDim.x) * blockDim.x)
         clear[v] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (blockIdx.x * norm_rows >= row_count) return; // a block that only clears
@@ -57,31 +59,41 @@ __global__ void __launch_bounds__(norm_warps * 32)
     for (uint32_t r = 0; r < each; ++r)
 #pragma unroll
         for (int band = 0; band < 8; ++band) sums[r][band] = 0.0f;
-    for (uint32_t v = lane; v < vectors; v += 32) {
-        uint4 packed[each];
+    // Three vectors of both rows are under way before the first is used (stores to `copy` stand between the trips).
+    constexpr uint32_t ahead = 3;
+    for (uint32_t base = lane; base < vectors; base += 32 * ahead) {
+        uint4 packed[ahead][each];
 #pragma unroll
-        for (uint32_t r = 0; r < each; ++r) {
-            packed[r] = make_uint4(0u, 0u, 0u, 0u);
-            if (first + r < row_count && SC_IN_BOUNDS(static_cast<size_t>(first + r) * vectors + v, static_cast<size_t>(row_count) * vectors))
-                packed[r] = rows[static_cast<size_t>(first + r) * vectors + v];
-        }
-        uint32_t const channel = v * 8;
+        for (uint32_t a = 0; a < ahead; ++a)
 #pragma unroll
-        for (uint32_t r = 0; r < each; ++r) {
-            if (copy != nullptr && first + r < row_count &&
-                SC_IN_BOUNDS(static_cast<size_t>(first + r) * vectors + v, static_cast<size_t>(row_count) * vectors))
-                copy[static_cast<size_t>(first + r) * vectors + v] = packed[r];
-            uint32_t const words[4] = {packed[r].x, packed[r].y, packed[r].z, packed[r].w};
-            float square = 0;
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                float const lo = __uint_as_float(words[w] << 16), hi = __uint_as_float(words[w] & 0xFFFF0000u);
-                square = fmaf(lo, lo, square);
-                square = fmaf(hi, hi, square);
+            for (uint32_t r = 0; r < each; ++r) {
+                uint32_t const v = base + 32 * a;
+                packed[a][r] = make_uint4(0u, 0u, 0u, 0u);
+                if (v < vectors && first + r < row_count &&
+                    SC_IN_BOUNDS(static_cast<size_t>(first + r) * vectors + v, static_cast<size_t>(row_count) * vectors))
+                    packed[a][r] = rows[static_cast<size_t>(first + r) * vectors + v];
             }
 #pragma unroll
-            for (int band = 0; band < 8; ++band)
-                if (band < ladder.count && channel >= ladder.begin(band) && channel < ladder.ends[band]) sums[r][band] += square;
+        for (uint32_t a = 0; a < ahead; ++a) {
+            uint32_t const v = base + 32 * a, channel = v * 8;
+            if (v >= vectors) break;
+#pragma unroll
+            for (uint32_t r = 0; r < each; ++r) {
+                if (copy != nullptr && first + r < row_count &&
+                    SC_IN_BOUNDS(static_cast<size_t>(first + r) * vectors + v, static_cast<size_t>(row_count) * vectors))
+                    copy[static_cast<size_t>(first + r) * vectors + v] = packed[a][r];
+                uint32_t const words[4] = {packed[a][r].x, packed[a][r].y, packed[a][r].z, packed[a][r].w};
+                float square = 0;
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    float const lo = __uint_as_float(words[w] << 16), hi = __uint_as_float(words[w] & 0xFFFF0000u);
+                    square = fmaf(lo, lo, square);
+                    square = fmaf(hi, hi, square);
+                }
+#pragma unroll
+                for (int band = 0; band < 8; ++band)
+                    if (band < ladder.count && channel >= ladder.begin(band) && channel < ladder.ends[band]) sums[r][band] += square;
+            }
         }
     }
     float running[each];
@@ -118,8 +130,10 @@ __global__ void __launch_bounds__(norm_warps * 32)
 }
 
 __global__ void __launch_bounds__(256)
-    transpose_kernel(__nv_bfloat16 const* __restrict__ in, __nv_bfloat16* __restrict__ out, uint32_t rows, uint32_t hidden) {
+    transpose_kernel(__nv_bfloat16 const* in, __nv_bfloat16* out, uint32_t rows, uint32_t hidden) {
     __shared__ __nv_bfloat16 tile[32][33];
+    let_dependents_start();
+    wait_for_kernels_before();
     uint32_t const column = blockIdx.x * 32 + threadIdx.x;
     for (uint32_t r = threadIdx.y; r < 32; r += 8) {
         uint32_t const row = blockIdx.y * 32 + r;
@@ -146,6 +160,8 @@ __device__ __forceinline__ void copy_vectors(uint4 const* src, uint4* dst, size_
 }
 
 __global__ void __launch_bounds__(256) pull_kernel(pull_request request) {
+    let_dependents_start();
+    wait_for_kernels_before();
     size_t const thread = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     size_t const threads = static_cast<size_t>(gridDim.x) * blockDim.x;
     for (int part = 0; part < 2; ++part)
@@ -169,7 +185,7 @@ template <bool vector_> __device__ __forceinline__ float4 load_rows(float const*
 }
 template <bool vector_>
 __global__ void __launch_bounds__(fold_warps * 32)
-    fold_partials_kernel(float const* __restrict__ partials, float* __restrict__ accumulators, uint32_t rows, uint32_t slots,
+    fold_partials_kernel(float const* partials, float* accumulators, uint32_t rows, uint32_t slots,
                          uint32_t quantities) {
     __shared__ float4 sums[fold_warps][32];
     uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -177,6 +193,8 @@ __global__ void __launch_bounds__(fold_warps * 32)
     uint32_t const quantity = blockIdx.y;
     float4 total = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     size_t const stride = static_cast<size_t>(quantities) * rows;
+    let_dependents_start();
+    wait_for_kernels_before();
     float const* const first = partials + static_cast<size_t>(quantity) * rows;
 #pragma unroll 4
     for (uint32_t slot = warp; slot < slots; slot += fold_warps)
@@ -215,7 +233,7 @@ constexpr uint32_t finish_warps = 8;
 // A fixed reduction tree, so the bits do not depend on anything but the inputs. All quantities go in one pass: a thread has
 // a 16-byte load of every quantity in flight at once, and the block meets twice instead of twice per quantity.
 template <uint32_t prefixes_>
-__device__ __forceinline__ void sum_summands(float const* __restrict__ accumulators, float* __restrict__ summands, uint32_t rows) {
+__device__ __forceinline__ void sum_summands(float const* accumulators, float* summands, uint32_t rows) {
     constexpr uint32_t quantities = 2 + prefixes_, prefixes = prefixes_, warps = finish_warps;
     __shared__ float scratch[quantities][warps];
     __shared__ float totals[quantities];
@@ -261,9 +279,10 @@ __device__ __forceinline__ void sum_summands(float const* __restrict__ accumulat
 
 template <uint32_t prefixes_>
 __global__ void __launch_bounds__(finish_warps * 32)
-    finish_kernel(uint4 const* __restrict__ queries, float const* __restrict__ inverse_norms,
-                  float const* __restrict__ accumulators, float const* __restrict__ query_gradient,
-                  uint4* __restrict__ gradient_out, float* __restrict__ summands, uint32_t rows, uint32_t hidden, ladder_t ladder) {
+    finish_kernel(uint4 const* queries, float const* inverse_norms, float const* accumulators, float const* query_gradient,
+                  uint4* gradient_out, float* summands, uint32_t rows, uint32_t hidden, ladder_t ladder) {
+    let_dependents_start();
+    wait_for_kernels_before();
     if (blockIdx.x == 0) {
         sum_summands<prefixes_>(accumulators, summands, rows);
         return;
@@ -287,26 +306,36 @@ __global__ void __launch_bounds__(finish_warps * 32)
     }
     __syncwarp();
     uint32_t const vectors = hidden / 8;
-#pragma unroll 3
-    for (uint32_t v = lane; v < vectors; v += 32) {
-        uint32_t const channel = v * 8;
-        if (!SC_IN_BOUNDS(static_cast<size_t>(row) * hidden + channel + 7, static_cast<size_t>(rows) * hidden)) continue;
-        uint4 const packed = queries[static_cast<size_t>(row) * vectors + v];
-        float4 const g0 = *reinterpret_cast<float4 const*>(query_gradient + static_cast<size_t>(row) * hidden + channel);
-        float4 const g1 = *reinterpret_cast<float4 const*>(query_gradient + static_cast<size_t>(row) * hidden + channel + 4);
-        uint32_t band = 0;
+    constexpr uint32_t ahead = 3; // vectors under way before the first is used
+    for (uint32_t base = lane; base < vectors; base += 32 * ahead) {
+        uint4 packed[ahead];
+        float4 g0[ahead], g1[ahead];
 #pragma unroll
-        for (uint32_t b = 0; b + 1 < prefixes_; ++b) band += channel >= ladder.ends[b] ? 1u : 0u;
-        float const fold = folds[warp][band];
-        uint32_t const words[4] = {packed.x, packed.y, packed.z, packed.w};
-        float const g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-        uint32_t out[4];
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            float const lo = __uint_as_float(words[w] << 16), hi = __uint_as_float(words[w] & 0xFFFF0000u);
-            out[w] = pack_bf16x2(fmaf(-fold, lo, g[2 * w]), fmaf(-fold, hi, g[2 * w + 1]));
+        for (uint32_t a = 0; a < ahead; ++a) {
+            uint32_t const v = base + 32 * a, channel = v * 8;
+            if (v >= vectors || !SC_IN_BOUNDS(static_cast<size_t>(row) * hidden + channel + 7, static_cast<size_t>(rows) * hidden)) continue;
+            packed[a] = queries[static_cast<size_t>(row) * vectors + v];
+            g0[a] = *reinterpret_cast<float4 const*>(query_gradient + static_cast<size_t>(row) * hidden + channel);
+            g1[a] = *reinterpret_cast<float4 const*>(query_gradient + static_cast<size_t>(row) * hidden + channel + 4);
         }
-        gradient_out[static_cast<size_t>(row) * vectors + v] = make_uint4(out[0], out[1], out[2], out[3]);
+#pragma unroll
+        for (uint32_t a = 0; a < ahead; ++a) {
+            uint32_t const v = base + 32 * a, channel = v * 8;
+            if (v >= vectors || !SC_IN_BOUNDS(static_cast<size_t>(row) * hidden + channel + 7, static_cast<size_t>(rows) * hidden)) continue;
+            uint32_t band = 0;
+#pragma unroll
+            for (uint32_t b = 0; b + 1 < prefixes_; ++b) band += channel >= ladder.ends[b] ? 1u : 0u;
+            float const fold = folds[warp][band];
+            uint32_t const words[4] = {packed[a].x, packed[a].y, packed[a].z, packed[a].w};
+            float const g[8] = {g0[a].x, g0[a].y, g0[a].z, g0[a].w, g1[a].x, g1[a].y, g1[a].z, g1[a].w};
+            uint32_t out[4];
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                float const lo = __uint_as_float(words[w] << 16), hi = __uint_as_float(words[w] & 0xFFFF0000u);
+                out[w] = pack_bf16x2(fmaf(-fold, lo, g[2 * w]), fmaf(-fold, hi, g[2 * w + 1]));
+            }
+            gradient_out[static_cast<size_t>(row) * vectors + v] = make_uint4(out[0], out[1], out[2], out[3]);
+        }
     }
 }
 
@@ -374,16 +403,16 @@ void launch_prefix_norms(void const* rows_bf16, void* copy_bf16, float* inverse_
     // A few rows make a few blocks, which would clear a wide gradient slowly: up to one block per multiprocessor helps them.
     size_t const clearing = (clear_floats / 4 + norm_warps * 32 - 1) / (norm_warps * 32);
     int const blocks = std::max(blocks_of(rows, norm_rows), static_cast<int>(std::min<size_t>(clearing, 148)));
-    prefix_norms_kernel<<<blocks, norm_warps * 32, 0, stream>>>(
-        static_cast<uint4 const*>(rows_bf16), static_cast<uint4*>(copy_bf16), inverse_norms, tile_max, rows, hidden, to_device(ladder),
+    launch_dependent(
+        true, prefix_norms_kernel, blocks, norm_warps * 32, 0, stream, static_cast<uint4 const*>(rows_bf16), static_cast<uint4*>(copy_bf16), inverse_norms, tile_max, rows, hidden, to_device(ladder),
         reinterpret_cast<float4*>(clear), clear_floats / 4);
     check_launch("prefix_norms");
 }
 
 void launch_transpose(void const* rows_bf16, void* transposed_bf16, uint32_t rows, uint32_t hidden, cudaStream_t stream) {
     dim3 const grid((hidden + 31) / 32, (rows + 31) / 32), block(32, 8);
-    transpose_kernel<<<grid, block, 0, stream>>>(static_cast<__nv_bfloat16 const*>(rows_bf16),
-                                                 static_cast<__nv_bfloat16*>(transposed_bf16), rows, hidden);
+    launch_dependent(true, transpose_kernel, grid, block, 0, stream, static_cast<__nv_bfloat16 const*>(rows_bf16),
+                     static_cast<__nv_bfloat16*>(transposed_bf16), rows, hidden);
     check_launch("transpose");
 }
 
@@ -393,7 +422,7 @@ void launch_pull(void const* src0, void* dst0, size_t bytes0, void const* src1, 
     pull_request request{};
     request.src[0] = src0, request.dst[0] = dst0, request.bytes[0] = bytes0;
     request.src[1] = src1, request.dst[1] = dst1, request.bytes[1] = bytes1;
-    pull_kernel<<<blocks < 1 ? 1 : blocks, 256, 0, stream>>>(request);
+    launch_dependent(true, pull_kernel, blocks < 1 ? 1 : blocks, 256, 0, stream, request);
     check_launch("pull");
 }
 
@@ -402,8 +431,8 @@ void launch_fold_partials(float const* partials, float* row_accumulators, uint32
     bool const vectors = rows % 4 == 0 && reinterpret_cast<uintptr_t>(partials) % 16 == 0 &&
                          reinterpret_cast<uintptr_t>(row_accumulators) % 16 == 0;
     dim3 const grid(blocks_of(rows, 128), quantities);
-    if (vectors) fold_partials_kernel<true><<<grid, fold_warps * 32, 0, stream>>>(partials, row_accumulators, rows, slots, quantities);
-    else fold_partials_kernel<false><<<grid, fold_warps * 32, 0, stream>>>(partials, row_accumulators, rows, slots, quantities);
+    launch_dependent(true, vectors ? fold_partials_kernel<true> : fold_partials_kernel<false>, grid, fold_warps * 32, 0, stream, partials,
+                     row_accumulators, rows, slots, quantities);
     check_launch("fold_partials");
 }
 
@@ -413,9 +442,9 @@ void launch_finish(void const* queries_bf16, float const* inverse_norms, float c
     if (rows % 4 || hidden % 8 || reinterpret_cast<uintptr_t>(row_accumulators) % 16)
         throw std::runtime_error("finish: rows must be a multiple of 4, hidden of 8 and the accumulators 16-byte aligned");
     auto launch = [&](auto kernel) {
-        kernel<<<1 + blocks_of(rows, finish_warps), finish_warps * 32, 0, stream>>>(
-            static_cast<uint4 const*>(queries_bf16), inverse_norms, row_accumulators, query_gradient,
-            static_cast<uint4*>(gradient_out_bf16), summands, rows, hidden, to_device(ladder));
+        launch_dependent(true, kernel, 1 + blocks_of(rows, finish_warps), finish_warps * 32, 0, stream,
+                         static_cast<uint4 const*>(queries_bf16), inverse_norms, row_accumulators, query_gradient,
+                         static_cast<uint4*>(gradient_out_bf16), summands, rows, hidden, to_device(ladder));
     };
     switch (ladder.count) {
     case 1: launch(finish_kernel<1>); break;

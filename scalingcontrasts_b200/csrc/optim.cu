@@ -18,6 +18,7 @@
 
 #include "api.h"
 #include "common.cuh"
+#include "launch.h"
 
 namespace sc {
 
@@ -50,6 +51,8 @@ __global__ void __launch_bounds__(256) adamw_kernel(const adamw_table table, con
     uint32_t index = 0;
     while (index + 1 < table.used && blockIdx.x >= table.first_block[index + 1]) ++index;
     adamw_tensor const t = table.tensors[index];
+    let_dependents_start();
+    wait_for_kernels_before();
     size_t const begin = static_cast<size_t>(blockIdx.x - table.first_block[index]) * adamw_block_elements;
     if (t.is_bf16 && t.vectorised) {
         size_t const at = begin + threadIdx.x * 8u;
@@ -128,7 +131,7 @@ void launch_adamw(adamw_tensor const* tensors, uint32_t count, float lr, float b
             ++table.used;
         }
         table.first_block[table.used] = blocks;
-        adamw_kernel<<<blocks, 256, 0, stream>>>(table, c);
+        launch_dependent(true, adamw_kernel, blocks, 256, 0, stream, table, c);
         cudaError_t const error = cudaGetLastError();
         if (error != cudaSuccess) throw std::runtime_error(std::string("adamw launch failed: ") + cudaGetErrorString(error));
         note_launch();

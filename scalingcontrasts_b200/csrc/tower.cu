@@ -13,6 +13,7 @@
 
 #include "api.h"
 #include "common.cuh"
+#include "launch.h"
 
 namespace sc {
 
@@ -57,10 +58,12 @@ __device__ __forceinline__ uint4 pack8(float const (&v)[8]) {
     return make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
 }
 
-__global__ void __launch_bounds__(256) gelu_forward_kernel(uint4 const* __restrict__ z, uint4* __restrict__ h, size_t vectors) {
+__global__ void __launch_bounds__(256) gelu_forward_kernel(uint4 const* z, uint4* h, size_t vectors) {
     // Four vectors per thread and trip, all loads issued before the first is used: the pass is bound by memory, and the
     // arithmetic of one vector would otherwise stand between consecutive loads.
     constexpr int batch = 4;
+    let_dependents_start();
+    wait_for_kernels_before();
     size_t const stride = static_cast<size_t>(gridDim.x) * blockDim.x;
     for (size_t index = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; index < vectors; index += batch * stride) {
         uint4 loaded[batch];
@@ -83,9 +86,10 @@ __global__ void __launch_bounds__(256) gelu_forward_kernel(uint4 const* __restri
 // and keeps eight column sums; the eight row groups are then added in shared memory in a fixed order.
 template <bool with_activation_>
 __global__ void __launch_bounds__(256)
-    column_partials_kernel(uint4 const* __restrict__ upstream, uint4 const* __restrict__ z, uint4* __restrict__ out,
-                           float* __restrict__ partials, uint32_t rows, uint32_t columns) {
+    column_partials_kernel(uint4 const* upstream, uint4 const* z, uint4* out, float* partials, uint32_t rows, uint32_t columns) {
     __shared__ float sums[8][tower_columns_per_block];
+    let_dependents_start();
+    wait_for_kernels_before();
     uint32_t const lane = threadIdx.x % 32, group = threadIdx.x / 32;
     uint32_t const column = blockIdx.x * tower_columns_per_block + lane * 8;
     uint32_t const first_row = blockIdx.y * tower_rows_per_block;
@@ -143,9 +147,10 @@ __global__ void __launch_bounds__(256)
 // the eight parts are then added in part order, so the sum's order is fixed whatever the scheduling (and eight loads per
 // column are in flight instead of one dependent chain).
 __global__ void __launch_bounds__(256)
-    fold_column_partials_kernel(float const* __restrict__ partials, float* __restrict__ out, uint32_t blocks, uint32_t columns,
-                                void* __restrict__ out_bf16) {
+    fold_column_partials_kernel(float const* partials, float* out, uint32_t blocks, uint32_t columns, void* out_bf16) {
     __shared__ float parts[8][32];
+    let_dependents_start();
+    wait_for_kernels_before();
     uint32_t const lane = threadIdx.x % 32, part = threadIdx.x / 32;
     uint32_t const column = blockIdx.x * 32 + lane;
     float total = 0;
@@ -182,7 +187,8 @@ void launch_gelu_forward(void const* z_bf16, void* h_bf16, size_t scalars, int m
     size_t const cap = static_cast<size_t>(multiprocessors > 0 ? multiprocessors : 148) * 16;
     if (blocks > cap) blocks = cap;
     if (blocks == 0) return;
-    gelu_forward_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(static_cast<uint4 const*>(z_bf16), static_cast<uint4*>(h_bf16), vectors);
+    launch_dependent(true, gelu_forward_kernel, static_cast<uint32_t>(blocks), 256, 0, stream, static_cast<uint4 const*>(z_bf16),
+                     static_cast<uint4*>(h_bf16), vectors);
     check_launch("gelu_forward");
 }
 
@@ -190,10 +196,10 @@ void launch_gelu_backward_bias(void const* upstream_bf16, void const* z_bf16, vo
                                uint32_t rows, uint32_t columns, cudaStream_t stream) {
     check_matrix(rows, columns, "gelu_backward_bias");
     dim3 const grid((columns + tower_columns_per_block - 1) / tower_columns_per_block, tower_partial_blocks(rows));
-    column_partials_kernel<true><<<grid, 256, 0, stream>>>(static_cast<uint4 const*>(upstream_bf16), static_cast<uint4 const*>(z_bf16),
-                                                            static_cast<uint4*>(dz_bf16), partials, rows, columns);
+    launch_dependent(true, column_partials_kernel<true>, grid, 256, 0, stream, static_cast<uint4 const*>(upstream_bf16),
+                     static_cast<uint4 const*>(z_bf16), static_cast<uint4*>(dz_bf16), partials, rows, columns);
     check_launch("gelu_backward_bias");
-    fold_column_partials_kernel<<<(columns + 31) / 32, 256, 0, stream>>>(partials, nullptr, grid.y, columns, bias_grad_bf16);
+    launch_dependent(true, fold_column_partials_kernel, (columns + 31) / 32, 256, 0, stream, partials, nullptr, grid.y, columns, bias_grad_bf16);
     check_launch("fold_column_partials");
 }
 
@@ -201,9 +207,10 @@ void launch_column_sums(void const* matrix_bf16, float* partials, void* sums_bf1
                         cudaStream_t stream) {
     check_matrix(rows, columns, "column_sums");
     dim3 const grid((columns + tower_columns_per_block - 1) / tower_columns_per_block, tower_partial_blocks(rows));
-    column_partials_kernel<false><<<grid, 256, 0, stream>>>(static_cast<uint4 const*>(matrix_bf16), nullptr, nullptr, partials, rows, columns);
+    launch_dependent(true, column_partials_kernel<false>, grid, 256, 0, stream, static_cast<uint4 const*>(matrix_bf16), nullptr, nullptr,
+                     partials, rows, columns);
     check_launch("column_sums");
-    fold_column_partials_kernel<<<(columns + 31) / 32, 256, 0, stream>>>(partials, nullptr, grid.y, columns, sums_bf16);
+    launch_dependent(true, fold_column_partials_kernel, (columns + 31) / 32, 256, 0, stream, partials, nullptr, grid.y, columns, sums_bf16);
     check_launch("fold_column_partials");
 }
 
