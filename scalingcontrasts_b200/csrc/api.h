@@ -70,10 +70,16 @@ void launch_expect_arrivals(control_view const& control, uint32_t arrivals, cuda
 void preload_collective_kernels();
 
 // -------- small loss kernels (loss_small.cu) ---------------------------------------------------------------------
-// `clear` (optional): `clear_floats` words, whole 16-byte vectors, that the same launch sets to zero.
+// `clear` (optional): `clear_floats` words, whole 16-byte vectors, that the same launch sets to zero. `learned` (optional): the
+// learned log scale and bias on the device, from which the launch makes the two scalars that the forward kernel takes.
+struct learned_scalars {
+    float const* log_scale;
+    float const* bias;
+    float* out; // {exp(log scale), bias}, or null
+};
 void launch_prefix_norms(void const* rows_bf16, void* copy_bf16, float* inverse_norms, float* tile_max, uint32_t rows,
                          uint32_t hidden, ladder_host const& ladder, cudaStream_t stream,
-                         float* clear = nullptr, size_t clear_floats = 0);
+                         float* clear = nullptr, size_t clear_floats = 0, learned_scalars learned = {});
 void launch_transpose(void const* rows_bf16, void* transposed_bf16, uint32_t rows, uint32_t hidden, cudaStream_t stream);
 void launch_pull(void const* src0, void* dst0, size_t bytes0, void const* src1, void* dst1, size_t bytes1, int blocks,
                  cudaStream_t stream);
@@ -82,6 +88,12 @@ void launch_fold_partials(float const* partials, float* row_accumulators, uint32
 void launch_finish(void const* queries_bf16, float const* inverse_norms, float const* row_accumulators,
                    float const* query_gradient, void* gradient_out_bf16, float* summands, uint32_t rows, uint32_t hidden,
                    ladder_host const& ladder, cudaStream_t stream);
+// kept[0..count) = summands, *loss = summands[0].
+void launch_keep_summands(float const* summands, float* kept, float* loss, uint32_t count, cudaStream_t stream);
+// out = gradient * bfloat16(*upstream) rounded to bfloat16 (stored as such or as float32), the scalar gradients summands[2] and
+// summands[1] times *upstream.
+void launch_scale_gradients(void const* gradient_bf16, float const* upstream, float const* summands, void* out, bool out_f32,
+                            float* scale_gradient, float* bias_gradient, size_t scalars, cudaStream_t stream);
 void launch_keyed_embeddings(void* rows_bf16, uint32_t rows, uint32_t hidden, uint64_t salt, float scale,
                              cudaStream_t stream);
 void launch_keyed_integers(float* out, size_t scalars, size_t first, uint32_t members, uint32_t member,

@@ -139,14 +139,15 @@ struct loss_plan {
     // cleared here, and every block adds to both, whatever came before it: what a launch does never hangs on what this object
     // remembers, so blocks captured in a graph and replayed any number of times sum up like blocks scored one by one. Where the
     // queries' norms are taken here too (`inverse_norms` not null), one launch does both: 52.1 -> 46.9 us for a step of 128 rows.
-    void begin_step(uint64_t queries, uint64_t inverse_norms, uint64_t tile_max, uint64_t stream_handle) {
+    // `cleared`: the launch that took them just before has cleared both already.
+    void begin_step(uint64_t queries, uint64_t inverse_norms, uint64_t tile_max, uint64_t stream_handle, bool cleared) {
         if (pending) throw std::runtime_error("LossPlan: begin_step with a backward still pending (join() was not called)");
         scored = 0;
         size_t const floats = static_cast<size_t>(rows_q) * (hidden + quantities);
         if (inverse_norms)
             sc::launch_prefix_norms(pointer<void>(queries), nullptr, pointer<float>(inverse_norms), pointer<float>(tile_max), rows_q,
                                     hidden, ladder, stream_of(stream_handle), pointer<float>(query_gradient), floats);
-        else runtime_check(cudaMemsetAsync(pointer<void>(query_gradient), 0, floats * 4, stream_of(stream_handle)), "cudaMemsetAsync");
+        else if (!cleared) runtime_check(cudaMemsetAsync(pointer<void>(query_gradient), 0, floats * 4, stream_of(stream_handle)), "cudaMemsetAsync");
     }
 
     void launch_pending_on_side() {
@@ -328,9 +329,21 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     });
 
     m.def("prefix_norms", [](uint64_t rows, uint64_t copy, uint64_t inverse_norms, uint64_t tile_max, uint32_t row_count,
-                             uint32_t hidden, std::vector<uint32_t> const& ends, uint64_t stream) {
+                             uint32_t hidden, std::vector<uint32_t> const& ends, uint64_t stream, uint64_t clear, uint64_t clear_floats,
+                             uint64_t log_scale, uint64_t bias, uint64_t scalars) {
         sc::launch_prefix_norms(pointer<void>(rows), pointer<void>(copy), pointer<float>(inverse_norms), pointer<float>(tile_max),
-                                row_count, hidden, ladder_of(ends), stream_of(stream));
+                                row_count, hidden, ladder_of(ends), stream_of(stream), pointer<float>(clear), clear_floats,
+                                sc::learned_scalars{pointer<float>(log_scale), pointer<float>(bias), pointer<float>(scalars)});
+    }, py::arg("rows"), py::arg("copy"), py::arg("inverse_norms"), py::arg("tile_max"), py::arg("row_count"), py::arg("hidden"),
+       py::arg("ends"), py::arg("stream"), py::arg("clear") = 0, py::arg("clear_floats") = 0, py::arg("log_scale") = 0,
+       py::arg("bias") = 0, py::arg("scalars") = 0);
+    m.def("keep_summands", [](uint64_t summands, uint64_t kept, uint64_t loss, uint32_t count, uint64_t stream) {
+        sc::launch_keep_summands(pointer<float>(summands), pointer<float>(kept), pointer<float>(loss), count, stream_of(stream));
+    });
+    m.def("scale_gradients", [](uint64_t gradient, uint64_t upstream, uint64_t summands, uint64_t out, bool out_f32,
+                                uint64_t scale_gradient, uint64_t bias_gradient, uint64_t scalars, uint64_t stream) {
+        sc::launch_scale_gradients(pointer<void>(gradient), pointer<float>(upstream), pointer<float>(summands), pointer<void>(out),
+                                   out_f32, pointer<float>(scale_gradient), pointer<float>(bias_gradient), scalars, stream_of(stream));
     });
     m.def("transpose", [](uint64_t rows, uint64_t out, uint32_t row_count, uint32_t hidden, uint64_t stream) {
         sc::launch_transpose(pointer<void>(rows), pointer<void>(out), row_count, hidden, stream_of(stream));
@@ -374,7 +387,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def_readwrite("transpose_candidates", &loss_plan::transpose_candidates)
         .def_readonly("overlap", &loss_plan::overlap)
         .def("enable_overlap", &loss_plan::enable_overlap, py::arg("second_cube"), py::arg("backward_multiprocessors"))
-        .def("begin_step", &loss_plan::begin_step, py::arg("queries"), py::arg("inverse_norms"), py::arg("tile_max"), py::arg("stream"))
+        .def("begin_step", &loss_plan::begin_step, py::arg("queries"), py::arg("inverse_norms"), py::arg("tile_max"), py::arg("stream"),
+             py::arg("cleared") = false)
         .def("join", &loss_plan::join, py::arg("stream"))
         .def("score", &loss_plan::score);
     m.attr("BOUNDS_BUILD") = sc::bounds_build();

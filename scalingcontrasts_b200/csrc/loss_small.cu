@@ -43,7 +43,7 @@ ladder_t to_device(ladder_host const& host) {
 constexpr uint32_t norm_rows = 64, norm_warps = 32;
 __global__ void __launch_bounds__(norm_warps * 32)
     prefix_norms_kernel(uint4 const* rows, uint4* copy, float* inverse_norms, float* tile_max, uint32_t row_count, uint32_t hidden, ladder_t ladder,
-                        float4* clear, size_t clear_vectors) {
+                        float4* clear, size_t clear_vectors, learned_scalars learned) {
     constexpr uint32_t each = norm_rows / norm_warps;
     __shared__ float largest[norm_warps][8];
     uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -53,6 +53,10 @@ __global__ void __launch_bounds__(norm_warps * 32)
     wait_for_kernels_before();
     for (size_t v = blockIdx.x * blockDim.x + threadIdx.x; v < clear_vectors; v += static_cast<size_t>(gridDim.x) * blockDim.x)
         clear[v] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (learned.out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
+        learned.out[0] = expf(*learned.log_scale);
+        learned.out[1] = *learned.bias;
+    }
     if (blockIdx.x * norm_rows >= row_count) return; // a block that only clears
     float sums[each][8];
 #pragma unroll
@@ -339,6 +343,44 @@ __global__ void __launch_bounds__(finish_warps * 32)
     }
 }
 
+// A step's summands for whoever differentiates the loss later (the span they were summed in is rewritten by the next step),
+// and the loss by itself.
+__global__ void keep_summands_kernel(float const* summands, float* kept, float* loss, uint32_t count) {
+    let_dependents_start();
+    wait_for_kernels_before();
+    if (threadIdx.x < count) kept[threadIdx.x] = summands[threadIdx.x];
+    if (threadIdx.x == 0) *loss = summands[0];
+}
+
+// The row gradients and the two scalar gradients times the upstream gradient (a device scalar), in one pass. The row gradients
+// are bfloat16 and so is their product with the upstream gradient's nearest bfloat16; it leaves in the embeddings' type.
+template <typename out_t>
+__global__ void __launch_bounds__(256)
+    scale_gradients_kernel(uint4 const* gradient, float const* upstream, float const* summands, out_t* out, float* scale_gradient,
+                           float* bias_gradient, size_t vectors) {
+    let_dependents_start();
+    wait_for_kernels_before();
+    float const whole = *upstream, factor = __bfloat162float(__float2bfloat16(whole));
+    if (blockIdx.x == 0 && threadIdx.x == 0) *scale_gradient = summands[2] * whole, *bias_gradient = summands[1] * whole;
+    for (size_t v = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; v < vectors; v += static_cast<size_t>(gridDim.x) * blockDim.x) {
+        uint4 const packed = gradient[v];
+        uint32_t const words[4] = {packed.x, packed.y, packed.z, packed.w};
+        uint32_t scaled[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+            scaled[w] = pack_bf16x2(__uint_as_float(words[w] << 16) * factor, __uint_as_float(words[w] & 0xFFFF0000u) * factor);
+        if constexpr (sizeof(out_t) == 2) {
+            reinterpret_cast<uint4*>(out)[v] = make_uint4(scaled[0], scaled[1], scaled[2], scaled[3]);
+        } else {
+            float4* const into = reinterpret_cast<float4*>(out) + 2 * v;
+            into[0] = make_float4(__uint_as_float(scaled[0] << 16), __uint_as_float(scaled[0] & 0xFFFF0000u),
+                                  __uint_as_float(scaled[1] << 16), __uint_as_float(scaled[1] & 0xFFFF0000u));
+            into[1] = make_float4(__uint_as_float(scaled[2] << 16), __uint_as_float(scaled[2] & 0xFFFF0000u),
+                                  __uint_as_float(scaled[3] << 16), __uint_as_float(scaled[3] & 0xFFFF0000u));
+        }
+    }
+}
+
 __device__ __forceinline__ uint64_t splitmix64(uint64_t value) {
     value = (value ^ (value >> 30)) * 0xBF58476D1CE4E5B9ull;
     value = (value ^ (value >> 27)) * 0x94D049BB133111EBull;
@@ -395,7 +437,8 @@ bool bounds_build() { return SC_BOUNDS != 0; }
 SC_DEFINE_BOUNDS_READER(bounds_record_small)
 
 void launch_prefix_norms(void const* rows_bf16, void* copy_bf16, float* inverse_norms, float* tile_max, uint32_t rows,
-                         uint32_t hidden, ladder_host const& ladder, cudaStream_t stream, float* clear, size_t clear_floats) {
+                         uint32_t hidden, ladder_host const& ladder, cudaStream_t stream, float* clear, size_t clear_floats,
+                         learned_scalars learned) {
     if (hidden % 8) throw std::runtime_error("prefix_norms: hidden must be a multiple of 8");
     if (tile_max != nullptr && rows % norm_rows) throw std::runtime_error("prefix_norms: rows must be a multiple of 64 for tile maxima");
     if (clear_floats % 4 || reinterpret_cast<uintptr_t>(clear) % 16)
@@ -405,7 +448,7 @@ void launch_prefix_norms(void const* rows_bf16, void* copy_bf16, float* inverse_
     int const blocks = std::max(blocks_of(rows, norm_rows), static_cast<int>(std::min<size_t>(clearing, 148)));
     launch_dependent(
         true, prefix_norms_kernel, blocks, norm_warps * 32, 0, stream, static_cast<uint4 const*>(rows_bf16), static_cast<uint4*>(copy_bf16), inverse_norms, tile_max, rows, hidden, to_device(ladder),
-        reinterpret_cast<float4*>(clear), clear_floats / 4);
+        reinterpret_cast<float4*>(clear), clear_floats / 4, learned);
     check_launch("prefix_norms");
 }
 
@@ -458,6 +501,27 @@ void launch_finish(void const* queries_bf16, float const* inverse_norms, float c
     default: throw std::runtime_error("finish: a ladder holds one to eight prefixes");
     }
     check_launch("finish");
+}
+
+void launch_keep_summands(float const* summands, float* kept, float* loss, uint32_t count, cudaStream_t stream) {
+    if (count == 0 || count > 32) throw std::runtime_error("keep_summands: one to 32 summands");
+    launch_dependent(true, keep_summands_kernel, 1, 32, 0, stream, summands, kept, loss, count);
+    check_launch("keep_summands");
+}
+
+void launch_scale_gradients(void const* gradient_bf16, float const* upstream, float const* summands, void* out, bool out_f32,
+                            float* scale_gradient, float* bias_gradient, size_t scalars, cudaStream_t stream) {
+    if (scalars % 8 || reinterpret_cast<uintptr_t>(gradient_bf16) % 16 || reinterpret_cast<uintptr_t>(out) % 16)
+        throw std::runtime_error("scale_gradients: whole, aligned vectors of eight");
+    uint32_t const blocks = static_cast<uint32_t>(std::min<size_t>((scalars / 8 + 255) / 256, 148 * 8));
+    uint4 const* const gradient = static_cast<uint4 const*>(gradient_bf16);
+    if (out_f32)
+        launch_dependent(true, scale_gradients_kernel<float>, blocks < 1 ? 1 : blocks, 256, 0, stream, gradient, upstream, summands,
+                         static_cast<float*>(out), scale_gradient, bias_gradient, scalars / 8);
+    else
+        launch_dependent(true, scale_gradients_kernel<__nv_bfloat16>, blocks < 1 ? 1 : blocks, 256, 0, stream, gradient, upstream,
+                         summands, static_cast<__nv_bfloat16*>(out), scale_gradient, bias_gradient, scalars / 8);
+    check_launch("scale_gradients");
 }
 
 void launch_keyed_embeddings(void* rows_bf16, uint32_t rows, uint32_t hidden, uint64_t salt, float scale,

@@ -28,21 +28,27 @@ from ..ladder import Matryoshka
 class _DeviceLoss(torch.autograd.Function):
     @staticmethod
     def forward(ctx, embeddings, logit_scale, logit_bias, module):
-        engine = module.engine
-        scalars = module._scalars
-        scalars[0] = logit_scale.detach().float().exp()
-        scalars[1] = logit_bias.detach().float()
+        from .._ext import native, stream_handle
+
+        engine, scalars, learned = module.engine, module._scalars, None
+        if logit_scale.dtype == torch.float32 and logit_bias.dtype == torch.float32 and logit_scale.is_cuda and logit_bias.is_cuda:
+            learned = (logit_scale, logit_bias)  # the step's first launch makes them into the two scalars
+        else:
+            scalars[0] = logit_scale.detach().float().exp()
+            scalars[1] = logit_bias.detach().float()
         source = embeddings.detach()
         if source.dtype != torch.bfloat16:
             source = source.to(torch.bfloat16)
         source = source.contiguous()
-        gradient, summands = engine.step(source, scalars=scalars)
-        kept = summands.clone()  # the payload is rewritten by the next step
+        gradient, summands = engine.step(source, scalars=scalars, learned=learned)
+        kept = torch.empty_like(summands)  # the payload is rewritten by the next step
+        loss = torch.empty((), dtype=torch.float32, device=kept.device)
+        native().keep_summands(summands.data_ptr(), kept.data_ptr(), loss.data_ptr(), kept.numel(), stream_handle())
         ctx.save_for_backward(gradient, kept)
         ctx.input_dtype = embeddings.dtype
         ctx.unit_upstream = bool(module.unit_upstream)
         module.last_summands = kept
-        return kept[0].clone()
+        return loss
 
     @staticmethod
     def backward(ctx, grad_output):
@@ -51,8 +57,28 @@ class _DeviceLoss(torch.autograd.Function):
             # The caller promised `loss.backward()` with nothing after the loss: the upstream gradient is one, and a pass
             # over the row gradients that multiplies them by it (25 MB in, 25 MB out per step) is left out.
             return gradient.to(ctx.input_dtype), summands[2], summands[1], None
+        if _DeviceLoss._plain(ctx, gradient, summands, grad_output):
+            from .._ext import native, stream_handle
+
+            scaled = torch.empty(gradient.shape, dtype=ctx.input_dtype, device=gradient.device)
+            by_scale, by_bias = torch.empty_like(grad_output), torch.empty_like(grad_output)
+            native().scale_gradients(gradient.data_ptr(), grad_output.data_ptr(), summands.data_ptr(), scaled.data_ptr(),
+                                     ctx.input_dtype == torch.float32, by_scale.data_ptr(), by_bias.data_ptr(), gradient.numel(),
+                                     stream_handle())
+            return scaled, by_scale, by_bias, None
         scaled = gradient * grad_output.to(gradient.dtype)
         return scaled.to(ctx.input_dtype), summands[2] * grad_output, summands[1] * grad_output, None
+
+    @staticmethod
+    def _plain(ctx, gradient, summands, grad_output) -> bool:
+        """Whether one launch does it all: nothing of this backward is differentiated again, and what the hooks on saved
+        tensors hand back is what was saved."""
+        return (not torch.is_grad_enabled() and type(grad_output) is torch.Tensor and grad_output.is_cuda
+                and grad_output.dtype == torch.float32 and grad_output.dim() == 0 and type(gradient) is torch.Tensor
+                and gradient.is_cuda and gradient.dtype == torch.bfloat16 and gradient.is_contiguous()
+                and gradient.data_ptr() % 16 == 0 and type(summands) is torch.Tensor and summands.is_cuda
+                and summands.dtype == torch.float32 and summands.is_contiguous()
+                and ctx.input_dtype in (torch.bfloat16, torch.float32))
 
 
 class _HostLoss(torch.autograd.Function):

@@ -13,31 +13,37 @@ training benchmark puts in front of the loss.
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 from torch import nn
+
+
+@functools.lru_cache(maxsize=None)
+def _multiprocessors(device: torch.device) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
 
 
 class _FusedTower(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight1, bias1, weight2, bias2, landing):
-        from .._ext import native
+        from .._ext import native, stream_handle
 
         ctx.landing = landing
-        ext, stream = native(), torch.cuda.current_stream().cuda_stream
+        ext, stream = native(), stream_handle()
         z = torch.addmm(bias1, x, weight1.t())
         h = torch.empty_like(z)
-        ext.gelu_forward(z.data_ptr(), h.data_ptr(), z.numel(), torch.cuda.get_device_properties(x.device).multi_processor_count,
-                         stream)
+        ext.gelu_forward(z.data_ptr(), h.data_ptr(), z.numel(), _multiprocessors(x.device), stream)
         y = torch.addmm(bias2, h, weight2.t())
         ctx.save_for_backward(x, weight1, weight2, z, h)
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        from .._ext import native
+        from .._ext import native, stream_handle
 
         x, weight1, weight2, z, h = ctx.saved_tensors
-        ext, stream = native(), torch.cuda.current_stream().cuda_stream
+        ext, stream = native(), stream_handle()
         dy = dy.contiguous()
         rows, mid, out = x.shape[0], weight1.shape[0], weight2.shape[0]
         partials = torch.empty(int(ext.tower_partial_blocks(rows)) * max(mid, out), dtype=torch.float32, device=x.device)

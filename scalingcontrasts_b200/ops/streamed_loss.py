@@ -41,7 +41,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from .._ext import native
+from .._ext import native, stream_handle as _stream
 from ..config import LossSpec, REFERENCE_SPEC, SUMMAND_SLOTS
 from ..ladder import Matryoshka
 
@@ -83,22 +83,22 @@ class BlockNorms:
         return self.scalars * 4
 
 
-def _stream(stream) -> int:
-    return (torch.cuda.current_stream() if stream is None else stream).cuda_stream
-
-
 def compute_block_norms(rows: torch.Tensor, ladder: Matryoshka, norms: BlockNorms, copy_to: Optional[torch.Tensor] = None,
-                        stream=None) -> None:
+                        stream=None, clear: Optional[torch.Tensor] = None,
+                        learned: Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor]] = None) -> None:
     """Fills ``norms`` for the bfloat16 block ``rows``; optionally copies the block to ``copy_to`` in the same pass
-    (used to publish a block into symmetric memory)."""
+    (used to publish a block into symmetric memory), sets the float32 span ``clear`` to zero, and makes a learned log scale
+    and bias into the two scalars that ``score`` takes (``learned`` = (log scale, bias, scalars), float32 on the device)."""
     _check_block(rows)
     copy_pointer = 0
     if copy_to is not None:
         if copy_to.shape != rows.shape or copy_to.dtype != torch.bfloat16 or not copy_to.is_contiguous():
             raise ValueError("copy_to must match the block")
         copy_pointer = copy_to.data_ptr()
+    pointers = (0, 0, 0) if learned is None else tuple(t.data_ptr() for t in learned)
     native().prefix_norms(rows.data_ptr(), copy_pointer, norms.inverse.data_ptr(), norms.tile_max.data_ptr(),
-                          rows.shape[0], rows.shape[1], list(ladder.ends), _stream(stream))
+                          rows.shape[0], rows.shape[1], ladder.ends, _stream(stream), 0 if clear is None else clear.data_ptr(),
+                          0 if clear is None else clear.numel(), *pointers)
 
 
 def _check_block(block: torch.Tensor) -> None:
@@ -148,7 +148,7 @@ class StreamedLoss:
         self.query_norms = BlockNorms(k, rows, device=self.device)
         self.candidate_norms = BlockNorms(k, self.candidate_rows, device=self.device)
         # One span, the gradient and the row accumulators behind it, so that a step clears both at once.
-        sums = torch.zeros(rows * (hidden + self.quantities), **f32)
+        self.sums = sums = torch.zeros(rows * (hidden + self.quantities), **f32)
         self.query_gradient = sums[:rows * hidden].view(rows, hidden)
         # Bias gradient, log-scale gradient, prefix losses, self coefficients of the blocks scored so far.
         self.row_accumulators = sums[rows * hidden:].view(self.quantities, rows)
@@ -203,15 +203,17 @@ class StreamedLoss:
                    self.status)
         return sum(t.numel() * t.element_size() for t in tensors)
 
-    def begin(self, queries: torch.Tensor, stream=None, query_norms: Optional[BlockNorms] = None) -> None:
-        """Clears the gradient and the row accumulators and takes the queries' prefix norms (computed here unless supplied)."""
+    def begin(self, queries: torch.Tensor, stream=None, query_norms: Optional[BlockNorms] = None,
+              cleared: bool = False) -> None:
+        """Clears the gradient and the row accumulators and takes the queries' prefix norms (computed here unless supplied).
+        ``cleared``: the launch that computed the supplied norms has cleared ``sums`` as well."""
         self._check_queries(queries)
         if query_norms is None:
             own = self.query_norms
             self._plan.begin_step(queries.data_ptr(), own.inverse.data_ptr(), own.tile_max.data_ptr(), _stream(stream))
             self._query_norms_view = own
         else:
-            self._plan.begin_step(0, 0, 0, _stream(stream))
+            self._plan.begin_step(0, 0, 0, _stream(stream), cleared)
             self._query_norms_view = query_norms
         self._begun = True
 
@@ -255,7 +257,7 @@ class StreamedLoss:
         qn = self._query_norms_view
         self._plan.join(s)
         ext.finish(queries.data_ptr(), qn.inverse.data_ptr(), self.row_accumulators.data_ptr(), self.query_gradient.data_ptr(),
-                   gradient_out.data_ptr(), summands.data_ptr(), self.rows, self.hidden, list(self.ladder.ends), s)
+                   gradient_out.data_ptr(), summands.data_ptr(), self.rows, self.hidden, self.ladder.ends, s)
         self._begun = False
         return gradient_out, summands
 

@@ -45,7 +45,7 @@ class FusedAdamW:
 
     @torch.no_grad()
     def step(self) -> None:
-        from ._ext import native
+        from ._ext import native, stream_handle
 
         group = self.param_groups[0]
         entries = []
@@ -61,7 +61,8 @@ class FusedAdamW:
         if not entries:
             return
         self.steps += 1
-        stream = torch.cuda.current_stream(self.params[0].device).cuda_stream
+        device = self.params[0].device.index
+        stream = stream_handle(None) if device == torch._C._cuda_getDevice() else torch.cuda.current_stream(device).cuda_stream
         native().adamw_step([entry[:6] for entry in entries], float(group["lr"]), float(group["betas"][0]), float(group["betas"][1]),
                             float(group["eps"]), float(group["weight_decay"]), self.steps, stream)
 

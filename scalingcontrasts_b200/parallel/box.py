@@ -116,7 +116,7 @@ class BoxLoss:
         the block before it, so only a remote block in first position costs a launch of its own. The staging buffers are
         used in rotation across calls, so that a buffer is written again only once every kernel reading it has finished
         (two buffers when the gradient GEMM runs in line, three when it overlaps the next block's forward)."""
-        from .._ext import native
+        from .._ext import native, stream_handle
 
         ahead = None  # the staging slot that the previous block's launch filled with this block
         for index, block in enumerate(blocks):
@@ -127,7 +127,7 @@ class BoxLoss:
                     ahead = self._take_slot()
                     request = self._pull(block, ahead)
                     native().pull(request.src0, request.dst0, request.bytes0, request.src1, request.dst1, request.bytes1,
-                                  self.loss.multiprocessors, (torch.cuda.current_stream() if stream is None else stream).cuda_stream)
+                                  self.loss.multiprocessors, stream_handle(stream))
                 candidates, norms = self.staged[ahead], self.staged_norms[ahead]
             following = blocks[index + 1] if index + 1 < len(blocks) else None
             pull, ahead = None, None
@@ -145,13 +145,13 @@ class BoxLoss:
     # ------------------------------------------------------------------------------------------------------
     def _core(self, beta: float, bias: float, scalars: Optional[torch.Tensor], gradient: torch.Tensor, reduce: bool,
               stream) -> None:
-        """Everything of a step after the publish pass. It touches only buffers this object (or its domain) owns plus
+        """Everything of a step after the publish pass (which has cleared the sums). It touches only buffers this object (or its domain) owns plus
         ``scalars`` and ``gradient``, which is what makes it replayable as a CUDA graph."""
         members, member, rows = self.members, self.member, self.rows
         if self.domain is not None:
             with phase("barrier: every block is published"):
                 self.domain.barrier(stream)
-        self.loss.begin(self.embeddings, stream, query_norms=self.norms)
+        self.loss.begin(self.embeddings, stream, query_norms=self.norms, cleared=True)
         blocks: List[SourceBlock] = [SourceBlock(member * rows, self.embeddings, self.norms)]
         for p in range(1, members):
             peer = (member + p) % members
@@ -170,7 +170,8 @@ class BoxLoss:
 
     def step(self, queries: torch.Tensor, beta: float = 10.0, bias: float = -10.0, scalars: Optional[torch.Tensor] = None,
              gradient_out: Optional[torch.Tensor] = None, stream=None, reduce: bool = True,
-             graph: Optional[bool] = None) -> Tuple[torch.Tensor, torch.Tensor]:
+             graph: Optional[bool] = None,
+             learned: Optional[Tuple[torch.Tensor, torch.Tensor]] = None) -> Tuple[torch.Tensor, torch.Tensor]:
         """Runs one step; returns ``(gradient [R,H] bf16, summands [SUMMAND_SLOTS] f32)``. With ``reduce`` the summands
         are the world's sums on return (stream order); without it they are this rank's share and a barrier closes the
         step instead.
@@ -178,9 +179,10 @@ class BoxLoss:
         With ``graph`` (default: the object's ``use_graphs``) everything after the publish pass is captured once per
         argument set as a CUDA graph and replayed afterwards, so a step costs the host two launches however many
         blocks it scores; the first call of an argument set runs eagerly, the second captures. Every member of the
-        domain must make the same choice in the same step."""
+        domain must make the same choice in the same step. ``learned``, a float32 log scale and bias on the device, fills
+        ``scalars`` in the publish launch."""
         with phase("publish: prefix norms + copy into symmetric memory"):
-            compute_block_norms(queries, self.ladder, self.norms, copy_to=self.embeddings, stream=stream)
+            self._publish(queries, stream, None if learned is None else (*learned, scalars))
         gradient = self.gradient if gradient_out is None else gradient_out
         _check_gradient(gradient, self.rows, self.hidden)
         if (self.use_graphs if graph is None else graph) and stream is None:
@@ -188,6 +190,12 @@ class BoxLoss:
         else:
             self._core(beta, bias, scalars, gradient, reduce, stream)
         return gradient, self.summands
+
+    def _publish(self, queries: torch.Tensor, stream, learned=None) -> None:
+        """Norms, the copy that peers read, and the clear of the step's sums, in one launch: the sums are this rank's own and
+        nothing reads them any more once the step before has finished (stream order)."""
+        compute_block_norms(queries, self.ladder, self.norms, copy_to=self.embeddings, stream=stream, clear=self.loss.sums,
+                            learned=learned)
 
     def _replay(self, beta: float, bias: float, scalars: Optional[torch.Tensor], gradient: torch.Tensor, reduce: bool) -> None:
         from .._ext import native
@@ -219,8 +227,8 @@ class BoxLoss:
                  pull: bool = True) -> Tuple[torch.Tensor, torch.Tensor]:
         """One rank of a ``world``-GPU step on this GPU alone: the own block stands in for every peer's."""
         rows = self.rows
-        compute_block_norms(queries, self.ladder, self.norms, copy_to=self.embeddings, stream=stream)
-        self.loss.begin(self.embeddings, stream, query_norms=self.norms)
+        self._publish(queries, stream)
+        self.loss.begin(self.embeddings, stream, query_norms=self.norms, cleared=True)
         for block in range(world):
             if block == 0 or not pull:
                 candidates, norms = self.embeddings, self.norms

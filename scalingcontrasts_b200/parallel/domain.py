@@ -30,7 +30,7 @@ from typing import List, Optional, Sequence
 
 import torch
 
-from .._ext import native
+from .._ext import native, stream_handle
 
 CONTROL_REGION = 4096  # bytes reserved at the start of every replica for the control block
 LATENCY_SLOT_BYTES = 64 << 10  # largest payload of the one-round all-reduce
@@ -340,9 +340,7 @@ class DeviceDomain(Domain):
         return self.tensor(self._payload_offset, (self.payload_scalars,), torch.float32, member)
 
     # collectives -----------------------------------------------------------------------------------------
-    @staticmethod
-    def _stream(stream) -> int:
-        return (torch.cuda.current_stream() if stream is None else stream).cuda_stream
+    _stream = staticmethod(stream_handle)
 
     def channel(self, index: int):
         """Control block ``index`` (0..15). Collectives that may be in flight at the same time (say the loss step on one

@@ -12,7 +12,7 @@ a training framework adds around it.
 from __future__ import annotations
 
 from collections import deque
-from typing import Deque, Dict, Optional, Tuple
+from typing import Deque, Dict, Optional
 
 import torch
 
@@ -61,7 +61,8 @@ class ContrastiveTrainer:
         self._copy_stream = torch.cuda.Stream(device=self.device)
         self._slots = [torch.empty(rows, in_features, dtype=torch.bfloat16, device=self.device) for _ in range(2)]
         self._slot_free = [torch.cuda.Event() for _ in range(2)]
-        self._fed: Deque[Tuple[int, torch.cuda.Event]] = deque()
+        self._slot_landed = [torch.cuda.Event() for _ in range(2)]
+        self._fed: Deque[int] = deque()
         self._next_slot = 0
         self._loss_host = torch.zeros(2, 16, dtype=torch.float32).pin_memory()
         # Status words of the tile kernels and of the two collective channels travel to the host with every loss, so a
@@ -91,9 +92,8 @@ class ContrastiveTrainer:
         self._copy_stream.wait_event(self._slot_free[slot])
         with torch.cuda.stream(self._copy_stream):
             self._slots[slot].copy_(batch, non_blocking=True)
-            landed = torch.cuda.Event()
-            landed.record(self._copy_stream)
-        self._fed.append((slot, landed))
+            self._slot_landed[slot].record(self._copy_stream)
+        self._fed.append(slot)
 
     def step(self, batch: Optional[torch.Tensor] = None) -> Optional[float]:
         """Runs one training step on the oldest fed batch (feeding ``batch`` first when given). Returns the loss of the
@@ -102,22 +102,22 @@ class ContrastiveTrainer:
             self.feed(batch)
         if not self._fed:
             raise RuntimeError("step() without a fed batch")
-        slot, landed = self._fed.popleft()
-        torch.cuda.current_stream().wait_event(landed)
-        loss = self.step_on_device(self._slots[slot])
-        self._slot_free[slot].record()
+        slot, current = self._fed.popleft(), torch.cuda.current_stream()
+        current.wait_event(self._slot_landed[slot])
+        self.step_on_device(self._slots[slot])
+        self._slot_free[slot].record(current)
         previous = self._collect_loss()
         index = self.steps_done % 2
         self._gather_report()
         self._report_host[index].copy_(self._report, non_blocking=True)
-        self._loss_events[index].record()
+        self._loss_events[index].record(current)
         self._loss_pending.append(index)
         return previous
 
     def _gather_report(self) -> None:
-        from ._ext import native
+        from ._ext import native, stream_handle
 
-        ext, stream = native(), torch.cuda.current_stream().cuda_stream
+        ext, stream = native(), stream_handle()
         base = self._report.data_ptr()
         spans = [(self.loss.last_summands.data_ptr(), base, 48)]
         spans += [(source.data_ptr(), base + 64 + 32 * position, 32) for position, source in enumerate(self._status_sources)]

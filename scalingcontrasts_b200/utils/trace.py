@@ -7,8 +7,8 @@ The reference has no tracing of any kind (its only instrument is the wall-clock 
 from __future__ import annotations
 
 import os
-from contextlib import contextmanager
-from typing import Iterator
+from contextlib import contextmanager, nullcontext
+from typing import ContextManager, Iterator
 
 _enabled = os.environ.get("SC_NVTX", "0") == "1"
 
@@ -22,11 +22,15 @@ def enabled() -> bool:
     return _enabled
 
 
+_nothing = nullcontext()
+
+
+def phase(name: str) -> ContextManager[None]:
+    return _range(name) if _enabled else _nothing
+
+
 @contextmanager
-def phase(name: str) -> Iterator[None]:
-    if not _enabled:
-        yield
-        return
+def _range(name: str) -> Iterator[None]:
     import torch
 
     torch.cuda.nvtx.range_push(name)
