@@ -148,8 +148,9 @@ struct forward_arguments {
     float gradient_scale;              // the loss passes 2 / live
     bool ordinary_launch;              // true: starts only once everything before it in the stream is complete (see launch.h)
 };
-// Returns the number of partial slots the launch fills: (column groups per tile) * rows_c / 64 / tiles_per_run.
+// Partial slots: room for what any launch of the shape fills, and how many this one does (one to a run, 64 columns and column group).
 uint32_t forward_partial_slots(uint32_t rows_c, uint32_t tiles_per_run);
+uint32_t forward_filled_slots(forward_arguments const& arguments);
 uint32_t forward_quantities(uint32_t prefixes);
 uint32_t forward_choose_tiles_per_run(uint32_t rows_q, uint32_t rows_c, int multiprocessors);
 bool forward_fused_supported(uint32_t hidden, uint32_t prefixes);

@@ -214,7 +214,8 @@ struct loss_plan {
         // The block's records are folded by the backward kernel, unless there is none, it comes later (the next block's records
         // are written before it has run) or its CTAs need not all run (split).
         bool const folds = !fused && !overlapping && backward_split == 1;
-        if (!folds) sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows_q, partial_slots, quantities, stream);
+        uint32_t const filled = sc::forward_filled_slots(a);
+        if (!folds) sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows_q, filled, quantities, stream);
         if (!fused) {
             sc::backward_arguments b{};
             b.gradient_cube_bf16 = pointer<void>(cube);
@@ -225,7 +226,7 @@ struct loss_plan {
             b.scale = static_cast<float>(2.0 / live), b.budget_ns = budget_ns, b.ordinary_launch = overlapping;
             if (folds) {
                 b.partials = pointer<float>(partials), b.row_accumulators = pointer<float>(accumulators);
-                b.partial_slots = partial_slots, b.quantities = quantities;
+                b.partial_slots = filled, b.quantities = quantities;
             }
             if (!overlapping) sc::launch_backward(b, stream);
             else {

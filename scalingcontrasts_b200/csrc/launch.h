@@ -22,17 +22,24 @@ namespace sc {
 __device__ __forceinline__ void let_dependents_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_kernels_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// `overlap` false: an ordinary launch. Errors are left for cudaGetLastError, as with the launch syntax.
+// `overlap` false: an ordinary launch. `cluster`: CTAs of a cluster. Errors are left for cudaGetLastError, as with the launch syntax.
+template <typename... parameters, typename... arguments>
+void launch_dependent_clusters(bool overlap, uint32_t cluster, void (*kernel)(parameters...), dim3 grid, dim3 block, size_t shared_bytes,
+                               cudaStream_t stream, arguments&&... values) {
+    cudaLaunchAttribute attributes[2]{};
+    attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[0].val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
+    attributes[1].id = cudaLaunchAttributeClusterDimension;
+    attributes[1].val.clusterDim.x = cluster, attributes[1].val.clusterDim.y = 1, attributes[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid, config.blockDim = block, config.dynamicSmemBytes = shared_bytes, config.stream = stream;
+    config.attrs = attributes, config.numAttrs = cluster > 1 ? 2 : 1;
+    cudaLaunchKernelEx(&config, kernel, static_cast<parameters>(values)...);
+}
 template <typename... parameters, typename... arguments>
 void launch_dependent(bool overlap, void (*kernel)(parameters...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream,
                       arguments&&... values) {
-    cudaLaunchAttribute attribute{};
-    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute.val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
-    cudaLaunchConfig_t config{};
-    config.gridDim = grid, config.blockDim = block, config.dynamicSmemBytes = shared_bytes, config.stream = stream;
-    config.attrs = &attribute, config.numAttrs = 1;
-    cudaLaunchKernelEx(&config, kernel, static_cast<parameters>(values)...);
+    launch_dependent_clusters(overlap, 1, kernel, grid, block, shared_bytes, stream, static_cast<arguments&&>(values)...);
 }
 
 } // namespace sc

@@ -3,7 +3,9 @@
 // the raw dot product (bfloat16) plus per-row partial sums. Optionally the same launch pulls the NEXT peer's block
 // from that peer's memory into local staging, so the NVLink transfer hides under this block's tensor-core work.
 //
-// Shape of the work. A tile is 128 query rows x 64 candidates. The hidden axis streams through shared memory in
+// Shape of the work. A tile is 128 query rows x 64 candidates, scored by one CTA, or 128 x 128, scored by a pair of CTAs (a cluster of
+// two): each loads half the rows and half the candidates, the UMMAs of the pair read both, and each CTA scores its 64 rows
+// against all 128 candidates, so that a cell costs a third fewer operand bytes. The hidden axis streams through shared memory in
 // stages of 64 channels (TMA, 128-byte swizzle), widest channels first. Every band of the ladder owns one 64-column
 // slot of tensor memory and the UMMAs of a 16-channel step accumulate into the slot of the band that contains the
 // step, so each channel is multiplied exactly once (depth H per cell, where a sweep-and-subtract scheme spends up to
@@ -21,13 +23,12 @@
 // from another GPU's memory), warp 19 the fused kernel's second issuer. The epilogue's four warpgroups run with 104
 // registers a thread, the helpers' with 64.
 //
-// What bounds it (B200, 4096 rows, H=768, K=5, then 90 us, now 88): nothing alone. Taking one resource away at a time gained little:
-// three of four UMMAs 4 us, the queries' loads 2 us, four of five bands' math 4 us, the cube's stores 6 us. A tile is a chain
-// (operands, UMMAs, epilogue, slots back to the issuer) of which two tiles are under way at once; tensor memory has no room
-// for a third. Of a tile's 9.6 k cycles the issuer issues for 5.9 k and waits for operands and slots in the others; an epilogue
-// warp waits for 1.3 k of its 10.6 k.
+// What bounds it (B200, one block of 4096 rows, H=768, K=5, off the diagonal: 75 us): the epilogue, which by itself takes about 60 (cells
+// 6.4 k of a tile's 9 k cycles: a warp's instructions wait for one another, and four warps to a scheduler do not hide all of it);
+// operands and UMMAs by themselves take about 30. One block of 16384 rows (1.13 ms): the memory side as well; a single CTA's loads and
+// the cube's stores without any arithmetic took 1.05 ms, and the GPU runs at its power limit.
 //
-// A CTA walks work items (row strip, run of consecutive candidate tiles) in a fixed round-robin order and writes one
+// A CTA or pair walks work items (row strip, run of consecutive candidate tiles) in a fixed round-robin order and writes one
 // partial record per (run, column quarter, row); the fold over records happens in a fixed order elsewhere, so the loss
 // summands do not depend on scheduling.
 //
@@ -45,14 +46,20 @@ namespace sc {
 
 namespace {
 
-constexpr uint32_t fwd_rows = 128;
-constexpr uint32_t fwd_cols = 64;
+constexpr uint32_t fwd_rows = 128; // of a strip: one CTA's, or a pair's
 constexpr uint32_t fwd_depth = 64;
-constexpr uint32_t fwd_max_stages = 6;
+constexpr uint32_t fwd_max_stages = 8;
+// The kernel's forms. A CTA scores tiles of 128 rows x 64 candidates by itself (`form_single`, and `form_fused`, which also runs the
+// gradient GEMM), or two CTAs, a cluster, score tiles of 128 x 128 together (`form_pair`, and `form_pair_apart` for blocks that
+// hold no row's own copy or partner: nothing of what those need is in it). See forward_form for which is taken when.
+enum form_t { form_single, form_pair, form_pair_apart, form_fused };
+__host__ __device__ constexpr bool fwd_paired(form_t form) { return form == form_pair || form == form_pair_apart; }
+__host__ __device__ constexpr uint32_t fwd_cols_for(form_t form) { return fwd_paired(form) ? 128u : 64u; }
+__host__ __device__ constexpr uint32_t fwd_ctas_for(form_t form) { return fwd_paired(form) ? 2u : 1u; }
 constexpr uint32_t fwd_max_slots = 8;
 // Tensor-memory slots of the score accumulators: all eight 64-column slots, or six when the last 128 columns hold the
 // gradient GEMM's accumulator.
-__host__ __device__ constexpr uint32_t fwd_slots_for(bool fused) { return fused ? 6u : 8u; }
+__host__ __device__ constexpr uint32_t fwd_slots_for(form_t form) { return form == form_fused ? 6u : 8u; }
 constexpr uint32_t fwd_slot_columns = 64;
 constexpr uint32_t fwd_tmem_columns = 512;
 // The gradient GEMM that the fused kernel runs beside the scoring: 128 rows x up to 128 channels per accumulator, the
@@ -72,7 +79,7 @@ constexpr uint32_t fz_max_tiles_per_run = 16;
 constexpr uint32_t fwd_epilogue_warps = 16; // four per scheduler
 constexpr uint32_t fwd_epilogue_threads = fwd_epilogue_warps * 32;
 constexpr uint32_t fwd_column_groups = fwd_epilogue_warps / 4;             // warps that share a lane quadrant
-constexpr uint32_t fwd_warp_columns = fwd_cols / fwd_column_groups;        // columns of a tile that one warp owns
+constexpr uint32_t fwd_warp_columns = fwd_slot_columns / fwd_column_groups; // columns of a tile that one warp owns
 // Columns a thread takes at a time: all bands' values of a chunk are held in registers together.
 // Ladders of seven and eight bands go band by band instead (`rolled`), sixteen columns at a time: their values do not fit the
 // registers, and eight bands times three forms of the cell math are more code than the instruction cache likes. One block
@@ -101,9 +108,11 @@ constexpr uint32_t fwd_epilogue_registers = 104, fwd_helper_registers = 64, fwd_
 static_assert(fwd_epilogue_threads * fwd_epilogue_registers + (fwd_threads - fwd_epilogue_threads) * fwd_helper_registers <=
                   fwd_threads * fwd_launch_registers,
               "the register split must not exceed what the block is launched with");
-constexpr uint32_t fwd_q_bytes = fwd_rows * fwd_depth * 2;
-constexpr uint32_t fwd_c_bytes = fwd_cols * fwd_depth * 2;
-constexpr uint32_t fwd_stage_bytes = fwd_q_bytes + fwd_c_bytes;
+// A CTA's share of a stage: its rows of the strip and its part of the tile's candidates.
+__host__ __device__ constexpr uint32_t fwd_own_rows(form_t form) { return fwd_rows / fwd_ctas_for(form); }
+__host__ __device__ constexpr uint32_t fwd_own_cols(form_t form) { return fwd_cols_for(form) / fwd_ctas_for(form); }
+__host__ __device__ constexpr uint32_t fwd_q_bytes(form_t form) { return fwd_own_rows(form) * fwd_depth * 2; }
+__host__ __device__ constexpr uint32_t fwd_stage_bytes(form_t form) { return fwd_q_bytes(form) + fwd_own_cols(form) * fwd_depth * 2; }
 constexpr uint32_t fwd_tile_barriers = 8;
 constexpr float log2_e = 1.4426950408889634f;
 // (logit + bias) * log2(e) below these: the series may be cut. At e < 2^-8 three terms leave out e^3 / 4 of log1p(e) (1.5e-8
@@ -136,15 +145,17 @@ struct fwd_tail {
     uint32_t abort_flag;
 };
 constexpr uint32_t fwd_tail_bytes = (sizeof(fwd_tail) + 127) / 128 * 128;
-// Ring of candidate norms, one entry per tile in flight: [prefixes][64 columns] inverse norms, then the [8] tile maxima.
-__host__ __device__ constexpr uint32_t fwd_norm_floats(uint32_t prefixes) { return prefixes * fwd_cols + 8; }
-__host__ __device__ constexpr uint32_t fwd_norm_bytes(uint32_t prefixes) { return fwd_norm_slots * fwd_norm_floats(prefixes) * 4; }
+// Ring of candidate norms, one entry per tile in flight: [prefixes][columns] inverse norms, then [8] maxima per 64 columns.
+__host__ __device__ constexpr uint32_t fwd_norm_floats(uint32_t prefixes, form_t form) {
+    return prefixes * fwd_cols_for(form) + 8 * (fwd_cols_for(form) / 64);
+}
+__host__ __device__ constexpr uint32_t fwd_norm_bytes(uint32_t prefixes, form_t form) { return fwd_norm_slots * fwd_norm_floats(prefixes, form) * 4; }
 // Per epilogue thread and band the row factor beta / |q_k|: in shared memory where the bands' values leave no registers for
 // it (chunks of eight columns times four or more bands), in registers otherwise. Band by band, the row's loss and
 // coefficient as well.
-__host__ __device__ constexpr bool fwd_factors_in_shared(uint32_t prefixes, bool fused) { return !fused && prefixes >= 4; }
-__host__ __device__ constexpr uint32_t fwd_factor_bytes(uint32_t prefixes, bool fused) {
-    return (fwd_rolled_for(prefixes) ? 3u : (fwd_factors_in_shared(prefixes, fused) ? 1u : 0u)) * prefixes * fwd_epilogue_threads * 4;
+__host__ __device__ constexpr bool fwd_factors_in_shared(uint32_t prefixes, form_t form) { return form != form_fused && prefixes >= 4; }
+__host__ __device__ constexpr uint32_t fwd_factor_bytes(uint32_t prefixes, form_t form) {
+    return (fwd_rolled_for(prefixes) ? 3u : (fwd_factors_in_shared(prefixes, form) ? 1u : 0u)) * prefixes * fwd_epilogue_threads * 4;
 }
 // Per epilogue warp and band (four in rotation when the bands go one by one) a patch of [32 rows][16 columns] bfloat16, from
 // which the gradient cube is written by TMA stores.
@@ -156,18 +167,18 @@ __host__ __device__ constexpr uint32_t fwd_store_bytes(uint32_t prefixes) {
 // Stages of the score operands: as many as the rest of the shared memory leaves room for. The fused kernel keeps room for
 // the gradient GEMM's stages and runs the scores on what is left (three at five prefixes, two at six).
 constexpr uint32_t fwd_shared_limit = 227 * 1024;
-__host__ __device__ constexpr uint32_t fwd_stages_for(uint32_t prefixes, bool fused) {
-    uint32_t const rest = 1024 + (fused ? fz_stages * fz_stage_bytes : 0u) + fwd_store_bytes(prefixes) + fwd_tail_bytes + fwd_norm_bytes(prefixes) + fwd_factor_bytes(prefixes, fused);
-    uint32_t const fit = (fwd_shared_limit - rest) / fwd_stage_bytes;
+__host__ __device__ constexpr uint32_t fwd_stages_for(uint32_t prefixes, form_t form) {
+    uint32_t const rest = 1024 + (form == form_fused ? fz_stages * fz_stage_bytes : 0u) + fwd_store_bytes(prefixes) + fwd_tail_bytes + fwd_norm_bytes(prefixes, form) + fwd_factor_bytes(prefixes, form);
+    uint32_t const fit = (fwd_shared_limit - rest) / fwd_stage_bytes(form);
     return fit < fwd_max_stages ? fit : fwd_max_stages;
 }
-static_assert(fwd_stages_for(8, false) >= 3 && fwd_stages_for(fz_max_prefixes, true) >= 2, "the score operands need a ring of stages");
-__host__ __device__ constexpr uint32_t fwd_stage_region_bytes(uint32_t prefixes, bool fused) {
-    return fwd_stages_for(prefixes, fused) * fwd_stage_bytes + (fused ? fz_stages * fz_stage_bytes : 0u);
+static_assert(fwd_stages_for(8, form_pair) >= 3 && fwd_stages_for(fz_max_prefixes, form_fused) >= 2, "the score operands need a ring of stages");
+__host__ __device__ constexpr uint32_t fwd_stage_region_bytes(uint32_t prefixes, form_t form) {
+    return fwd_stages_for(prefixes, form) * fwd_stage_bytes(form) + (form == form_fused ? fz_stages * fz_stage_bytes : 0u);
 }
-__host__ __device__ constexpr uint32_t fwd_shared_bytes(uint32_t prefixes, bool fused) {
-    return 1024 + fwd_stage_region_bytes(prefixes, fused) + fwd_store_bytes(prefixes) + fwd_tail_bytes + fwd_norm_bytes(prefixes) +
-           fwd_factor_bytes(prefixes, fused);
+__host__ __device__ constexpr uint32_t fwd_shared_bytes(uint32_t prefixes, form_t form) {
+    return 1024 + fwd_stage_region_bytes(prefixes, form) + fwd_store_bytes(prefixes) + fwd_tail_bytes + fwd_norm_bytes(prefixes, form) +
+           fwd_factor_bytes(prefixes, form);
 }
 
 struct fwd_params {
@@ -179,7 +190,7 @@ struct fwd_params {
     uint32_t* status;
     uint32_t rows_q, rows_c, hidden;
     ladder_t ladder;
-    uint32_t tiles_per_run, runs_per_strip, items;
+    uint32_t tiles_per_run, tiles_per_strip, runs_per_strip, items; // a strip's last run may be shorter
     float beta, bias, weight;
     float const* scalars; // optional device copy of {beta, bias}: learnable values never visit the host
     uint64_t query_base, candidate_base;
@@ -322,37 +333,52 @@ __device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, wa
 }
 constexpr uint32_t sleep_gemm_ns = 500; // the fused kernel's gradient GEMM runs a whole item behind
 
-// A CTA's items: every gridDim.x-th of the list.
-__device__ __forceinline__ uint32_t item_count(uint32_t items) { return (items + gridDim.x - 1 - blockIdx.x) / gridDim.x; }
-__device__ __forceinline__ uint32_t item_at(uint32_t n) { return blockIdx.x + n * gridDim.x; }
+// The items of a CTA or pair: every so many-th of the list.
+template <form_t form_> __device__ __forceinline__ uint32_t item_count(uint32_t items) {
+    uint32_t const walkers = gridDim.x / fwd_ctas_for(form_), walker = blockIdx.x / fwd_ctas_for(form_);
+    return (items + walkers - 1 - walker) / walkers;
+}
+template <form_t form_> __device__ __forceinline__ uint32_t item_at(uint32_t n) {
+    return blockIdx.x / fwd_ctas_for(form_) + n * (gridDim.x / fwd_ctas_for(form_));
+}
+
+// Tiles of a strip's run: a divisor of the tiles of 64, but not always of those of 128.
+template <form_t form_> __device__ __forceinline__ uint32_t run_length(fwd_params const& p, uint32_t run) {
+    if constexpr (!fwd_paired(form_)) return p.tiles_per_run;
+    else return min(p.tiles_per_run, p.tiles_per_strip - run * p.tiles_per_run);
+}
 
 // The producer also brings the candidates' inverse norms of a tile (and their maxima) into the ring the epilogue warps read
 // them from: plain loads at the start of the tile, stored once the tile's operand loads have been issued.
-template <int prefixes_>
+template <int prefixes_, form_t form_>
 __device__ __forceinline__ void producer_role(CUtensorMap const* q_map, CUtensorMap const* c_map, fwd_params const& p,
                                               uint32_t stages_base, float* norm_ring, fwd_tail* tail,
-                                              wait_context const& ctx, uint32_t const stages) {
+                                              wait_context const& ctx, uint32_t const rank) {
+    constexpr uint32_t stages = fwd_stages_for(prefixes_, form_), columns = fwd_cols_for(form_), halves = columns / 32;
     bool const elected = elect_one();
     uint32_t const lane = threadIdx.x % 32;
     uint32_t stage = 0, phase = 0, tile_local = 0;
     uint32_t const chunks = p.hidden / fwd_depth;
-    uint32_t const column_tiles = p.rows_c / fwd_cols;
+    uint32_t const maxima = p.rows_c / 64;
     phase_timer timer(p);
     timer.only_if(elected);
-    for (uint32_t n = 0, count = item_count(p.items); n < count; ++n) {
-        uint32_t const item = item_at(n);
+    for (uint32_t n = 0, count = item_count<form_>(p.items); n < count; ++n) {
+        uint32_t const item = item_at<form_>(n);
         uint32_t const strip = item / p.runs_per_strip, run = item % p.runs_per_strip;
-        for (uint32_t t = 0; t < p.tiles_per_run; ++t, ++tile_local) {
-            uint32_t const column_tile = run * p.tiles_per_run + t;
-            float norms[2 * prefixes_], largest = 0.0f;
+        for (uint32_t t = 0, length = run_length<form_>(p, run); t < length; ++t, ++tile_local) {
+            uint32_t const first_column = (run * p.tiles_per_run + t) * columns;
+            float norms[halves * prefixes_], largest = 0.0f;
 #pragma unroll
-            for (int j = 0; j < 2 * prefixes_; ++j) {
-                size_t const at = static_cast<size_t>(j / 2) * p.rows_c + column_tile * fwd_cols + (j % 2) * 32u + lane;
-                norms[j] = SC_IN_BOUNDS(at, static_cast<size_t>(prefixes_) * p.rows_c) ? *(p.c_inv + at) : 0.0f;
+            for (int j = 0; j < static_cast<int>(halves) * prefixes_; ++j) {
+                uint32_t const column = first_column + (j % halves) * 32u + lane; // the last tile of a pair may be half empty
+                size_t const at = static_cast<size_t>(j / halves) * p.rows_c + column;
+                norms[j] = column < p.rows_c && SC_IN_BOUNDS(at, static_cast<size_t>(prefixes_) * p.rows_c) ? *(p.c_inv + at) : 0.0f;
             }
-            if (lane < prefixes_ &&
-                SC_IN_BOUNDS(static_cast<size_t>(lane) * column_tiles + column_tile, static_cast<size_t>(prefixes_) * column_tiles))
-                largest = *(p.c_tile_max + static_cast<size_t>(lane) * column_tiles + column_tile);
+            // Lane 8 h + k: band k's largest inverse norm among the tile's h-th 64 columns.
+            uint32_t const maximum = first_column / 64 + lane / 8;
+            if (lane % 8 < prefixes_ && lane / 8 < columns / 64 && maximum < maxima &&
+                SC_IN_BOUNDS(static_cast<size_t>(lane % 8) * maxima + maximum, static_cast<size_t>(prefixes_) * maxima))
+                largest = *(p.c_tile_max + static_cast<size_t>(lane % 8) * maxima + maximum);
             bool ok = true;
             if (elected) {
                 for (int chunk = static_cast<int>(chunks) - 1; chunk >= 0; --chunk) {
@@ -361,11 +387,21 @@ __device__ __forceinline__ void producer_role(CUtensorMap const* q_map, CUtensor
                     if (!ok) break;
                     timer.lap(1);
                     uint32_t const full = smem_u32(&tail->stage_full[stage]);
-                    uint32_t const destination = stages_base + stage * fwd_stage_bytes;
-                    mbar_arrive_expect_tx(full, fwd_stage_bytes);
-                    tma_load_2d(destination, q_map, full, chunk * static_cast<int>(fwd_depth), static_cast<int>(strip * fwd_rows));
-                    tma_load_2d(destination + fwd_q_bytes, c_map, full, chunk * static_cast<int>(fwd_depth),
-                                static_cast<int>(column_tile * fwd_cols));
+                    uint32_t const destination = stages_base + stage * fwd_stage_bytes(form_);
+                    int const x = chunk * static_cast<int>(fwd_depth);
+                    int const q_row = static_cast<int>(strip * fwd_rows + rank * fwd_own_rows(form_));
+                    int const c_row = static_cast<int>(first_column + rank * fwd_own_cols(form_));
+                    if constexpr (fwd_paired(form_)) {
+                        // The first CTA's barrier counts both CTAs' bytes, whichever arrive first.
+                        uint32_t const counted = smem_of(full, 0);
+                        if (rank == 0) mbar_arrive_expect_tx(full, 2 * fwd_stage_bytes(form_));
+                        tma_load_2d_pair(destination, q_map, counted, x, q_row);
+                        tma_load_2d_pair(destination + fwd_q_bytes(form_), c_map, counted, x, c_row);
+                    } else {
+                        mbar_arrive_expect_tx(full, fwd_stage_bytes(form_));
+                        tma_load_2d(destination, q_map, full, x, q_row);
+                        tma_load_2d(destination + fwd_q_bytes(form_), c_map, full, x, c_row);
+                    }
                     if (++stage == stages) stage = 0, phase ^= 1u;
                 }
             }
@@ -374,10 +410,10 @@ __device__ __forceinline__ void producer_role(CUtensorMap const* q_map, CUtensor
             if (!__all_sync(0xFFFFFFFFu, mbar_wait_lane(smem_u32(&tail->norms_empty[entry]), ((tile_local / fwd_norm_slots) & 1u) ^ 1u,
                                                         ctx, site_fwd_norms_empty, item)))
                 return;
-            float* const into = norm_ring + entry * fwd_norm_floats(prefixes_);
+            float* const into = norm_ring + entry * fwd_norm_floats(prefixes_, form_);
 #pragma unroll
-            for (int j = 0; j < 2 * prefixes_; ++j) into[(j / 2) * fwd_cols + (j % 2) * 32u + lane] = norms[j];
-            if (lane < 8) into[prefixes_ * fwd_cols + lane] = largest;
+            for (int j = 0; j < static_cast<int>(halves) * prefixes_; ++j) into[(j / halves) * columns + (j % halves) * 32u + lane] = norms[j];
+            if (lane < columns / 8) into[prefixes_ * columns + lane] = largest;
             __syncwarp();
             if (elected) mbar_arrive(smem_u32(&tail->norms_full[entry]));
         }
@@ -385,11 +421,11 @@ __device__ __forceinline__ void producer_role(CUtensorMap const* q_map, CUtensor
     timer.flush(p, 0, 2);
 }
 
-template <int prefixes_, bool fused_>
+template <int prefixes_, form_t form_>
 __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_base, fwd_tail* tail, uint32_t tmem_base,
                                          wait_context const& ctx) {
-    constexpr uint32_t fwd_slots = fwd_slots_for(fused_);
-    constexpr uint32_t idesc = umma_idesc_bf16(fwd_rows, fwd_cols);
+    constexpr uint32_t fwd_slots = fwd_slots_for(form_);
+    constexpr uint32_t idesc = umma_idesc_bf16(fwd_rows, fwd_cols_for(form_));
     constexpr uint32_t parked = fwd_parked_bands_for(prefixes_);
     constexpr uint32_t descriptor_high = (1024u >> 4) | (1u << 14) | (2u << 29); // stride 1024 B, version 1, 128-byte swizzle
     if (!elect_one()) return;
@@ -397,6 +433,14 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
     uint32_t const low_base = ((stages_base & 0x3FFFFu) >> 4) | (1u << 16);
     uint32_t stage = 0, phase = 0, unit = 0, tile_local = 0, seen = 0, seen_parked = 0;
     phase_timer timer(p);
+    auto multiply = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate) {
+        if constexpr (fwd_paired(form_)) umma_bf16_pair(d, a, b, idesc, accumulate);
+        else umma_bf16(d, a, b, idesc, accumulate);
+    };
+    auto commit = [&](uint32_t bar) { // to both CTAs of a pair
+        if constexpr (fwd_paired(form_)) umma_commit_pair(smem_of(bar, 0)), umma_commit_pair(smem_of(bar, 1));
+        else umma_commit(bar);
+    };
     // The next band's slot, once it is free. The slot's last user was unit - fwd_slots, a band of tile `needed`; the
     // epilogue must have read it out. Releases are observed here strictly in tile order, per barrier array, so a barrier's
     // parity can never be a full turn ahead of the one waited for: tile X + fwd_slots cannot even be issued before tile X's release has been
@@ -421,9 +465,8 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
         ++unit;
         return true;
     };
-    for (uint32_t n = 0, count = item_count(p.items); n < count; ++n) {
-        uint32_t const item = item_at(n);
-        for (uint32_t t = 0; t < p.tiles_per_run; ++t) {
+    for (uint32_t n = 0, count = item_count<form_>(p.items); n < count; ++n) {
+        for (uint32_t t = 0, length = run_length<form_>(p, item_at<form_>(n) % p.runs_per_strip); t < length; ++t) {
             for (int chunk = static_cast<int>(chunks) - 1; chunk >= 0; --chunk) {
                 uint32_t const starts = p.band_starts[chunk];
                 timer.lap(0);
@@ -431,31 +474,31 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
                     return;
                 timer.lap(1);
                 tcgen05_fence_after();
-                uint32_t const low = low_base + stage * (fwd_stage_bytes >> 4);
+                uint32_t const low = low_base + stage * (fwd_stage_bytes(form_) >> 4);
                 uint64_t q_descriptor, c_descriptor;
                 asm("mov.b64 %0, {%1, %2};" : "=l"(q_descriptor) : "r"(low), "r"(descriptor_high));
-                asm("mov.b64 %0, {%1, %2};" : "=l"(c_descriptor) : "r"(low + (fwd_q_bytes >> 4)), "r"(descriptor_high));
+                asm("mov.b64 %0, {%1, %2};" : "=l"(c_descriptor) : "r"(low + (fwd_q_bytes(form_) >> 4)), "r"(descriptor_high));
                 uint32_t const empty = smem_u32(&tail->stage_empty[stage]);
                 // A step of 16 channels advances both descriptors by 32 bytes. Steps run from the chunk's top down; a band
                 // that starts inside the chunk (its edge is not a multiple of 64) takes the step-by-step way.
                 if ((starts & 0x00FFFFFFu) == 0u) {
                     if (starts != 0u && !take_slot()) return;
-                    umma_bf16(slot_address, q_descriptor + 6, c_descriptor + 6, idesc, starts != 0u ? 0u : 1u);
-                    umma_bf16(slot_address, q_descriptor + 4, c_descriptor + 4, idesc, 1u);
-                    umma_bf16(slot_address, q_descriptor + 2, c_descriptor + 2, idesc, 1u);
-                    umma_bf16(slot_address, q_descriptor, c_descriptor, idesc, 1u);
+                    multiply(slot_address, q_descriptor + 6, c_descriptor + 6, starts != 0u ? 0u : 1u);
+                    multiply(slot_address, q_descriptor + 4, c_descriptor + 4, 1u);
+                    multiply(slot_address, q_descriptor + 2, c_descriptor + 2, 1u);
+                    multiply(slot_address, q_descriptor, c_descriptor, 1u);
                 } else {
 #pragma unroll 1
                     for (int sub = 3; sub >= 0; --sub) {
                         bool const begins = ((starts >> (8 * sub)) & 0xFFu) != 0u;
                         if (begins && !take_slot()) return;
-                        umma_bf16(slot_address, q_descriptor + 2u * sub, c_descriptor + 2u * sub, idesc, begins ? 0u : 1u);
+                        multiply(slot_address, q_descriptor + 2u * sub, c_descriptor + 2u * sub, begins ? 0u : 1u);
                     }
                 }
-                umma_commit(empty);
-                if (++stage == fwd_stages_for(prefixes_, fused_)) stage = 0, phase ^= 1u;
+                commit(empty);
+                if (++stage == fwd_stages_for(prefixes_, form_)) stage = 0, phase ^= 1u;
             }
-            umma_commit(smem_u32(&tail->tile_full[tile_local % fwd_tile_barriers]));
+            commit(smem_u32(&tail->tile_full[tile_local % fwd_tile_barriers]));
             ++tile_local;
         }
     }
@@ -463,14 +506,14 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
 }
 
 // Position of a CTA in its walk over (work item, tile of the run).
-struct tile_cursor {
+template <form_t form_> struct tile_cursor {
     uint32_t n, t, strip, run;
     __device__ __forceinline__ void go_to(fwd_params const& p, uint32_t to) {
-        uint32_t const item = item_at(to);
+        uint32_t const item = item_at<form_>(to);
         n = to, t = 0, strip = item / p.runs_per_strip, run = item % p.runs_per_strip;
     }
     __device__ __forceinline__ void advance(fwd_params const& p) {
-        if (++t == p.tiles_per_run) go_to(p, n + 1);
+        if (++t == run_length<form_>(p, run)) go_to(p, n + 1);
     }
     __device__ __forceinline__ uint32_t column_tile(fwd_params const& p) const { return run * p.tiles_per_run + t; }
 };
@@ -494,8 +537,8 @@ __device__ __noinline__ void fz_drain_chunks(float* destination, uint32_t chunks
 }
 
 // Where band `band` of the tile whose widest band is unit `first_unit` of the ring has its slot.
-template <int prefixes_, bool fused_> __device__ __forceinline__ uint32_t band_slot(uint32_t first_unit, uint32_t band) {
-    return ((first_unit + (prefixes_ - 1 - band)) % fwd_slots_for(fused_)) * fwd_slot_columns;
+template <int prefixes_, form_t form_> __device__ __forceinline__ uint32_t band_slot(uint32_t first_unit, uint32_t band) {
+    return ((first_unit + (prefixes_ - 1 - band)) % fwd_slots_for(form_)) * fwd_slot_columns;
 }
 
 // In a patch that the diagonal crosses, a row's own copy and its pair partner: each thread scores its two cells (where the
@@ -518,7 +561,7 @@ __device__ __forceinline__ float pick_column(uint32_t const (&d)[16], uint32_t c
     for (int c = 0; c < 2; ++c) two[c] = (column & 2u) ? four[c + 2] : four[c];
     return __uint_as_float((column & 1u) ? two[1] : two[0]);
 }
-template <int prefixes_, bool fused_>
+template <int prefixes_, form_t form_>
 __device__ __noinline__ special_sums special_cells(uint32_t lane_base, uint32_t first_unit, float const* norms,
                                                    float const* q_inv, uint32_t rows_q, float beta, float bias,
                                                    int own_column, int partner_column, uint32_t spec_code, uint32_t sums,
@@ -529,7 +572,7 @@ __device__ __noinline__ special_sums special_cells(uint32_t lane_base, uint32_t 
 #pragma unroll 1
     for (int k = 0; k < prefixes_; ++k) {
         uint32_t d[16];
-        tmem_load<16>(lane_base + band_slot<prefixes_, fused_>(first_unit, k), d);
+        tmem_load<16>(lane_base + band_slot<prefixes_, form_>(first_unit, k), d);
         float const inv_q = *(q_inv + static_cast<size_t>(k) * rows_q);
         float const row_beta = row_factor(beta, inv_q);
         float const without_row_factor = row_beta != 0.0f ? __fdividef(1.0f, row_beta) : 0.0f;
@@ -538,13 +581,13 @@ __device__ __noinline__ special_sums special_cells(uint32_t lane_base, uint32_t 
         own_dot += pick_column(d, static_cast<uint32_t>(own_column));
         partner_dot += pick_column(d, static_cast<uint32_t>(partner_column));
         if (own_column >= 0) {
-            cell_outcome const cell = cell_general(own_dot, inv_q, norms[k * fwd_cols + own_column], beta, bias, true, false, spec_code);
+            cell_outcome const cell = cell_general(own_dot, inv_q, norms[k * fwd_cols_for(form_) + own_column], beta, bias, true, false, spec_code);
             loss += cell.loss;
             total.cell += cell.cell, total.own_logit += cell.cell * beta;
         }
         if (partner_column >= 0) {
             cell_outcome const cell =
-                cell_general(partner_dot, inv_q, norms[k * fwd_cols + partner_column], beta, bias, false, true, spec_code);
+                cell_general(partner_dot, inv_q, norms[k * fwd_cols_for(form_) + partner_column], beta, bias, false, true, spec_code);
             loss += cell.loss;
             total.cell += cell.cell;
             partner_raw = cell.raw * without_row_factor;
@@ -567,17 +610,22 @@ __device__ __noinline__ special_sums special_cells(uint32_t lane_base, uint32_t 
 // What it costs: eleven packed float32 instructions per pair of cells and prefix, two cycles each, and one exponential per
 // cell, eight cycles; about 5000 cycles of a tile's 9700 at K=5 are bound by these. One block of 4096 rows, H=768, K=5: 98 ->
 // 88 us off the diagonal, 123 -> 89 us on it, against the form that parked every band in tensor memory.
-template <int prefixes_, bool fused_>
+template <int prefixes_, form_t form_>
 __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_params const& p, fwd_tail* tail,
                                               uint32_t store_base, float const* norm_ring, float* row_factors, uint32_t tmem_base,
-                                              wait_context const& ctx, uint32_t warp, uint32_t lane) {
-    constexpr uint32_t fwd_slots = fwd_slots_for(fused_);
+                                              wait_context const& ctx, uint32_t warp, uint32_t lane, uint32_t rank) {
+    constexpr uint32_t fwd_slots = fwd_slots_for(form_);
     constexpr int columns = fwd_chunk_columns_for(prefixes_);
     constexpr int parked = fwd_parked_bands_for(prefixes_);
     constexpr bool rolled = fwd_rolled_for(prefixes_);
     constexpr int warp_columns = fwd_warp_columns;
     uint32_t const quadrant = warp % 4, group = warp / 4;
-    uint32_t const row_local = quadrant * 32 + lane;
+    // Where the warp's patch lies in the strip and in the tile. A CTA of a pair has half the strip's rows; the upper half of its
+    // tensor-memory lanes holds the same rows' products with the tile's second 64 candidates.
+    uint32_t const patch_row = fwd_paired(form_) ? rank * fwd_own_rows(form_) + quadrant % 2 * 32 : quadrant * 32;
+    uint32_t const column_half = fwd_paired(form_) ? quadrant / 2 : 0u;
+    uint32_t const patch_column = column_half * 64 + group * fwd_warp_columns;
+    uint32_t const row_local = patch_row + lane;
     uint32_t const lane_base = tmem_base + ((quadrant * 32u) << 16) + group * warp_columns;
     uint32_t const quantities = 2 + 2 * prefixes_;
     float const beta = p.scalars != nullptr ? *p.scalars : p.beta;
@@ -585,12 +633,12 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
     uint32_t tile_local = 0;
     uint32_t const warp_store_base = store_base + warp * fwd_store_patches(prefixes_) * fwd_store_patch_bytes;
 
-    tile_cursor cursor;
+    tile_cursor<form_> cursor;
     cursor.go_to(p, 0);
-    uint32_t const items = item_count(p.items);
+    uint32_t const items = item_count<form_>(p.items);
     // Per-row sums of the item, in registers or in the thread's own words of shared memory; `coefficient` is kept without the
     // row factor beta / |q_k|. Lane k of a warp holds the largest inverse norm of the warp's rows at band k (`rows_max`).
-    constexpr bool shared_factors = fwd_factors_in_shared(prefixes_, fused_);
+    constexpr bool shared_factors = fwd_factors_in_shared(prefixes_, form_);
     constexpr int factor_stride = shared_factors ? fwd_epilogue_threads : 1;
     float own_factors[shared_factors ? 1 : prefixes_];
     float* const row_beta = shared_factors ? row_factors + threadIdx.x : own_factors;
@@ -606,6 +654,10 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
         }
     };
     float g = 0.0f, own_logit = 0.0f, rows_max = 0.0f;
+    auto give_back = [&](uint64_t* barrier) { // slots, to the issuer: in a pair the first CTA's
+        if constexpr (fwd_paired(form_)) mbar_arrive_cluster(smem_of(smem_u32(barrier), 0));
+        else mbar_arrive(smem_u32(barrier));
+    };
     uint32_t row = 0;
     phase_timer timer(p);
     timer.only_if(threadIdx.x == 0);
@@ -625,7 +677,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
                 break;
             }
             tcgen05_fence_after();
-            uint32_t const item = item_at(drained / p.tile_count);
+            uint32_t const item = item_at<form_>(drained / p.tile_count);
             uint32_t const word = p.tiles[drained % p.tile_count];
             float* const destination = p.gradient +
                                        (static_cast<size_t>(item / p.runs_per_strip) * fwd_rows + row_local) * p.hidden +
@@ -645,7 +697,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
 
     uint32_t strip_now = 0xFFFFFFFFu;
     while (cursor.n < items) {
-        if constexpr (fused_) drain(items_done * p.tile_count, false);
+        if constexpr (form_ == form_fused) drain(items_done * p.tile_count, false);
         uint32_t const strip = cursor.strip, run = cursor.run;
         if (strip != strip_now) {
             strip_now = strip;
@@ -667,15 +719,16 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
             }
             g = 0.0f, own_logit = 0.0f;
         }
-        uint32_t const column = cursor.column_tile(p) * fwd_cols + group * warp_columns;
+        uint32_t const column = cursor.column_tile(p) * fwd_cols_for(form_) + patch_column;
         uint32_t const entry = tile_local % fwd_norm_slots;
-        float const* const norms_now = norm_ring + entry * fwd_norm_floats(prefixes_) + group * warp_columns;
+        float const* const norms_now = norm_ring + entry * fwd_norm_floats(prefixes_, form_) + patch_column;
         // Does the diagonal cross this warp's patch? It does when the patch's columns come within one of its rows (a row's
         // own copy, or its pair partner next to it); then each row's own and partner cells are scored apart, and the others
         // as everywhere. Decided per warp, so that of a tile on the diagonal only the patches it crosses pay for that.
-        uint64_t const first_row = p.query_base + static_cast<uint64_t>(strip) * fwd_rows + quadrant * 32u;
+        uint64_t const first_row = p.query_base + static_cast<uint64_t>(strip) * fwd_rows + patch_row;
         uint64_t const first_column = p.candidate_base + column;
-        bool const special = first_column - first_row + warp_columns < 32u + 1 + warp_columns;
+        uint64_t const odd = first_row & 1u; // then the first row's partner lies a row before, the last one's a row behind the patch's
+        bool const special = form_ != form_pair_apart && first_column - first_row + (warp_columns - 1) + odd < 32u + (warp_columns - 1) + 2 * odd;
 
         timer.lap(0);
         if (!mbar_wait(smem_u32(&tail->tile_full[tile_local % fwd_tile_barriers]), (tile_local / fwd_tile_barriers) & 1u, ctx,
@@ -685,11 +738,21 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
         if (!mbar_wait(smem_u32(&tail->norms_full[entry]), (tile_local / fwd_norm_slots) & 1u, ctx, site_fwd_norms_full, tile_local))
             return;
         timer.lap(1);
+        if (fwd_paired(form_) && column >= p.rows_c) {
+            // The second half of the last tile, where the candidates are an odd number of 64s: nothing to score.
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                give_back(&tail->tile_taken[tile_local % fwd_slots]);
+                if (parked > 0) give_back(&tail->tile_parked_taken[tile_local % fwd_slots]);
+                mbar_arrive(smem_u32(&tail->norms_empty[entry]));
+            }
+        } else {
         // Bands in which some cosine of the patch may sit on the floor (one bit each).
         uint32_t floors = 0;
         {
             bool const may = lane < prefixes_ &&
-                             rows_max * norm_ring[entry * fwd_norm_floats(prefixes_) + prefixes_ * fwd_cols + lane % 8u] >= 100.0f;
+                             rows_max * norm_ring[entry * fwd_norm_floats(prefixes_, form_) + prefixes_ * fwd_cols_for(form_) + column_half * 8u + lane % 8u] >= 100.0f;
             floors = __ballot_sync(0xFFFFFFFFu, may);
         }
 
@@ -711,7 +774,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
             if (own_at >= 0 && own_at < warp_columns) own_column = static_cast<int>(own_at);
             if ((p.spec_code & 1u) != 0u && partner_at >= 0 && partner_at < warp_columns) partner_column = static_cast<int>(partner_at);
             special_sums const total =
-                special_cells<prefixes_, fused_>(lane_base, first_unit, norms_now, p.q_inv + row, p.rows_q, beta, bias, own_column,
+                special_cells<prefixes_, form_>(lane_base, first_unit, norms_now, p.q_inv + row, p.rows_q, beta, bias, own_column,
                                                  partner_column, p.spec_code, sums, sums_stride);
             g += total.cell, own_logit += total.own_logit;
             apart = (own_column >= 0 ? 1u << own_column : 0u) | (partner_column >= 0 ? 0x10001u << partner_column : 0u);
@@ -727,9 +790,9 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
         // gradient cube at the tile's place, or (fused kernel) of this CTA's scratch buffer of the item,
         // [band][128 rows][tiles_per_run * 64 candidates], at the tile's place in the run.
         auto store_patches = [&](int patch, int band) {
-            uint32_t const store_x = fused_ ? cursor.t * fwd_cols + group * warp_columns : column;
-            uint32_t const store_y = fused_ ? quadrant * 32u : strip * fwd_rows + quadrant * 32u;
-            uint32_t const store_z = fused_ ? (blockIdx.x * 2u + (items_done & 1u)) * prefixes_ : 0u;
+            uint32_t const store_x = form_ == form_fused ? cursor.t * fwd_cols_for(form_) + patch_column : column;
+            uint32_t const store_y = form_ == form_fused ? patch_row : strip * fwd_rows + patch_row;
+            uint32_t const store_z = form_ == form_fused ? (blockIdx.x * 2u + (items_done & 1u)) * prefixes_ : 0u;
             asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
                              reinterpret_cast<uint64_t>(cube_map)),
                          "r"(warp_store_base + patch * fwd_store_patch_bytes), "r"(store_x), "r"(store_y), "r"(store_z + band)
@@ -756,7 +819,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
                 pair_t inv_c[columns / 2];
 #pragma unroll
                 for (int c = 0; c < columns / 2; c += 2) {
-                    float4 const quad = *reinterpret_cast<float4 const*>(norms_now + k * fwd_cols + first + 2 * c);
+                    float4 const quad = *reinterpret_cast<float4 const*>(norms_now + k * fwd_cols_for(form_) + first + 2 * c);
                     inv_c[c] = pack2(quad.x, quad.y), inv_c[c + 1] = pack2(quad.z, quad.w);
                 }
                 if ((floors >> k) & 1u) {
@@ -838,7 +901,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
                     // scored apart are looked for only in patches that have any: for every patch it cost 2 % at four bands,
                     // 3 % at five and 6 % at six. Up to four bands there are registers to look ahead of the loop, which then
                     // has no branch in it (K=4, 4096 rows, H=768: 101.4 -> 98.7 us; in the fused form and with more bands it costs spills).
-                    constexpr bool ahead = !fused_ && prefixes_ <= 4;
+                    constexpr bool ahead = form_ != form_fused && prefixes_ <= 4;
                     auto natural = [&](int const c) { return fma2(prefix[c], mul2(inv_c[c], row_beta2), pack2(bias, bias)); };
                     if constexpr (ahead) {
 #pragma unroll
@@ -899,19 +962,19 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
             };
             auto load_bands = [&](auto& d, int const from, int const to) {
 #pragma unroll
-                for (int k = from; k < to; ++k) tmem_load<columns>(lane_base + band_slot<prefixes_, fused_>(first_unit, k) + first, d[k - from]);
+                for (int k = from; k < to; ++k) tmem_load<columns>(lane_base + band_slot<prefixes_, form_>(first_unit, k) + first, d[k - from]);
                 tmem_load_wait();
             };
             auto release_slots = [&](uint64_t* barriers) { // this warp is done with the tile's slots (or one kind of them)
                 if (first + columns != warp_columns) return;
                 tcgen05_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&barriers[tile_local % fwd_slots]));
+                if (lane == 0) give_back(&barriers[tile_local % fwd_slots]);
             };
             if constexpr (rolled) {
 #pragma unroll 1
                 for (int k = 0; k < prefixes_; ++k) {
-                    uint32_t const address = lane_base + band_slot<prefixes_, fused_>(first_unit, k);
+                    uint32_t const address = lane_base + band_slot<prefixes_, form_>(first_unit, k);
                     uint32_t d[columns];
                     tmem_load<columns>(address, d);
                     tmem_load_wait();
@@ -925,8 +988,8 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
                 for (int k = prefixes_ - 1; k >= 0; k -= 2) {
                     int const below = k > 0 ? k - 1 : 0, patch = ((prefixes_ - 1 - k) / 2 % 2) * 2;
                     uint32_t upper[columns], lower[columns];
-                    tmem_load<columns>(lane_base + band_slot<prefixes_, fused_>(first_unit, k), upper);
-                    tmem_load<columns>(lane_base + band_slot<prefixes_, fused_>(first_unit, below), lower);
+                    tmem_load<columns>(lane_base + band_slot<prefixes_, form_>(first_unit, k), upper);
+                    tmem_load<columns>(lane_base + band_slot<prefixes_, form_>(first_unit, below), lower);
                     tmem_load_wait();
                     if (k == prefixes_ - 1) release_slots(tail->tile_taken);
                     if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
@@ -949,7 +1012,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
 #pragma unroll
                     for (int k = 0; k < parked; ++k) {
                         score_band(k, d[k]);
-                        tmem_store_8(lane_base + band_slot<prefixes_, fused_>(first_unit, k) + first, d[k]);
+                        tmem_store_8(lane_base + band_slot<prefixes_, form_>(first_unit, k) + first, d[k]);
                     }
                 }
                 {
@@ -984,12 +1047,13 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
         }
         if (lane == 0) mbar_arrive(smem_u32(&tail->norms_empty[entry])); // every lane's reads are behind a __syncwarp above
         timer.lap(3);
-        if (cursor.t + 1 == p.tiles_per_run) {
+        }
+        if (cursor.t + 1 == run_length<form_>(p, run)) {
             // One partial record per (run, column group, row); the 1/N weight and the mirror cell's factor two go in here.
-            uint32_t const slot = run * fwd_column_groups + group;
+            uint32_t const slot = (run * (fwd_cols_for(form_) / 64) + column_half) * fwd_column_groups + group;
             float* record = p.partials + static_cast<size_t>(slot) * quantities * p.rows_q + row;
             if (SC_IN_BOUNDS((static_cast<size_t>(slot) * quantities + quantities - 1) * p.rows_q + row,
-                             static_cast<size_t>(p.runs_per_strip) * fwd_column_groups * quantities * p.rows_q)) {
+                             static_cast<size_t>(p.runs_per_strip) * (fwd_cols_for(form_) / 64) * fwd_column_groups * quantities * p.rows_q)) {
                 auto put = [&](uint32_t quantity, float value) { record[static_cast<size_t>(quantity) * p.rows_q] = value; };
                 // sum of cell gradient * logit: the coefficients are exactly that, except for a row's own copy, whose logit
                 // is the scale itself and which moves no dot product
@@ -1006,7 +1070,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
                 put(0, p.weight * g);
                 put(1, p.weight * logits);
             }
-            if constexpr (fused_) {
+            if constexpr (form_ == form_fused) {
                 // The item's patches of this warp are in memory once its bulk stores have completed (not merely been
                 // read out of the staging buffers); then the gradient GEMM's producer may load them.
                 if (lane == 0) {
@@ -1026,7 +1090,7 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
     timer.flush(p, 5, 4);
     // The staging buffers must outlive the stores that read them.
     if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-    if constexpr (fused_) drain(items_done * p.tile_count, true);
+    if constexpr (form_ == form_fused) drain(items_done * p.tile_count, true);
 }
 
 // ---- fused kernel: the gradient GEMM's two roles ------------------------------------------------------------------
@@ -1038,15 +1102,15 @@ __device__ __forceinline__ void fz_producer_role(fz_maps const* maps, fwd_params
     if (!elect_one()) return;
     uint32_t stage = 0, phase = 0, local = 0;
     phase_timer timer(p);
-    for (uint32_t count = item_count(p.items); local < count; ++local) {
-        uint32_t const item = item_at(local);
+    for (uint32_t count = item_count<form_fused>(p.items); local < count; ++local) {
+        uint32_t const item = item_at<form_fused>(local);
         uint32_t const buffer = local & 1u;
         timer.lap(0);
         if (!mbar_wait_relaxed(smem_u32(&tail->fz_item_stored[buffer]), (local >> 1) & 1u, ctx, site_fz_item_stored, item, sleep_gemm_ns))
             return;
         timer.lap(1);
         fence_proxy_async_all();
-        uint32_t const first_candidate = (item % p.runs_per_strip) * p.tiles_per_run * fwd_cols;
+        uint32_t const first_candidate = (item % p.runs_per_strip) * p.tiles_per_run * fwd_cols_for(form_fused);
         for (uint32_t which = 0; which < p.tile_count; ++which) {
             uint32_t const word = p.tiles[which];
             uint32_t const band = word & 0xFu, channel0 = ((word >> 4) & 0xFFFu) * 16u, width = (word >> 16) * 16u;
@@ -1086,8 +1150,7 @@ __device__ __forceinline__ void fz_mma_role(fwd_params const& p, uint32_t stages
     uint32_t const accumulator = tmem_base + fz_accumulator_column;
     uint32_t stage = 0, phase = 0, unit = 0;
     phase_timer timer(p);
-    for (uint32_t n = 0, count = item_count(p.items); n < count; ++n) {
-        uint32_t const item = item_at(n);
+    for (uint32_t n = 0, count = item_count<form_fused>(p.items); n < count; ++n) {
         for (uint32_t which = 0; which < p.tile_count; ++which, ++unit) {
             uint32_t const idesc = umma_idesc_bf16(128, (p.tiles[which] >> 16) * 16u);
             // The accumulator's previous contents must have left tensor memory (an arrival per epilogue warp).
@@ -1139,18 +1202,18 @@ __device__ __forceinline__ void pull_role(pull_request const& request, uint32_t 
     }
 }
 
-template <int prefixes_, bool fused_>
+template <int prefixes_, form_t form_>
 __global__ void __launch_bounds__(fwd_threads, 1)
     forward_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap c_map,
                    const __grid_constant__ CUtensorMap cube_map, const __grid_constant__ fz_maps gemm_maps,
                    const fwd_params p) {
-    constexpr uint32_t fwd_slots = fwd_slots_for(fused_);
-    constexpr uint32_t stages = fwd_stages_for(prefixes_, fused_);
+    constexpr uint32_t fwd_slots = fwd_slots_for(form_);
+    constexpr uint32_t stages = fwd_stages_for(prefixes_, form_);
     extern __shared__ uint8_t raw_shared[];
     uint32_t const raw_address = smem_u32(raw_shared);
     uint32_t const stages_base = (raw_address + 1023u) & ~1023u;
-    uint32_t const gemm_stages_base = stages_base + stages * fwd_stage_bytes;
-    uint32_t const store_base = stages_base + fwd_stage_region_bytes(prefixes_, fused_);
+    uint32_t const gemm_stages_base = stages_base + stages * fwd_stage_bytes(form_);
+    uint32_t const store_base = stages_base + fwd_stage_region_bytes(prefixes_, form_);
     fwd_tail* tail = reinterpret_cast<fwd_tail*>(raw_shared + (store_base - raw_address) + fwd_store_bytes(prefixes_));
     uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 
@@ -1160,15 +1223,15 @@ __global__ void __launch_bounds__(fwd_threads, 1)
             mbar_init(smem_u32(&tail->stage_empty[i]), 1);
         }
         for (uint32_t i = 0; i < fwd_slots; ++i) {
-            mbar_init(smem_u32(&tail->tile_taken[i]), fwd_epilogue_warps);
-            mbar_init(smem_u32(&tail->tile_parked_taken[i]), fwd_epilogue_warps);
+            mbar_init(smem_u32(&tail->tile_taken[i]), fwd_ctas_for(form_) * fwd_epilogue_warps);
+            mbar_init(smem_u32(&tail->tile_parked_taken[i]), fwd_ctas_for(form_) * fwd_epilogue_warps);
         }
         for (uint32_t i = 0; i < fwd_tile_barriers; ++i) mbar_init(smem_u32(&tail->tile_full[i]), 1);
         for (uint32_t i = 0; i < fwd_norm_slots; ++i) {
             mbar_init(smem_u32(&tail->norms_full[i]), 1);
             mbar_init(smem_u32(&tail->norms_empty[i]), fwd_epilogue_warps);
         }
-        if constexpr (fused_) {
+        if constexpr (form_ == form_fused) {
             for (uint32_t i = 0; i < fz_stages; ++i) {
                 mbar_init(smem_u32(&tail->fz_stage_full[i]), 1);
                 mbar_init(smem_u32(&tail->fz_stage_empty[i]), 1);
@@ -1181,22 +1244,34 @@ __global__ void __launch_bounds__(fwd_threads, 1)
         fence_barrier_init();
     }
     if (warp == fwd_mma_warp) {
-        tmem_alloc(smem_u32(&tail->tmem_base), fwd_tmem_columns);
-        tmem_relinquish();
+        if constexpr (fwd_paired(form_)) {
+            tmem_alloc_pair(smem_u32(&tail->tmem_base), fwd_tmem_columns);
+            tmem_relinquish_pair();
+        } else {
+            tmem_alloc(smem_u32(&tail->tmem_base), fwd_tmem_columns);
+            tmem_relinquish();
+        }
     }
     if (warp == fwd_producer_warp && lane == 0) {
         tma_prefetch_descriptor(&q_map);
         tma_prefetch_descriptor(&c_map);
     }
-    if constexpr (fused_) {
+    if constexpr (form_ == form_fused) {
         if (warp == fwd_first_pull_warp && lane == 0) {
             tma_prefetch_descriptor(&gemm_maps.patches);
             for (uint32_t i = 0; i < fz_candidate_maps; ++i) tma_prefetch_descriptor(&gemm_maps.candidates[i]);
         }
     }
-    // Everything up to here may run beside the end of the kernel before.
     let_dependents_start();
+    uint32_t rank = 0;
+    if constexpr (fwd_paired(form_)) {
+        rank = cluster_rank();
+        cluster_sync(); // the other CTA's barriers are set up
+    }
+    // Everything up to here may run beside the end of the kernel before.
     wait_for_kernels_before();
+    // (Both CTAs of a pair read the same: only kernels before this one have written it, or waits of this one that ran out, long after
+    // its CTAs have started; should they ever disagree, the other's waits run out too.)
     if (threadIdx.x == 0) tail->abort_flag = status_poisoned(p.status) ? 1u : 0u;
     tcgen05_fence_before();
     __syncthreads();
@@ -1209,21 +1284,21 @@ __global__ void __launch_bounds__(fwd_threads, 1)
     if (poisoned) {
     } else if (warp < fwd_epilogue_warps) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(fwd_epilogue_registers));
-        epilogue_role<prefixes_, fused_>(&cube_map, p, tail, store_base, norm_ring, norm_ring + fwd_norm_bytes(prefixes_) / 4, tmem_base, ctx, warp,
-                                         lane);
+        epilogue_role<prefixes_, form_>(&cube_map, p, tail, store_base, norm_ring, norm_ring + fwd_norm_bytes(prefixes_, form_) / 4, tmem_base, ctx, warp,
+                                         lane, rank);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(fwd_helper_registers));
         if (warp == fwd_producer_warp) {
-            producer_role<prefixes_>(&q_map, &c_map, p, stages_base, norm_ring, tail, ctx, stages);
+            producer_role<prefixes_, form_>(&q_map, &c_map, p, stages_base, norm_ring, tail, ctx, rank);
         } else if (warp == fwd_mma_warp) {
-            mma_role<prefixes_, fused_>(p, stages_base, tail, tmem_base, ctx);
+            if (rank == 0) mma_role<prefixes_, form_>(p, stages_base, tail, tmem_base, ctx);
         } else if (warp == fwd_first_pull_warp) {
             // The pull is a short copy at the start of the launch; the gradient GEMM's first item is not ready before the
             // epilogue warps have scored a whole item, so the same warp serves both.
             pull_role(p.pull, threadIdx.x - fwd_first_pull_warp * 32);
-            if constexpr (fused_) fz_producer_role(&gemm_maps, p, gemm_stages_base, tail, ctx, prefixes_);
+            if constexpr (form_ == form_fused) fz_producer_role(&gemm_maps, p, gemm_stages_base, tail, ctx, prefixes_);
         } else if (warp == fz_mma_warp) {
-            if constexpr (fused_) fz_mma_role(p, gemm_stages_base, tail, tmem_base, ctx);
+            if constexpr (form_ == form_fused) fz_mma_role(p, gemm_stages_base, tail, tmem_base, ctx);
         }
     }
 
@@ -1235,61 +1310,126 @@ __global__ void __launch_bounds__(fwd_threads, 1)
         uint64_t const start = global_timer_ns();
         while (global_timer_ns() - start < 200000ull) __nanosleep(1000);
     }
-    __syncthreads();
+    // A pair's barriers and operands are used by both CTAs until both are done.
+    if constexpr (fwd_paired(form_)) cluster_sync();
+    else __syncthreads();
     if (warp == fwd_mma_warp) {
         tcgen05_fence_after();
-        tmem_dealloc(tmem_base, fwd_tmem_columns);
+        if constexpr (fwd_paired(form_)) tmem_dealloc_pair(tmem_base, fwd_tmem_columns);
+        else tmem_dealloc(tmem_base, fwd_tmem_columns);
     }
 }
 
 // ---- host side --------------------------------------------------------------------------------------------------
-template <int prefixes_, bool fused_>
+template <int prefixes_, form_t form_>
 void launch_instance(CUtensorMap const& q_map, CUtensorMap const& c_map, CUtensorMap const& cube_map, fz_maps const& gemm_maps,
                      fwd_params const& p, int blocks, cudaStream_t stream, bool overlap) {
     // The attribute is per device; a process drives one GPU, but a second one costs only the repeat of a cheap call.
-    static int prepared_device = -1;
+    static int prepared_device = -1, resident = 0;
     int device = 0;
     cudaGetDevice(&device);
     if (prepared_device != device) {
-        require(cudaFuncSetAttribute(forward_kernel<prefixes_, fused_>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     fwd_shared_bytes(prefixes_, fused_)),
+        require(cudaFuncSetAttribute(forward_kernel<prefixes_, form_>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     fwd_shared_bytes(prefixes_, form_)),
                 "raising the forward kernel's shared memory");
+        resident = 1 << 30;
+        if constexpr (fwd_paired(form_)) {
+            // How many pairs the device holds at a time: the walk over the items assumes that all of them run.
+            cudaLaunchAttribute attribute{};
+            attribute.id = cudaLaunchAttributeClusterDimension;
+            attribute.val.clusterDim.x = 2, attribute.val.clusterDim.y = 1, attribute.val.clusterDim.z = 1;
+            cudaLaunchConfig_t config{};
+            config.gridDim = 2, config.blockDim = fwd_threads, config.dynamicSmemBytes = fwd_shared_bytes(prefixes_, form_);
+            config.attrs = &attribute, config.numAttrs = 1;
+            require(cudaOccupancyMaxActiveClusters(&resident, forward_kernel<prefixes_, form_>, &config), "asking for the resident pairs");
+            if (resident < 1) throw std::runtime_error("forward: the device holds no pair of CTAs");
+            resident *= 2;
+        }
         prepared_device = device;
     }
-    launch_dependent(overlap, forward_kernel<prefixes_, fused_>, blocks, fwd_threads, fwd_shared_bytes(prefixes_, fused_), stream, q_map, c_map,
-                     cube_map, gemm_maps, p);
+    launch_dependent_clusters(overlap, fwd_ctas_for(form_), forward_kernel<prefixes_, form_>, blocks < resident ? blocks : resident, fwd_threads,
+                              fwd_shared_bytes(prefixes_, form_), stream, q_map, c_map, cube_map, gemm_maps, p);
 }
 
-template <bool fused_>
+template <form_t form_>
 void launch_for_count(uint32_t count, CUtensorMap const& q_map, CUtensorMap const& c_map, CUtensorMap const& cube_map,
                       fz_maps const& gemm_maps, fwd_params const& p, int blocks, cudaStream_t stream, bool overlap) {
     switch (count) {
-    case 1: launch_instance<1, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
-    case 2: launch_instance<2, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
-    case 3: launch_instance<3, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
-    case 4: launch_instance<4, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
-    case 5: launch_instance<5, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
-    case 6: launch_instance<6, fused_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
+    case 1: launch_instance<1, form_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
+    case 2: launch_instance<2, form_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
+    case 3: launch_instance<3, form_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
+    case 4: launch_instance<4, form_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
+    case 5: launch_instance<5, form_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
+    case 6: launch_instance<6, form_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap); break;
     default:
-        if constexpr (!fused_) {
-            if (count == 7) launch_instance<7, false>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap);
-            else launch_instance<8, false>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap);
+        if constexpr (form_ != form_fused) {
+            if (count == 7) launch_instance<7, form_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap);
+            else launch_instance<8, form_>(q_map, c_map, cube_map, gemm_maps, p, blocks, stream, overlap);
         }
         break;
     }
 }
 
+template <form_t form_> void preload_form() {
+    cudaFuncAttributes attributes;
+    require(cudaFuncGetAttributes(&attributes, forward_kernel<1, form_>), "preload forward<1>");
+    require(cudaFuncGetAttributes(&attributes, forward_kernel<2, form_>), "preload forward<2>");
+    require(cudaFuncGetAttributes(&attributes, forward_kernel<3, form_>), "preload forward<3>");
+    require(cudaFuncGetAttributes(&attributes, forward_kernel<4, form_>), "preload forward<4>");
+    require(cudaFuncGetAttributes(&attributes, forward_kernel<5, form_>), "preload forward<5>");
+    require(cudaFuncGetAttributes(&attributes, forward_kernel<6, form_>), "preload forward<6>");
+    if constexpr (form_ != form_fused) {
+        require(cudaFuncGetAttributes(&attributes, forward_kernel<7, form_>), "preload forward<7>");
+        require(cudaFuncGetAttributes(&attributes, forward_kernel<8, form_>), "preload forward<8>");
+    }
+}
+
 } // namespace
 
-uint32_t forward_partial_slots(uint32_t rows_c, uint32_t tiles_per_run) {
-    return fwd_column_groups * (rows_c / fwd_cols) / tiles_per_run;
+// Which form a launch takes; by sizes and numbers alone, so that a block takes the same one however much of the GPU it gets.
+// - Every tile of 64 at once on the GPU: a single CTA each. A pair's barriers and commits across CTAs cost a launch 0.7 us (128 rows,
+//   H=768, K=5: 11.6 against 12.4 us; 1024 rows 12.2 against 13.0).
+// - A block without the rows' own copies: the pair's form that has nothing of the diagonal in it (one block of 4096 rows, H=768, K=5: 74.7
+//   us against 80.7 with a single CTA and 82.3 with a pair that can score the diagonal; 2944 rows, H=832, K=4: 44.8, 49.3, 50.8;
+//   16384 rows, H=768, K=5: 1130, 1248, 1215; every cell in the general form, 8192 rows, H=512, K=4: 328, 359, 371).
+// - A block with them: a pair loads a third fewer operand bytes per cell, and where those weigh more than the cells' arithmetic, which
+//   goes with the channels per band, it is faster: H=1024, K=1, 8192 rows 166 against 175 us, H=768, K=3, 4096 rows 69 against 78,
+//   H=1024, K=4 81 against 86, K=7 145 against 153. It is not for few channels (H=512, K=4, 4096 rows 70 against 66; H=832, K=4, 2944
+//   rows 51 against 49.5), and in between for large launches, which run at the GPU's power limit (H=768, K=5: 4096
+//   rows 83.4 against 82.1, 16384 rows 1229 against 1270; H=1024, K=6: 4096 rows 124 either way, 8192 rows 418 against 454).
+static form_t forward_form(forward_arguments const& a) {
+    if (a.fused) return form_fused;
+    uint32_t const column_tiles = a.rows_c / 64, bands = a.ladder.count;
+    uint64_t const singles = static_cast<uint64_t>(a.rows_q / fwd_rows) * column_tiles;
+    if (column_tiles % 2) return form_pair; // the only one that can do without half a tile
+    if (singles <= 148) return form_single;
+    // A row's own copy is the candidate of the same number, its partner the other of the pair 2m, 2m + 1.
+    uint64_t const first = a.query_base & ~1ull, behind = (a.query_base + a.rows_q + 1) & ~1ull;
+    bool const apart = a.candidate_base >= behind || a.candidate_base + a.rows_c <= first;
+    if (apart) return form_pair_apart;
+    bool const large = static_cast<uint64_t>(a.rows_q) * a.rows_c >= (1ull << 26);
+    return bands >= 7 || a.hidden >= (large ? 144 : 256) * bands ? form_pair : form_single;
 }
+// A run is `tiles_per_run` tiles, of 64 candidates or, in a pair, of 128, and has one record per 64 columns of a tile and column group. A
+// pair's last run may be shorter.
+static uint32_t runs_of(form_t form, uint32_t rows_c, uint32_t tiles_per_run) {
+    uint32_t const tiles = (rows_c + fwd_cols_for(form) - 1) / fwd_cols_for(form);
+    return (tiles + tiles_per_run - 1) / tiles_per_run;
+}
+static uint32_t slots_of(form_t form, uint32_t rows_c, uint32_t tiles_per_run) {
+    return fwd_column_groups * (fwd_cols_for(form) / 64) * runs_of(form, rows_c, tiles_per_run);
+}
+uint32_t forward_partial_slots(uint32_t rows_c, uint32_t tiles_per_run) {
+    uint32_t const single = slots_of(form_single, rows_c, tiles_per_run), pair = slots_of(form_pair, rows_c, tiles_per_run);
+    return single > pair ? single : pair;
+}
+uint32_t forward_filled_slots(forward_arguments const& a) { return slots_of(forward_form(a), a.rows_c, a.tiles_per_run); }
 uint32_t forward_quantities(uint32_t prefixes) { return 2 + 2 * prefixes; }
 
 uint32_t forward_choose_tiles_per_run(uint32_t rows_q, uint32_t rows_c, int multiprocessors) {
-    uint32_t const strips = rows_q / fwd_rows, column_tiles = rows_c / fwd_cols;
+    uint32_t const strips = rows_q / fwd_rows, column_tiles = rows_c / 64;
     uint32_t best = 1;
-    for (uint32_t t = 1; t <= 32 && column_tiles % t == 0; t *= 2)
+    for (uint32_t t = 1; t <= 32 && column_tiles % t == 0 && (t == 1 || 2 * t <= column_tiles); t *= 2)
         if (static_cast<uint64_t>(strips) * (column_tiles / t) >= 6ull * static_cast<uint64_t>(multiprocessors)) best = t;
     return best;
 }
@@ -1300,7 +1440,7 @@ bool forward_fused_supported(uint32_t hidden, uint32_t prefixes) { return prefix
 // gradient once per item: runs of at least four tiles keep those additions rare, longer runs are taken while enough
 // items remain to balance the GPU.
 uint32_t forward_choose_tiles_per_run_fused(uint32_t rows_q, uint32_t rows_c, int multiprocessors) {
-    uint32_t const strips = rows_q / fwd_rows, column_tiles = rows_c / fwd_cols;
+    uint32_t const strips = rows_q / fwd_rows, column_tiles = rows_c / fwd_cols_for(form_fused);
     uint32_t best = 1;
     for (uint32_t t = 1; t <= fz_max_tiles_per_run && column_tiles % t == 0; t *= 2)
         if (t <= 4 || static_cast<uint64_t>(strips) * (column_tiles / t) >= 6ull * static_cast<uint64_t>(multiprocessors)) best = t;
@@ -1309,18 +1449,18 @@ uint32_t forward_choose_tiles_per_run_fused(uint32_t rows_q, uint32_t rows_c, in
 
 // Two buffers per CTA of [prefixes][128 rows][tiles_per_run * 64 candidates] bfloat16.
 size_t forward_fused_scratch_bytes(uint32_t prefixes, uint32_t tiles_per_run, int multiprocessors) {
-    return static_cast<size_t>(multiprocessors) * 2 * prefixes * fwd_rows * tiles_per_run * fwd_cols * 2;
+    return static_cast<size_t>(multiprocessors) * 2 * prefixes * fwd_rows * tiles_per_run * fwd_cols_for(form_fused) * 2;
 }
 
 void launch_forward(forward_arguments const& a, cudaStream_t stream) {
-    if (a.rows_q % fwd_rows || a.rows_c % fwd_cols || a.hidden % fwd_depth || a.hidden > 4096)
+    if (a.rows_q % fwd_rows || a.rows_c % 64 || a.hidden % fwd_depth || a.hidden > 4096)
         throw std::runtime_error("forward: rows must be multiples of 128 (queries) and 64 (candidates), hidden of 64 up to 4096");
     if (a.ladder.count < 1 || a.ladder.count > 8 || a.ladder.ends[a.ladder.count - 1] != a.hidden)
         throw std::runtime_error("forward: the ladder's widest prefix must equal hidden");
     for (uint32_t band = 0, begin = 0; band < a.ladder.count; begin = a.ladder.ends[band++])
         if (a.ladder.ends[band] % 16 || a.ladder.ends[band] <= begin)
             throw std::runtime_error("forward: band edges must ascend in multiples of 16");
-    uint32_t const column_tiles = a.rows_c / fwd_cols;
+    uint32_t const column_tiles = a.rows_c / 64;
     if (a.tiles_per_run == 0 || column_tiles % a.tiles_per_run)
         throw std::runtime_error("forward: tiles_per_run must divide the number of candidate tiles");
     if (a.pull.bytes[0] % 16 || a.pull.bytes[1] % 16) throw std::runtime_error("forward: pull sizes must be multiples of 16");
@@ -1333,8 +1473,10 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
     p.rows_q = a.rows_q, p.rows_c = a.rows_c, p.hidden = a.hidden;
     p.ladder.count = a.ladder.count;
     for (int i = 0; i < 8; ++i) p.ladder.ends[i] = a.ladder.ends[i];
+    form_t const form = forward_form(a);
     p.tiles_per_run = a.tiles_per_run;
-    p.runs_per_strip = column_tiles / a.tiles_per_run;
+    p.tiles_per_strip = fwd_paired(form) ? (column_tiles + 1) / 2 : column_tiles;
+    p.runs_per_strip = runs_of(form, a.rows_c, a.tiles_per_run);
     p.items = (a.rows_q / fwd_rows) * p.runs_per_strip;
     p.beta = a.beta, p.bias = a.bias, p.weight = a.weight;
     p.scalars = a.scalars;
@@ -1352,9 +1494,10 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
         }
         p.band_starts[chunk] = word;
     }
-    int blocks = static_cast<int>(p.items < static_cast<uint32_t>(a.multiprocessors) ? p.items : a.multiprocessors);
-    if ((a.pull.bytes[0] | a.pull.bytes[1]) != 0 && blocks < a.multiprocessors / 2) blocks = a.multiprocessors / 2;
-    if (blocks < 1) blocks = 1;
+    int const ctas = static_cast<int>(fwd_ctas_for(form)), walkers = a.multiprocessors / ctas;
+    int blocks = static_cast<int>(p.items < static_cast<uint32_t>(walkers) ? p.items : walkers);
+    if ((a.pull.bytes[0] | a.pull.bytes[1]) != 0 && blocks < walkers / 2) blocks = walkers / 2;
+    blocks = (blocks < 1 ? 1 : blocks) * ctas;
 
     if (a.fused) {
         if (!forward_fused_supported(a.hidden, a.ladder.count))
@@ -1366,8 +1509,8 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
             throw std::runtime_error("forward: the fused kernel needs its scratch, the transposed candidates and the gradient");
     }
     // Everything above is checked before the first driver or runtime call.
-    CUtensorMap const q_map = cached_operand_map(a.queries_bf16, a.hidden, a.rows_q, fwd_depth, fwd_rows);
-    CUtensorMap const c_map = cached_operand_map(a.candidates_bf16, a.hidden, a.rows_c, fwd_depth, fwd_cols);
+    CUtensorMap const q_map = cached_operand_map(a.queries_bf16, a.hidden, a.rows_q, fwd_depth, fwd_own_rows(form));
+    CUtensorMap const c_map = cached_operand_map(a.candidates_bf16, a.hidden, a.rows_c, fwd_depth, fwd_own_cols(form));
     fz_maps gemm_maps{};
     if (!a.fused) {
         // The warps' patches of the gradient cube [K, rows_q, rows_c]: boxes of all bands x 32 rows x 16 candidates, staged under the
@@ -1377,7 +1520,11 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
         cuuint32_t const box[3] = {fwd_warp_columns, 32, fwd_rolled_for(static_cast<int>(a.ladder.count)) ? 1u : a.ladder.count};
         CUtensorMap const cube_map =
             cached_map(a.gradient_cube_bf16, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
-        launch_for_count<false>(a.ladder.count, q_map, c_map, cube_map, gemm_maps, p, blocks, stream, !a.ordinary_launch);
+        switch (form) {
+        case form_single: launch_for_count<form_single>(a.ladder.count, q_map, c_map, cube_map, gemm_maps, p, blocks, stream, !a.ordinary_launch); break;
+        case form_pair: launch_for_count<form_pair>(a.ladder.count, q_map, c_map, cube_map, gemm_maps, p, blocks, stream, !a.ordinary_launch); break;
+        default: launch_for_count<form_pair_apart>(a.ladder.count, q_map, c_map, cube_map, gemm_maps, p, blocks, stream, !a.ordinary_launch); break;
+        }
     } else {
         p.gradient = a.query_gradient, p.gradient_scale = a.gradient_scale;
         for (uint32_t band = 0, begin = 0; band < a.ladder.count; begin = a.ladder.ends[band++])
@@ -1388,7 +1535,7 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
             }
         // Scratch of gradient patches: [CTA and buffer][band][128 rows][run of candidates], written in the warps' boxes
         // (under the 32-byte swizzle), read back as the GEMM's A operand (128 rows x 64 candidates, swizzled).
-        uint64_t const run = static_cast<uint64_t>(a.tiles_per_run) * fwd_cols;
+        uint64_t const run = static_cast<uint64_t>(a.tiles_per_run) * fwd_cols_for(form_fused);
         cuuint64_t const dims[3] = {run, fwd_rows, static_cast<cuuint64_t>(blocks) * 2 * a.ladder.count};
         cuuint64_t const strides[2] = {run * 2, run * fwd_rows * 2};
         cuuint32_t const store_box[3] = {fwd_warp_columns, 32, a.ladder.count};
@@ -1403,7 +1550,7 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
             gemm_maps.candidates[index] =
                 cached_operand_map(a.transposed_candidates, a.rows_c, a.hidden, fz_depth, channels <= a.hidden ? channels : 16u);
         }
-        launch_for_count<true>(a.ladder.count, q_map, c_map, store_map, gemm_maps, p, blocks, stream, !a.ordinary_launch);
+        launch_for_count<form_fused>(a.ladder.count, q_map, c_map, store_map, gemm_maps, p, blocks, stream, !a.ordinary_launch);
     }
     cudaError_t const error = cudaGetLastError();
     if (error != cudaSuccess) throw std::runtime_error(std::string("forward launch failed: ") + cudaGetErrorString(error));
@@ -1413,21 +1560,10 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
 SC_DEFINE_BOUNDS_READER(bounds_record_forward)
 
 void preload_forward_kernels() {
-    cudaFuncAttributes attributes;
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<1, false>), "preload forward<1>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<2, false>), "preload forward<2>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<3, false>), "preload forward<3>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<4, false>), "preload forward<4>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<5, false>), "preload forward<5>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<6, false>), "preload forward<6>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<7, false>), "preload forward<7>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<8, false>), "preload forward<8>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<1, true>), "preload fused forward<1>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<2, true>), "preload fused forward<2>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<3, true>), "preload fused forward<3>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<4, true>), "preload fused forward<4>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<5, true>), "preload fused forward<5>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<6, true>), "preload fused forward<6>");
+    preload_form<form_single>();
+    preload_form<form_pair>();
+    preload_form<form_pair_apart>();
+    preload_form<form_fused>();
 }
 
 } // namespace sc

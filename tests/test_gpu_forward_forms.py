@@ -1,0 +1,98 @@
+"""The forward kernel's forms (one CTA per tile, pairs of CTAs, pairs without anything of the diagonal) at the sizes and places where the
+choice between them, or a tile of theirs, ends: each block against float64, own copies and partners inside, beside and astride."""
+import pytest
+import torch
+
+from scalingcontrasts_b200 import LossSpec, Matryoshka, StreamedLoss
+from scalingcontrasts_b200._ext import native, stream_handle
+from scalingcontrasts_b200.cpu.streamed import CpuStreamedLoss
+
+pytestmark = pytest.mark.gpu
+
+# As for the forms of the cell math: the functions are good to about 1e-7, sums of rows * columns terms in float32; the gradient leaves
+# through bfloat16 cubes and a bfloat16 store.
+SUMMAND_TOLERANCE, GRADIENT_TOLERANCE = 2e-5, 8e-3
+
+
+def _rows(rows, hidden, seed):
+    generator = torch.Generator(device="cuda").manual_seed(seed)
+    values = torch.randn(rows, hidden, device="cuda", generator=generator)
+    values[1::2] = 0.6 * values[0::2] + 0.8 * values[1::2]
+    return torch.nn.functional.normalize(values, dim=1).to(torch.bfloat16)
+
+
+def _check(queries, block, ladder, spec, query_base, candidate_base, beta=10.0, bias=-10.0):
+    rows, hidden = queries.shape
+    live = rows + block.shape[0]
+    loss = StreamedLoss(rows, hidden, ladder, spec, "cuda", candidate_rows=block.shape[0])
+    for scratch in (loss.partials, loss.similarity_gradients):
+        scratch.fill_(float("nan"))
+    loss.begin(queries)
+    loss.score(queries, block, query_base, candidate_base, beta, bias, live)
+    gradient, summands = loss.finish(queries)
+    loss.check()
+    reference = CpuStreamedLoss(rows, hidden, ladder, spec, torch.float64, "cuda")
+    reference.begin(queries)
+    reference.score(queries, block, query_base, candidate_base, beta, bias, live)
+    expected, sums = reference.finish(queries, torch.empty(rows, hidden, dtype=torch.float64, device="cuda"))
+    assert float((gradient.double() - expected).norm() / expected.norm()) < GRADIENT_TOLERANCE
+    assert torch.allclose(summands[4:4 + ladder.count].double(), sums[4:4 + ladder.count].double(), rtol=SUMMAND_TOLERANCE, atol=0.0)
+
+
+@pytest.mark.parametrize("rows,candidates", [(1152, 1024), (1280, 1024), (128, 9472), (128, 9600), (2432, 512), (1152, 1152),
+                                             (4736, 5248)])  # the last: runs of two tiles, 41 tiles to a strip
+@pytest.mark.parametrize("prefixes", [1, 4, 5, 8])
+def test_both_sides_of_one_wave(rows, candidates, prefixes):
+    """148 tiles of 64 candidates go to single CTAs, more to pairs or to a walk over the tiles."""
+    ladder = Matryoshka(tuple(64 * (k + 1) for k in range(prefixes)))
+    queries, block = _rows(rows, ladder.hidden, 1), _rows(candidates, ladder.hidden, 2)
+    for base in (0, 128 * 1024):
+        _check(queries, block, ladder, LossSpec("pairs"), 0, base)
+
+
+@pytest.mark.parametrize("spec", [LossSpec("self"), LossSpec("pairs"), LossSpec("pairs", "skip")], ids=lambda s: f"{s.positives}-{s.diagonal}")
+@pytest.mark.parametrize("query_base,candidate_base", [(0, 0), (1536, 0), (0, 1536), (0, 1535), (1535, 0), (1537, 0), (0, 1537), (1, 1537),
+                                                       (1537, 1), (3, 0), (0, 17), (1520, 0), (64, 0)])
+def test_own_copies_and_partners_wherever_they_lie(spec, query_base, candidate_base):
+    """Blocks side by side hold no own copies; where a number is odd a partner can be just across the border."""
+    ladder = Matryoshka((48, 160, 256))
+    queries, block = _rows(1536, ladder.hidden, 3), _rows(1536, ladder.hidden, 4)
+    _check(queries, block, ladder, spec, query_base, candidate_base)
+
+
+@pytest.mark.parametrize("prefixes", [1, 3, 5, 6, 8])
+@pytest.mark.parametrize("rows_c", [64, 192, 1088])
+def test_an_odd_number_of_64_candidates(prefixes, rows_c):
+    """The native launch takes candidates in 64s: the last tile of a pair is then half empty, and what lies behind the cube and the
+    norms is neither read into the sums nor written."""
+    ext, rows_q, ladder = native(), 256, Matryoshka(tuple(64 * (k + 1) for k in range(prefixes)))
+    hidden = ladder.hidden
+    queries, block = _rows(rows_q, hidden, 5), _rows(rows_c, hidden, 6)
+    quantities, slots = ext.forward_quantities(prefixes), ext.forward_partial_slots(rows_c, 1)
+    f32 = dict(dtype=torch.float32, device="cuda")
+
+    def norms(values):
+        inverse, largest = torch.empty(prefixes, values.shape[0], **f32), torch.empty(prefixes, values.shape[0] // 64, **f32)
+        ext.prefix_norms(values.data_ptr(), 0, inverse.data_ptr(), largest.data_ptr(), values.shape[0], hidden, list(ladder.ends), stream_handle())
+        return inverse, largest
+
+    (q_inverse, _), (c_inverse, c_largest) = norms(queries), norms(block)
+    cube = torch.full((prefixes * rows_q * rows_c + 4096,), 7.0, dtype=torch.bfloat16, device="cuda")
+    partials = torch.full((slots * quantities * rows_q + 4096,), 7.0, **f32)
+    status = torch.zeros(8, dtype=torch.int32, device="cuda")
+    ext.forward(queries=queries.data_ptr(), candidates=block.data_ptr(), q_inv=q_inverse.data_ptr(), c_inv=c_inverse.data_ptr(),
+                c_tile_max=c_largest.data_ptr(), cube=cube.data_ptr(), partials=partials.data_ptr(), status=status.data_ptr(), rows_q=rows_q,
+                rows_c=rows_c, hidden=hidden, ends=list(ladder.ends), tiles_per_run=1, beta=10.0, bias=-10.0, weight=1.0, scalars=0,
+                query_base=0, candidate_base=0, spec_code=LossSpec("pairs").code(), budget_ns=10 ** 9, pull_src0=0, pull_dst0=0,
+                pull_bytes0=0, pull_src1=0, pull_dst1=0, pull_bytes1=0, sms=148, stream=stream_handle())
+    torch.cuda.synchronize()
+    assert not status.any() and (cube[-4096:] == 7.0).all() and (partials[-4096:] == 7.0).all()
+    rows = torch.arange(rows_q, device="cuda")[:, None]
+    columns = torch.arange(rows_c, device="cuda")[None, :]
+    losses = partials[:-4096].view(slots, quantities, rows_q).double().sum((0, 2))[2:2 + prefixes]
+    for k, end in enumerate(ladder.ends):
+        cosine = torch.nn.functional.normalize(queries[:, :end].double(), dim=1) @ torch.nn.functional.normalize(block[:, :end].double(), dim=1).T
+        logits = 10.0 * torch.where(rows == columns, 1.0, cosine) - 10.0
+        signs = torch.where(((rows ^ 1) == columns) | ((rows == columns) & (LossSpec("pairs").diagonal == "own")), 1.0, -1.0)
+        expected = torch.nn.functional.softplus(-signs * logits).sum()
+        assert float(losses[k]) == pytest.approx(float(expected), rel=SUMMAND_TOLERANCE)
