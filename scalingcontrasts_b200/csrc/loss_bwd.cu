@@ -339,21 +339,36 @@ uint32_t plan_tiles(uint32_t rows_q, ladder_host const& ladder, uint32_t split, 
     bool const two_blocks = static_cast<uint64_t>(row_blocks / 2) * plain_tiles * split >= 2ull * static_cast<uint64_t>(multiprocessors);
     // One-block tiles that make a little more than one CTA per multiprocessor leave most of the chip idle in a second round
     // (4096 rows, H=768, K=5: 192 CTAs on 148, 58 us). Cut to 128 channels they run two to a multiprocessor, each with half
-    // the ring and half the tensor memory, as long as all of them are resident at once: 47 us. A launch of one round stays
-    // with 256 channels, and so does one with more CTAs than two per multiprocessor, which would start a third round (neither line
-    // has been measured closely: launches that fill a part of one round, and widths between 128 and 256 channels, have not).
+    // the ring and half the tensor memory, as long as all of them are resident at once: 47 us. One with more CTAs than two per
+    // multiprocessor, which would start a third round, stays with 256 channels.
     uint64_t const rounds_of = static_cast<uint64_t>(row_blocks) * split;
     shared = !two_blocks && rounds_of * plain_tiles > static_cast<uint64_t>(multiprocessors) && narrow_tiles <= bwd_max_tiles &&
              rounds_of * narrow_tiles <= 2ull * static_cast<uint64_t>(multiprocessors);
-    uint32_t const widest = shared ? bwd_shared_width : bwd_max_width;
+    uint32_t widest = shared ? bwd_shared_width : bwd_max_width;
+    // A launch of one round takes as long as its longest CTA: the narrowest width with which all tiles still run at once. With tiles of 256
+    // channels wherever a band has them: 1024 rows, H=768, K=5 13.9 us in 48 CTAs, now 7.9 in 128; 3072 rows, H=512, K=4 26.7 -> 19.8;
+    // 2944 rows, H=832, K=4 26.5 -> 22.8. Tiles narrower than a box of 64 channels still load whole ones, but 512 rows take 5.2 us
+    // with 32 channels against 5.9 with 64.
+    bool const one_round = !two_blocks && rounds_of * plain_tiles <= static_cast<uint64_t>(multiprocessors);
+    if (one_round)
+        for (uint32_t width = 32; width < bwd_max_width; width += 16) {
+            uint64_t tiles_of = 0;
+            for (uint32_t band = 0, from = 0; band < ladder.count; from = ladder.ends[band++]) tiles_of += (ladder.ends[band] - from + width - 1) / width;
+            if (rounds_of * tiles_of > static_cast<uint64_t>(multiprocessors) || tiles_of > bwd_max_tiles) continue;
+            widest = width;
+            break;
+        }
     begin = 0;
     for (uint32_t band = 0; band < ladder.count; ++band) {
         uint32_t const end = ladder.ends[band];
+        // A band's tiles are as equal as multiples of 16 can be, where one of them is the last to end.
+        uint32_t const pieces = (end - begin + widest - 1) / widest;
+        uint32_t const equal = one_round ? ((end - begin + pieces - 1) / pieces + 15) / 16 * 16 : widest;
         for (uint32_t channel = begin; channel < end;) {
             if (tile_count == bwd_max_tiles) throw std::runtime_error("backward: too many channel tiles for one launch");
             uint32_t const left = end - channel;
             bool const whole_band = two_blocks && left == end - begin && left > bwd_max_width && left <= bwd_wide_width;
-            uint32_t const width = whole_band || left <= widest ? left : widest;
+            uint32_t const width = whole_band || left <= equal ? left : equal;
             tiles[tile_count++] = bwd_tile{band, channel, width, two_blocks && !whole_band ? 2u : 1u, 0u, 1u};
             channel += width;
         }
