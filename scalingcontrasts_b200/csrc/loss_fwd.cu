@@ -1393,9 +1393,9 @@ template <form_t form_> void preload_form() {
 //   us against 80.7 with a single CTA and 82.3 with a pair that can score the diagonal; 2944 rows, H=832, K=4: 44.8, 49.3, 50.8;
 //   16384 rows, H=768, K=5: 1130, 1248, 1215; every cell in the general form, 8192 rows, H=512, K=4: 328, 359, 371).
 // - A block with them: a pair loads a third fewer operand bytes per cell, and where those weigh more than the cells' arithmetic, which
-//   goes with the channels per band, it is faster: H=1024, K=1, 8192 rows 166 against 175 us, H=768, K=3, 4096 rows 69 against 78,
-//   H=1024, K=4 81 against 86, K=7 145 against 153. It is not for few channels (H=512, K=4, 4096 rows 70 against 66; H=832, K=4, 2944
-//   rows 51 against 49.5), and in between for large launches, which run at the GPU's power limit (H=768, K=5: 4096
+//   goes with the channels per band, it is faster: H=1024, K=1, 4096 rows 44.5 against 45.9 us, 8192 rows 166 against 175, K=7, 4096
+//   rows 145 against 153. It is not for few channels (H=512, K=4, 4096 rows 70 against 66; H=832, K=4, 2944 rows 51 against 49.5; H=512,
+//   K=2, 6144 rows 98 against 92), and in between for large launches, which run at the GPU's power limit (H=768, K=5: 4096
 //   rows 83.4 against 82.1, 16384 rows 1229 against 1270; H=1024, K=6: 4096 rows 124 either way, 8192 rows 418 against 454).
 static form_t forward_form(forward_arguments const& a) {
     if (a.fused) return form_fused;
@@ -1408,7 +1408,7 @@ static form_t forward_form(forward_arguments const& a) {
     bool const apart = a.candidate_base >= behind || a.candidate_base + a.rows_c <= first;
     if (apart) return form_pair_apart;
     bool const large = static_cast<uint64_t>(a.rows_q) * a.rows_c >= (1ull << 26);
-    return bands >= 7 || a.hidden >= (large ? 144 : 256) * bands ? form_pair : form_single;
+    return bands >= 7 || a.hidden >= (large ? 144 : 320) * bands ? form_pair : form_single;
 }
 // A run is `tiles_per_run` tiles, of 64 candidates or, in a pair, of 128, and has one record per 64 columns of a tile and column group. A
 // pair's last run may be shorter.
@@ -1426,11 +1426,19 @@ uint32_t forward_partial_slots(uint32_t rows_c, uint32_t tiles_per_run) {
 uint32_t forward_filled_slots(forward_arguments const& a) { return slots_of(forward_form(a), a.rows_c, a.tiles_per_run); }
 uint32_t forward_quantities(uint32_t prefixes) { return 2 + 2 * prefixes; }
 
+// The run length (a power of two that divides the tiles of 64) after which the busiest pair is done first: its tiles, and an eighth of a
+// tile for every run's record, which the epilogue writes and the backward launch folds. With at least six runs to a walker
+// instead (2944 and 3072 rows: runs of one tile, 184 and 192 records to a row) the fold took longer than the gradient GEMM that
+// hides it: three blocks of 2944 rows, H=832, K=4, took 274 us, with runs of two tiles 237.
 uint32_t forward_choose_tiles_per_run(uint32_t rows_q, uint32_t rows_c, int multiprocessors) {
-    uint32_t const strips = rows_q / fwd_rows, column_tiles = rows_c / 64;
+    uint64_t const strips = rows_q / fwd_rows, column_tiles = rows_c / 64, tiles = (column_tiles + 1) / 2;
+    uint64_t const walkers = multiprocessors > 1 ? static_cast<uint64_t>(multiprocessors) / 2 : 1;
     uint32_t best = 1;
-    for (uint32_t t = 1; t <= 32 && column_tiles % t == 0 && (t == 1 || 2 * t <= column_tiles); t *= 2)
-        if (static_cast<uint64_t>(strips) * (column_tiles / t) >= 6ull * static_cast<uint64_t>(multiprocessors)) best = t;
+    uint64_t least = ~0ull;
+    for (uint32_t t = 1; t <= 32 && column_tiles % t == 0 && (t == 1 || t <= tiles); t *= 2) {
+        uint64_t const runs = (strips * ((tiles + t - 1) / t) + walkers - 1) / walkers; // of the busiest pair
+        if (runs * (8 * t + 1) < least) least = runs * (8 * t + 1), best = t;
+    }
     return best;
 }
 
