@@ -184,7 +184,9 @@ void launch_backward(backward_arguments const& arguments, cudaStream_t stream);
 std::vector<std::array<uint32_t, 6>> backward_plan(uint32_t rows_q, ladder_host const& ladder, uint32_t split,
                                                     int multiprocessors, uint32_t* ctas);
 
-void preload_loss_kernels();
+// A kernel is loaded when it is first used, which must not fall into a time when another rank's kernel waits for this one's.
+void preload_backward_kernels();
+void preload_forward_kernels(uint32_t prefixes, bool fused); // the forms one ladder length can take
 
 // -------- projector tower (tower.cu) -----------------------------------------------------------------------------
 // Elementwise passes between the tower's library GEMMs. bfloat16 matrices are row-major with a multiple of 8 columns.

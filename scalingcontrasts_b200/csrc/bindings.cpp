@@ -288,8 +288,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("make_control", &make_control);
     m.def("preload_kernels", []() {
         sc::preload_collective_kernels();
-        sc::preload_loss_kernels();
+        sc::preload_backward_kernels();
     });
+    m.def("preload_forward", &sc::preload_forward_kernels, py::arg("prefixes"), py::arg("fused"));
 
     m.def("barrier", [](control_handle const& c, uint64_t stream) { sc::launch_barrier(c.view, stream_of(stream)); });
     m.def("expect_arrivals", [](control_handle const& c, uint32_t arrivals, uint64_t stream) {

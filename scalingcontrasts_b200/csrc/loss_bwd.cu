@@ -470,7 +470,6 @@ void launch_backward(backward_arguments const& a, cudaStream_t stream) {
     note_launch();
 }
 
-void preload_forward_kernels();
 std::vector<std::array<uint32_t, 6>> backward_plan(uint32_t rows_q, ladder_host const& ladder, uint32_t split,
                                                     int multiprocessors, uint32_t* ctas) {
     if (rows_q % bwd_rows || split < 1) throw std::runtime_error("backward_plan: rows must be a multiple of 128 and split positive");
@@ -487,11 +486,10 @@ std::vector<std::array<uint32_t, 6>> backward_plan(uint32_t rows_q, ladder_host 
 
 SC_DEFINE_BOUNDS_READER(bounds_record_backward)
 
-void preload_loss_kernels() {
+void preload_backward_kernels() {
     cudaFuncAttributes attributes;
     require(cudaFuncGetAttributes(&attributes, backward_kernel<false>), "preload backward");
     require(cudaFuncGetAttributes(&attributes, backward_kernel<true>), "preload backward (row-major candidates)");
-    preload_forward_kernels();
 }
 
 } // namespace sc

@@ -1370,17 +1370,14 @@ void launch_for_count(uint32_t count, CUtensorMap const& q_map, CUtensorMap cons
     }
 }
 
-template <form_t form_> void preload_form() {
+template <int prefixes_> void preload_count(bool fused) {
     cudaFuncAttributes attributes;
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<1, form_>), "preload forward<1>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<2, form_>), "preload forward<2>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<3, form_>), "preload forward<3>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<4, form_>), "preload forward<4>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<5, form_>), "preload forward<5>");
-    require(cudaFuncGetAttributes(&attributes, forward_kernel<6, form_>), "preload forward<6>");
-    if constexpr (form_ != form_fused) {
-        require(cudaFuncGetAttributes(&attributes, forward_kernel<7, form_>), "preload forward<7>");
-        require(cudaFuncGetAttributes(&attributes, forward_kernel<8, form_>), "preload forward<8>");
+    if (!fused) {
+        require(cudaFuncGetAttributes(&attributes, forward_kernel<prefixes_, form_single>), "preload forward (single)");
+        require(cudaFuncGetAttributes(&attributes, forward_kernel<prefixes_, form_pair>), "preload forward (pair)");
+        require(cudaFuncGetAttributes(&attributes, forward_kernel<prefixes_, form_pair_apart>), "preload forward (pair, apart)");
+    } else if constexpr (prefixes_ <= static_cast<int>(fz_max_prefixes)) {
+        require(cudaFuncGetAttributes(&attributes, forward_kernel<prefixes_, form_fused>), "preload forward (fused)");
     }
 }
 
@@ -1567,11 +1564,18 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
 
 SC_DEFINE_BOUNDS_READER(bounds_record_forward)
 
-void preload_forward_kernels() {
-    preload_form<form_single>();
-    preload_form<form_pair>();
-    preload_form<form_pair_apart>();
-    preload_form<form_fused>();
+void preload_forward_kernels(uint32_t prefixes, bool fused) {
+    switch (prefixes) {
+    case 1: preload_count<1>(fused); break;
+    case 2: preload_count<2>(fused); break;
+    case 3: preload_count<3>(fused); break;
+    case 4: preload_count<4>(fused); break;
+    case 5: preload_count<5>(fused); break;
+    case 6: preload_count<6>(fused); break;
+    case 7: preload_count<7>(fused); break;
+    case 8: preload_count<8>(fused); break;
+    default: throw std::runtime_error("preload: a ladder holds one to eight prefixes");
+    }
 }
 
 } // namespace sc

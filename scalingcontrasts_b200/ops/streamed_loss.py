@@ -176,6 +176,8 @@ class StreamedLoss:
                                   self.partials.data_ptr(), self.row_accumulators.data_ptr(), self.status.data_ptr(),
                                   self.budget_ns, self.multiprocessors)
         self._plan.transpose_candidates = self.transpose_candidates
+        with torch.cuda.device(self.device):
+            ext.preload_forward(k, self.fused)
         # With ``overlap_backward`` a block's gradient GEMM runs on a second stream, on a few multiprocessors, beside the
         # next block's forward kernel (whose grid shrinks by as many), and a step's last one runs alone in finish(). It
         # takes a second gradient cube, and the caller must leave a block's candidates in place until the block after
