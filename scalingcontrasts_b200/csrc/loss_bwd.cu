@@ -12,6 +12,9 @@
 // 257 to 384 channels, one block x the whole band, so that the band's cube, the traffic this kernel is bound by, is read
 // from DRAM once instead of once per 256-channel tile.
 //
+// Where it pays, two CTAs with consecutive row blocks of a tile, a cluster, run their UMMAs together (256 rows) and load half of the
+// tile's candidates each.
+//
 // Warp roles (192 threads): warps 0-3 epilogue (tensor-memory lanes 32*w..; before that the fold of the forward launch's
 // partial records, if asked for), warp 4 TMA producer, warp 5 UMMA issuer and tensor-memory owner. The producer's and the issuer's loops are run by one elected lane each. The epilogue adds its scaled accumulators with
 // vector reductions (fire and forget: no read of the old value comes back to the SM). With `split == 1` each output
@@ -137,7 +140,7 @@ __device__ __forceinline__ void fold_share(bwd_params const& p, uint32_t warp, u
     }
 }
 
-template <bool mn_major_>
+template <bool mn_major_, bool pair_>
 __global__ void __launch_bounds__(bwd_threads, 1)
     backward_kernel(const __grid_constant__ CUtensorMap cube_map, const __grid_constant__ bwd_candidate_boxes candidates,
                     const bwd_params p) {
@@ -150,14 +153,21 @@ __global__ void __launch_bounds__(bwd_threads, 1)
     while (tile_index + p.tiles[tile_index].group < p.tile_count &&
            blockIdx.x >= p.tiles[tile_index + p.tiles[tile_index].group].first_cta)
         tile_index += p.tiles[tile_index].group;
-    uint32_t const within = blockIdx.x - p.tiles[tile_index].first_cta, group = p.tiles[tile_index].group;
+    uint32_t const group = p.tiles[tile_index].group, rank = pair_ ? cluster_rank() : 0u;
+    uint32_t within = blockIdx.x - p.tiles[tile_index].first_cta;
+    // A pair takes one tile of the group for the rows of two CTAs, one after the other.
+    if constexpr (pair_) within = (within / 2 / group * 2 + rank) * group + within / 2 % group;
     tile_index += within % group;
     bwd_tile const tile = p.tiles[tile_index];
     // Stage geometry: [row blocks of the cube, 16 KB each][candidate tile of the tile's width]. MN-major candidates come in
     // whole boxes of 64 channels (8 KB), K-major ones in rows of 128 bytes per channel; either way a stage is a multiple of
     // 1 KB, so every stage starts on a swizzle atom.
     bool const wide = tile.width > bwd_max_width;
-    uint32_t const candidate_bytes = mn_major_ ? ((tile.width + 63u) / 64u) * bwd_mn_box_bytes : tile.width * bwd_depth * 2u;
+    // A pair's UMMAs take N in steps of 32 channels (what the last one has beyond the tile is never read), half of them from
+    // either CTA.
+    uint32_t const pair_width = (tile.width + 31u) / 32u * 32u;
+    uint32_t const boxes = ((pair_ ? pair_width / 2 : tile.width) + 63u) / 64u; // MN-major: whole boxes of 64 channels, the last one partly used
+    uint32_t const candidate_bytes = mn_major_ ? boxes * bwd_mn_box_bytes : tile.width * bwd_depth * 2u;
     uint32_t const stage_bytes = tile.blocks * bwd_a_bytes + candidate_bytes;
     // One-block tiles (small launches) take as deep a ring as fits: 0.187 -> 0.181 ms per 4096-row block. Two-block tiles
     // stay at three stages: deeper rings for the narrow, DRAM-bound ones made a 16384-row launch slower (1.82 -> 1.85 ms per
@@ -185,13 +195,19 @@ __global__ void __launch_bounds__(bwd_threads, 1)
         return;
     }
     if (warp == 5) {
-        tmem_alloc(smem_u32(&tail->tmem_base), p.tmem_columns);
-        tmem_relinquish();
+        if constexpr (pair_) {
+            tmem_alloc_pair(smem_u32(&tail->tmem_base), p.tmem_columns);
+            tmem_relinquish_pair();
+        } else {
+            tmem_alloc(smem_u32(&tail->tmem_base), p.tmem_columns);
+            tmem_relinquish();
+        }
     }
     if (warp == 4 && lane == 0) {
         tma_prefetch_descriptor(&cube_map);
-        for (uint32_t i = 0; i < bwd_candidate_maps; ++i) tma_prefetch_descriptor(&candidates.maps[i]);
+        for (uint32_t i = 0; i < (mn_major_ ? 1u : bwd_candidate_maps); ++i) tma_prefetch_descriptor(&candidates.maps[i]);
     }
+    if constexpr (pair_) cluster_sync(); // the other CTA's barriers are set up
     // Everything up to here may run beside the end of the kernel before.
     wait_for_kernels_before();
     if (threadIdx.x == 0) tail->abort_flag = status_poisoned(p.status) ? 1u : 0u;
@@ -208,12 +224,23 @@ __global__ void __launch_bounds__(bwd_threads, 1)
     } else if (warp == 4) {
         if (elect_one()) {
             uint32_t stage = 0, phase = 0;
-            uint32_t const boxes = (tile.width + 63u) / 64u; // MN-major: whole boxes of 64 channels, the last one partly used
-            uint32_t const bytes = blocks * bwd_a_bytes + (mn_major_ ? boxes * bwd_mn_box_bytes : tile.width * bwd_depth * 2);
+            uint32_t const bytes = blocks * bwd_a_bytes + candidate_bytes;
             for (uint32_t chunk = chunk_begin; chunk < chunk_end; ++chunk) {
                 if (!mbar_wait(smem_u32(&tail->stage_empty[stage]), phase ^ 1u, ctx, site_bwd_stage_empty, chunk)) break;
                 uint32_t const full = smem_u32(&tail->stage_full[stage]);
                 uint32_t const destination = stages_base + stage * stage_bytes;
+                if constexpr (pair_) {
+                    // The first CTA's barrier counts both CTAs' bytes, whichever arrive first.
+                    uint32_t const counted = smem_of(full, 0);
+                    if (rank == 0) mbar_arrive_expect_tx(full, 2 * bytes);
+                    tma_load_3d_pair(destination, &cube_map, counted, static_cast<int>(chunk * bwd_depth), static_cast<int>(first_block * bwd_rows),
+                                     static_cast<int>(tile.band));
+                    for (uint32_t box = 0; box < boxes; ++box)
+                        tma_load_2d_pair(destination + b_offset + box * bwd_mn_box_bytes, &candidates.maps[0], counted,
+                                         static_cast<int>(tile.channel0 + rank * (pair_width / 2) + box * 64u), static_cast<int>(chunk * bwd_depth));
+                    if (++stage == stages) stage = 0, phase ^= 1u;
+                    continue;
+                }
                 mbar_arrive_expect_tx(full, bytes);
                 for (uint32_t block = 0; block < blocks; ++block)
                     tma_load_3d(destination + block * bwd_a_bytes, &cube_map, full, static_cast<int>(chunk * bwd_depth),
@@ -241,13 +268,21 @@ __global__ void __launch_bounds__(bwd_threads, 1)
             }
         }
     } else if (warp == 5) {
-        if (elect_one()) {
+        if (rank == 0 && elect_one()) {
             // A tile wider than one UMMA's 256 columns is issued in two pieces; the second starts 256 channels on, which is
             // 32 KB into the candidate stage in either layout (four 8 KB boxes, or 256 rows of 128 bytes).
             uint32_t const major = mn_major_ ? umma_idesc_b_mn_major : 0u;
             uint32_t const width0 = wide ? bwd_max_width : tile.width;
-            uint32_t const idesc0 = umma_idesc_bf16(bwd_rows, width0) | major;
+            uint32_t const idesc0 = (pair_ ? umma_idesc_bf16(2 * bwd_rows, pair_width) : umma_idesc_bf16(bwd_rows, width0)) | major;
             uint32_t const idesc1 = wide ? (umma_idesc_bf16(bwd_rows, tile.width - bwd_max_width) | major) : 0u;
+            auto multiply = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+                if constexpr (pair_) umma_bf16_pair(d, a, b, idesc, accumulate);
+                else umma_bf16(d, a, b, idesc, accumulate);
+            };
+            auto commit = [&](uint32_t bar) {
+                if constexpr (pair_) umma_commit_pair(smem_of(bar, 0)), umma_commit_pair(smem_of(bar, 1));
+                else umma_commit(bar);
+            };
             constexpr uint32_t descriptor_high = (1024u >> 4) | (1u << 14) | (2u << 29); // stride 1024 B, version 1, 128-byte swizzle
             uint32_t const low_base = ((stages_base & 0x3FFFFu) >> 4) | (1u << 16);
             // The B operand's leading offset (bits 16-29 of the low word) and its advance per 16 candidates.
@@ -266,19 +301,19 @@ __global__ void __launch_bounds__(bwd_threads, 1)
                 // Straight-line runs of four: with a loop over the row blocks around them and the wide tile's test between them, a
                 // chunk took 457 cycles to issue (64 channels, nothing to load) and 730 (256 channels), now 255 and 540.
                 auto four_steps = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t idesc) {
-                    umma_bf16(d, a, b, idesc, accumulate);
-                    umma_bf16(d, a + 2u, b + b_step, idesc, 1u);
-                    umma_bf16(d, a + 4u, b + 2u * b_step, idesc, 1u);
-                    umma_bf16(d, a + 6u, b + 3u * b_step, idesc, 1u);
+                    multiply(d, a, b, idesc, accumulate);
+                    multiply(d, a + 2u, b + b_step, idesc, 1u);
+                    multiply(d, a + 4u, b + 2u * b_step, idesc, 1u);
+                    multiply(d, a + 6u, b + 3u * b_step, idesc, 1u);
                 };
                 four_steps(tmem_base, a_descriptor, b_descriptor, idesc0);
-                if (blocks == 2) four_steps(tmem_base + bwd_block_columns, a_descriptor + (bwd_a_bytes >> 4), b_descriptor, idesc0);
-                if (wide) four_steps(tmem_base + bwd_max_width, a_descriptor, b_descriptor + ((bwd_max_width * bwd_depth * 2u) >> 4), idesc1);
+                if (!pair_ && blocks == 2) four_steps(tmem_base + bwd_block_columns, a_descriptor + (bwd_a_bytes >> 4), b_descriptor, idesc0);
+                if (!pair_ && wide) four_steps(tmem_base + bwd_max_width, a_descriptor, b_descriptor + ((bwd_max_width * bwd_depth * 2u) >> 4), idesc1);
                 accumulate = 1;
-                umma_commit(smem_u32(&tail->stage_empty[stage]));
+                commit(smem_u32(&tail->stage_empty[stage]));
                 if (++stage == stages) stage = 0, phase ^= 1u;
             }
-            if (ok) umma_commit(smem_u32(&tail->accumulated));
+            if (ok) commit(smem_u32(&tail->accumulated));
         }
     } else {
         if (p.partials != nullptr) fold_share(p, warp, lane);
@@ -312,10 +347,13 @@ __global__ void __launch_bounds__(bwd_threads, 1)
         uint64_t const start = global_timer_ns();
         while (global_timer_ns() - start < 200000ull) __nanosleep(1000);
     }
-    __syncthreads();
+    // A pair's barriers and operands are used by both CTAs until both are done.
+    if constexpr (pair_) cluster_sync();
+    else __syncthreads();
     if (warp == 5) {
         tcgen05_fence_after();
-        tmem_dealloc(tmem_base, p.tmem_columns);
+        if constexpr (pair_) tmem_dealloc_pair(tmem_base, p.tmem_columns);
+        else tmem_dealloc(tmem_base, p.tmem_columns);
     }
 }
 
@@ -456,15 +494,23 @@ void launch_backward(backward_arguments const& a, cudaStream_t stream) {
     // Per device, once: the shared-memory limit of the kernel.
     static int prepared_device = -1;
     if (prepared_device != device) {
-        require(cudaFuncSetAttribute(backward_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd_shared_bytes),
-                "raising the backward kernel's shared memory");
-        require(cudaFuncSetAttribute(backward_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd_shared_bytes),
-                "raising the backward kernel's shared memory");
+        for (auto* kernel : {backward_kernel<false, false>, backward_kernel<true, false>, backward_kernel<true, true>})
+            require(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd_shared_bytes),
+                    "raising the backward kernel's shared memory");
         prepared_device = device;
     }
     dim3 const grid(ctas, a.split, 1);
-    launch_dependent(!a.ordinary_launch, mn_major ? backward_kernel<true> : backward_kernel<false>, grid, bwd_threads, shared_bytes, stream,
-                     cube_map, candidates, p);
+    // Pairs of CTAs, each with one row block of a tile, load half of its candidates each: where a launch of one-block tiles is more than one
+    // round (4096 rows, H=768, K=5 44.5 -> 40.8 us, 6144 rows, H=1024, K=2 85 -> 78). In one round the barriers across CTAs cost more
+    // than that (1024 rows 7.6 -> 9 us), as with bands narrower than a pair's UMMA (2048 rows, H=2048, K=8 28 -> 30); in a large launch, whose
+    // two-block CTAs share their candidates already, it changed nothing (16384 rows, H=1024, K=5, a whole step 2.09 ms either way).
+    bool pair = mn_major && a.rows_q / bwd_rows % 2 == 0 && static_cast<uint64_t>(ctas) * a.split > static_cast<uint64_t>(multiprocessors);
+    for (uint32_t i = 0; i < p.tile_count; ++i)
+        pair = pair && p.tiles[i].blocks == 1 && p.tiles[i].width >= 32 && p.tiles[i].width <= bwd_max_width;
+    if (pair) launch_dependent_clusters(!a.ordinary_launch, 2, backward_kernel<true, true>, grid, bwd_threads, shared_bytes, stream, cube_map, candidates, p);
+    else
+        launch_dependent(!a.ordinary_launch, mn_major ? backward_kernel<true, false> : backward_kernel<false, false>, grid, bwd_threads, shared_bytes,
+                         stream, cube_map, candidates, p);
     cudaError_t const error = cudaGetLastError();
     if (error != cudaSuccess) throw std::runtime_error(std::string("backward launch failed: ") + cudaGetErrorString(error));
     note_launch();
@@ -488,8 +534,9 @@ SC_DEFINE_BOUNDS_READER(bounds_record_backward)
 
 void preload_backward_kernels() {
     cudaFuncAttributes attributes;
-    require(cudaFuncGetAttributes(&attributes, backward_kernel<false>), "preload backward");
-    require(cudaFuncGetAttributes(&attributes, backward_kernel<true>), "preload backward (row-major candidates)");
+    require(cudaFuncGetAttributes(&attributes, backward_kernel<false, false>), "preload backward");
+    require(cudaFuncGetAttributes(&attributes, backward_kernel<true, false>), "preload backward (row-major candidates)");
+    require(cudaFuncGetAttributes(&attributes, backward_kernel<true, true>), "preload backward (pairs)");
 }
 
 } // namespace sc

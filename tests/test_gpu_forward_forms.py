@@ -96,3 +96,31 @@ def test_an_odd_number_of_64_candidates(prefixes, rows_c):
         signs = torch.where(((rows ^ 1) == columns) | ((rows == columns) & (LossSpec("pairs").diagonal == "own")), 1.0, -1.0)
         expected = torch.nn.functional.softplus(-signs * logits).sum()
         assert float(losses[k]) == pytest.approx(float(expected), rel=SUMMAND_TOLERANCE)
+
+
+@pytest.mark.parametrize("rows_q,ends", [(4096, [48, 96, 192, 384, 768]), (3584, [64, 112, 1024]), (4864, [1024]), (4096, [32, 272, 1024]),
+                                         (3328, [96, 768, 1104]), (4096, [16, 1024]), (4992, [1024])])
+@pytest.mark.parametrize("rows_c", [64, 448])
+def test_backward_in_pairs_of_ctas(rows_q, ends, rows_c):
+    """Launches of more than one round of one-block tiles: pairs, whose UMMAs take channels in steps of 32, and the ones that stay with
+    single CTAs (a band of 16, an odd number of row blocks). Float32 sums of bfloat16 products against the same in float64."""
+    ext, hidden = native(), ends[-1]
+    tiles, ctas = ext.backward_plan(rows_q, ends, 1, 148)
+    assert ctas > 148 and all(t[3] == 1 for t in tiles)
+    generator = torch.Generator(device="cuda").manual_seed(7)
+    cube = (torch.randn(len(ends), rows_q, rows_c, device="cuda", generator=generator) * 0.1).to(torch.bfloat16)
+    candidates = torch.randn(rows_c, hidden, device="cuda", generator=generator).to(torch.bfloat16)
+    status = torch.zeros(8, dtype=torch.int32, device="cuda")
+    begins = [0] + ends[:-1]
+    expected = 1.0 + 0.5 * torch.cat([cube[b].double() @ candidates.double()[:, begins[b]:ends[b]] for b in range(len(ends))], dim=1)
+    outcomes = []
+    for _ in range(2):
+        gradient = torch.ones(rows_q, hidden, device="cuda")
+        ext.backward(cube.data_ptr(), 0, gradient.data_ptr(), status.data_ptr(), rows_q, rows_c, hidden, ends, 1, 0.5, 10 ** 9,
+                     stream_handle(), candidates.data_ptr())
+        torch.cuda.synchronize()
+        assert not status.any()
+        # one float32 sum of rows_c products per element: 448 * 2^-24 of the terms' size at most, and one rounding of the whole
+        assert float((gradient.double() - expected).norm() / expected.norm()) < 1e-5
+        outcomes.append(gradient)
+    assert torch.equal(outcomes[0], outcomes[1])
