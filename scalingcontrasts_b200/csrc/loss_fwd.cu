@@ -24,8 +24,8 @@
 // registers a thread, the helpers' with 64.
 //
 // What bounds it (B200, one block of 4096 rows, H=768, K=5, off the diagonal: 75 us): the epilogue, which by itself takes about 60 (cells
-// 6.4 k of a tile's 9 k cycles: a warp's instructions wait for one another, and four warps to a scheduler do not hide all of it);
-// operands and UMMAs by themselves take about 30. One block of 16384 rows (1.13 ms): the memory side as well; a single CTA's loads and
+// 6.4 k of a tile's 9 k cycles: a warp's instructions wait for one another, and four warps to a scheduler do not hide all of it).
+// A single CTA's operands and UMMAs by themselves took 41. One block of 16384 rows (1.13 ms): the memory side as well; a single CTA's loads and
 // the cube's stores without any arithmetic took 1.05 ms, and the GPU runs at its power limit.
 //
 // A CTA or pair walks work items (row strip, run of consecutive candidate tiles) in a fixed round-robin order and writes one

@@ -79,9 +79,9 @@ def render(rows: List[Dict[str, object]]) -> str:
         lines.append(f"| `{row['source']}` | `{row['name']}` | {row['registers']} | {row['spill_stores']} | {row['spill_loads']} | "
                      f"{row['stack']} | {row['shared']} |")
     lines += ["",
-              "Dynamic shared memory (set by the launchers), K the number of prefixes: `forward_kernel<K, false>` as many 24 KB stages as",
-              "fit beside 16 KB of store patches per band (four bands in rotation from K = 7 on), norms and row factors: six for K <= 4",
-              "(226,944 bytes at K = 4), five at K = 5 (221,824), four above; `forward_kernel<K, true>` (fused) two 32 KB stages of the",
+              "Dynamic shared memory (set by the launchers), K the number of prefixes: `forward_kernel<K, form>` (forms: 0 one CTA per tile,",
+              "1 pairs of CTAs, 2 pairs without anything of the diagonal, 3 fused) as many stages as fit, up to eight (24 KB each, in a pair",
+              "16 KB), beside 16 KB of store patches per band (four bands in rotation from K = 7 on), norms and row factors; fused two 32 KB stages of the",
               "gradient GEMM and six to two scoring stages (227,968 bytes, three stages, at K = 5); `backward_kernel` 214,128 bytes (a 208 KB",
               "ring of three to six stages, a stage being the CTA's row blocks of the cube plus its tile's candidates), or half the ring",
               "where two CTAs share a multiprocessor. Threads per block: 640 (forward; 96 registers at launch, 104 in the epilogue's",
