@@ -16,7 +16,7 @@ this is the framework layer around its ``StreamedLoss`` contract (scalingcontras
 from __future__ import annotations
 
 import math
-from typing import Optional
+from typing import Optional, Tuple
 
 import torch
 from torch import nn
@@ -57,28 +57,36 @@ class _DeviceLoss(torch.autograd.Function):
             # The caller promised `loss.backward()` with nothing after the loss: the upstream gradient is one, and a pass
             # over the row gradients that multiplies them by it (25 MB in, 25 MB out per step) is left out.
             return gradient.to(ctx.input_dtype), summands[2], summands[1], None
-        if _DeviceLoss._plain(ctx, gradient, summands, grad_output):
+        addresses = _DeviceLoss._plain(ctx, gradient, summands, grad_output)
+        if addresses is not None:
             from .._ext import native, stream_handle
 
             scaled = torch.empty(gradient.shape, dtype=ctx.input_dtype, device=gradient.device)
             by_scale, by_bias = torch.empty_like(grad_output), torch.empty_like(grad_output)
-            native().scale_gradients(gradient.data_ptr(), grad_output.data_ptr(), summands.data_ptr(), scaled.data_ptr(),
-                                     ctx.input_dtype == torch.float32, by_scale.data_ptr(), by_bias.data_ptr(), gradient.numel(),
-                                     stream_handle())
+            native().scale_gradients(*addresses, scaled.data_ptr(), ctx.input_dtype == torch.float32, by_scale.data_ptr(),
+                                     by_bias.data_ptr(), gradient.numel(), stream_handle())
             return scaled, by_scale, by_bias, None
         scaled = gradient * grad_output.to(gradient.dtype)
         return scaled.to(ctx.input_dtype), summands[2] * grad_output, summands[1] * grad_output, None
 
     @staticmethod
-    def _plain(ctx, gradient, summands, grad_output) -> bool:
-        """Whether one launch does it all: nothing of this backward is differentiated again, and what the hooks on saved
-        tensors hand back is what was saved."""
-        return (not torch.is_grad_enabled() and type(grad_output) is torch.Tensor and grad_output.is_cuda
-                and grad_output.dtype == torch.float32 and grad_output.dim() == 0 and type(gradient) is torch.Tensor
-                and gradient.is_cuda and gradient.dtype == torch.bfloat16 and gradient.is_contiguous()
-                and gradient.data_ptr() % 16 == 0 and type(summands) is torch.Tensor and summands.is_cuda
-                and summands.dtype == torch.float32 and summands.is_contiguous()
-                and ctx.input_dtype in (torch.bfloat16, torch.float32))
+    def _plain(ctx, gradient, summands, grad_output) -> Optional[Tuple[int, int, int]]:
+        """The addresses of the row gradients, the upstream gradient and the summands where one launch does it all, else None:
+        nothing of this backward is differentiated again, what the hooks on saved tensors hand back is what was saved, and each
+        tensor's values are what lies in its memory. (An upstream gradient with a batch axis of a ``vmap``, which
+        ``is_grads_batched`` is too, calls itself a 0-d tensor and has no memory of its own.)"""
+        if (torch.is_grad_enabled() or type(grad_output) is not torch.Tensor or not grad_output.is_cuda
+                or grad_output.dtype != torch.float32 or grad_output.dim() != 0 or grad_output.is_neg()
+                or type(gradient) is not torch.Tensor or not gradient.is_cuda or gradient.dtype != torch.bfloat16
+                or not gradient.is_contiguous() or type(summands) is not torch.Tensor or not summands.is_cuda
+                or summands.dtype != torch.float32 or not summands.is_contiguous()
+                or ctx.input_dtype not in (torch.bfloat16, torch.float32)):
+            return None
+        try:
+            addresses = gradient.data_ptr(), grad_output.data_ptr(), summands.data_ptr()
+        except RuntimeError:
+            return None
+        return addresses if all(addresses) and addresses[0] % 16 == 0 else None
 
 
 class _HostLoss(torch.autograd.Function):
