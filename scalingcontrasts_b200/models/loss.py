@@ -155,7 +155,9 @@ class MatryoshkaSigmoidLoss(nn.Module):
 
             device_domain = domain if domain is not None and hasattr(domain, "alloc") else None
             self.engine = BoxLoss(rows, hidden, self.ladder, spec, device_domain, device)
-            self.register_buffer("_scalars", torch.zeros(2, dtype=torch.float32, device=device), persistent=False)
+            # {logit scale, bias} as the kernels read and write them, two float32 words: not a buffer, which `.to(torch.bfloat16)` or
+            # `.half()` would shrink under them.
+            self._scalars = torch.zeros(2, dtype=torch.float32, device=self.engine.device)
 
     def forward(self, embeddings: torch.Tensor) -> torch.Tensor:
         if tuple(embeddings.shape) != (self.rows, self.hidden):

@@ -50,3 +50,17 @@ def test_a_lazily_negated_upstream_gradient():
     for one, other in zip(torch.autograd.grad(loss, inputs, negated, retain_graph=True),
                           torch.autograd.grad(loss, inputs, torch.tensor(-0.5, device="cuda"))):
         assert torch.equal(one, other)
+
+
+@pytest.mark.parametrize("cast", [torch.bfloat16, torch.float16, torch.float64])
+def test_a_module_cast_to_another_type(cast):
+    """The kernels' two scalars stay float32 words whatever the module's parameters become, and when these come back."""
+    module, embeddings = _module(init_logit_scale=2.0, init_logit_bias=-3.0), _embeddings()  # exact in every type
+    expected = [module(embeddings).detach().clone()] + [g.clone() for g in torch.autograd.grad(module(embeddings), _inputs(module, embeddings))]
+    for kind in (cast, torch.float32):
+        module.to(kind)
+        assert module.logit_scale.dtype == kind and module._scalars.dtype == torch.float32 and module._scalars.numel() == 2
+        loss = module(embeddings)
+        gradients = torch.autograd.grad(loss, _inputs(module, embeddings))
+        assert torch.equal(loss.detach(), expected[0]) and torch.equal(gradients[0], expected[1])
+        assert torch.equal(gradients[1], expected[2].to(kind)) and torch.equal(gradients[2], expected[3].to(kind))
