@@ -31,7 +31,7 @@ class _DeviceLoss(torch.autograd.Function):
         from .._ext import native, stream_handle
 
         engine, scalars, learned = module.engine, module._scalars, None
-        if logit_scale.dtype == torch.float32 and logit_bias.dtype == torch.float32 and logit_scale.is_cuda and logit_bias.is_cuda:
+        if _DeviceLoss._is_word(logit_scale, scalars.device) and _DeviceLoss._is_word(logit_bias, scalars.device):
             learned = (logit_scale, logit_bias)  # the step's first launch makes them into the two scalars
         else:
             scalars[0] = logit_scale.detach().float().exp()
@@ -68,6 +68,12 @@ class _DeviceLoss(torch.autograd.Function):
             return scaled, by_scale, by_bias, None
         scaled = gradient * grad_output.to(gradient.dtype)
         return scaled.to(ctx.input_dtype), summands[2] * grad_output, summands[1] * grad_output, None
+
+    @staticmethod
+    def _is_word(value, device) -> bool:
+        """Whether a kernel of ``device`` can read the value as one float32 word."""
+        return (type(value) in (torch.Tensor, nn.Parameter) and value.dtype == torch.float32 and value.numel() == 1
+                and value.device == device and not value.is_neg())
 
     @staticmethod
     def _plain(ctx, gradient, summands, grad_output) -> Optional[Tuple[int, int, int]]:

@@ -95,7 +95,13 @@ def compute_block_norms(rows: torch.Tensor, ladder: Matryoshka, norms: BlockNorm
         if copy_to.shape != rows.shape or copy_to.dtype != torch.bfloat16 or not copy_to.is_contiguous():
             raise ValueError("copy_to must match the block")
         copy_pointer = copy_to.data_ptr()
-    pointers = (0, 0, 0) if learned is None else tuple(t.data_ptr() for t in learned)
+    pointers = (0, 0, 0)
+    if learned is not None:
+        for name, tensor, least in zip(("the log scale", "the bias", "scalars"), learned, (1, 1, 2)):
+            _check_words(name, tensor, least, rows.device)
+        pointers = tuple(t.data_ptr() for t in learned)
+    if clear is not None:
+        _check_words("clear", clear, 0, rows.device)
     native().prefix_norms(rows.data_ptr(), copy_pointer, norms.inverse.data_ptr(), norms.tile_max.data_ptr(),
                           rows.shape[0], rows.shape[1], ladder.ends, _stream(stream), 0 if clear is None else clear.data_ptr(),
                           0 if clear is None else clear.numel(), *pointers)
@@ -106,6 +112,14 @@ def _check_block(block: torch.Tensor) -> None:
         raise ValueError("a block must be a contiguous CUDA bfloat16 matrix")
     if block.data_ptr() % 16:
         raise ValueError("a block must start on a 16-byte boundary")
+
+
+def _check_words(name: str, words: torch.Tensor, least: int, device: torch.device) -> None:
+    """What a kernel of ``device`` reads or writes by its address as float32 words."""
+    if not isinstance(words, torch.Tensor) or words.dtype != torch.float32 or words.numel() < least or not words.is_contiguous():
+        raise ValueError(f"{name} must be a contiguous float32 span of at least {least} values")
+    if words.device != device and (words.is_cuda or not words.is_pinned()):
+        raise ValueError(f"{name} must lie on {device}")
 
 
 class StreamedLoss:
@@ -233,6 +247,8 @@ class StreamedLoss:
         _check_block(candidates)
         if tuple(candidates.shape) != (self.candidate_rows, self.hidden):
             raise ValueError(f"candidates must be [{self.candidate_rows}, {self.hidden}]")
+        if scalars is not None:
+            _check_words("scalars", scalars, 2, queries.device)
         if candidate_norms is None:
             compute_block_norms(candidates, self.ladder, self.candidate_norms, stream=stream)
             candidate_norms = self.candidate_norms

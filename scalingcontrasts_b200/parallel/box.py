@@ -28,7 +28,7 @@ import torch
 
 from ..config import LossSpec, REFERENCE_SPEC, SUMMAND_SLOTS
 from ..ladder import Matryoshka
-from ..ops.streamed_loss import BlockNorms, PullRequest, StreamedLoss, compute_block_norms
+from ..ops.streamed_loss import BlockNorms, PullRequest, StreamedLoss, _check_words, compute_block_norms
 from ..utils.trace import phase
 
 
@@ -181,6 +181,10 @@ class BoxLoss:
         blocks it scores; the first call of an argument set runs eagerly, the second captures. Every member of the
         domain must make the same choice in the same step. ``learned``, a float32 log scale and bias on the device, fills
         ``scalars`` in the publish launch."""
+        if scalars is not None:
+            _check_words("scalars", scalars, 2, queries.device)  # before anything is launched that other ranks wait for
+        elif learned is not None:
+            raise ValueError("a learned log scale and bias fill `scalars`: both must be given")
         with phase("publish: prefix norms + copy into symmetric memory"):
             self._publish(queries, stream, None if learned is None else (*learned, scalars))
         gradient = self.gradient if gradient_out is None else gradient_out
