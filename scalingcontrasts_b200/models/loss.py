@@ -40,19 +40,32 @@ class _DeviceLoss(torch.autograd.Function):
         if source.dtype != torch.bfloat16:
             source = source.to(torch.bfloat16)
         source = source.contiguous()
-        gradient, summands = engine.step(source, scalars=scalars, learned=learned)
+        ctx.unit_upstream, ctx.shared = bool(module.unit_upstream), None
+        # The row gradients are this call's own, as the summands below: another forward may come before this one's backward. A
+        # captured step writes the engine's one buffer, so a copy is kept, except where the caller promised (`unit_upstream`) to
+        # differentiate before the next step; that is then checked.
+        if not engine.use_graphs:
+            gradient, summands = engine.step(source, scalars=scalars, gradient_out=torch.empty_like(engine.gradient), learned=learned)
+        else:
+            gradient, summands = engine.step(source, scalars=scalars, learned=learned)
+            if ctx.unit_upstream:
+                ctx.shared = engine, engine.gradient_writes
+            else:
+                gradient = gradient.clone()
         kept = torch.empty_like(summands)  # the payload is rewritten by the next step
         loss = torch.empty((), dtype=torch.float32, device=kept.device)
         native().keep_summands(summands.data_ptr(), kept.data_ptr(), loss.data_ptr(), kept.numel(), stream_handle())
         ctx.save_for_backward(gradient, kept)
         ctx.input_dtype = embeddings.dtype
-        ctx.unit_upstream = bool(module.unit_upstream)
         module.last_summands = kept
         return loss
 
     @staticmethod
     def backward(ctx, grad_output):
         gradient, summands = ctx.saved_tensors
+        if ctx.shared is not None and ctx.shared[0].gradient_writes != ctx.shared[1]:
+            raise RuntimeError("the row gradients of this forward have been overwritten by a later step: with captured steps and "
+                               "unit_upstream, backward must run before the next forward")
         if ctx.unit_upstream:
             # The caller promised `loss.backward()` with nothing after the loss: the upstream gradient is one, and a pass
             # over the row gradients that multiplies them by it (25 MB in, 25 MB out per step) is left out.

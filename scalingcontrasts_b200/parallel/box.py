@@ -92,6 +92,7 @@ class BoxLoss:
         self.staged = [torch.empty(rows, hidden, dtype=torch.bfloat16, device=self.device) for _ in range(self._slots)]
         self.staged_norms = [BlockNorms(k, rows, device=self.device) for _ in range(self._slots)]
         self.gradient = torch.empty(rows, hidden, dtype=torch.bfloat16, device=self.device)
+        self.gradient_writes = 0  # how many steps have written it
         self._cursor = 0
         self.use_graphs = False
         self._graphs = {}
@@ -188,6 +189,7 @@ class BoxLoss:
         with phase("publish: prefix norms + copy into symmetric memory"):
             self._publish(queries, stream, None if learned is None else (*learned, scalars))
         gradient = self.gradient if gradient_out is None else gradient_out
+        self.gradient_writes += gradient_out is None
         _check_gradient(gradient, self.rows, self.hidden)
         if (self.use_graphs if graph is None else graph) and stream is None:
             self._replay(float(beta), float(bias), scalars, gradient, bool(reduce))
@@ -231,6 +233,7 @@ class BoxLoss:
                  pull: bool = True) -> Tuple[torch.Tensor, torch.Tensor]:
         """One rank of a ``world``-GPU step on this GPU alone: the own block stands in for every peer's."""
         rows = self.rows
+        self.gradient_writes += 1
         self._publish(queries, stream)
         self.loss.begin(self.embeddings, stream, query_norms=self.norms, cleared=True)
         for block in range(world):

@@ -64,3 +64,38 @@ def test_a_module_cast_to_another_type(cast):
         gradients = torch.autograd.grad(loss, _inputs(module, embeddings))
         assert torch.equal(loss.detach(), expected[0]) and torch.equal(gradients[0], expected[1])
         assert torch.equal(gradients[1], expected[2].to(kind)) and torch.equal(gradients[2], expected[3].to(kind))
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_two_forwards_before_a_backward(dtype, graphs):
+    """Each forward's gradients are its own, also when another forward, or a step of the engine, comes before the backward."""
+    module = _module()
+    module.engine.use_graphs = graphs
+    first, second = _embeddings(1, dtype), _embeddings(2, dtype)
+    expected = [torch.autograd.grad(module(x), _inputs(module, x)) for x in (first, second)]
+    for _ in range(3):  # of a captured step: in line, captured, replayed
+        a, b = module(first), module(second)
+        module.engine.step(_embeddings(3).detach())
+        gradients = torch.autograd.grad(a + 2.0 * b, [first, second, module.logit_scale, module.logit_bias])
+        assert torch.equal(gradients[0], expected[0][0]) and torch.equal(gradients[1], 2.0 * expected[1][0])
+        for value, one, other in zip(gradients[2:], expected[0][1:], expected[1][1:]):
+            assert torch.equal(value, one + 2.0 * other)
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_the_promise_of_a_bare_backward(graphs):
+    """``unit_upstream`` hands the row gradients on as they are; with captured steps these lie in the engine's one buffer, and a
+    backward that comes after the next step is refused instead of handing on that step's."""
+    module, first, second = _module(), _embeddings(1), _embeddings(2)
+    expected = [torch.autograd.grad(module(x), x)[0] for x in (first, second)]
+    module.unit_upstream, module.engine.use_graphs = True, graphs
+    for _ in range(3):
+        for x, gradient in zip((first, second), expected):
+            assert torch.equal(torch.autograd.grad(module(x), x)[0], gradient)
+    late, _ = module(first), module(second)
+    if graphs:
+        with pytest.raises(RuntimeError, match="overwritten by a later step"):
+            torch.autograd.grad(late, first)
+    else:
+        assert torch.equal(torch.autograd.grad(late, first)[0], expected[0])
