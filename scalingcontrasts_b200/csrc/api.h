@@ -83,8 +83,9 @@ void launch_prefix_norms(void const* rows_bf16, void* copy_bf16, float* inverse_
 void launch_transpose(void const* rows_bf16, void* transposed_bf16, uint32_t rows, uint32_t hidden, cudaStream_t stream);
 void launch_pull(void const* src0, void* dst0, size_t bytes0, void const* src1, void* dst1, size_t bytes1, int blocks,
                  cudaStream_t stream);
+// `ordinary_launch`: starts only once everything before it in the stream is complete (see launch.h).
 void launch_fold_partials(float const* partials, float* row_accumulators, uint32_t rows, uint32_t slots,
-                          uint32_t quantities, cudaStream_t stream);
+                          uint32_t quantities, cudaStream_t stream, bool ordinary_launch = false);
 void launch_finish(void const* queries_bf16, float const* inverse_norms, float const* row_accumulators,
                    float const* query_gradient, void* gradient_out_bf16, float* summands, uint32_t rows, uint32_t hidden,
                    ladder_host const& ladder, cudaStream_t stream);

@@ -215,7 +215,8 @@ struct loss_plan {
         // are written before it has run) or its CTAs need not all run (split).
         bool const folds = !fused && !overlapping && backward_split == 1;
         uint32_t const filled = sc::forward_filled_slots(a);
-        if (!folds) sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows_q, filled, quantities, stream);
+        if (!folds)
+            sc::launch_fold_partials(pointer<float>(partials), pointer<float>(accumulators), rows_q, filled, quantities, stream, overlapping);
         if (!fused) {
             sc::backward_arguments b{};
             b.gradient_cube_bf16 = pointer<void>(cube);

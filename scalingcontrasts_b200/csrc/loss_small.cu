@@ -470,11 +470,11 @@ void launch_pull(void const* src0, void* dst0, size_t bytes0, void const* src1, 
 }
 
 void launch_fold_partials(float const* partials, float* row_accumulators, uint32_t rows, uint32_t slots,
-                          uint32_t quantities, cudaStream_t stream) {
+                          uint32_t quantities, cudaStream_t stream, bool ordinary_launch) {
     bool const vectors = rows % 4 == 0 && reinterpret_cast<uintptr_t>(partials) % 16 == 0 &&
                          reinterpret_cast<uintptr_t>(row_accumulators) % 16 == 0;
     dim3 const grid(blocks_of(rows, 128), quantities);
-    launch_dependent(true, vectors ? fold_partials_kernel<true> : fold_partials_kernel<false>, grid, fold_warps * 32, 0, stream, partials,
+    launch_dependent(!ordinary_launch, vectors ? fold_partials_kernel<true> : fold_partials_kernel<false>, grid, fold_warps * 32, 0, stream, partials,
                      row_accumulators, rows, slots, quantities);
     check_launch("fold_partials");
 }
