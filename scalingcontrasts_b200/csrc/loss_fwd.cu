@@ -331,6 +331,13 @@ __device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, wa
         if (mbar_try_wait(bar, parity)) return true;
     return mbar_wait_sleeping(bar, parity, ctx.status, ctx.budget_ns, ctx.abort_flag, site, detail, 0u);
 }
+// The same for tensor-memory slots that both CTAs of a pair give back.
+__device__ __forceinline__ bool mbar_wait_lane_cluster(uint32_t bar, uint32_t parity, wait_context const& ctx, uint32_t site, uint32_t detail) {
+#pragma unroll 1
+    for (int spin = 0; spin < 16; ++spin)
+        if (mbar_try_wait_cluster(bar, parity)) return true;
+    return mbar_wait_sleeping(bar, parity, ctx.status, ctx.budget_ns, ctx.abort_flag, site, detail, 0u) && mbar_try_wait_cluster(bar, parity);
+}
 constexpr uint32_t sleep_gemm_ns = 500; // the fused kernel's gradient GEMM runs a whole item behind
 
 // The items of a CTA or pair: every so many-th of the list.
@@ -454,7 +461,9 @@ __device__ __forceinline__ void mma_role(fwd_params const& p, uint32_t stages_ba
             uint32_t& observed = was_parked ? seen_parked : seen;
             timer.lap(0);
             while (observed <= needed) {
-                if (!mbar_wait_lane(smem_u32(&barriers[observed % fwd_slots]), (observed / fwd_slots) & 1u, ctx, site_fwd_slot_empty, unit))
+                uint32_t const given_back = smem_u32(&barriers[observed % fwd_slots]), parity = (observed / fwd_slots) & 1u;
+                if (!(fwd_paired(form_) ? mbar_wait_lane_cluster(given_back, parity, ctx, site_fwd_slot_empty, unit)
+                                        : mbar_wait_lane(given_back, parity, ctx, site_fwd_slot_empty, unit)))
                     return false;
                 ++observed;
             }
