@@ -182,10 +182,12 @@ class BoxLoss:
         blocks it scores; the first call of an argument set runs eagerly, the second captures. Every member of the
         domain must make the same choice in the same step. ``learned``, a float32 log scale and bias on the device, fills
         ``scalars`` in the publish launch."""
-        if scalars is not None:
-            _check_words("scalars", scalars, 2, queries.device)  # before anything is launched that other ranks wait for
-        elif learned is not None:
-            raise ValueError("a learned log scale and bias fill `scalars`: both must be given")
+        # Before anything is launched that other ranks wait for (a learned pair and the scalars it fills: by the publish launch).
+        if learned is not None:
+            if scalars is None:
+                raise ValueError("a learned log scale and bias fill `scalars`: both must be given")
+        elif scalars is not None:
+            _check_words("scalars", scalars, 2, queries.device)
         with phase("publish: prefix norms + copy into symmetric memory"):
             self._publish(queries, stream, None if learned is None else (*learned, scalars))
         gradient = self.gradient if gradient_out is None else gradient_out
