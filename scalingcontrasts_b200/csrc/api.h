@@ -137,7 +137,8 @@ struct forward_arguments {
     // it spends in 0 producer issue, 1 producer waiting for a free stage, 2 UMMA issue, 3 UMMA waiting for a stage,
     // 4 UMMA waiting for a slot, 5 epilogue between tiles, 6 epilogue waiting for a tile, 7 cell pass, 8 suffix pass.
     unsigned long long* trace;
-    int multiprocessors;
+    int multiprocessors;        // for the launch to walk over
+    int device_multiprocessors; // of the whole GPU
     // The fused form: the same launch also folds the gradient patches into `query_gradient` (tensor-core GEMM beside
     // the scoring), so no gradient cube exists. `gradient_cube_bf16` is then unused; the patches of a work item pass
     // through `fused_scratch_bf16` (forward_fused_scratch_bytes() bytes, contents meaningless between launches).

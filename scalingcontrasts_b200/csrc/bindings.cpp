@@ -198,6 +198,7 @@ struct loss_plan {
         a.pull.src[1] = pointer<void>(pull_src1), a.pull.dst[1] = pointer<void>(pull_dst1), a.pull.bytes[1] = pull_bytes1;
         // a forward that has the previous block's backward beside it leaves that kernel its multiprocessors
         a.multiprocessors = overlapping && pending ? multiprocessors - backward_multiprocessors : multiprocessors;
+        a.device_multiprocessors = multiprocessors;
         a.fused = fused, a.fused_scratch_bf16 = pointer<void>(cube), a.fused_scratch_bytes = gradients_bytes;
         a.transposed_candidates = pointer<void>(transposed), a.query_gradient = pointer<float>(query_gradient);
         a.gradient_scale = static_cast<float>(2.0 / live);
@@ -452,7 +453,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
               a.query_base = query_base, a.candidate_base = candidate_base, a.spec_code = spec_code, a.budget_ns = budget_ns;
               a.pull.src[0] = pointer<void>(pull_src0), a.pull.dst[0] = pointer<void>(pull_dst0), a.pull.bytes[0] = pull_bytes0;
               a.pull.src[1] = pointer<void>(pull_src1), a.pull.dst[1] = pointer<void>(pull_dst1), a.pull.bytes[1] = pull_bytes1;
-              a.multiprocessors = sms;
+              a.multiprocessors = a.device_multiprocessors = sms;
               a.trace = pointer<unsigned long long>(trace);
               a.fused = fused, a.fused_scratch_bf16 = pointer<void>(fused_scratch), a.fused_scratch_bytes = fused_scratch_bytes;
               a.transposed_candidates = pointer<void>(transposed), a.query_gradient = pointer<float>(query_gradient);

@@ -200,7 +200,7 @@ struct fwd_params {
     unsigned long long* trace; // optional: phase cycle counters of CTA 0 (see forward_trace_slots in api.h)
     // One word per 64-channel chunk, one byte per 16-channel step of the chunk: non-zero when, walking the channels
     // downwards, the step is the first of a band (the topmost step, or the step just below a band's first channel).
-    // Kept in the kernel's parameters so that the UMMA warp reads it through the uniform datapath. hidden <= 4096.
+    // Kept in the kernel's parameters: the issuer's lane has them without a load from global memory. hidden <= 4096.
     uint32_t band_starts[64];
     // Fused kernel only. The gradient GEMM's channel tiles, one word each: band | first channel / 16 << 4 | width / 16
     // << 16; a tile never crosses a band edge, so its A operand is one band's patch.
@@ -377,13 +377,12 @@ __device__ __forceinline__ void producer_role(CUtensorMap const* q_map, CUtensor
             float norms[halves * prefixes_], largest = 0.0f;
 #pragma unroll
             for (int j = 0; j < static_cast<int>(halves) * prefixes_; ++j) {
-                uint32_t const column = first_column + (j % halves) * 32u + lane; // the last tile of a pair may be half empty
-                size_t const at = static_cast<size_t>(j / halves) * p.rows_c + column;
-                norms[j] = column < p.rows_c && SC_IN_BOUNDS(at, static_cast<size_t>(prefixes_) * p.rows_c) ? *(p.c_inv + at) : 0.0f;
+                size_t const at = static_cast<size_t>(j / halves) * p.rows_c + first_column + (j % halves) * 32u + lane;
+                norms[j] = SC_IN_BOUNDS(at, static_cast<size_t>(prefixes_) * p.rows_c) ? *(p.c_inv + at) : 0.0f;
             }
             // Lane 8 h + k: band k's largest inverse norm among the tile's h-th 64 columns.
             uint32_t const maximum = first_column / 64 + lane / 8;
-            if (lane % 8 < prefixes_ && lane / 8 < columns / 64 && maximum < maxima &&
+            if (lane % 8 < prefixes_ && lane / 8 < columns / 64 &&
                 SC_IN_BOUNDS(static_cast<size_t>(lane % 8) * maxima + maximum, static_cast<size_t>(prefixes_) * maxima))
                 largest = *(p.c_tile_max + static_cast<size_t>(lane % 8) * maxima + maximum);
             bool ok = true;
@@ -747,16 +746,6 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
         if (!mbar_wait(smem_u32(&tail->norms_full[entry]), (tile_local / fwd_norm_slots) & 1u, ctx, site_fwd_norms_full, tile_local))
             return;
         timer.lap(1);
-        if (fwd_paired(form_) && column >= p.rows_c) {
-            // The second half of the last tile, where the candidates are an odd number of 64s: nothing to score.
-            tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                give_back(&tail->tile_taken[tile_local % fwd_slots]);
-                if (parked > 0) give_back(&tail->tile_parked_taken[tile_local % fwd_slots]);
-                mbar_arrive(smem_u32(&tail->norms_empty[entry]));
-            }
-        } else {
         // Bands in which some cosine of the patch may sit on the floor (one bit each).
         uint32_t floors = 0;
         {
@@ -1056,7 +1045,6 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
         }
         if (lane == 0) mbar_arrive(smem_u32(&tail->norms_empty[entry])); // every lane's reads are behind a __syncwarp above
         timer.lap(3);
-        }
         if (cursor.t + 1 == run_length<form_>(p, run)) {
             // One partial record per (run, column group, row); the 1/N weight and the mirror cell's factor two go in here.
             uint32_t const slot = (run * (fwd_cols_for(form_) / 64) + column_half) * fwd_column_groups + group;
@@ -1393,7 +1381,7 @@ template <int prefixes_> void preload_count(bool fused) {
 } // namespace
 
 // Which form a launch takes; by sizes and numbers alone, so that a block takes the same one however much of the GPU it gets.
-// - Every tile of 64 at once on the GPU: a single CTA each. A pair's barriers and commits across CTAs cost a launch 0.7 us (128 rows,
+// - Every tile of 64 at once on the GPU, or an odd number of them (a pair's tile is two): a single CTA each. A pair's barriers and commits across CTAs cost a launch 0.7 us (128 rows,
 //   H=768, K=5: 11.6 against 12.4 us; 1024 rows 12.2 against 13.0).
 // - A block without the rows' own copies: the pair's form that has nothing of the diagonal in it (one block of 4096 rows, H=768, K=5: 74.7
 //   us against 80.7 with a single CTA and 82.3 with a pair that can score the diagonal; 2944 rows, H=832, K=4: 44.8, 49.3, 50.8;
@@ -1407,8 +1395,7 @@ static form_t forward_form(forward_arguments const& a) {
     if (a.fused) return form_fused;
     uint32_t const column_tiles = a.rows_c / 64, bands = a.ladder.count;
     uint64_t const singles = static_cast<uint64_t>(a.rows_q / fwd_rows) * column_tiles;
-    if (column_tiles % 2) return form_pair; // the only one that can do without half a tile
-    if (singles <= 148) return form_single;
+    if (column_tiles % 2 || singles <= static_cast<uint64_t>(a.device_multiprocessors)) return form_single;
     // A row's own copy is the candidate of the same number, its partner the other of the pair 2m, 2m + 1.
     uint64_t const first = a.query_base & ~1ull, behind = (a.query_base + a.rows_q + 1) & ~1ull;
     bool const apart = a.candidate_base >= behind || a.candidate_base + a.rows_c <= first;
@@ -1419,8 +1406,7 @@ static form_t forward_form(forward_arguments const& a) {
 // A run is `tiles_per_run` tiles, of 64 candidates or, in a pair, of 128, and has one record per 64 columns of a tile and column group. A
 // pair's last run may be shorter.
 static uint32_t runs_of(form_t form, uint32_t rows_c, uint32_t tiles_per_run) {
-    uint32_t const tiles = (rows_c + fwd_cols_for(form) - 1) / fwd_cols_for(form);
-    return (tiles + tiles_per_run - 1) / tiles_per_run;
+    return (rows_c / fwd_cols_for(form) + tiles_per_run - 1) / tiles_per_run;
 }
 static uint32_t slots_of(form_t form, uint32_t rows_c, uint32_t tiles_per_run) {
     return fwd_column_groups * (fwd_cols_for(form) / 64) * runs_of(form, rows_c, tiles_per_run);
@@ -1437,7 +1423,7 @@ uint32_t forward_quantities(uint32_t prefixes) { return 2 + 2 * prefixes; }
 // instead (2944 and 3072 rows: runs of one tile, 184 and 192 records to a row) the fold took longer than the gradient GEMM that
 // hides it: three blocks of 2944 rows, H=832, K=4, took 274 us, with runs of two tiles 237.
 uint32_t forward_choose_tiles_per_run(uint32_t rows_q, uint32_t rows_c, int multiprocessors) {
-    uint64_t const strips = rows_q / fwd_rows, column_tiles = rows_c / 64, tiles = (column_tiles + 1) / 2;
+    uint64_t const strips = rows_q / fwd_rows, column_tiles = rows_c / 64, tiles = (column_tiles + 1) / 2; // of 128
     uint64_t const walkers = multiprocessors > 1 ? static_cast<uint64_t>(multiprocessors) / 2 : 1;
     uint32_t best = 1;
     uint64_t least = ~0ull;
@@ -1478,7 +1464,8 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
     if (a.tiles_per_run == 0 || column_tiles % a.tiles_per_run)
         throw std::runtime_error("forward: tiles_per_run must divide the number of candidate tiles");
     if (a.pull.bytes[0] % 16 || a.pull.bytes[1] % 16) throw std::runtime_error("forward: pull sizes must be multiples of 16");
-    if (a.multiprocessors < 1) throw std::runtime_error("forward: the multiprocessor count must be positive");
+    if (a.multiprocessors < 1 || a.multiprocessors > a.device_multiprocessors)
+        throw std::runtime_error("forward: the multiprocessor count must be positive and the device's at most");
 
     fwd_params p{};
     p.q_inv = a.query_inverse_norms, p.c_inv = a.candidate_inverse_norms, p.c_tile_max = a.candidate_tile_max;
@@ -1489,7 +1476,7 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
     for (int i = 0; i < 8; ++i) p.ladder.ends[i] = a.ladder.ends[i];
     form_t const form = forward_form(a);
     p.tiles_per_run = a.tiles_per_run;
-    p.tiles_per_strip = fwd_paired(form) ? (column_tiles + 1) / 2 : column_tiles;
+    p.tiles_per_strip = a.rows_c / fwd_cols_for(form);
     p.runs_per_strip = runs_of(form, a.rows_c, a.tiles_per_run);
     p.items = (a.rows_q / fwd_rows) * p.runs_per_strip;
     p.beta = a.beta, p.bias = a.bias, p.weight = a.weight;

@@ -98,6 +98,44 @@ def test_an_odd_number_of_64_candidates(prefixes, rows_c):
         assert float(losses[k]) == pytest.approx(float(expected), rel=SUMMAND_TOLERANCE)
 
 
+@pytest.mark.parametrize("rows_q,rows_c", [(256, 64), (256, 1088), (1152, 1088), (1280, 1088), (1280, 1024)])
+@pytest.mark.parametrize("prefixes,candidate_base", [(1, 0), (4, 64), (5, 0), (5, 4096), (8, 0), (8, 4096)])
+def test_the_cube_and_the_records_at_odd_and_even_numbers_of_64_candidates(rows_q, rows_c, prefixes, candidate_base):
+    """Every gradient of the cube against float64, and exactly as many records as there are runs, column groups and rows. An odd number
+    of 64 candidates has none of 128: single CTAs take it, on and off the diagonal."""
+    ext, ladder = native(), Matryoshka(tuple(64 * (k + 1) for k in range(prefixes)))
+    hidden, quantities, slots = ladder.hidden, ext.forward_quantities(prefixes), ext.forward_partial_slots(rows_c, 1)
+    assert slots == 4 * (rows_c // 64)
+    queries, block = _rows(rows_q, hidden, 8), _rows(rows_c, hidden, 9)
+    f32 = dict(dtype=torch.float32, device="cuda")
+    inverse = []
+    for values in (queries, block):
+        inverse.append((torch.empty(prefixes, values.shape[0], **f32), torch.empty(prefixes, values.shape[0] // 64, **f32)))
+        ext.prefix_norms(values.data_ptr(), 0, inverse[-1][0].data_ptr(), inverse[-1][1].data_ptr(), values.shape[0], hidden,
+                         list(ladder.ends), stream_handle())
+    cube = torch.full((prefixes, rows_q, rows_c), float("nan"), dtype=torch.bfloat16, device="cuda")
+    partials = torch.full((slots, quantities, rows_q), float("nan"), **f32)
+    status = torch.zeros(8, dtype=torch.int32, device="cuda")
+    ext.forward(queries=queries.data_ptr(), candidates=block.data_ptr(), q_inv=inverse[0][0].data_ptr(), c_inv=inverse[1][0].data_ptr(),
+                c_tile_max=inverse[1][1].data_ptr(), cube=cube.data_ptr(), partials=partials.data_ptr(), status=status.data_ptr(),
+                rows_q=rows_q, rows_c=rows_c, hidden=hidden, ends=list(ladder.ends), tiles_per_run=1, beta=10.0, bias=-10.0, weight=1.0,
+                scalars=0, query_base=0, candidate_base=candidate_base, spec_code=LossSpec("pairs").code(), budget_ns=10 ** 9,
+                pull_src0=0, pull_dst0=0, pull_bytes0=0, pull_src1=0, pull_dst1=0, pull_bytes1=0, sms=148, stream=stream_handle())
+    torch.cuda.synchronize()
+    assert not status.any() and partials.isfinite().all()
+    rows, columns = torch.arange(rows_q, device="cuda")[:, None], candidate_base + torch.arange(rows_c, device="cuda")[None, :]
+    own, signs = rows == columns, torch.where((rows ^ 1) == columns, 1.0, -1.0)  # a row's own copy moves no dot product
+    below = torch.zeros(rows_q, rows_c, dtype=torch.float64, device="cuda")
+    for k in reversed(range(prefixes)):
+        end = ladder.ends[k]
+        q, c = queries[:, :end].double(), block[:, :end].double()
+        inverses = 1.0 / (q.norm(dim=1)[:, None] * c.norm(dim=1)[None, :])
+        logits = 10.0 * (q @ c.T) * inverses - 10.0
+        below += torch.where(own, 0.0, -signs * torch.sigmoid(-signs * logits) * 10.0 * inverses)
+        # bfloat16 has eight significant bits: rounding to the nearest moves a value by 2^-8 of itself at most, and so the whole
+        assert float((cube[k].double() - below).norm() / below.norm()) < 2.0 ** -8
+
+
 @pytest.mark.parametrize("rows_q,ends", [(4096, [48, 96, 192, 384, 768]), (3584, [64, 112, 1024]), (4864, [1024]), (4096, [32, 272, 1024]),
                                          (3328, [96, 768, 1104]), (4096, [16, 1024]), (4992, [1024])])
 @pytest.mark.parametrize("rows_c", [64, 448])
