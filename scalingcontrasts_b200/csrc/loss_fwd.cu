@@ -1381,16 +1381,21 @@ template <int prefixes_> void preload_count(bool fused) {
 } // namespace
 
 // Which form a launch takes; by sizes and numbers alone, so that a block takes the same one however much of the GPU it gets.
-// - Every tile of 64 at once on the GPU, or an odd number of them (a pair's tile is two): a single CTA each. A pair's barriers and commits across CTAs cost a launch 0.7 us (128 rows,
-//   H=768, K=5: 11.6 against 12.4 us; 1024 rows 12.2 against 13.0).
+// - Every tile of 64 at once on the GPU, or an odd number of them (a pair's tile is two): a single CTA each. A pair's barriers and
+//   commits across CTAs cost a launch 0.7 us (128 rows, H=768, K=5: 11.6 against 12.4 us; 1024 rows 12.2 against 13.0).
 // - A block without the rows' own copies: the pair's form that has nothing of the diagonal in it (one block of 4096 rows, H=768, K=5: 74.7
 //   us against 80.7 with a single CTA and 82.3 with a pair that can score the diagonal; 2944 rows, H=832, K=4: 44.8, 49.3, 50.8;
 //   16384 rows, H=768, K=5: 1130, 1248, 1215; every cell in the general form, 8192 rows, H=512, K=4: 328, 359, 371).
-// - A block with them: a pair loads a third fewer operand bytes per cell, and where those weigh more than the cells' arithmetic, which
-//   goes with the channels per band, it is faster: H=1024, K=1, 4096 rows 44.5 against 45.9 us, 8192 rows 166 against 175, K=7, 4096
-//   rows 145 against 153. It is not for few channels (H=512, K=4, 4096 rows 70 against 66; H=832, K=4, 2944 rows 51 against 49.5; H=512,
-//   K=2, 6144 rows 98 against 92), and in between for large launches, which run at the GPU's power limit (H=768, K=5: 4096
-//   rows 83.4 against 82.1, 16384 rows 1229 against 1270; H=1024, K=6: 4096 rows 124 either way, 8192 rows 418 against 454).
+// - A block with them: a pair loads a third fewer operand bytes per cell but carries the diagonal's code beside two CTAs' hand-overs, and
+//   spills a little more (4 to 36 bytes at K = 4, 5, 6 and 8). Measured for 256 to 2048 channels, one to eight bands, 2048 to 16384 rows,
+//   in turn, single CTA against pair in us:
+//   1536 channels and more, a pair everywhere (1 to 19 %): K=5 4096 rows 110.4 against 104.0, K=6 16384 rows 2363 against 2209.
+//   Seven and eight bands, from 512 channels on: H=512, K=7 4096 rows 134.3 against 132.1, K=8 16384 rows 2307 against 2075; at
+//   H=256, K=8 a pair takes 1 % more. Six bands, from 768 channels on: H=768 4096 rows 101.8 against 99.8, H=1024 125.0 against 114.2.
+//   Fewer bands, where the operands weigh more than the cells: H=768, K=2 4096 rows 45.5 against 43.8, H=1024, K=1 45.1 against 43.4; not at
+//   256 channels a band and less: H=768, K=3 54.7 against 56.4, H=1024, K=4 2048 rows 23.5 against 24.2, 4096 rows 74.0 against 74.4,
+//   H=512, K=4 63.5 against 67.8. Large launches, which run at the GPU's power limit, gain from 768 channels on: 16384 rows, H=768, K=3
+//   979 against 900, K=5 1332 against 1320, H=1024, K=5 1488 against 1394, but H=512, K=3 772 against 813.
 static form_t forward_form(forward_arguments const& a) {
     if (a.fused) return form_fused;
     uint32_t const column_tiles = a.rows_c / 64, bands = a.ladder.count;
@@ -1401,7 +1406,9 @@ static form_t forward_form(forward_arguments const& a) {
     bool const apart = a.candidate_base >= behind || a.candidate_base + a.rows_c <= first;
     if (apart) return form_pair_apart;
     bool const large = static_cast<uint64_t>(a.rows_q) * a.rows_c >= (1ull << 26);
-    return bands >= 7 || a.hidden >= (large ? 144 : 320) * bands ? form_pair : form_single;
+    bool const pair = a.hidden >= 1536 || (bands >= 7 && a.hidden >= 512) || (bands == 6 && a.hidden >= 768) || a.hidden >= 320 * bands ||
+                      (large && a.hidden >= 768 && a.hidden >= 144 * bands);
+    return pair ? form_pair : form_single;
 }
 // A run is `tiles_per_run` tiles, of 64 candidates or, in a pair, of 128, and has one record per 64 columns of a tile and column group. A
 // pair's last run may be shorter.

@@ -50,6 +50,16 @@ def test_both_sides_of_one_wave(rows, candidates, prefixes):
         _check(queries, block, ladder, LossSpec("pairs"), 0, base)
 
 
+@pytest.mark.parametrize("ends", [(64, 128, 256, 384, 512, 768), (64, 128, 256, 384, 512, 704), (96, 192, 384, 768, 1536), (96, 192, 384, 768, 1472),
+                                  (64, 128, 192, 256, 320, 448, 512), (64, 128, 192, 256, 320, 384, 448), (320, 640), (320, 576), (320,), (256,)])
+@pytest.mark.parametrize("base", [0, 1])
+def test_both_sides_of_the_lines_for_blocks_with_own_copies(ends, base):
+    """Channels and bands at which a block that holds the rows' own copies changes from single CTAs to pairs."""
+    ladder = Matryoshka(ends)
+    queries, block = _rows(1280, ladder.hidden, 10), _rows(1280, ladder.hidden, 11)
+    _check(queries, block, ladder, LossSpec("pairs"), 0, base)
+
+
 @pytest.mark.parametrize("spec", [LossSpec("self"), LossSpec("pairs"), LossSpec("pairs", "skip")], ids=lambda s: f"{s.positives}-{s.diagonal}")
 @pytest.mark.parametrize("query_base,candidate_base", [(0, 0), (1536, 0), (0, 1536), (0, 1535), (1535, 0), (1537, 0), (0, 1537), (1, 1537),
                                                        (1537, 1), (3, 0), (0, 17), (1520, 0), (64, 0)])
