@@ -357,12 +357,13 @@ __global__ void keep_summands_kernel(float const* summands, float* kept, float* 
 template <typename out_t>
 __global__ void __launch_bounds__(256)
     scale_gradients_kernel(uint4 const* gradient, float const* upstream, float const* summands, out_t* out, float* scale_gradient,
-                           float* bias_gradient, size_t vectors) {
+                           float* bias_gradient, size_t scalars) {
     let_dependents_start();
     wait_for_kernels_before();
     float const whole = *upstream, factor = __bfloat162float(__float2bfloat16(whole));
     if (blockIdx.x == 0 && threadIdx.x == 0) *scale_gradient = summands[2] * whole, *bias_gradient = summands[1] * whole;
-    for (size_t v = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; v < vectors; v += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    for (size_t v = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; v < scalars / 8; v += static_cast<size_t>(gridDim.x) * blockDim.x) {
+        if (!SC_IN_BOUNDS(v * 8 + 7, scalars)) continue;
         uint4 const packed = gradient[v];
         uint32_t const words[4] = {packed.x, packed.y, packed.z, packed.w};
         uint32_t scaled[4];
@@ -517,10 +518,10 @@ void launch_scale_gradients(void const* gradient_bf16, float const* upstream, fl
     uint4 const* const gradient = static_cast<uint4 const*>(gradient_bf16);
     if (out_f32)
         launch_dependent(true, scale_gradients_kernel<float>, blocks < 1 ? 1 : blocks, 256, 0, stream, gradient, upstream, summands,
-                         static_cast<float*>(out), scale_gradient, bias_gradient, scalars / 8);
+                         static_cast<float*>(out), scale_gradient, bias_gradient, scalars);
     else
         launch_dependent(true, scale_gradients_kernel<__nv_bfloat16>, blocks < 1 ? 1 : blocks, 256, 0, stream, gradient, upstream,
-                         summands, static_cast<__nv_bfloat16*>(out), scale_gradient, bias_gradient, scalars / 8);
+                         summands, static_cast<__nv_bfloat16*>(out), scale_gradient, bias_gradient, scalars);
     check_launch("scale_gradients");
 }
 

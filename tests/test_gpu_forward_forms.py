@@ -172,3 +172,38 @@ def test_backward_in_pairs_of_ctas(rows_q, ends, rows_c):
         assert float((gradient.double() - expected).norm() / expected.norm()) < 1e-5
         outcomes.append(gradient)
     assert torch.equal(outcomes[0], outcomes[1])
+
+
+@pytest.mark.parametrize("rows,candidates,ends,candidate_base", [
+    (128, 128, (64, 256), 0),                     # single CTAs
+    (1280, 1280, (320,), 0),                      # pairs, with own copies
+    (1280, 1280, (64, 256), 4096),                # pairs, without
+    (4096, 512, (48, 96, 192, 384, 768), 4096),   # the backward in pairs as well
+])
+def test_a_failure_recorded_before_is_left_at_once(rows, candidates, ends, candidate_base):
+    """Kernels that find a failure in the status block score and add nothing, whatever their form, give everything back and leave; once
+    the block is clear the same launches work."""
+    ladder = Matryoshka(ends)
+    queries, block = _rows(rows, ladder.hidden, 12), _rows(candidates, ladder.hidden, 13)
+    loss = StreamedLoss(rows, ladder.hidden, ladder, LossSpec("pairs"), "cuda", candidate_rows=candidates)
+
+    def scored():
+        loss.begin(queries)
+        loss.score(queries, block, 0, candidate_base, 10.0, -10.0, rows + candidates)
+        torch.cuda.synchronize()
+        return loss.query_gradient.clone(), loss.row_accumulators.clone()
+
+    expected = scored()
+    loss.status[0] = 2
+    for scratch in (loss.partials, loss.similarity_gradients):
+        scratch.fill_(7.0)
+    for _ in range(3):
+        gradient, accumulators = scored()
+        assert not gradient.any() and not accumulators.any()
+        assert (loss.partials == 7.0).all() and (loss.similarity_gradients == 7.0).all()
+    with pytest.raises(RuntimeError, match="gave up"):
+        loss.check()
+    loss.status.zero_()
+    again = scored()
+    loss.check()
+    assert torch.equal(again[0], expected[0]) and torch.equal(again[1], expected[1])
