@@ -16,7 +16,8 @@
 // tile's candidates each.
 //
 // Warp roles (192 threads): warps 0-3 epilogue (tensor-memory lanes 32*w..; before that the fold of the forward launch's
-// partial records, if asked for), warp 4 TMA producer, warp 5 UMMA issuer and tensor-memory owner. The producer's and the issuer's loops are run by one elected lane each. The epilogue adds its scaled accumulators with
+// partial records, if asked for), warp 4 TMA producer, warp 5 UMMA issuer and tensor-memory owner. The producer's
+// and the issuer's loops are run by one elected lane each. The epilogue adds its scaled accumulators with
 // vector reductions (fire and forget: no read of the old value comes back to the SM). With `split == 1` each output
 // element receives exactly one addition per launch, so the sum's order is the launches' stream order and the result
 // is deterministic; with a larger split the candidate range is divided and the order of a launch's partial sums is not.
@@ -319,25 +320,25 @@ __global__ void __launch_bounds__(bwd_threads, 1)
         if (p.partials != nullptr) fold_share(p, warp, lane);
         if (mbar_wait(smem_u32(&tail->accumulated), 0u, ctx, site_bwd_accumulated, tile_index)) {
             tcgen05_fence_after();
-          for (uint32_t block = 0; block < blocks; ++block) {
-            uint32_t const row = (first_block + block) * bwd_rows + warp * 32 + lane;
-            float* destination = p.query_gradient + static_cast<size_t>(row) * p.hidden + tile.channel0;
-            uint32_t const lane_base = tmem_base + ((warp * 32u) << 16) + block * bwd_block_columns;
-            for (uint32_t column = 0; column < tile.width; column += 16) {
-                if (!SC_WARP_IN_BOUNDS(static_cast<size_t>(row) * p.hidden + tile.channel0 + column + 15,
-                                       static_cast<size_t>(p.rows_q) * p.hidden))
-                    break;
-                uint32_t values[16];
-                tmem_load_16(lane_base + column, values);
-                tmem_load_wait();
+            for (uint32_t block = 0; block < blocks; ++block) {
+                uint32_t const row = (first_block + block) * bwd_rows + warp * 32 + lane;
+                float* destination = p.query_gradient + static_cast<size_t>(row) * p.hidden + tile.channel0;
+                uint32_t const lane_base = tmem_base + ((warp * 32u) << 16) + block * bwd_block_columns;
+                for (uint32_t column = 0; column < tile.width; column += 16) {
+                    if (!SC_WARP_IN_BOUNDS(static_cast<size_t>(row) * p.hidden + tile.channel0 + column + 15,
+                                           static_cast<size_t>(p.rows_q) * p.hidden))
+                        break;
+                    uint32_t values[16];
+                    tmem_load_16(lane_base + column, values);
+                    tmem_load_wait();
 #pragma unroll
-                for (int v = 0; v < 4; ++v)
-                    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(destination + column + 4 * v),
-                                 "f"(p.scale * __uint_as_float(values[4 * v])), "f"(p.scale * __uint_as_float(values[4 * v + 1])),
-                                 "f"(p.scale * __uint_as_float(values[4 * v + 2])), "f"(p.scale * __uint_as_float(values[4 * v + 3]))
-                                 : "memory");
+                    for (int v = 0; v < 4; ++v)
+                        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(destination + column + 4 * v),
+                                     "f"(p.scale * __uint_as_float(values[4 * v])), "f"(p.scale * __uint_as_float(values[4 * v + 1])),
+                                     "f"(p.scale * __uint_as_float(values[4 * v + 2])), "f"(p.scale * __uint_as_float(values[4 * v + 3]))
+                                     : "memory");
+                }
             }
-          }
         }
     }
 
@@ -507,7 +508,9 @@ void launch_backward(backward_arguments const& a, cudaStream_t stream) {
     bool pair = mn_major && a.rows_q / bwd_rows % 2 == 0 && static_cast<uint64_t>(ctas) * a.split > static_cast<uint64_t>(multiprocessors);
     for (uint32_t i = 0; i < p.tile_count; ++i)
         pair = pair && p.tiles[i].blocks == 1 && p.tiles[i].width >= 32 && p.tiles[i].width <= bwd_max_width;
-    if (pair) launch_dependent_clusters(!a.ordinary_launch, 2, backward_kernel<true, true>, grid, bwd_threads, shared_bytes, stream, cube_map, candidates, p);
+    if (pair)
+        launch_dependent_clusters(!a.ordinary_launch, 2, backward_kernel<true, true>, grid, bwd_threads, shared_bytes, stream, cube_map,
+                                  candidates, p);
     else
         launch_dependent(!a.ordinary_launch, mn_major ? backward_kernel<true, false> : backward_kernel<false, false>, grid, bwd_threads, shared_bytes,
                          stream, cube_map, candidates, p);

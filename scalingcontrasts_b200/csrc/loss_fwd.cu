@@ -19,8 +19,8 @@
 //
 // Warp roles (640 threads): warps 0-15 epilogue (warp w owns tensor-memory lanes 32*(w%4).. and the 16 columns w/4 of
 // the tile; four warps per scheduler keep the issue slots busy), warp 16 TMA producer (and the candidates' norms), warp 17
-// UMMA issuer and tensor-memory owner (each loop run by one elected lane), warp 18 peer pull (plain 16-byte loads from the peer's replica, plain stores to local staging; never a TMA load
-// from another GPU's memory), warp 19 the fused kernel's second issuer. The epilogue's four warpgroups run with 104
+// UMMA issuer and tensor-memory owner (each loop run by one elected lane), warp 18 peer pull (plain 16-byte loads from the
+// peer's replica, plain stores to local staging; never a TMA load from another GPU's memory), warp 19 the fused kernel's second issuer. The epilogue's four warpgroups run with 104
 // registers a thread, the helpers' with 64.
 //
 // What bounds it (B200, one block of 4096 rows, H=768, K=5, off the diagonal: 75 us): the epilogue, which by itself takes about 60 (cells
@@ -168,7 +168,8 @@ __host__ __device__ constexpr uint32_t fwd_store_bytes(uint32_t prefixes) {
 // the gradient GEMM's stages and runs the scores on what is left (three at five prefixes, two at six).
 constexpr uint32_t fwd_shared_limit = 227 * 1024;
 __host__ __device__ constexpr uint32_t fwd_stages_for(uint32_t prefixes, form_t form) {
-    uint32_t const rest = 1024 + (form == form_fused ? fz_stages * fz_stage_bytes : 0u) + fwd_store_bytes(prefixes) + fwd_tail_bytes + fwd_norm_bytes(prefixes, form) + fwd_factor_bytes(prefixes, form);
+    uint32_t const rest = 1024 + (form == form_fused ? fz_stages * fz_stage_bytes : 0u) + fwd_store_bytes(prefixes) + fwd_tail_bytes +
+                          fwd_norm_bytes(prefixes, form) + fwd_factor_bytes(prefixes, form);
     uint32_t const fit = (fwd_shared_limit - rest) / fwd_stage_bytes(form);
     return fit < fwd_max_stages ? fit : fwd_max_stages;
 }
@@ -736,7 +737,8 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
         uint64_t const first_row = p.query_base + static_cast<uint64_t>(strip) * fwd_rows + patch_row;
         uint64_t const first_column = p.candidate_base + column;
         uint64_t const odd = first_row & 1u; // then the first row's partner lies a row before, the last one's a row behind the patch's
-        bool const special = form_ != form_pair_apart && first_column - first_row + (warp_columns - 1) + odd < 32u + (warp_columns - 1) + 2 * odd;
+        bool const special = form_ != form_pair_apart &&
+                             first_column - first_row + (warp_columns - 1) + odd < 32u + (warp_columns - 1) + 2 * odd;
 
         timer.lap(0);
         if (!mbar_wait(smem_u32(&tail->tile_full[tile_local % fwd_tile_barriers]), (tile_local / fwd_tile_barriers) & 1u, ctx,
@@ -750,7 +752,8 @@ __device__ __forceinline__ void epilogue_role(CUtensorMap const* cube_map, fwd_p
         uint32_t floors = 0;
         {
             bool const may = lane < prefixes_ &&
-                             rows_max * norm_ring[entry * fwd_norm_floats(prefixes_, form_) + prefixes_ * fwd_cols_for(form_) + column_half * 8u + lane % 8u] >= 100.0f;
+                             rows_max * norm_ring[entry * fwd_norm_floats(prefixes_, form_) + prefixes_ * fwd_cols_for(form_) +
+                                                  column_half * 8u + lane % 8u] >= 100.0f;
             floors = __ballot_sync(0xFFFFFFFFu, may);
         }
 
@@ -1281,8 +1284,8 @@ __global__ void __launch_bounds__(fwd_threads, 1)
     if (poisoned) {
     } else if (warp < fwd_epilogue_warps) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(fwd_epilogue_registers));
-        epilogue_role<prefixes_, form_>(&cube_map, p, tail, store_base, norm_ring, norm_ring + fwd_norm_bytes(prefixes_, form_) / 4, tmem_base, ctx, warp,
-                                         lane, rank);
+        epilogue_role<prefixes_, form_>(&cube_map, p, tail, store_base, norm_ring, norm_ring + fwd_norm_bytes(prefixes_, form_) / 4,
+                                        tmem_base, ctx, warp, lane, rank);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(fwd_helper_registers));
         if (warp == fwd_producer_warp) {
@@ -1387,7 +1390,7 @@ template <int prefixes_> void preload_count(bool fused) {
 //   us against 80.7 with a single CTA and 82.3 with a pair that can score the diagonal; 2944 rows, H=832, K=4: 44.8, 49.3, 50.8;
 //   16384 rows, H=768, K=5: 1130, 1248, 1215; every cell in the general form, 8192 rows, H=512, K=4: 328, 359, 371).
 // - A block with them: a pair loads a third fewer operand bytes per cell but carries the diagonal's code beside two CTAs' hand-overs, and
-//   spills a little more (4 to 36 bytes at K = 4, 5, 6 and 8). Measured for 256 to 2048 channels, one to eight bands, 2048 to 16384 rows,
+//   spills a little more (4 to 36 bytes from K = 4 on; alone 12 at K = 4). Measured for 256 to 2048 channels, one to eight bands, 2048 to 16384 rows,
 //   in turn, single CTA against pair in us:
 //   1536 channels and more, a pair everywhere (1 to 19 %): K=5 4096 rows 110.4 against 104.0, K=6 16384 rows 2363 against 2209.
 //   Seven and eight bands, from 512 channels on: H=512, K=7 4096 rows 134.3 against 132.1, K=8 16384 rows 2307 against 2075; at
@@ -1529,9 +1532,15 @@ void launch_forward(forward_arguments const& a, cudaStream_t stream) {
         CUtensorMap const cube_map =
             cached_map(a.gradient_cube_bf16, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
         switch (form) {
-        case form_single: launch_for_count<form_single>(a.ladder.count, q_map, c_map, cube_map, gemm_maps, p, blocks, stream, !a.ordinary_launch); break;
-        case form_pair: launch_for_count<form_pair>(a.ladder.count, q_map, c_map, cube_map, gemm_maps, p, blocks, stream, !a.ordinary_launch); break;
-        default: launch_for_count<form_pair_apart>(a.ladder.count, q_map, c_map, cube_map, gemm_maps, p, blocks, stream, !a.ordinary_launch); break;
+        case form_single:
+            launch_for_count<form_single>(a.ladder.count, q_map, c_map, cube_map, gemm_maps, p, blocks, stream, !a.ordinary_launch);
+            break;
+        case form_pair:
+            launch_for_count<form_pair>(a.ladder.count, q_map, c_map, cube_map, gemm_maps, p, blocks, stream, !a.ordinary_launch);
+            break;
+        default:
+            launch_for_count<form_pair_apart>(a.ladder.count, q_map, c_map, cube_map, gemm_maps, p, blocks, stream, !a.ordinary_launch);
+            break;
         }
     } else {
         p.gradient = a.query_gradient, p.gradient_scale = a.gradient_scale;

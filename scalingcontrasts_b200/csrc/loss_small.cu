@@ -42,8 +42,8 @@ ladder_t to_device(ladder_host const& host) {
 // edges are multiples of 16 channels, so a vector never straddles two bands.
 constexpr uint32_t norm_rows = 64, norm_warps = 32;
 __global__ void __launch_bounds__(norm_warps * 32)
-    prefix_norms_kernel(uint4 const* rows, uint4* copy, float* inverse_norms, float* tile_max, uint32_t row_count, uint32_t hidden, ladder_t ladder,
-                        float4* clear, size_t clear_vectors, learned_scalars learned) {
+    prefix_norms_kernel(uint4 const* rows, uint4* copy, float* inverse_norms, float* tile_max, uint32_t row_count, uint32_t hidden,
+                        ladder_t ladder, float4* clear, size_t clear_vectors, learned_scalars learned) {
     constexpr uint32_t each = norm_rows / norm_warps;
     __shared__ float largest[norm_warps][8];
     uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -362,7 +362,8 @@ __global__ void __launch_bounds__(256)
     wait_for_kernels_before();
     float const whole = *upstream, factor = __bfloat162float(__float2bfloat16(whole));
     if (blockIdx.x == 0 && threadIdx.x == 0) *scale_gradient = summands[2] * whole, *bias_gradient = summands[1] * whole;
-    for (size_t v = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; v < scalars / 8; v += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    size_t const threads = static_cast<size_t>(gridDim.x) * blockDim.x;
+    for (size_t v = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; v < scalars / 8; v += threads) {
         if (!SC_IN_BOUNDS(v * 8 + 7, scalars)) continue;
         uint4 const packed = gradient[v];
         uint32_t const words[4] = {packed.x, packed.y, packed.z, packed.w};
@@ -447,9 +448,9 @@ void launch_prefix_norms(void const* rows_bf16, void* copy_bf16, float* inverse_
     // A few rows make a few blocks, which would clear a wide gradient slowly: up to one block per multiprocessor helps them.
     size_t const clearing = (clear_floats / 4 + norm_warps * 32 - 1) / (norm_warps * 32);
     int const blocks = std::max(blocks_of(rows, norm_rows), static_cast<int>(std::min<size_t>(clearing, 148)));
-    launch_dependent(
-        true, prefix_norms_kernel, blocks, norm_warps * 32, 0, stream, static_cast<uint4 const*>(rows_bf16), static_cast<uint4*>(copy_bf16), inverse_norms, tile_max, rows, hidden, to_device(ladder),
-        reinterpret_cast<float4*>(clear), clear_floats / 4, learned);
+    launch_dependent(true, prefix_norms_kernel, blocks, norm_warps * 32, 0, stream, static_cast<uint4 const*>(rows_bf16),
+                     static_cast<uint4*>(copy_bf16), inverse_norms, tile_max, rows, hidden, to_device(ladder),
+                     reinterpret_cast<float4*>(clear), clear_floats / 4, learned);
     check_launch("prefix_norms");
 }
 
