@@ -435,6 +435,9 @@ int blocks_of(size_t items, int per_block) { return static_cast<int>((items + pe
 
 } // namespace
 
+// How far passes over memory spread; no result depends on it.
+constexpr size_t b200_multiprocessors = 148;
+
 bool bounds_build() { return SC_BOUNDS != 0; }
 SC_DEFINE_BOUNDS_READER(bounds_record_small)
 
@@ -447,7 +450,7 @@ void launch_prefix_norms(void const* rows_bf16, void* copy_bf16, float* inverse_
         throw std::runtime_error("prefix_norms: the span to clear must be whole, aligned vectors");
     // A few rows make a few blocks, which would clear a wide gradient slowly: up to one block per multiprocessor helps them.
     size_t const clearing = (clear_floats / 4 + norm_warps * 32 - 1) / (norm_warps * 32);
-    int const blocks = std::max(blocks_of(rows, norm_rows), static_cast<int>(std::min<size_t>(clearing, 148)));
+    int const blocks = std::max(blocks_of(rows, norm_rows), static_cast<int>(std::min<size_t>(clearing, b200_multiprocessors)));
     launch_dependent(true, prefix_norms_kernel, blocks, norm_warps * 32, 0, stream, static_cast<uint4 const*>(rows_bf16),
                      static_cast<uint4*>(copy_bf16), inverse_norms, tile_max, rows, hidden, to_device(ladder),
                      reinterpret_cast<float4*>(clear), clear_floats / 4, learned);
@@ -515,7 +518,7 @@ void launch_scale_gradients(void const* gradient_bf16, float const* upstream, fl
                             float* scale_gradient, float* bias_gradient, size_t scalars, cudaStream_t stream) {
     if (scalars % 8 || reinterpret_cast<uintptr_t>(gradient_bf16) % 16 || reinterpret_cast<uintptr_t>(out) % 16)
         throw std::runtime_error("scale_gradients: whole, aligned vectors of eight");
-    uint32_t const blocks = static_cast<uint32_t>(std::min<size_t>((scalars / 8 + 255) / 256, 148 * 8));
+    uint32_t const blocks = static_cast<uint32_t>(std::min<size_t>((scalars / 8 + 255) / 256, b200_multiprocessors * 8));
     uint4 const* const gradient = static_cast<uint4 const*>(gradient_bf16);
     if (out_f32)
         launch_dependent(true, scale_gradients_kernel<float>, blocks < 1 ? 1 : blocks, 256, 0, stream, gradient, upstream, summands,

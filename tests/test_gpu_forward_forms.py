@@ -73,8 +73,8 @@ def test_own_copies_and_partners_wherever_they_lie(spec, query_base, candidate_b
 @pytest.mark.parametrize("prefixes", [1, 3, 5, 6, 8])
 @pytest.mark.parametrize("rows_c", [64, 192, 1088])
 def test_an_odd_number_of_64_candidates(prefixes, rows_c):
-    """The native launch takes candidates in 64s: the last tile of a pair is then half empty, and what lies behind the cube and the
-    norms is neither read into the sums nor written."""
+    """The native launch takes candidates in 64s, which single CTAs score: what lies behind the cube and the norms is neither read into
+    the sums nor written."""
     ext, rows_q, ladder = native(), 256, Matryoshka(tuple(64 * (k + 1) for k in range(prefixes)))
     hidden = ladder.hidden
     queries, block = _rows(rows_q, hidden, 5), _rows(rows_c, hidden, 6)
